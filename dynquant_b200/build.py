@@ -21,7 +21,7 @@ INCLUDE = ROOT / "include"
 OBJ_DIR = PKG / "lib" / "obj"
 LIB_PATH = PKG / "lib" / "libdynquant_b200.so"
 
-SOURCES = ["dq_capi.cu", "dq_dequant.cu", "dq_gemv.cu", "dq_gemv_mma.cu", "dq_gemv_plan.cu", "dq_gemv_rows.cu", "dq_gemv_stream_multi.cu", "dq_gemv_stream_sliced.cu", "dq_moe.cu", "dq_peer.cu", "dq_probe.cu"]
+SOURCES = ["dq_capi.cu", "dq_dequant.cu", "dq_encode.cu", "dq_gemv.cu", "dq_gemv_mma.cu", "dq_gemv_plan.cu", "dq_gemv_rows.cu", "dq_gemv_stream_multi.cu", "dq_gemv_stream_sliced.cu", "dq_moe.cu", "dq_peer.cu", "dq_probe.cu"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -91,12 +91,13 @@ TORCH_SHIM_PATH = PKG / "lib" / "libdynquant_b200_torch.so"
 
 
 def build_torch_shim(force: bool = False, verbose: bool = False) -> Path | None:
-    """Compile ``csrc/dq_torch_shim.cpp`` -- the C++ CUDA backend of ``torch.ops.dynquant.{gemv,
-    dequant}`` -- against the installed torch and link it to the C-ABI library beside it.  It is
-    optional: without it the operators are implemented by a Python function over ctypes (same
-    kernels, more host time per call).  Returns None when no C++ compiler is available."""
-    src = CSRC / "dq_torch_shim.cpp"
-    if not force and not _stale(TORCH_SHIM_PATH, [src, INCLUDE / "dynquant_b200.h", LIB_PATH]):
+    """Compile the torch side against the installed torch and link it to the C-ABI library beside
+    it: ``csrc/dq_torch_shim.cpp`` (the C++ CUDA backend of ``torch.ops.dynquant.{gemv, dequant}``)
+    and ``csrc/dq_torch_host.cpp`` (the Python module ``_host``, one C call per public entry point).
+    Optional: without it the operators are Python functions over ctypes (same kernels, more host
+    time per call).  Returns None when no C++ compiler is available."""
+    sources = [CSRC / "dq_torch_shim.cpp", CSRC / "dq_torch_host.cpp"]
+    if not force and not _stale(TORCH_SHIM_PATH, [*sources, INCLUDE / "dynquant_b200.h", LIB_PATH]):
         return TORCH_SHIM_PATH
     gxx = shutil.which("g++")
     if gxx is None or not LIB_PATH.exists():
@@ -107,20 +108,30 @@ def build_torch_shim(force: bool = False, verbose: bool = False) -> Path | None:
     from torch.utils import cpp_extension
 
     torch_lib = Path(torch.__file__).parent / "lib"
-    cmd = [gxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
-           "-I", str(INCLUDE), "-I", sysconfig.get_paths()["include"], "-I", "/usr/local/cuda/include"]
+    flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden",
+             "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
+             "-I", str(INCLUDE), "-I", sysconfig.get_paths()["include"], "-I", "/usr/local/cuda/include"]
     for p in cpp_extension.include_paths():
-        cmd += ["-isystem", p]
-    cmd += [str(src), "-o", str(TORCH_SHIM_PATH), "-L", str(LIB_PATH.parent), "-ldynquant_b200",
-            "-L", str(torch_lib), "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
-            "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"]
-    if verbose:
-        print(" ".join(cmd), flush=True)
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        sys.stderr.write(res.stdout + res.stderr)
-        raise RuntimeError("g++ failed on dq_torch_shim.cpp")
+        flags += ["-isystem", p]
+    objects = [OBJ_DIR / (src.stem + ".o") for src in sources]
+
+    def run(cmd: list[str]) -> None:
+        if verbose:
+            print(" ".join(cmd), flush=True)
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            sys.stderr.write(res.stdout + res.stderr)
+            raise RuntimeError(f"g++ failed on {cmd[-1]}")
+
+    OBJ_DIR.mkdir(parents=True, exist_ok=True)
+    compiles = [[gxx, *flags, "-c", "-o", str(obj), str(src)] for src, obj in zip(sources, objects)
+                if force or _stale(obj, [src, INCLUDE / "dynquant_b200.h"])]
+    if compiles:
+        with ThreadPoolExecutor(max_workers=len(compiles)) as pool:
+            list(pool.map(run, compiles))
+    run([gxx, "-shared", "-o", str(TORCH_SHIM_PATH), *map(str, objects), "-L", str(LIB_PATH.parent), "-ldynquant_b200",
+         "-L", str(torch_lib), "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda",
+         "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"])
     return TORCH_SHIM_PATH
 
 

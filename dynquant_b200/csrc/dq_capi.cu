@@ -5,6 +5,7 @@
 // resolve_geometry (packages/dynquant-kernels/csrc/include/dynquant/geometry.h:63-132):
 // nothing is derived by guesswork, everything is either passed in or implied
 // by a shape, and every implication is checked.
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 
@@ -31,7 +32,7 @@ int64_t launches_so_far() { return g_launches.load(std::memory_order_relaxed); }
 const DeviceInfo* device_info() {
   constexpr int kMaxDevices = 64;
   static DeviceInfo cache[kMaxDevices];
-  static bool ready[kMaxDevices] = {false};
+  static std::atomic<bool> ready[kMaxDevices];
   static std::mutex mu;
   int device = 0;
   cudaError_t err = cudaGetDevice(&device);
@@ -39,8 +40,9 @@ const DeviceInfo* device_info() {
     fail(DQ_ERR_CUDA, "cudaGetDevice failed: %s", cudaGetErrorString(err));
     return nullptr;
   }
+  if (ready[device].load(std::memory_order_acquire)) return &cache[device];
   std::lock_guard<std::mutex> lock(mu);
-  if (!ready[device]) {
+  if (!ready[device].load(std::memory_order_relaxed)) {
     DeviceInfo info = {};
     info.device = device;
     err = cudaDeviceGetAttribute(&info.sm_count, cudaDevAttrMultiProcessorCount, device);
@@ -53,9 +55,57 @@ const DeviceInfo* device_info() {
       return nullptr;
     }
     cache[device] = info;
-    ready[device] = true;
+    ready[device].store(true, std::memory_order_release);
   }
   return &cache[device];
+}
+
+namespace {
+// A direct-mapped table per thread: no lock, and a collision only costs asking again.
+struct KernelFact {
+  const void* kernel;
+  int device, threads;
+  size_t bytes;
+  int value;
+};
+constexpr int kFacts = 512;
+
+KernelFact& fact_slot(KernelFact* table, const void* kernel, int device, size_t mix) {
+  const size_t h = (reinterpret_cast<uintptr_t>(kernel) >> 4) * 0x9E3779B97F4A7C15ull + mix * 0xC2B2AE3D27D4EB4Full + static_cast<size_t>(device);
+  return table[(h >> 32) % kFacts];
+}
+}  // namespace
+
+cudaError_t allow_shared_bytes(const void* kernel, size_t bytes) {
+  static thread_local KernelFact table[kFacts];
+  int device = 0;
+  if (const cudaError_t err = cudaGetDevice(&device)) return err;
+  KernelFact& f = fact_slot(table, kernel, device, 0);
+  if (f.kernel == kernel && f.device == device && f.bytes >= bytes) return cudaSuccess;
+  // Always all that the device allows, so that no thread ever lowers what another one relies on.
+  const DeviceInfo* dev = device_info();
+  cudaFuncAttributes attr = {};
+  if (dev == nullptr) return cudaErrorInvalidDevice;
+  if (const cudaError_t err = cudaFuncGetAttributes(&attr, kernel)) return err;
+  const size_t most = static_cast<size_t>(dev->max_smem_optin) - attr.sharedSizeBytes;
+  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(std::max(most, bytes)));
+  if (err == cudaSuccess) f = {kernel, device, 0, std::max(most, bytes), 0};
+  return err;
+}
+
+cudaError_t resident_ctas_of(int* per_sm, const void* kernel, int threads, size_t bytes) {
+  static thread_local KernelFact table[kFacts];
+  int device = 0;
+  if (const cudaError_t err = cudaGetDevice(&device)) return err;
+  KernelFact& f = fact_slot(table, kernel, device, bytes * 2048 + static_cast<size_t>(threads));
+  if (f.kernel != kernel || f.device != device || f.threads != threads || f.bytes != bytes) {
+    int n = 0;
+    if (const cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, bytes)) return err;
+    f = {kernel, device, threads, bytes, n};
+  }
+  *per_sm = f.value;
+  return cudaSuccess;
 }
 
 }  // namespace dq

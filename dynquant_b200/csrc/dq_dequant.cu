@@ -29,63 +29,103 @@ namespace dq {
 namespace {
 
 constexpr int kDequantThreads = 256;
+constexpr int kRowsInFlight = 4;
 
 struct DequantArgs {
   const uint32_t* packed;
   const void* scales;
   const void* offsets;
   void* out;
+  const void* ids;       // null, or the packed row of every output row
+  int ids_are_32;        // int32 ids (else int64)
+  int table_rows;        // rows of the packed tensor (ids lie below it)
   int meta_dtype, out_dtype;
-  int rows;
+  int rows;              // output rows
   int words_per_row, num_groups, words_per_group, group_values, in_features;
   int blocks_per_group, blocks_per_row;
 };
 
-// 8 consecutive values of one row per thread.  `group_shift` >= 0: the group size is 2^shift.
+// Which packed row an output row comes from: itself, or (an embedding lookup) the id at its place.
+// An id outside the table gives -1.
+__device__ __forceinline__ int source_row(const DequantArgs& a, int row) {
+  if (a.ids == nullptr) return row;
+  const int64_t id = a.ids_are_32 ? static_cast<int64_t>(__ldg(static_cast<const int*>(a.ids) + row))
+                                  : static_cast<int64_t>(__ldg(static_cast<const long long*>(a.ids) + row));
+  return id >= 0 && id < a.table_rows ? static_cast<int>(id) : -1;
+}
+
+// 8 consecutive values of kRowsInFlight rows per thread and round.  `group_shift` >= 0: the group
+// size is 2^shift.
+//
+// Bound by the stores (2 bytes written per value, bits/8 read).  With one row per round a thread
+// had one word and two metadata loads in flight and then waited: the rows of a round are
+// independent, so their loads are all issued before the first is used (the octet, its group and
+// its bit position are the same in every row).
 template <int BITS>
 __global__ void __launch_bounds__(kDequantThreads) dequant_octet_kernel(const DequantArgs a, int octets_per_row,
                                                                         int group_shift) {
   const bool has_offsets = a.offsets != nullptr;
   constexpr uint32_t kMask = (1u << BITS) - 1u;
-  for (int row = blockIdx.y; row < a.rows; row += gridDim.y) {
-    const uint32_t* src = a.packed + static_cast<int64_t>(row) * a.words_per_row;
-    for (int o = blockIdx.x * kDequantThreads + threadIdx.x; o < octets_per_row; o += gridDim.x * kDequantThreads) {
-      const int bit = o * 8 * BITS;
-      const int word = bit >> 5;
-      // the octet's 8 * BITS bits (64 at 8-bit: two whole words)
-      uint32_t lo, hi = 0u;
-      if constexpr (BITS == 8) {
-        const uint2 v = __ldg(reinterpret_cast<const uint2*>(src) + o);
-        lo = v.x, hi = v.y;
-      } else if constexpr (BITS == 4) {
-        lo = __ldg(src + word);
-      } else if constexpr (BITS == 2) {
-        lo = __ldg(src + word) >> (bit & 31);
-      } else {
-        const uint32_t w0 = __ldg(src + word);
-        const uint32_t w1 = (bit & 31) > 8 ? __ldg(src + word + 1) : 0u;  // 24 bits from bit (bit & 31)
-        lo = __funnelshift_r(w0, w1, bit & 31);
+  constexpr int U = kRowsInFlight;
+  const int o = blockIdx.x * kDequantThreads + threadIdx.x;
+  if (o >= octets_per_row) return;
+  const int bit = o * 8 * BITS;
+  const int word = bit >> 5;
+  const int value0 = o * 8;
+  const int g = group_shift >= 0 ? (value0 >> group_shift) : value0 / a.group_values;
+  const bool fused = a.meta_dtype != DQ_F32;  // q * scale is exact in fp32: one fma is multiply, then add
+  for (int row0 = blockIdx.y; row0 < a.rows; row0 += gridDim.y * U) {
+    uint32_t lo[U], hi[U];
+    float scale[U], offset[U];
+    bool known[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int row = row0 + u * static_cast<int>(gridDim.y);
+      lo[u] = hi[u] = 0u, scale[u] = offset[u] = 0.0f, known[u] = true;
+      if (row < a.rows) {
+        const int from = source_row(a, row);
+        known[u] = from >= 0;
+        if (from >= 0) {
+          const uint32_t* src = a.packed + static_cast<int64_t>(from) * a.words_per_row;
+          // the octet's 8 * BITS bits (64 at 8-bit: two whole words)
+          if constexpr (BITS == 8) {
+            const uint2 v = __ldg(reinterpret_cast<const uint2*>(src) + o);
+            lo[u] = v.x, hi[u] = v.y;
+          } else {
+            lo[u] = __ldg(src + word);
+            if constexpr (BITS == 3) hi[u] = (bit & 31) > 8 ? __ldg(src + word + 1) : 0u;  // 24 bits from bit (bit & 31)
+          }
+          const int64_t meta = static_cast<int64_t>(from) * a.num_groups + g;
+          scale[u] = load_f32(a.scales, meta, a.meta_dtype);
+          if (has_offsets) offset[u] = load_f32(a.offsets, meta, a.meta_dtype);
+        }
       }
-      const int value0 = o * 8;
-      const int g = group_shift >= 0 ? (value0 >> group_shift) : value0 / a.group_values;
-      const int64_t meta = static_cast<int64_t>(row) * a.num_groups + g;
-      const float scale = load_f32(a.scales, meta, a.meta_dtype);
-      const float offset = has_offsets ? load_f32(a.offsets, meta, a.meta_dtype) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int row = row0 + u * static_cast<int>(gridDim.y);
+      if (row >= a.rows) break;
+      if constexpr (BITS == 2) lo[u] >>= bit & 31;
+      if constexpr (BITS == 3) lo[u] = __funnelshift_r(lo[u], hi[u], bit & 31);
       float vals[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         uint32_t q;
         if constexpr (BITS == 8) {
-          q = ((i < 4 ? lo : hi) >> (8 * (i & 3))) & 0xFFu;
+          q = ((i < 4 ? lo[u] : hi[u]) >> (8 * (i & 3))) & 0xFFu;
         } else {
-          q = (lo >> (BITS * i)) & kMask;
+          q = (lo[u] >> (BITS * i)) & kMask;
         }
         // float(q) without the conversion unit (a quarter-rate pipe): 2^23 + q is exactly
         // representable, so OR-ing q into the mantissa of 2^23 and subtracting 2^23 is exact
         const float qf = __uint_as_float(0x4B000000u | q) - 8388608.0f;
-        float v = __fmul_rn(qf, scale);
-        if (has_offsets) v = __fadd_rn(v, offset);
-        vals[i] = v;
+        if (fused && has_offsets) {
+          vals[i] = __fmaf_rn(qf, scale[u], offset[u]);
+        } else {
+          vals[i] = __fmul_rn(qf, scale[u]);
+          if (has_offsets) vals[i] = __fadd_rn(vals[i], offset[u]);
+        }
+        if (!known[u]) vals[i] = __int_as_float(0x7FC00000);
       }
       const int64_t out_base = static_cast<int64_t>(row) * a.in_features + value0;
       if (a.out_dtype == DQ_F32) {
@@ -128,11 +168,16 @@ __global__ void __launch_bounds__(kDequantThreads) dequant_kernel(const DequantA
     if (live <= 0) {
       continue;
     }
-    const uint32_t* src = a.packed + static_cast<int64_t>(row) * a.words_per_row + word_base;
-    const int64_t meta = static_cast<int64_t>(row) * a.num_groups + g;
+    const int64_t out_base = static_cast<int64_t>(row) * a.in_features + value_base;
+    const int from = source_row(a, row);
+    if (from < 0) {
+      for (int j = 0; j < live; ++j) store_f32(a.out, out_base + j, a.out_dtype, __int_as_float(0x7FC00000));
+      continue;
+    }
+    const uint32_t* src = a.packed + static_cast<int64_t>(from) * a.words_per_row + word_base;
+    const int64_t meta = static_cast<int64_t>(from) * a.num_groups + g;
     const float scale = load_f32(a.scales, meta, a.meta_dtype);
     const float offset = has_offsets ? load_f32(a.offsets, meta, a.meta_dtype) : 0.0f;
-    const int64_t out_base = static_cast<int64_t>(row) * a.in_features + value_base;
 
     if (live == VB && words_left >= WB) {
       uint32_t w[WB];
@@ -209,21 +254,22 @@ __global__ void __launch_bounds__(kDequantThreads) dequant_kernel(const DequantA
 }  // namespace
 }  // namespace dq
 
-extern "C" int32_t dq_dequant(const dq_weight* w, void* out, int32_t out_dtype, void* stream) {
-  dq_geometry g;
-  if (const int32_t rc = dq_resolve_geometry("dequant", w, &g)) return rc;
-  DQ_REQUIRE(dq::dtype_ok(out_dtype), "dequant: unsupported output dtype tag %d", out_dtype);
-  if (w->rows == 0) return DQ_OK;
-  DQ_REQUIRE(out != nullptr, "dequant: null output pointer");
+namespace dq {
+namespace {
 
-  dq::DequantArgs a = {};
+int32_t launch_dequant(const dq_weight* w, const dq_geometry& g, const void* ids, int ids_are_32, int64_t rows, void* out,
+                       int32_t out_dtype, cudaStream_t s) {
+  DequantArgs a = {};
   a.packed = static_cast<const uint32_t*>(w->packed);
   a.scales = w->scales;
   a.offsets = w->offsets;
   a.out = out;
+  a.ids = ids;
+  a.ids_are_32 = ids_are_32;
+  a.table_rows = static_cast<int>(w->rows);
   a.meta_dtype = w->meta_dtype;
   a.out_dtype = out_dtype;
-  a.rows = static_cast<int>(w->rows);
+  a.rows = static_cast<int>(rows);
   a.words_per_row = g.words_per_row;
   a.num_groups = g.num_groups;
   a.words_per_group = g.words_per_group;
@@ -232,12 +278,11 @@ extern "C" int32_t dq_dequant(const dq_weight* w, void* out, int32_t out_dtype, 
   a.blocks_per_group = g.blocks_per_group;
   a.blocks_per_row = g.blocks_per_row;
 
-  const dq::DeviceInfo* dev = dq::device_info();
+  const DeviceInfo* dev = device_info();
   if (dev == nullptr) return DQ_ERR_CUDA;
-  auto s = static_cast<cudaStream_t>(stream);
   // The octet kernel: whole octets per row and per group, 16-byte aligned output rows, and
   // (8-bit) 8-byte aligned packed rows.
-  const size_t out_elem = static_cast<size_t>(dq::dtype_size(out_dtype));
+  const size_t out_elem = static_cast<size_t>(dtype_size(out_dtype));
   const bool octets = a.in_features % 8 == 0 && a.group_values % 8 == 0 &&
                       reinterpret_cast<uintptr_t>(out) % 16 == 0 && (a.in_features * out_elem) % 16 == 0 &&
                       (w->bits != 8 || (reinterpret_cast<uintptr_t>(a.packed) % 8 == 0 && a.words_per_row % 2 == 0));
@@ -248,43 +293,68 @@ extern "C" int32_t dq_dequant(const dq_weight* w, void* out, int32_t out_dtype, 
       shift = 0;
       while ((1 << shift) < a.group_values) ++shift;
     }
-    const int gx = static_cast<int>(std::min<int64_t>(dq::ceil_div(octets_per_row, dq::kDequantThreads), 64));
-    const int gy = static_cast<int>(std::min<int64_t>(a.rows, std::max<int64_t>(1, (static_cast<int64_t>(dev->sm_count) * 64) / gx)));
+    const int64_t gx = ceil_div(octets_per_row, kDequantThreads);
+    // a round per CTA where that fills the chip; few rows (an embedding lookup): a row per CTA
+    const int64_t want = ceil_div(a.rows, kRowsInFlight);
+    const int64_t gy = std::min<int64_t>(want * gx >= dev->sm_count * 4 ? want : a.rows, 65535);
     const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
     switch (w->bits) {
       case 2:
-        dq::dequant_octet_kernel<2><<<grid, dq::kDequantThreads, 0, s>>>(a, octets_per_row, shift);
+        dequant_octet_kernel<2><<<grid, kDequantThreads, 0, s>>>(a, octets_per_row, shift);
         break;
       case 3:
-        dq::dequant_octet_kernel<3><<<grid, dq::kDequantThreads, 0, s>>>(a, octets_per_row, shift);
+        dequant_octet_kernel<3><<<grid, kDequantThreads, 0, s>>>(a, octets_per_row, shift);
         break;
       case 4:
-        dq::dequant_octet_kernel<4><<<grid, dq::kDequantThreads, 0, s>>>(a, octets_per_row, shift);
+        dequant_octet_kernel<4><<<grid, kDequantThreads, 0, s>>>(a, octets_per_row, shift);
         break;
       default:
-        dq::dequant_octet_kernel<8><<<grid, dq::kDequantThreads, 0, s>>>(a, octets_per_row, shift);
+        dequant_octet_kernel<8><<<grid, kDequantThreads, 0, s>>>(a, octets_per_row, shift);
         break;
     }
     DQ_CHECK_LAUNCH("dequant");
     return DQ_OK;
   }
   const int64_t total = static_cast<int64_t>(a.rows) * a.blocks_per_row;
-  const int64_t want = dq::ceil_div(total, dq::kDequantThreads);
+  const int64_t want = ceil_div(total, kDequantThreads);
   const int grid = static_cast<int>(std::min<int64_t>(want, static_cast<int64_t>(dev->sm_count) * 32));
   switch (w->bits) {
     case 2:
-      dq::dequant_kernel<2><<<grid, dq::kDequantThreads, 0, s>>>(a);
+      dequant_kernel<2><<<grid, kDequantThreads, 0, s>>>(a);
       break;
     case 3:
-      dq::dequant_kernel<3><<<grid, dq::kDequantThreads, 0, s>>>(a);
+      dequant_kernel<3><<<grid, kDequantThreads, 0, s>>>(a);
       break;
     case 4:
-      dq::dequant_kernel<4><<<grid, dq::kDequantThreads, 0, s>>>(a);
+      dequant_kernel<4><<<grid, kDequantThreads, 0, s>>>(a);
       break;
     default:
-      dq::dequant_kernel<8><<<grid, dq::kDequantThreads, 0, s>>>(a);
+      dequant_kernel<8><<<grid, kDequantThreads, 0, s>>>(a);
       break;
   }
   DQ_CHECK_LAUNCH("dequant");
   return DQ_OK;
+}
+
+}  // namespace
+}  // namespace dq
+
+extern "C" int32_t dq_dequant(const dq_weight* w, void* out, int32_t out_dtype, void* stream) {
+  dq_geometry g;
+  if (const int32_t rc = dq_resolve_geometry("dequant", w, &g)) return rc;
+  DQ_REQUIRE(dq::dtype_ok(out_dtype), "dequant: unsupported output dtype tag %d", out_dtype);
+  if (w->rows == 0) return DQ_OK;
+  DQ_REQUIRE(out != nullptr, "dequant: null output pointer");
+  return dq::launch_dequant(w, g, nullptr, 0, w->rows, out, out_dtype, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int32_t dq_dequant_rows(const dq_weight* w, const void* ids, int32_t ids_are_int32, int64_t count, void* out,
+                                   int32_t out_dtype, void* stream) {
+  dq_geometry g;
+  if (const int32_t rc = dq_resolve_geometry("dequant_rows", w, &g)) return rc;
+  DQ_REQUIRE(dq::dtype_ok(out_dtype), "dequant_rows: unsupported output dtype tag %d", out_dtype);
+  DQ_REQUIRE(count >= 0 && count < (1LL << 31), "dequant_rows: bad row count %lld", static_cast<long long>(count));
+  if (count == 0) return DQ_OK;
+  DQ_REQUIRE(ids != nullptr && out != nullptr, "dequant_rows: null pointer");
+  return dq::launch_dequant(w, g, ids, ids_are_int32 != 0, count, out, out_dtype, static_cast<cudaStream_t>(stream));
 }

@@ -358,8 +358,7 @@ template <typename Kernel>
 int32_t launch(Kernel kernel, const GemvArgs& args, int grid, size_t smem, cudaStream_t stream,
                const char* what /* kernel name, for dq_last_kernel */) {
   if (smem > 48 * 1024) {
-    DQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(smem)));
+    DQ_CUDA(allow_shared(kernel, smem));
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));

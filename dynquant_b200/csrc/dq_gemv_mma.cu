@@ -445,13 +445,13 @@ template <typename Kernel>
 int32_t launch_mma_kernel(Kernel kernel, const GemvArgs& a, MmaParams p, int threads, size_t smem,
                           const DeviceInfo& dev, cudaStream_t stream) {
   if (smem > 48 * 1024) {
-    DQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    DQ_CUDA(allow_shared(kernel, smem));
   }
   int grid = static_cast<int>(ceil_div(p.tiles, p.rw));
   if (p.kw == 1) {
     // persistent: no more CTAs than the device holds at once; warps stride over the tiles
     int per_sm = 0;
-    DQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+    DQ_CUDA(resident_ctas(&per_sm, kernel, threads, smem));
     grid = std::min(grid, std::max(1, per_sm) * dev.sm_count);
   }
   cudaLaunchConfig_t cfg = {};
@@ -540,9 +540,9 @@ int32_t launch_stream(const GemvArgs& a, const DeviceInfo& dev, int tiles, int s
     return DQ_ERR_UNSUPPORTED;
   }
   auto run = [&](auto kernel) -> int32_t {
-    DQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    DQ_CUDA(allow_shared(kernel, smem));
     int per_sm = 0;
-    DQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, stream::kThreads, smem));
+    DQ_CUDA(resident_ctas(&per_sm, kernel, stream::kThreads, smem));
     const int resident = std::max(1, per_sm) * dev.sm_count;
     int grid = std::min(static_cast<int>(ceil_div(tiles, stream::kWarps)), resident);
     // Strided tiles unless that leaves the busiest SM well above the average.  Several rounds:
@@ -815,7 +815,7 @@ int32_t try_tile(const GemvArgs* jobs, const int* bits, int n, const DeviceInfo&
 
   auto run = [&](auto kernel) -> int32_t {
     if (smem > 48 * 1024) {
-      DQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+      DQ_CUDA(allow_shared(kernel, smem));
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(grid));

@@ -917,9 +917,9 @@ int32_t dq_plan_create(const dq_gemv_job* jobs, int32_t num_jobs, void* workspac
   plan->smem = fixed + (tables ? table_bytes : 0) + static_cast<size_t>(nb) * kWarps * kSlotBytes;
 
   auto set_attr = [&](auto kernel) -> int32_t {
-    DQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(plan->smem)));
+    DQ_CUDA(allow_shared(kernel, plan->smem));
     int per_sm = 0;
-    DQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, plan->smem));
+    DQ_CUDA(resident_ctas(&per_sm, kernel, kThreads, plan->smem));
     if (per_sm < 1) return fail(DQ_ERR_UNSUPPORTED, "plan_create: the kernel does not fit an SM with %zu bytes of shared memory", plan->smem);
     return DQ_OK;
   };

@@ -592,7 +592,7 @@ int32_t launch_mb(const GemvArgs& a, const Params& p, int max_slices, bool force
   const int row_ctas = static_cast<int>(ceil_div(p.tiles, kWarps));
   auto run = [&](auto kernel, auto tag) -> int32_t {
     constexpr int TAG = decltype(tag)::value;
-    DQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    DQ_CUDA(allow_shared(kernel, smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(row_ctas));
     cfg.blockDim = dim3(kThreads);

@@ -138,9 +138,9 @@ int32_t launch_gemv_stream_fused(const GemvArgs* jobs, const int* bits, int n, c
   if (smem > static_cast<size_t>(dev->max_smem_optin)) return DQ_OK;
 
   auto run = [&](auto kernel) -> int32_t {
-    DQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    DQ_CUDA(allow_shared(kernel, smem));
     int per_sm = 0;
-    DQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, stream::kThreads, smem));
+    DQ_CUDA(resident_ctas(&per_sm, kernel, stream::kThreads, smem));
     const int resident = std::max(1, per_sm) * dev->sm_count;
     // CTAs in proportion to the jobs' bytes, every job at least one, no job more CTAs than tiles
     int grid = 0;

@@ -43,7 +43,7 @@ int active_clusters(int tag, Kernel kernel, int slices, size_t smem) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess ||
+  if (allow_shared(kernel, smem) != cudaSuccess ||
       cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
     (void)cudaGetLastError();
     n = 0;
@@ -104,7 +104,7 @@ int32_t launch_sliced(const GemvArgs& a, const DeviceInfo& dev, cudaStream_t str
     }
     const size_t smem = smem_for(slices);
     if (smem > static_cast<size_t>(dev.max_smem_optin)) return DQ_OK;
-    DQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    DQ_CUDA(allow_shared(kernel, smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(row_groups), static_cast<unsigned>(slices));
     cfg.blockDim = dim3(stream::kThreads);

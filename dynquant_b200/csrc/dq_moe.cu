@@ -766,7 +766,7 @@ template <typename Kernel>
 int32_t launch_pdl(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t stream, const MoeArgs& args,
                    const char* what) {
   if (smem > 48 * 1024) {
-    DQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    DQ_CUDA(allow_shared(kernel, smem));
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
@@ -932,7 +932,7 @@ int32_t launch_down_by_token(const dq_weight& w, const dq_geometry& g, const Moe
   auto run = [&](auto kernel, size_t smem) -> int32_t {
     if (smem > static_cast<size_t>(dev->max_smem_optin)) return DQ_OK;  // not taken
     if (smem > 48 * 1024) {
-      DQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+      DQ_CUDA(allow_shared(kernel, smem));
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;

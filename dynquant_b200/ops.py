@@ -433,7 +433,11 @@ def _kernel_args(qt: QuantTensor):
 
 def dequantize(qt: QuantTensor, *, dtype: torch.dtype | None = None) -> torch.Tensor:
     """Reconstruct the dense tensor (``runtime/ops.py:163-181``)."""
-    dense = dequant(*_kernel_args(qt))
+    dense = None
+    if _host is not None and qt.layout == "linear" and not torch.compiler.is_compiling():
+        dense = _host.dequant(qt.packed, qt.scales, qt.offsets, qt.bits, qt.group_size, qt.in_features)
+    if dense is None:
+        dense = dequant(*_kernel_args(qt))
     dense = dense.reshape(qt.logical_shape)
     return dense if dtype is None else dense.to(dtype)
 
@@ -446,6 +450,10 @@ def quantized_matmul(x: torch.Tensor, qt: QuantTensor, bias: torch.Tensor | None
         )
     if len(qt.logical_shape) != 2:
         raise ValueError(f"quantized_matmul expects a 2-D weight; this tensor is {qt.logical_shape}.")
+    if _host is not None and qt.layout == "linear" and not torch.compiler.is_compiling():
+        out = _host.matmul(x, qt.packed, qt.scales, qt.offsets, qt.bits, qt.group_size, qt.in_features, bias)
+        if out is not None:
+            return out
     lead = x.shape[:-1]
     flat = x.reshape(-1, qt.in_features)
     if bias is not None and bias.dtype != flat.dtype:
@@ -470,6 +478,10 @@ def embedding_lookup(qt: QuantTensor, ids: torch.Tensor) -> torch.Tensor:
     """Gather rows of a packed table, then dequantize only those (``runtime/ops.py:234-260``)."""
     if len(qt.logical_shape) != 2:
         raise ValueError(f"embedding table must be 2-D, got {qt.logical_shape}")
+    if _host is not None and qt.layout == "linear" and not torch.compiler.is_compiling():
+        out = _host.embedding(ids, qt.packed, qt.scales, qt.offsets, qt.bits, qt.group_size, qt.in_features)
+        if out is not None:
+            return out
     flat_ids = ids.reshape(-1)
     packed, scales, offsets, bits, group_values, in_features = _kernel_args(qt)
     rows = packed.index_select(0, flat_ids)
@@ -488,6 +500,9 @@ _libs: list[torch.library.Library] = []
 
 
 _native_backend = False
+# The compiled host path (csrc/dq_torch_host.cpp): one C call per entry point.  Its functions
+# return None for whatever they do not take, and the Python code below them then runs.
+_host = None
 
 
 def torch_ops_backend() -> str:
@@ -509,9 +524,25 @@ def _load_torch_shim() -> bool:
     try:
         _lib.load()
         torch.ops.load_library(str(path))
+        _load_host(path)
     except (OSError, RuntimeError, _lib.LibraryUnavailableError):
         return False  # built against another torch, or the C-ABI library is missing: Python backend
     return True
+
+
+def _load_host(path) -> None:
+    from importlib.machinery import ExtensionFileLoader
+    from importlib.util import module_from_spec, spec_from_file_location
+
+    global _host
+    name = f"{__package__}._host"
+    try:
+        spec = spec_from_file_location(name, str(path), loader=ExtensionFileLoader(name, str(path)))
+        module = module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _host = module
+    except ImportError:
+        _host = None  # a shim built without the module: the Python path serves every call
 
 
 def register_torch_ops() -> bool:

@@ -22,6 +22,7 @@ Mirrors the contract of the reference's serving plugins without importing a fram
 
 from __future__ import annotations
 
+import struct
 from dataclasses import dataclass
 from typing import Any, Sequence
 
@@ -75,6 +76,13 @@ class FusedPackedGeometry:
         self.out_features = row
         self.qweight_numel = qoff
         self.scale_numel = soff
+        # the shards as csrc/dq_torch_host.cpp reads them: eight int64 each
+        self.table = b"".join(
+            struct.pack("8q", p.spec.out_features, p.words_per_row, p.num_groups,
+                        row_geometry(p.spec.bits, p.spec.group_size, in_features).effective_group, in_features,
+                        p.qweight_offset, p.scale_offset, p.spec.bits)
+            for p in plans
+        )
 
     def __len__(self) -> int:
         return len(self._plans)
@@ -263,6 +271,11 @@ class DynQuantLinearMethod:
 
     def apply(self, layer: torch.nn.Module, x: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
         geometry: FusedPackedGeometry = layer.dynquant_geometry
+        if ops._host is not None and not torch.compiler.is_compiling():
+            params = layer._parameters
+            out = ops._host.fused(x, params.get("qweight"), params.get("scales"), params.get("offsets"), geometry.table, bias)
+            if out is not None:
+                return out
         shards = [self.shard_tensor(layer, i) for i in range(len(geometry))]
         lead = x.shape[:-1]
         flat = x.reshape(-1, geometry.in_features)

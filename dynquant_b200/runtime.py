@@ -104,9 +104,14 @@ class _PackedModule(nn.Module):
 
 
 def _encode(weight: torch.Tensor, bits: int, group_size: int, symmetric: bool) -> QuantTensor:
-    """Min/max encoding of a dense weight on its own device's host copy (no clip search: the
-    reference's encoder search is outside this package)."""
+    """Min/max encoding of a dense weight: ``dq_encode`` where the weight is on the GPU and of a
+    shape that kernel takes, else on the host (no clip search: the reference's encoder search is
+    outside this package)."""
     w = weight.detach()
+    if w.is_cuda and ops._host is not None:
+        parts = ops._host.encode(w, bits, group_size, symmetric)  # the same bits, on the GPU
+        if parts is not None:
+            return QuantTensor(*parts, bits, group_size, w.shape[-1], tuple(w.shape), symmetric=symmetric)
     meta = w.dtype if w.dtype in (torch.float16, torch.bfloat16) else torch.float16
     qt = QuantTensor.from_dense(w.cpu(), bits=bits, group_size=group_size, symmetric=symmetric, compute_dtype=meta)
     return qt.to(w.device)
@@ -126,6 +131,13 @@ class DynQuantLinear(_PackedModule):
         return cls(_encode(linear.weight, bits, group_size, symmetric), linear.bias)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        if ops._host is not None and not torch.compiler.is_compiling():
+            # straight from the registered buffers to the library: no view object, no geometry
+            spec, held = self.spec, self.holder._buffers
+            out = ops._host.matmul(x, held["qweight"], held["scales"], held["offsets"], spec.bits, spec.group_size,
+                                   spec.in_features, self._buffers["bias"])
+            if out is not None:
+                return out
         return ops.quantized_matmul(x, self.weight_qt, self.bias)
 
 
@@ -146,6 +158,12 @@ class DynQuantEmbedding(_PackedModule):
         return cls(_encode(embedding.weight, bits, group_size, symmetric), padding_idx=embedding.padding_idx)
 
     def forward(self, ids: torch.Tensor) -> torch.Tensor:
+        if ops._host is not None and not torch.compiler.is_compiling():
+            spec, held = self.spec, self.holder._buffers
+            out = ops._host.embedding(ids, held["qweight"], held["scales"], held["offsets"], spec.bits, spec.group_size,
+                                      spec.in_features)
+            if out is not None:
+                return out
         return ops.embedding_lookup(self.weight_qt, ids)
 
 

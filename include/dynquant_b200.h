@@ -120,6 +120,20 @@ DQ_API int32_t dq_resolve_geometry(const char* op, const dq_weight* w, dq_geomet
  * dtype; any dq_dtype is accepted here.  w = float(q)*scale, then + offset,
  * in fp32, one rounding to out_dtype. */
 DQ_API int32_t dq_dequant(const dq_weight* w, void* out, int32_t out_dtype, void* stream);
+/* Embedding lookup (reference: embedding_lookup, runtime/ops.py:234-260, three gathers and a
+ * dequant): out [count, in_features] = the dense rows `ids` (device array of int64, or int32) of
+ * the table, in one launch.  An id outside the table gives a row of NaN. */
+DQ_API int32_t dq_dequant_rows(const dq_weight* w, const void* ids, int32_t ids_are_int32, int64_t count,
+                               void* out, int32_t out_dtype, void* stream);
+
+/* ---- encode (reference: QuantTensor.from_dense, quant/tensor.py:239-396, without clipping) ----
+ * Min/max group quantization of a dense [rows, in_features] matrix into packed words
+ * [rows, groups * group_values * bits / 32] and scales / offsets [rows, groups] of meta_dtype;
+ * rows are padded with zeros to whole groups.  Bit-identical to the host encoder.  Groups of 32,
+ * 64, 128 or 256 values and in_features % 8 == 0, else DQ_ERR_UNSUPPORTED (nothing launched). */
+DQ_API int32_t dq_encode(const void* w, int32_t w_dtype, int64_t rows, int64_t in_features, int32_t bits,
+                         int64_t group_values, int32_t symmetric, void* packed, void* scales, void* offsets,
+                         int32_t meta_dtype, void* stream);
 
 /* ---- achievable-bandwidth probes (reference: achievable_bandwidth,
  *      packages/dynquant-core/src/dynquant/commands/bench.py:95-120, which times
