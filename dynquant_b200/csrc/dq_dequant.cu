@@ -18,8 +18,7 @@
 // the group size multiples of 8): a thread produces 8 consecutive values -- one 16-byte
 // store for a 16-bit output, so a warp writes 512 contiguous bytes per store instruction --
 // from the 8 * BITS bits at bit 8 * BITS * octet of its row (the packed row is one
-// contiguous LSB-first bit string: groups are whole numbers of 32-value blocks).  Rows run
-// over blockIdx.y and octets over blockIdx.x, so no thread divides anything.  dequant_kernel
+// contiguous LSB-first bit string: groups are whole numbers of 32-value blocks).  dequant_kernel
 // is the general one: one thread per block of 16/32/8/4 values at 2/3/4/8-bit, any tail.
 #include <algorithm>
 
@@ -28,8 +27,7 @@
 namespace dq {
 namespace {
 
-constexpr int kDequantThreads = 256;
-constexpr int kRowsInFlight = 4;
+constexpr int kDequantThreads = 128;
 
 struct DequantArgs {
   const uint32_t* packed;
@@ -54,93 +52,92 @@ __device__ __forceinline__ int source_row(const DequantArgs& a, int row) {
   return id >= 0 && id < a.table_rows ? static_cast<int>(id) : -1;
 }
 
-// 8 consecutive values of kRowsInFlight rows per thread and round.  `group_shift` >= 0: the group
-// size is 2^shift.
+// U runs of 8 consecutive values per thread, kDequantThreads octets apart, so that a CTA
+// writes one contiguous stretch of the output and the grid writes the output front to back.
+// `group_shift` >= 0: the group size is 2^shift.  `per_row_magic` = ceil(2^64 / octets_per_row):
+// the high half of its product with an octet's number is the octet's row (exact below 2^32).
 //
-// Bound by the stores (2 bytes written per value, bits/8 read).  With one row per round a thread
-// had one word and two metadata loads in flight and then waited: the rows of a round are
-// independent, so their loads are all issued before the first is used (the octet, its group and
-// its bit position are the same in every row).
-template <int BITS>
-__global__ void __launch_bounds__(kDequantThreads) dequant_octet_kernel(const DequantArgs a, int octets_per_row,
+// Bound by the stores (2 bytes written per value, bits/8 read): 14336 x 4096 at 3 / 4 / 8 bits takes
+// 39 / 37 / 37 us where filling the output with zeros takes 33.  (Octets over blockIdx.x and rows
+// over blockIdx.y, one octet per thread: 52 / 44 / 44 -- and 14 us against 10 on 14080 x 768, whose
+// rows left most threads of a CTA idle.)  256 threads and 4 octets: 43; 2 octets: 39 to 41.
+template <int BITS, int U>
+__global__ void __launch_bounds__(kDequantThreads) dequant_octet_kernel(const DequantArgs a, unsigned octets_per_row,
+                                                                        unsigned long long per_row_magic, unsigned total,
                                                                         int group_shift) {
   const bool has_offsets = a.offsets != nullptr;
   constexpr uint32_t kMask = (1u << BITS) - 1u;
-  constexpr int U = kRowsInFlight;
-  const int o = blockIdx.x * kDequantThreads + threadIdx.x;
-  if (o >= octets_per_row) return;
-  const int bit = o * 8 * BITS;
-  const int word = bit >> 5;
-  const int value0 = o * 8;
-  const int g = group_shift >= 0 ? (value0 >> group_shift) : value0 / a.group_values;
   const bool fused = a.meta_dtype != DQ_F32;  // q * scale is exact in fp32: one fma is multiply, then add
-  for (int row0 = blockIdx.y; row0 < a.rows; row0 += gridDim.y * U) {
-    uint32_t lo[U], hi[U];
-    float scale[U], offset[U];
-    bool known[U];
+  const unsigned first = blockIdx.x * (kDequantThreads * U) + threadIdx.x;
+  uint32_t lo[U], hi[U];
+  float scale[U], offset[U];
+  bool known[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int row = row0 + u * static_cast<int>(gridDim.y);
-      lo[u] = hi[u] = 0u, scale[u] = offset[u] = 0.0f, known[u] = true;
-      if (row < a.rows) {
-        const int from = source_row(a, row);
-        known[u] = from >= 0;
-        if (from >= 0) {
-          const uint32_t* src = a.packed + static_cast<int64_t>(from) * a.words_per_row;
-          // the octet's 8 * BITS bits (64 at 8-bit: two whole words)
-          if constexpr (BITS == 8) {
-            const uint2 v = __ldg(reinterpret_cast<const uint2*>(src) + o);
-            lo[u] = v.x, hi[u] = v.y;
-          } else {
-            lo[u] = __ldg(src + word);
-            if constexpr (BITS == 3) hi[u] = (bit & 31) > 8 ? __ldg(src + word + 1) : 0u;  // 24 bits from bit (bit & 31)
-          }
-          const int64_t meta = static_cast<int64_t>(from) * a.num_groups + g;
-          scale[u] = load_f32(a.scales, meta, a.meta_dtype);
-          if (has_offsets) offset[u] = load_f32(a.offsets, meta, a.meta_dtype);
+  for (int u = 0; u < U; ++u) {
+    const unsigned at = first + u * kDequantThreads;
+    lo[u] = hi[u] = 0u, scale[u] = offset[u] = 0.0f, known[u] = true;
+    if (at < total) {
+      const int row = static_cast<int>(__umul64hi(at, per_row_magic));
+      const int o = static_cast<int>(at - row * octets_per_row);
+      const int from = source_row(a, row);
+      known[u] = from >= 0;
+      if (from >= 0) {
+        const int bit = o * 8 * BITS;
+        const int word = bit >> 5;
+        const uint32_t* src = a.packed + static_cast<int64_t>(from) * a.words_per_row;
+        // the octet's 8 * BITS bits (64 at 8-bit: two whole words)
+        if constexpr (BITS == 8) {
+          const uint2 v = __ldg(reinterpret_cast<const uint2*>(src) + o);
+          lo[u] = v.x, hi[u] = v.y;
+        } else {
+          lo[u] = __ldg(src + word);
+          if constexpr (BITS == 3) hi[u] = (bit & 31) > 8 ? __ldg(src + word + 1) : 0u;  // 24 bits from bit (bit & 31)
         }
+        const int g = group_shift >= 0 ? ((o * 8) >> group_shift) : (o * 8) / a.group_values;
+        const int64_t meta = static_cast<int64_t>(from) * a.num_groups + g;
+        scale[u] = load_f32(a.scales, meta, a.meta_dtype);
+        if (has_offsets) offset[u] = load_f32(a.offsets, meta, a.meta_dtype);
+        if constexpr (BITS == 2) lo[u] >>= bit & 31;
+        if constexpr (BITS == 3) lo[u] = __funnelshift_r(lo[u], hi[u], bit & 31);
       }
     }
+  }
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int row = row0 + u * static_cast<int>(gridDim.y);
-      if (row >= a.rows) break;
-      if constexpr (BITS == 2) lo[u] >>= bit & 31;
-      if constexpr (BITS == 3) lo[u] = __funnelshift_r(lo[u], hi[u], bit & 31);
-      float vals[8];
+  for (int u = 0; u < U; ++u) {
+    const unsigned at = first + u * kDequantThreads;
+    if (at >= total) break;
+    float vals[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        uint32_t q;
-        if constexpr (BITS == 8) {
-          q = ((i < 4 ? lo[u] : hi[u]) >> (8 * (i & 3))) & 0xFFu;
-        } else {
-          q = (lo[u] >> (BITS * i)) & kMask;
-        }
-        // float(q) without the conversion unit (a quarter-rate pipe): 2^23 + q is exactly
-        // representable, so OR-ing q into the mantissa of 2^23 and subtracting 2^23 is exact
-        const float qf = __uint_as_float(0x4B000000u | q) - 8388608.0f;
-        if (fused && has_offsets) {
-          vals[i] = __fmaf_rn(qf, scale[u], offset[u]);
-        } else {
-          vals[i] = __fmul_rn(qf, scale[u]);
-          if (has_offsets) vals[i] = __fadd_rn(vals[i], offset[u]);
-        }
-        if (!known[u]) vals[i] = __int_as_float(0x7FC00000);
-      }
-      const int64_t out_base = static_cast<int64_t>(row) * a.in_features + value0;
-      if (a.out_dtype == DQ_F32) {
-        float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + out_base);
-        dst[0] = make_float4(vals[0], vals[1], vals[2], vals[3]);
-        dst[1] = make_float4(vals[4], vals[5], vals[6], vals[7]);
+    for (int i = 0; i < 8; ++i) {
+      uint32_t q;
+      if constexpr (BITS == 8) {
+        q = ((i < 4 ? lo[u] : hi[u]) >> (8 * (i & 3))) & 0xFFu;
       } else {
-        uint32_t p16[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          p16[j] = round_pair_to_16(vals[2 * j], vals[2 * j + 1], a.out_dtype);
-        }
-        *reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(a.out) + out_base) =
-            make_uint4(p16[0], p16[1], p16[2], p16[3]);
+        q = (lo[u] >> (BITS * i)) & kMask;
       }
+      // float(q) without the conversion unit (a quarter-rate pipe): 2^23 + q is exactly
+      // representable, so OR-ing q into the mantissa of 2^23 and subtracting 2^23 is exact
+      const float qf = __uint_as_float(0x4B000000u | q) - 8388608.0f;
+      if (fused && has_offsets) {
+        vals[i] = __fmaf_rn(qf, scale[u], offset[u]);
+      } else {
+        vals[i] = __fmul_rn(qf, scale[u]);
+        if (has_offsets) vals[i] = __fadd_rn(vals[i], offset[u]);
+      }
+      if (!known[u]) vals[i] = __int_as_float(0x7FC00000);
+    }
+    // rows are whole octets, so octet `at` of the output starts at value 8 * at
+    if (a.out_dtype == DQ_F32) {
+      float4* dst = reinterpret_cast<float4*>(a.out) + static_cast<size_t>(at) * 2;
+      dst[0] = make_float4(vals[0], vals[1], vals[2], vals[3]);
+      dst[1] = make_float4(vals[4], vals[5], vals[6], vals[7]);
+    } else {
+      uint32_t p16[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        p16[j] = round_pair_to_16(vals[2 * j], vals[2 * j + 1], a.out_dtype);
+      }
+      reinterpret_cast<uint4*>(a.out)[at] = make_uint4(p16[0], p16[1], p16[2], p16[3]);
     }
   }
 }
@@ -286,30 +283,32 @@ int32_t launch_dequant(const dq_weight* w, const dq_geometry& g, const void* ids
   const bool octets = a.in_features % 8 == 0 && a.group_values % 8 == 0 &&
                       reinterpret_cast<uintptr_t>(out) % 16 == 0 && (a.in_features * out_elem) % 16 == 0 &&
                       (w->bits != 8 || (reinterpret_cast<uintptr_t>(a.packed) % 8 == 0 && a.words_per_row % 2 == 0));
-  if (octets) {
-    const int octets_per_row = a.in_features / 8;
+  const int64_t num_octets = static_cast<int64_t>(a.rows) * (a.in_features / 8);
+  if (octets && a.in_features > 8 && num_octets < (int64_t{1} << 32)) {
+    const unsigned per_row = static_cast<unsigned>(a.in_features / 8);
+    const unsigned long long magic = ~0ull / per_row + 1;  // ceil(2^64 / per_row)
     int shift = -1;
     if ((a.group_values & (a.group_values - 1)) == 0) {
       shift = 0;
       while ((1 << shift) < a.group_values) ++shift;
     }
-    const int64_t gx = ceil_div(octets_per_row, kDequantThreads);
-    // a round per CTA where that fills the chip; few rows (an embedding lookup): a row per CTA
-    const int64_t want = ceil_div(a.rows, kRowsInFlight);
-    const int64_t gy = std::min<int64_t>(want * gx >= dev->sm_count * 4 ? want : a.rows, 65535);
-    const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
+    const unsigned total = static_cast<unsigned>(num_octets);
+    // Four octets per thread from a full wave of such threads on; below it more CTAs are worth more
+    // than loads in flight (6912 x 1024, 0.9 M octets: 7.1 us with one, 8.3 with four).
+    const bool four = num_octets >= static_cast<int64_t>(dev->sm_count) * 2048 * 4;
+    const unsigned grid = static_cast<unsigned>(ceil_div(num_octets, kDequantThreads * (four ? 4 : 1)));
     switch (w->bits) {
       case 2:
-        dequant_octet_kernel<2><<<grid, kDequantThreads, 0, s>>>(a, octets_per_row, shift);
+        (four ? dequant_octet_kernel<2, 4> : dequant_octet_kernel<2, 1>)<<<grid, kDequantThreads, 0, s>>>(a, per_row, magic, total, shift);
         break;
       case 3:
-        dequant_octet_kernel<3><<<grid, kDequantThreads, 0, s>>>(a, octets_per_row, shift);
+        (four ? dequant_octet_kernel<3, 4> : dequant_octet_kernel<3, 1>)<<<grid, kDequantThreads, 0, s>>>(a, per_row, magic, total, shift);
         break;
       case 4:
-        dequant_octet_kernel<4><<<grid, kDequantThreads, 0, s>>>(a, octets_per_row, shift);
+        (four ? dequant_octet_kernel<4, 4> : dequant_octet_kernel<4, 1>)<<<grid, kDequantThreads, 0, s>>>(a, per_row, magic, total, shift);
         break;
       default:
-        dequant_octet_kernel<8><<<grid, kDequantThreads, 0, s>>>(a, octets_per_row, shift);
+        (four ? dequant_octet_kernel<8, 4> : dequant_octet_kernel<8, 1>)<<<grid, kDequantThreads, 0, s>>>(a, per_row, magic, total, shift);
         break;
     }
     DQ_CHECK_LAUNCH("dequant");

@@ -1,0 +1,499 @@
+// Packed matrix x many activation rows on the fifth-generation tensor cores:
+//   out[m, n] = sum_k x[m, k] * (q[n, k] * s[n, g] + o[n, g]) (+ bias[n])
+// for prefill and large batches, in ONE pass -- the reference (and this library before) writes the
+// dense matrix out and reads it back for a library GEMM (runtime/ops.py:205-231).
+//
+// A CTA computes 128 weight rows x n_tile activation rows (16..256) with the weights as the A
+// operand of tcgen05.mma:
+//   * warp 2 streams packed 128 x 128-value tiles into shared memory by TMA (they are 4..16 KB, so
+//     a ring of them keeps HBM busy), warp 0 the activation in 64-value slabs with the 128-byte
+//     swizzle, both zero-filled past the edges of their tensors;
+//   * two warpgroups (warps 4..11) decode, one 64-value half of a tile each: a thread owns one
+//     weight row, so its scale and offset are two registers and its packed words one contiguous
+//     piece of shared memory; the 16-bit weights go straight to TENSOR MEMORY (tcgen05.st) in the
+//     natural order -- not to shared memory, whose bandwidth the activation needs;
+//   * warp 1 issues the MMAs (A from tensor memory, B from shared memory), accumulating in tensor
+//     memory; two accumulator tiles where they fit (n_tile <= 192), so that the decode of the next
+//     tile runs under the epilogue of this one.
+// What bounds it: with n_tile >= 144 the tensor pipe (128 x n_tile x 64 take 2 n_tile cycles), below
+// that the decode (about 290 cycles per 128 x 64 values on the SM's four schedulers).
+//
+// Small matrices: the reduction axis is sliced over a thread-block cluster (grid.y), each CTA leaves
+// its fp32 tile in its own shared memory and the CTAs of the cluster add a share of the columns
+// each, in slice order, over distributed shared memory -- deterministic.
+//
+// Every wait is bounded (dq_umma.cuh): when one runs out the block stops issuing, drains its own
+// copies, frees its tensor memory, leaves its output unwritten and raises the device's error word
+// (dq_gemm_status).
+#include <algorithm>
+#include <cmath>
+
+#include "dq_gemm_umma.cuh"
+#include "dq_gemv.cuh"
+#include "dq_umma_decode.cuh"
+
+namespace dq {
+namespace {
+
+using namespace umma;
+
+constexpr int kJobs = 4;
+constexpr int kThreads = 384;          // warps 0..3: TMA x, MMA, TMA weights, tensor memory; 4..11 decode
+constexpr int kDecodeWarp0 = 4;
+constexpr int kASlots = 4;             // operand tiles of 128 x 64 in tensor memory, 32 columns each
+constexpr int kAColumns = kASlots * 32;
+constexpr int kMaxRing = 16;
+
+struct Job {
+  CUtensorMap wmap;
+  const void* scales;
+  const void* offsets;                 // may be null
+  const void* bias;                    // may be null; element 0 belongs to output column 0 of this job
+  int64_t col0;
+  int rows, row_tiles, bits, num_groups, group_shift, meta_dtype;  // group = 64 << group_shift
+};
+
+struct Params {
+  Job job[kJobs];
+  CUtensorMap xmap;
+  void* out;
+  int64_t out_stride;
+  int jobs, m, chunks;                 // chunks of 128 values of K
+  int row_tiles, tiles;                // over all jobs; tiles = row_tiles x token tiles
+  int n_tile, d_buffers, tmem_columns;
+  int x_slots, w_slots, w_bytes;       // rings; bytes of a weight slot
+  int slices;
+  uint32_t ring_offset, barrier_offset;
+};
+
+__device__ unsigned int g_gemm_failed = 0;
+
+// One warpgroup's half of the chunks [c0, c1) of a row tile; false once a wait has run out.
+template <int BITS, bool BF16>
+__device__ bool decode_tile(const Job& job, int row0, int c0, int c1, int half, unsigned char* w_ring, int w_slots, int w_bytes,
+                            uint32_t bars_w_full, uint32_t bars_w_empty, uint32_t bars_a_full, uint32_t bars_a_empty,
+                            uint32_t a_tmem, uint32_t& w_at, uint32_t& stage, volatile int* failed) {
+  const int lane = threadIdx.x & 31;
+  const int warp4 = (threadIdx.x >> 5) & 3;
+  const int r = warp4 * 32 + lane;
+  const int row = min(row0 + r, job.rows - 1);
+  const unsigned short* s_row = static_cast<const unsigned short*>(job.scales) + static_cast<int64_t>(row) * job.num_groups;
+  const unsigned short* o_row =
+      job.offsets == nullptr ? nullptr : static_cast<const unsigned short*>(job.offsets) + static_cast<int64_t>(row) * job.num_groups;
+  const bool mbf = job.meta_dtype == DQ_BF16;
+  auto widen = [&](unsigned short v) -> float {
+    return mbf ? __uint_as_float(static_cast<uint32_t>(v) << 16) : __half2float(__ushort_as_half(v));
+  };
+  auto group_of = [&](int c) -> int { return min((2 * c + half) >> job.group_shift, job.num_groups - 1); };
+  int g = group_of(c0);
+  unsigned short s_next = __ldg(s_row + g), o_next = o_row != nullptr ? __ldg(o_row + g) : 0;
+  Affine<BITS> affine;
+  int g_have = -1;
+  for (int c = c0; c < c1; ++c) {
+    if (g != g_have) {
+      affine.set(widen(s_next), o_row != nullptr ? widen(o_next) : 0.0f);
+      g_have = g;
+    }
+    // the next tile's metadata travels while this one is decoded
+    g = group_of(min(c + 1, c1 - 1));
+    if (g != g_have) {
+      s_next = __ldg(s_row + g);
+      if (o_row != nullptr) o_next = __ldg(o_row + g);
+    }
+    const uint32_t slot = w_at % static_cast<uint32_t>(w_slots);
+    if (!mbar_wait(bars_w_full + slot * 8, (w_at / static_cast<uint32_t>(w_slots)) & 1, failed)) return false;
+    uint32_t w[2 * BITS];
+    read_row64<BITS>(w_ring + slot * w_bytes, r, half, w);
+    const uint32_t a_slot = stage % kASlots;
+    uint32_t v[32];
+    decode32<BITS, BF16>(w, affine, v);
+    decode32<BITS, BF16>(w + BITS, affine, v + 16);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bars_w_empty + slot * 8);  // (the words are in registers)
+    if (!mbar_wait(bars_a_empty + a_slot * 8, ((stage / kASlots) & 1) ^ 1, failed)) return false;
+    fence_after_sync();
+    const uint32_t dst = a_tmem + a_slot * 32 + (static_cast<uint32_t>(warp4 * 32) << 16);
+    tmem_st16(dst, v);
+    tmem_st16(dst + 16, v + 16);
+    tmem_wait_st();
+    fence_before_sync();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bars_a_full + a_slot * 8);
+    ++w_at;
+    stage += 2;
+  }
+  return true;
+}
+
+template <bool BF16>
+__global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_constant__ Params p) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  // control block at the front: failure flag, tensor memory address, barriers
+  volatile int* failed = reinterpret_cast<volatile int*>(smem);
+  const uint32_t base = smem_addr(smem);
+  const uint32_t bars = base + p.barrier_offset;
+  const uint32_t bar_x_full = bars, bar_x_empty = bar_x_full + kMaxRing * 8, bar_w_full = bar_x_empty + kMaxRing * 8,
+                 bar_w_empty = bar_w_full + kMaxRing * 8, bar_a_full = bar_w_empty + kMaxRing * 8, bar_a_empty = bar_a_full + kASlots * 8,
+                 bar_d_full = bar_a_empty + kASlots * 8, bar_d_empty = bar_d_full + 2 * 8, bar_drain = bar_d_empty + 2 * 8;
+  const int x_bytes = p.n_tile * 128;
+  unsigned char* x_ring = smem + p.ring_offset;
+  unsigned char* w_ring = x_ring + p.x_slots * x_bytes;
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    *failed = 0;
+    for (int i = 0; i < p.x_slots; ++i) mbar_init(bar_x_full + i * 8, 1), mbar_init(bar_x_empty + i * 8, 1);
+    for (int i = 0; i < p.w_slots; ++i) mbar_init(bar_w_full + i * 8, 1), mbar_init(bar_w_empty + i * 8, 8);
+    for (int i = 0; i < kASlots; ++i) mbar_init(bar_a_full + i * 8, 4), mbar_init(bar_a_empty + i * 8, 1);
+    for (int i = 0; i < 2; ++i) mbar_init(bar_d_full + i * 8, 1), mbar_init(bar_d_empty + i * 8, 8);
+    mbar_init(bar_drain, 1);
+    fence_mbar_init();
+    tma_prefetch_map(&p.xmap);
+  }
+  if (warp == 3) tmem_alloc(base + 4, static_cast<uint32_t>(p.tmem_columns));
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + 4);
+  const uint32_t d_tmem = tmem + kAColumns;
+  pdl_launch_dependents();
+
+  // this CTA's share of the reduction axis (slices: as equal as possible, in chunks)
+  const int slice = static_cast<int>(blockIdx.y);
+  const int c0 = static_cast<int>(static_cast<int64_t>(p.chunks) * slice / p.slices);
+  const int c1 = static_cast<int>(static_cast<int64_t>(p.chunks) * (slice + 1) / p.slices);
+
+  auto job_of = [&](int row_tile, int& local) -> int {
+    int j = 0;
+    local = row_tile;
+    while (j + 1 < p.jobs && local >= p.job[j].row_tiles) local -= p.job[j++].row_tiles;
+    return j;
+  };
+
+  if (warp == 0 || warp == 2) {
+    if (elect_one()) {
+      const bool weights = warp == 2;
+      if (!weights) pdl_wait_prior_grid();  // the activation is the previous kernel's; weights are nobody's
+      const uint32_t full = weights ? bar_w_full : bar_x_full, empty = weights ? bar_w_empty : bar_x_empty;
+      const uint32_t slots = static_cast<uint32_t>(weights ? p.w_slots : p.x_slots);
+      uint32_t at = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
+        int local;
+        const Job& job = p.job[job_of(tile % p.row_tiles, local)];
+        const int token0 = (tile / p.row_tiles) * p.n_tile;
+        const int count = weights ? c1 - c0 : 2 * (c1 - c0);
+        const int bytes = weights ? 2048 * job.bits : x_bytes;
+        for (int i = 0; i < count; ++i, ++at) {
+          const uint32_t slot = at % slots;
+          if (!(ok = mbar_wait(empty + slot * 8, ((at / slots) & 1) ^ 1, failed))) break;
+          mbar_expect(full + slot * 8, static_cast<uint32_t>(bytes));
+          if (weights) {
+            tma_load_2d(smem_addr(w_ring) + slot * p.w_bytes, &job.wmap, (c0 + i) * 4 * job.bits, local * 128, full + slot * 8);
+          } else {
+            tma_load_2d(smem_addr(x_ring) + slot * x_bytes, &p.xmap, c0 * 128 + i * 64, token0, full + slot * 8);
+          }
+        }
+      }
+      if (!ok || *failed != 0) {  // wait for the copies in flight
+        for (uint32_t k = at > slots ? at - slots : 0; k < at; ++k) {
+          for (int i = 0; i < kSpins && !mbar_try(full + (k % slots) * 8, (k / slots) & 1); ++i) {
+          }
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint32_t idesc = mma_descriptor(BF16, p.n_tile);
+      uint32_t stage = 0, d_at = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x, ++d_at) {
+        const uint32_t buffer = d_at % static_cast<uint32_t>(p.d_buffers);
+        if (!mbar_wait(bar_d_empty + buffer * 8, ((d_at / p.d_buffers) & 1) ^ 1, failed)) break;
+        fence_after_sync();
+        const uint32_t d = d_tmem + buffer * p.n_tile;
+        for (int i = 0; i < 2 * (c1 - c0); ++i, ++stage) {
+          const uint32_t xs = stage % static_cast<uint32_t>(p.x_slots), as = stage % kASlots;
+          if (!(ok = mbar_wait(bar_x_full + xs * 8, (stage / p.x_slots) & 1, failed))) break;
+          if (!(ok = mbar_wait(bar_a_full + as * 8, (stage / kASlots) & 1, failed))) break;
+          fence_after_sync();
+          const uint64_t b = smem_descriptor(smem_addr(x_ring) + xs * x_bytes);
+          const uint32_t a = tmem + as * 32;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) mma_ts(d, a + k * 8, b + k * 2, idesc, i > 0 || k > 0);
+          mma_commit(bar_a_empty + as * 8);
+          mma_commit(bar_x_empty + xs * 8);
+        }
+        if (ok) mma_commit(bar_d_full + buffer * 8);
+      }
+      if (*failed != 0) {  // MMAs in flight read and write tensor memory: it is freed after them
+        mma_commit(bar_drain);
+        for (int i = 0; i < kSpins && !mbar_try(bar_drain, 0); ++i) {
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp >= kDecodeWarp0) {
+    const int half = (warp - kDecodeWarp0) >> 2;
+    const int warp4 = warp & 3;
+    const int r = warp4 * 32 + lane;
+    uint32_t w_at = 0, stage = static_cast<uint32_t>(half), d_at = 0;
+    for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, ++d_at) {
+      int local;
+      const Job& job = p.job[job_of(tile % p.row_tiles, local)];
+      bool ok;
+#define DQ_DECODE(B)                                                                                                             \
+  ok = decode_tile<B, BF16>(job, local * 128, c0, c1, half, w_ring, p.w_slots, p.w_bytes, bar_w_full, bar_w_empty, bar_a_full, \
+                            bar_a_empty, tmem, w_at, stage, failed)
+      switch (job.bits) {
+        case 2: DQ_DECODE(2); break;
+        case 3: DQ_DECODE(3); break;
+        case 4: DQ_DECODE(4); break;
+        default: DQ_DECODE(8); break;
+      }
+#undef DQ_DECODE
+      if (!ok) break;
+      const uint32_t buffer = d_at % static_cast<uint32_t>(p.d_buffers);
+      if (!mbar_wait(bar_d_full + buffer * 8, (d_at / p.d_buffers) & 1, failed)) break;
+      fence_after_sync();
+      // the two warpgroups share the columns
+      const int split = (p.n_tile / 2 + 15) / 16 * 16;
+      const int first = half == 0 ? 0 : split, last = half == 0 ? split : p.n_tile;
+      const uint32_t src = d_tmem + buffer * p.n_tile + (static_cast<uint32_t>(warp4 * 32) << 16);
+      const int row = local * 128 + r;
+      const int token0 = (tile / p.row_tiles) * p.n_tile;
+      const float bias = job.bias != nullptr && row < job.rows ? load_f32(job.bias, row, BF16 ? DQ_BF16 : DQ_F16) : 0.0f;
+      unsigned short* dst = static_cast<unsigned short*>(p.out) + job.col0 + row;
+      float* red = reinterpret_cast<float*>(smem + p.ring_offset);
+      for (int col = first; col < last; col += 16) {
+        uint32_t v[16];
+        tmem_ld16(src + col, v);
+        tmem_wait_ld();
+        if (p.slices > 1) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) red[(col + i) * 128 + r] = __uint_as_float(v[i]);
+        } else if (row < job.rows) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const int token = token0 + col + i;
+            if (token < p.m) {
+              dst[static_cast<int64_t>(token) * p.out_stride] =
+                  static_cast<unsigned short>(round_to_16(__uint_as_float(v[i]) + bias, BF16 ? DQ_BF16 : DQ_F16));
+            }
+          }
+        }
+      }
+      fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_d_empty + buffer * 8);
+    }
+  }
+
+  __syncthreads();
+  if (p.slices > 1) {  // one tile per cluster: add the slices' columns, a share of them per CTA
+    cluster_sync();
+    const int tile = blockIdx.x;
+    int local;
+    const Job& job = p.job[job_of(tile % p.row_tiles, local)];
+    const int per = (p.n_tile + p.slices - 1) / p.slices;
+    const int first = slice * per, last = min(first + per, p.n_tile);
+    const int row = local * 128 + (threadIdx.x & 127);
+    const int token0 = (tile / p.row_tiles) * p.n_tile;
+    if (*failed == 0 && row < job.rows) {
+      const float bias = job.bias != nullptr ? load_f32(job.bias, row, BF16 ? DQ_BF16 : DQ_F16) : 0.0f;
+      unsigned short* dst = static_cast<unsigned short*>(p.out) + job.col0 + row;
+      const uint32_t red = base + p.ring_offset + (threadIdx.x & 127) * 4;
+      for (int col = first + (threadIdx.x >> 7); col < last && token0 + col < p.m; col += kThreads / 128) {
+        float sum = 0.0f;
+        for (int s = 0; s < p.slices; ++s) sum += cluster_ld(red + col * 512, s);
+        dst[static_cast<int64_t>(token0 + col) * p.out_stride] =
+            static_cast<unsigned short>(round_to_16(sum + bias, BF16 ? DQ_BF16 : DQ_F16));
+      }
+    }
+    cluster_sync();  // nobody leaves while its sums are being read
+  }
+  if (threadIdx.x == 0 && *failed != 0) atomicOr(&g_gemm_failed, 1u);
+  fence_after_sync();
+  if (warp == 3) tmem_free(tmem, static_cast<uint32_t>(p.tmem_columns));
+}
+
+// ---------------------------------------------------------------------------
+// Host
+// ---------------------------------------------------------------------------
+
+constexpr uint32_t kBarrierOffset = 64;
+constexpr uint32_t kRingOffset = 1024;
+
+bool encode_map(CUtensorMap* map, CUtensorMapDataType type, const void* base, int64_t inner, int64_t outer, int64_t row_bytes,
+                int box_inner, int box_outer, CUtensorMapSwizzle swizzle) {
+  static const auto encode = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      fn = nullptr;
+    }
+    return reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(fn);
+  }();
+  if (encode == nullptr) return false;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(inner), static_cast<cuuint64_t>(outer)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_bytes)};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_inner), static_cast<cuuint32_t>(box_outer)};
+  const cuuint32_t step[2] = {1, 1};
+  return encode(map, type, 2, const_cast<void*>(base), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+CUtensorMapSwizzle weight_swizzle(int bits) {
+  return bits == 2 ? CU_TENSOR_MAP_SWIZZLE_32B : bits == 3 ? CU_TENSOR_MAP_SWIZZLE_NONE : bits == 4 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                                                                                     : CU_TENSOR_MAP_SWIZZLE_128B;
+}
+
+// 64 << shift values per group, or -1.
+int group_shift_of(int group_values) {
+  for (int s = 0; s < 16; ++s) {
+    if (group_values == (64 << s)) return s;
+  }
+  return -1;
+}
+
+bool geometry_ok(const GemvArgs& a, int bits) {
+  const bool x16 = a.x_dtype == DQ_BF16 || a.x_dtype == DQ_F16, meta16 = a.meta_dtype == DQ_BF16 || a.meta_dtype == DQ_F16;
+  if (!x16 || !meta16 || a.out_dtype != a.x_dtype || a.in_features % 8 != 0 || group_shift_of(a.group_values) < 0) return false;
+  if (a.words_per_group * 32 != a.group_values * bits || a.words_per_row % 4 != 0) return false;
+  return reinterpret_cast<uintptr_t>(a.x) % 16 == 0 && reinterpret_cast<uintptr_t>(a.packed) % 16 == 0;
+}
+
+struct Shape {
+  int n_tile, token_tiles, slices;
+};
+
+// Token tiles and slices of the reduction axis with the least estimated time: waves of CTAs times
+// the cycles of one (stages of 64 values, each bound by the decode or by the tensor pipe, plus a
+// start and an end per tile).
+Shape pick_shape(int m, int row_tiles, int chunks, int sm_count) {
+  Shape best = {};
+  double best_cost = 1e30;
+  const int min_tiles = static_cast<int>(ceil_div(m, 256));
+  for (int tt = min_tiles; tt <= min_tiles + 2; ++tt) {
+    const int n = static_cast<int>(ceil_div(ceil_div(m, tt), 16) * 16);
+    if (n * (tt - 1) >= m) continue;
+    for (int s = 1; s <= 8 && s <= chunks; ++s) {
+      const int resident = s == 1 ? sm_count : (s <= 2 ? sm_count : s <= 4 ? sm_count - 8 : sm_count - 20) / s * s;
+      const double ctas = static_cast<double>(row_tiles) * tt * s;
+      const double waves = std::ceil(ctas / resident);
+      const double stage = std::max(300.0, 2.0 * n);
+      const double overlap = s == 1 && n <= 192 ? 0.0 : 10.0 * n;  // an epilogue that nothing hides
+      const double cost = waves * (2.0 * static_cast<double>(ceil_div(chunks, s)) * stage + overlap + (s > 1 ? 1500.0 : 0.0)) + 10.0 * n + 3000.0;
+      if (cost < best_cost) best_cost = cost, best = {n, tt, s};
+    }
+  }
+  return best;
+}
+
+}  // namespace
+
+int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaStream_t stream, bool* taken) {
+  *taken = false;
+  const DeviceInfo* dev = device_info();
+  if (dev == nullptr) return DQ_ERR_CUDA;
+  if (count < 1 || count > kJobs) return DQ_OK;
+  Params p = {};
+  const GemvArgs& a = args[0];
+  int w_bytes = 0;
+  for (int i = 0; i < count; ++i) {
+    const GemvArgs& b = args[i];
+    if (!geometry_ok(b, bits[i]) || b.x != a.x || b.m != a.m || b.out != a.out || b.out_stride != a.out_stride ||
+        b.in_features != a.in_features || b.rows < 1) {
+      return DQ_OK;
+    }
+    Job& job = p.job[i];
+    if (!encode_map(&job.wmap, CU_TENSOR_MAP_DATA_TYPE_INT32, b.packed, b.words_per_row, b.rows, static_cast<int64_t>(b.words_per_row) * 4,
+                    4 * bits[i], 128, weight_swizzle(bits[i]))) {
+      return DQ_OK;
+    }
+    job.scales = b.scales;
+    job.offsets = b.offsets;
+    job.col0 = b.out_col0;
+    job.bias = b.bias == nullptr ? nullptr : static_cast<const unsigned short*>(b.bias) + b.out_col0;
+    job.rows = b.rows;
+    job.row_tiles = static_cast<int>(ceil_div(b.rows, 128));
+    job.bits = bits[i];
+    job.num_groups = b.num_groups;
+    job.group_shift = group_shift_of(b.group_values);
+    job.meta_dtype = b.meta_dtype;
+    p.row_tiles += job.row_tiles;
+    w_bytes = std::max(w_bytes, 2048 * bits[i]);
+  }
+  p.jobs = count;
+  p.m = a.m;
+  p.out = a.out;
+  p.out_stride = a.out_stride;
+  p.chunks = static_cast<int>(ceil_div(a.in_features, 128));
+  Shape shape = pick_shape(a.m, p.row_tiles, p.chunks, dev->sm_count);
+  if (const int n = tuning_int("DQ_B200_UMMA_N", 0)) shape.n_tile = n, shape.token_tiles = static_cast<int>(ceil_div(a.m, n));
+  if (const int s = tuning_int("DQ_B200_UMMA_SLICES", 0)) shape.slices = s;
+  p.n_tile = shape.n_tile;
+  p.slices = shape.slices;
+  p.tiles = p.row_tiles * shape.token_tiles;
+  if (!encode_map(&p.xmap, a.x_dtype == DQ_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a.x, a.in_features, a.m,
+                  static_cast<int64_t>(a.in_features) * 2, 64, p.n_tile, CU_TENSOR_MAP_SWIZZLE_128B)) {
+    return DQ_OK;
+  }
+  const int grid_x = p.slices > 1 ? p.tiles : std::min(p.tiles, dev->sm_count);
+  p.d_buffers = p.slices == 1 && p.tiles > grid_x && p.n_tile <= 192 ? 2 : 1;
+  p.tmem_columns = 128;
+  while (p.tmem_columns < kAColumns + p.d_buffers * p.n_tile) p.tmem_columns *= 2;
+  const int x_bytes = p.n_tile * 128;
+  p.w_bytes = w_bytes;
+  p.x_slots = std::clamp(131072 / x_bytes, 4, 8);
+  const int budget = dev->max_smem_optin - static_cast<int>(kRingOffset) - 1024;
+  p.w_slots = std::clamp((budget - p.x_slots * x_bytes) / w_bytes, 2, 12);
+  p.barrier_offset = kBarrierOffset;
+  p.ring_offset = kRingOffset;
+  const size_t smem = kRingOffset + static_cast<size_t>(p.x_slots) * x_bytes + static_cast<size_t>(p.w_slots) * w_bytes;
+
+  auto run = [&](auto kernel) -> int32_t {
+    DQ_CUDA(allow_shared(kernel, smem));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(grid_x), static_cast<unsigned>(p.slices));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (p.slices > 1) {
+      attr[n].id = cudaLaunchAttributeClusterDimension;
+      attr[n].val.clusterDim.x = 1;
+      attr[n].val.clusterDim.y = static_cast<unsigned>(p.slices);
+      attr[n].val.clusterDim.z = 1;
+      ++n;
+    }
+    if (pdl_enabled_for_rows()) {
+      attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[n].val.programmaticStreamSerializationAllowed = 1;
+      ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    DQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
+    DQ_CHECK_LAUNCH("gemm");
+    note_kernel("gemm_umma_kernel");
+    *taken = true;
+    return DQ_OK;
+  };
+  return a.x_dtype == DQ_BF16 ? run(gemm_umma_kernel<true>) : run(gemm_umma_kernel<false>);
+}
+
+}  // namespace dq
+
+extern "C" int32_t dq_gemm_status(void* stream) {
+  auto s = static_cast<cudaStream_t>(stream);
+  unsigned int word = 0;
+  DQ_CUDA(cudaMemcpyFromSymbolAsync(&word, dq::g_gemm_failed, sizeof(word), 0, cudaMemcpyDeviceToHost, s));
+  DQ_CUDA(cudaStreamSynchronize(s));
+  if (word != 0u) return dq::fail(DQ_ERR_DEVICE, "gemm: a wait inside a block ran out; an output of this device is incomplete");
+  return DQ_OK;
+}

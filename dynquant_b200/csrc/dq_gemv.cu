@@ -30,6 +30,7 @@
 #include <cstdlib>
 
 #include "dq_decode.cuh"
+#include "dq_gemm_umma.cuh"
 #include "dq_gemv.cuh"
 #include "dq_peer_push.cuh"
 
@@ -711,6 +712,50 @@ int32_t dq_gemv_shards_rows(const void* x, int32_t x_dtype, int64_t m, const dq_
     row0 += rows_here;
   }
   return flush();
+}
+
+int32_t dq_gemm_shards(const void* x, int32_t x_dtype, int64_t m, const dq_weight* shards, int32_t num_shards,
+                       const void* bias, void* out, int64_t out_stride, int32_t out_dtype, void* stream) {
+  DQ_REQUIRE(shards != nullptr && num_shards > 0, "gemm_shards: need at least one shard");
+  DQ_REQUIRE(dq::dtype_ok(x_dtype) && dq::dtype_ok(out_dtype), "gemm_shards: bad dtype tag");
+  DQ_REQUIRE(m >= 0 && m < (1LL << 31), "gemm_shards: bad row count %lld", static_cast<long long>(m));
+  int64_t total = 0;
+  for (int i = 0; i < num_shards; ++i) {
+    dq_geometry g;
+    if (const int32_t rc = dq_resolve_geometry("gemm_shards", &shards[i], &g)) return rc;
+    DQ_REQUIRE(shards[i].in_features == shards[0].in_features, "gemm_shards: shard %d has in_features=%lld but shard 0 has %lld", i,
+               static_cast<long long>(shards[i].in_features), static_cast<long long>(shards[0].in_features));
+    total += shards[i].rows;
+  }
+  DQ_REQUIRE(out_stride >= total, "gemm_shards: out_stride=%lld is smaller than the %lld rows of the shards",
+             static_cast<long long>(out_stride), static_cast<long long>(total));
+  if (m == 0 || total == 0) return DQ_OK;
+  DQ_REQUIRE(x != nullptr && out != nullptr, "gemm_shards: null activation or output pointer");
+  const auto refuse = [] {
+    return dq::fail(DQ_ERR_UNSUPPORTED, "gemm_shards: a geometry the tensor-core kernel does not take (dequantize + dense serves it)");
+  };
+  if (dq::force_general() || !dq::mma_enabled_for_rows()) return refuse();
+  constexpr int kBatch = 4;
+  dq::GemvArgs args[kBatch];
+  int bits[kBatch];
+  int live = 0;
+  int64_t col0 = 0;
+  for (int i = 0; i < num_shards; ++i) {
+    if (shards[i].rows > 0) {
+      dq_geometry g;
+      dq_resolve_geometry("gemm_shards", &shards[i], &g);
+      args[live] = dq::make_args(x, x_dtype, m, shards[i], g, bias, out, out_stride, col0, out_dtype);
+      bits[live++] = shards[i].bits;
+    }
+    col0 += shards[i].rows;
+    if (live == kBatch || (live > 0 && i + 1 == num_shards)) {
+      bool taken = false;
+      if (const int32_t rc = dq::launch_gemm_umma(args, bits, live, static_cast<cudaStream_t>(stream), &taken)) return rc;
+      if (!taken) return refuse();
+      live = 0;
+    }
+  }
+  return DQ_OK;
 }
 
 int32_t dq_gemv_sequence(const dq_gemv_job* jobs, int32_t num_jobs, void* stream) {

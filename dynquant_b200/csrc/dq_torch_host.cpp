@@ -171,6 +171,7 @@ PyObject* multiply(const at::Tensor* x, const dq_weight* w, int n, const at::Ten
   const int64_t k = w[0].in_features;
   if (x->device() != q.device() || x->size(-1) != k || x->numel() == 0 || total == 0) return unhandled();
   const int64_t m = x->numel() / k;
+  if (m > DQ_GEMV_CHUNKED_MAX_ROWS && at::autocast::is_autocast_enabled(at::kCUDA)) return unhandled();  // (a dense matmul casts)
   const at::Tensor* bias = nullptr;
   if (bias_o != Py_None) {
     bias = tensor(bias_o);
@@ -179,7 +180,6 @@ PyObject* multiply(const at::Tensor* x, const dq_weight* w, int n, const at::Ten
       return unhandled();
     }
   }
-  if (m > DQ_GEMV_CHUNKED_MAX_ROWS) return unhandled();
   return on_device(q.device(), [&](cudaStream_t stream) {
     const at::Tensor flat = x->is_contiguous() ? *x : x->contiguous();
     at::Tensor cast;
@@ -191,6 +191,13 @@ PyObject* multiply(const at::Tensor* x, const dq_weight* w, int n, const at::Ten
     sizes.back() = total;
     at::Tensor out = new_cuda(sizes, x->scalar_type(), q.device());
     const int tag = tag_of(x->scalar_type());
+    if (m > DQ_GEMV_CHUNKED_MAX_ROWS) {
+      const int32_t rc = dq_gemm_shards(flat.const_data_ptr(), tag, m, w, n, bias == nullptr ? nullptr : cast.const_data_ptr(),
+                                        out.data_ptr(), total, tag, stream);
+      if (rc == DQ_ERR_UNSUPPORTED) return at::Tensor();
+      check(rc);
+      return out;
+    }
     check(dq_gemv_shards_rows(flat.const_data_ptr(), tag, m, w, n, bias == nullptr ? nullptr : cast.const_data_ptr(),
                               out.data_ptr(), total, tag, stream));
     return out;

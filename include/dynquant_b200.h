@@ -104,7 +104,7 @@ DQ_API int64_t dq_launch_count(void);
  * ("gemv_mma_stream_kernel", "gemv_mma_stream_multi_kernel", "gemv_mma_stream_sliced_kernel", "gemv_mma_tile_kernel",
  * "gemv_mma_kernel", "gemv_fast_kernel",
  * "gemv_general_kernel", "gemv_plan_kernel", "gemv_rows_kernel", "moe_grouped_kernel", "moe_combine_kernel",
- * "moe_down_token_kernel"; "" before the first launch).  No reference
+ * "moe_down_token_kernel", "gemm_umma_kernel"; "" before the first launch).  No reference
  * counterpart: the reference has two kernels and a documented rule between them
  * (csrc/gemv/gemv.cu:566-598); here a test uses this to prove which kernel it exercised. */
 DQ_API const char* dq_last_kernel(void);
@@ -176,6 +176,16 @@ DQ_API int32_t dq_gemv_shards(const void* x, int32_t x_dtype, int64_t m, const d
 DQ_API int32_t dq_gemv_shards_rows(const void* x, int32_t x_dtype, int64_t m, const dq_weight* shards,
                                    int32_t num_shards, const void* bias, void* out, int64_t out_stride,
                                    int32_t out_dtype, void* stream);
+/* The same product for any number of activation rows (prefill), in one launch per four shards on
+ * the tcgen05 tensor cores: no dense weight is written.  16-bit activations and metadata, out_dtype
+ * == x_dtype, groups of 64 * 2^n values, in_features % 8 == 0, 16-byte aligned x and packed rows;
+ * anything else returns DQ_ERR_UNSUPPORTED (outputs then undefined): dequantize + dense serves it. */
+DQ_API int32_t dq_gemm_shards(const void* x, int32_t x_dtype, int64_t m, const dq_weight* shards,
+                              int32_t num_shards, const void* bias, void* out, int64_t out_stride,
+                              int32_t out_dtype, void* stream);
+/* Synchronises `stream`; DQ_ERR_DEVICE once a bounded wait inside one of these kernels has run out
+ * on the current device (its output is then incomplete; the context stays usable). */
+DQ_API int32_t dq_gemm_status(void* stream);
 
 /* One GEMV of a sequence; see dq_gemv_sequence. */
 typedef struct dq_gemv_job {
