@@ -8,9 +8,9 @@
 //   * warp 2 streams packed 128 x 128-value tiles into shared memory by TMA (they are 4..16 KB, so
 //     a ring of them keeps HBM busy), warp 0 the activation in 64-value slabs with the 128-byte
 //     swizzle, both zero-filled past the edges of their tensors;
-//   * two warpgroups (warps 4..11) decode, one 64-value half of a tile each: a thread owns one
-//     weight row, so its scale and offset are two registers and its packed words one contiguous
-//     piece of shared memory; the 16-bit weights go straight to TENSOR MEMORY (tcgen05.st) in the
+//   * four warpgroups (warps 4..19) decode, 64 values of K in turn: a thread owns one weight row, so
+//     its scale and offset are two registers and its packed words one contiguous piece of shared
+//     memory; the 16-bit weights go straight to TENSOR MEMORY (tcgen05.st) in the
 //     natural order -- not to shared memory, whose bandwidth the activation needs;
 //   * warp 1 issues the MMAs (A from tensor memory, B from shared memory), accumulating in tensor
 //     memory; two accumulator tiles where they fit (n_tile <= 192), so that the decode of the next
@@ -38,10 +38,10 @@ namespace {
 using namespace umma;
 
 constexpr int kJobs = 4;
-constexpr int kThreads = 384;          // warps 0..3: TMA x, MMA, TMA weights, tensor memory; 4..11 decode
-constexpr int kDecodeWarp0 = 4;
-constexpr int kASlots = 4;             // operand tiles of 128 x 64 in tensor memory, 32 columns each
-constexpr int kAColumns = kASlots * 32;
+constexpr int kDecodeWarp0 = 4;        // warps 0..3: TMA x, MMA, TMA weights, tensor memory
+constexpr int kGroups = 4;             // decoding warpgroups: 64-value stage i belongs to group i % 4
+constexpr int kThreads = (kDecodeWarp0 + 4 * kGroups) * 32;
+constexpr int kMaxASlots = 8;          // operand tiles of 128 x 64 in tensor memory, 32 columns each
 constexpr int kMaxRing = 16;
 
 struct Job {
@@ -50,7 +50,7 @@ struct Job {
   const void* offsets;                 // may be null
   const void* bias;                    // may be null; element 0 belongs to output column 0 of this job
   int64_t col0;
-  int rows, row_tiles, bits, num_groups, group_shift, meta_dtype;  // group = 64 << group_shift
+  int rows, row_tiles, bits, num_groups, group_shift;  // group = 64 << group_shift
 };
 
 struct Params {
@@ -60,7 +60,7 @@ struct Params {
   int64_t out_stride;
   int jobs, m, chunks;                 // chunks of 128 values of K
   int row_tiles, tiles;                // over all jobs; tiles = row_tiles x token tiles
-  int n_tile, d_buffers, tmem_columns;
+  int n_tile, d_buffers, a_slots, tmem_columns;
   int x_slots, w_slots, w_bytes;       // rings; bytes of a weight slot
   int slices;
   uint32_t ring_offset, barrier_offset;
@@ -68,11 +68,26 @@ struct Params {
 
 __device__ unsigned int g_gemm_failed = 0;
 
-// One warpgroup's half of the chunks [c0, c1) of a row tile; false once a wait has run out.
-template <int BITS, bool BF16>
-__device__ bool decode_tile(const Job& job, int row0, int c0, int c1, int half, unsigned char* w_ring, int w_slots, int w_bytes,
-                            uint32_t bars_w_full, uint32_t bars_w_empty, uint32_t bars_a_full, uint32_t bars_a_empty,
-                            uint32_t a_tmem, uint32_t& w_at, uint32_t& stage, volatile int* failed) {
+struct Bars {
+  uint32_t x_full, x_empty, w_full, w_empty, a_full, a_empty, d_full, d_empty, drain;
+};
+
+// Where a role stands in a ring: a slot and the parity of its pass (run-time divisions would cost the
+// single-thread roles more than their work: 0.3 us per stage, measured).
+struct Cursor {
+  uint32_t slot = 0, pass = 0;
+  __device__ __forceinline__ void advance(uint32_t slots, uint32_t by = 1) {
+    slot += by;
+    if (slot >= slots) slot -= slots, pass ^= 1;  // (by <= slots)
+  }
+};
+
+// Warpgroup `group`'s stages of the `stages` of a row tile, numbered from `stage0` on over the life of
+// the block; chunk c0 + i / 2 and half i % 2 of it are stage stage0 + i.  False once a wait has run out.
+template <int BITS, bool BF16, bool MBF16>
+__device__ bool decode_tile(const Job& job, const Params& p, int row0, int c0, int group, uint32_t stage0, int stages,
+                            const unsigned char* w_ring, const Bars& bars, uint32_t tmem, Cursor& w_at, Cursor& a_at,
+                            volatile int* failed) {
   const int lane = threadIdx.x & 31;
   const int warp4 = (threadIdx.x >> 5) & 3;
   const int r = warp4 * 32 + lane;
@@ -80,61 +95,66 @@ __device__ bool decode_tile(const Job& job, int row0, int c0, int c1, int half, 
   const unsigned short* s_row = static_cast<const unsigned short*>(job.scales) + static_cast<int64_t>(row) * job.num_groups;
   const unsigned short* o_row =
       job.offsets == nullptr ? nullptr : static_cast<const unsigned short*>(job.offsets) + static_cast<int64_t>(row) * job.num_groups;
-  const bool mbf = job.meta_dtype == DQ_BF16;
   auto widen = [&](unsigned short v) -> float {
-    return mbf ? __uint_as_float(static_cast<uint32_t>(v) << 16) : __half2float(__ushort_as_half(v));
+    return MBF16 ? __uint_as_float(static_cast<uint32_t>(v) << 16) : __half2float(__ushort_as_half(v));
   };
-  auto group_of = [&](int c) -> int { return min((2 * c + half) >> job.group_shift, job.num_groups - 1); };
-  int g = group_of(c0);
+  const int first = static_cast<int>((static_cast<uint32_t>(group) - stage0) & (kGroups - 1));
+  auto group_of = [&](int i) -> int { return min((2 * c0 + i) >> job.group_shift, job.num_groups - 1); };
+  if (first >= stages) return true;
+  int g = group_of(first), g_have = -1;
   unsigned short s_next = __ldg(s_row + g), o_next = o_row != nullptr ? __ldg(o_row + g) : 0;
-  Affine<BITS> affine;
-  int g_have = -1;
-  for (int c = c0; c < c1; ++c) {
+  Affine<BITS, MBF16> affine;
+  for (int i = first; i < stages; i += kGroups) {
     if (g != g_have) {
-      affine.set(widen(s_next), o_row != nullptr ? widen(o_next) : 0.0f);
+      affine.set(s_next, o_row != nullptr ? widen(o_next) : 0.0f);
       g_have = g;
     }
-    // the next tile's metadata travels while this one is decoded
-    g = group_of(min(c + 1, c1 - 1));
+    // the next stage's metadata travels while this one is decoded
+    g = i + kGroups < stages ? group_of(i + kGroups) : g;
     if (g != g_have) {
       s_next = __ldg(s_row + g);
       if (o_row != nullptr) o_next = __ldg(o_row + g);
     }
-    const uint32_t slot = w_at % static_cast<uint32_t>(w_slots);
-    if (!mbar_wait(bars_w_full + slot * 8, (w_at / static_cast<uint32_t>(w_slots)) & 1, failed)) return false;
+    const uint32_t slot = w_at.slot, a_slot = a_at.slot;
+    if (!mbar_wait(bars.w_full + slot * 8, w_at.pass, failed)) return false;
     uint32_t w[2 * BITS];
-    read_row64<BITS>(w_ring + slot * w_bytes, r, half, w);
-    const uint32_t a_slot = stage % kASlots;
-    uint32_t v[32];
-    decode32<BITS, BF16>(w, affine, v);
-    decode32<BITS, BF16>(w + BITS, affine, v + 16);
+    read_row64<BITS>(w_ring + slot * p.w_bytes, r, i & 1, w);
+    uint32_t v[16];
+    decode32<BITS, BF16, MBF16>(w, affine, v);
     __syncwarp();
-    if (lane == 0) mbar_arrive(bars_w_empty + slot * 8);  // (the words are in registers)
-    if (!mbar_wait(bars_a_empty + a_slot * 8, ((stage / kASlots) & 1) ^ 1, failed)) return false;
+    if (lane == 0) mbar_arrive(bars.w_empty + slot * 8);  // (the words are in registers)
+    if (!mbar_wait(bars.a_empty + a_slot * 8, a_at.pass ^ 1, failed)) return false;
     fence_after_sync();
-    const uint32_t dst = a_tmem + a_slot * 32 + (static_cast<uint32_t>(warp4 * 32) << 16);
+    const uint32_t dst = tmem + a_slot * 32 + (static_cast<uint32_t>(warp4 * 32) << 16);
     tmem_st16(dst, v);
-    tmem_st16(dst + 16, v + 16);
+    decode32<BITS, BF16, MBF16>(w + BITS, affine, v);
+    tmem_st16(dst + 16, v);
     tmem_wait_st();
     fence_before_sync();
     __syncwarp();
-    if (lane == 0) mbar_arrive(bars_a_full + a_slot * 8);
-    ++w_at;
-    stage += 2;
+    if (lane == 0) mbar_arrive(bars.a_full + a_slot * 8);
+    w_at.advance(static_cast<uint32_t>(p.w_slots), kGroups / 2);
+    a_at.advance(static_cast<uint32_t>(p.a_slots), kGroups);
   }
   return true;
 }
 
-template <bool BF16>
+template <bool BF16, bool MBF16>
 __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   // control block at the front: failure flag, tensor memory address, barriers
   volatile int* failed = reinterpret_cast<volatile int*>(smem);
   const uint32_t base = smem_addr(smem);
-  const uint32_t bars = base + p.barrier_offset;
-  const uint32_t bar_x_full = bars, bar_x_empty = bar_x_full + kMaxRing * 8, bar_w_full = bar_x_empty + kMaxRing * 8,
-                 bar_w_empty = bar_w_full + kMaxRing * 8, bar_a_full = bar_w_empty + kMaxRing * 8, bar_a_empty = bar_a_full + kASlots * 8,
-                 bar_d_full = bar_a_empty + kASlots * 8, bar_d_empty = bar_d_full + 2 * 8, bar_drain = bar_d_empty + 2 * 8;
+  Bars bars;
+  bars.x_full = base + p.barrier_offset;
+  bars.x_empty = bars.x_full + kMaxRing * 8;
+  bars.w_full = bars.x_empty + kMaxRing * 8;
+  bars.w_empty = bars.w_full + kMaxRing * 8;
+  bars.a_full = bars.w_empty + kMaxRing * 8;
+  bars.a_empty = bars.a_full + kMaxASlots * 8;
+  bars.d_full = bars.a_empty + kMaxASlots * 8;
+  bars.d_empty = bars.d_full + 2 * 8;
+  bars.drain = bars.d_empty + 2 * 8;
   const int x_bytes = p.n_tile * 128;
   unsigned char* x_ring = smem + p.ring_offset;
   unsigned char* w_ring = x_ring + p.x_slots * x_bytes;
@@ -143,11 +163,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
 
   if (threadIdx.x == 0) {
     *failed = 0;
-    for (int i = 0; i < p.x_slots; ++i) mbar_init(bar_x_full + i * 8, 1), mbar_init(bar_x_empty + i * 8, 1);
-    for (int i = 0; i < p.w_slots; ++i) mbar_init(bar_w_full + i * 8, 1), mbar_init(bar_w_empty + i * 8, 8);
-    for (int i = 0; i < kASlots; ++i) mbar_init(bar_a_full + i * 8, 4), mbar_init(bar_a_empty + i * 8, 1);
-    for (int i = 0; i < 2; ++i) mbar_init(bar_d_full + i * 8, 1), mbar_init(bar_d_empty + i * 8, 8);
-    mbar_init(bar_drain, 1);
+    for (int i = 0; i < p.x_slots; ++i) mbar_init(bars.x_full + i * 8, 1), mbar_init(bars.x_empty + i * 8, 1);
+    for (int i = 0; i < p.w_slots; ++i) mbar_init(bars.w_full + i * 8, 1), mbar_init(bars.w_empty + i * 8, 8);
+    for (int i = 0; i < p.a_slots; ++i) mbar_init(bars.a_full + i * 8, 4), mbar_init(bars.a_empty + i * 8, 1);
+    for (int i = 0; i < 2; ++i) mbar_init(bars.d_full + i * 8, 1), mbar_init(bars.d_empty + i * 8, 4 * kGroups);
+    mbar_init(bars.drain, 1);
     fence_mbar_init();
     tma_prefetch_map(&p.xmap);
   }
@@ -156,7 +176,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + 4);
-  const uint32_t d_tmem = tmem + kAColumns;
+  const uint32_t d_tmem = tmem + p.a_slots * 32;
   pdl_launch_dependents();
 
   // this CTA's share of the reduction axis (slices: as equal as possible, in chunks)
@@ -175,9 +195,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
     if (elect_one()) {
       const bool weights = warp == 2;
       if (!weights) pdl_wait_prior_grid();  // the activation is the previous kernel's; weights are nobody's
-      const uint32_t full = weights ? bar_w_full : bar_x_full, empty = weights ? bar_w_empty : bar_x_empty;
+      const uint32_t full = weights ? bars.w_full : bars.x_full, empty = weights ? bars.w_empty : bars.x_empty;
       const uint32_t slots = static_cast<uint32_t>(weights ? p.w_slots : p.x_slots);
-      uint32_t at = 0;
+      Cursor at;
+      uint32_t issued = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
         int local;
@@ -185,9 +206,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
         const int token0 = (tile / p.row_tiles) * p.n_tile;
         const int count = weights ? c1 - c0 : 2 * (c1 - c0);
         const int bytes = weights ? 2048 * job.bits : x_bytes;
-        for (int i = 0; i < count; ++i, ++at) {
-          const uint32_t slot = at % slots;
-          if (!(ok = mbar_wait(empty + slot * 8, ((at / slots) & 1) ^ 1, failed))) break;
+        for (int i = 0; i < count; ++i, ++issued, at.advance(slots)) {
+          const uint32_t slot = at.slot;
+          if (!(ok = mbar_wait(empty + slot * 8, at.pass ^ 1, failed))) break;
           mbar_expect(full + slot * 8, static_cast<uint32_t>(bytes));
           if (weights) {
             tma_load_2d(smem_addr(w_ring) + slot * p.w_bytes, &job.wmap, (c0 + i) * 4 * job.bits, local * 128, full + slot * 8);
@@ -197,7 +218,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
         }
       }
       if (!ok || *failed != 0) {  // wait for the copies in flight
-        for (uint32_t k = at > slots ? at - slots : 0; k < at; ++k) {
+        for (uint32_t k = issued > slots ? issued - slots : 0; k < issued; ++k) {
           for (int i = 0; i < kSpins && !mbar_try(full + (k % slots) * 8, (k / slots) & 1); ++i) {
           }
         }
@@ -207,46 +228,50 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
   } else if (warp == 1) {
     if (elect_one()) {
       const uint32_t idesc = mma_descriptor(BF16, p.n_tile);
-      uint32_t stage = 0, d_at = 0;
+      Cursor x_at, a_at, d_at;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x, ++d_at) {
-        const uint32_t buffer = d_at % static_cast<uint32_t>(p.d_buffers);
-        if (!mbar_wait(bar_d_empty + buffer * 8, ((d_at / p.d_buffers) & 1) ^ 1, failed)) break;
+      for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x, d_at.advance(static_cast<uint32_t>(p.d_buffers))) {
+        const uint32_t buffer = d_at.slot;
+        if (!mbar_wait(bars.d_empty + buffer * 8, d_at.pass ^ 1, failed)) break;
         fence_after_sync();
         const uint32_t d = d_tmem + buffer * p.n_tile;
-        for (int i = 0; i < 2 * (c1 - c0); ++i, ++stage) {
-          const uint32_t xs = stage % static_cast<uint32_t>(p.x_slots), as = stage % kASlots;
-          if (!(ok = mbar_wait(bar_x_full + xs * 8, (stage / p.x_slots) & 1, failed))) break;
-          if (!(ok = mbar_wait(bar_a_full + as * 8, (stage / kASlots) & 1, failed))) break;
+        for (int i = 0; i < 2 * (c1 - c0); ++i) {
+          const uint32_t xs = x_at.slot, as = a_at.slot;
+          if (!(ok = mbar_wait(bars.x_full + xs * 8, x_at.pass, failed))) break;
+          if (!(ok = mbar_wait(bars.a_full + as * 8, a_at.pass, failed))) break;
           fence_after_sync();
           const uint64_t b = smem_descriptor(smem_addr(x_ring) + xs * x_bytes);
           const uint32_t a = tmem + as * 32;
 #pragma unroll
           for (int k = 0; k < 4; ++k) mma_ts(d, a + k * 8, b + k * 2, idesc, i > 0 || k > 0);
-          mma_commit(bar_a_empty + as * 8);
-          mma_commit(bar_x_empty + xs * 8);
+          mma_commit(bars.a_empty + as * 8);
+          mma_commit(bars.x_empty + xs * 8);
+          x_at.advance(static_cast<uint32_t>(p.x_slots));
+          a_at.advance(static_cast<uint32_t>(p.a_slots));
         }
-        if (ok) mma_commit(bar_d_full + buffer * 8);
+        if (ok) mma_commit(bars.d_full + buffer * 8);
       }
       if (*failed != 0) {  // MMAs in flight read and write tensor memory: it is freed after them
-        mma_commit(bar_drain);
-        for (int i = 0; i < kSpins && !mbar_try(bar_drain, 0); ++i) {
+        mma_commit(bars.drain);
+        for (int i = 0; i < kSpins && !mbar_try(bars.drain, 0); ++i) {
         }
       }
     }
     __syncwarp();
   } else if (warp >= kDecodeWarp0) {
-    const int half = (warp - kDecodeWarp0) >> 2;
+    const int group = (warp - kDecodeWarp0) >> 2;
     const int warp4 = warp & 3;
     const int r = warp4 * 32 + lane;
-    uint32_t w_at = 0, stage = static_cast<uint32_t>(half), d_at = 0;
-    for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, ++d_at) {
+    const int stages = 2 * (c1 - c0);
+    uint32_t stage = 0;
+    Cursor w_at, a_at, d_at;
+    w_at.advance(static_cast<uint32_t>(p.w_slots), static_cast<uint32_t>(group / 2));
+    a_at.advance(static_cast<uint32_t>(p.a_slots), static_cast<uint32_t>(group));
+    for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, d_at.advance(static_cast<uint32_t>(p.d_buffers)), stage += stages) {
       int local;
       const Job& job = p.job[job_of(tile % p.row_tiles, local)];
       bool ok;
-#define DQ_DECODE(B)                                                                                                             \
-  ok = decode_tile<B, BF16>(job, local * 128, c0, c1, half, w_ring, p.w_slots, p.w_bytes, bar_w_full, bar_w_empty, bar_a_full, \
-                            bar_a_empty, tmem, w_at, stage, failed)
+#define DQ_DECODE(B) ok = decode_tile<B, BF16, MBF16>(job, p, local * 128, c0, group, stage, stages, w_ring, bars, tmem, w_at, a_at, failed)
       switch (job.bits) {
         case 2: DQ_DECODE(2); break;
         case 3: DQ_DECODE(3); break;
@@ -255,19 +280,16 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
       }
 #undef DQ_DECODE
       if (!ok) break;
-      const uint32_t buffer = d_at % static_cast<uint32_t>(p.d_buffers);
-      if (!mbar_wait(bar_d_full + buffer * 8, (d_at / p.d_buffers) & 1, failed)) break;
+      const uint32_t buffer = d_at.slot;
+      if (!mbar_wait(bars.d_full + buffer * 8, d_at.pass, failed)) break;
       fence_after_sync();
-      // the two warpgroups share the columns
-      const int split = (p.n_tile / 2 + 15) / 16 * 16;
-      const int first = half == 0 ? 0 : split, last = half == 0 ? split : p.n_tile;
       const uint32_t src = d_tmem + buffer * p.n_tile + (static_cast<uint32_t>(warp4 * 32) << 16);
       const int row = local * 128 + r;
       const int token0 = (tile / p.row_tiles) * p.n_tile;
       const float bias = job.bias != nullptr && row < job.rows ? load_f32(job.bias, row, BF16 ? DQ_BF16 : DQ_F16) : 0.0f;
       unsigned short* dst = static_cast<unsigned short*>(p.out) + job.col0 + row;
       float* red = reinterpret_cast<float*>(smem + p.ring_offset);
-      for (int col = first; col < last; col += 16) {
+      for (int col = group * 16; col < p.n_tile; col += kGroups * 16) {  // the warpgroups share the columns
         uint32_t v[16];
         tmem_ld16(src + col, v);
         tmem_wait_ld();
@@ -287,7 +309,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
       }
       fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_d_empty + buffer * 8);
+      if (lane == 0) mbar_arrive(bars.d_empty + buffer * 8);
     }
   }
 
@@ -406,7 +428,7 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
   for (int i = 0; i < count; ++i) {
     const GemvArgs& b = args[i];
     if (!geometry_ok(b, bits[i]) || b.x != a.x || b.m != a.m || b.out != a.out || b.out_stride != a.out_stride ||
-        b.in_features != a.in_features || b.rows < 1) {
+        b.in_features != a.in_features || b.meta_dtype != a.meta_dtype || b.rows < 1) {
       return DQ_OK;
     }
     Job& job = p.job[i];
@@ -423,7 +445,6 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
     job.bits = bits[i];
     job.num_groups = b.num_groups;
     job.group_shift = group_shift_of(b.group_values);
-    job.meta_dtype = b.meta_dtype;
     p.row_tiles += job.row_tiles;
     w_bytes = std::max(w_bytes, 2048 * bits[i]);
   }
@@ -443,9 +464,12 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
     return DQ_OK;
   }
   const int grid_x = p.slices > 1 ? p.tiles : std::min(p.tiles, dev->sm_count);
+  // Tensor memory: operand slots (eight where there is room: a warpgroup then works two stages
+  // ahead) and the accumulators (two where a CTA has several tiles and both fit).
   p.d_buffers = p.slices == 1 && p.tiles > grid_x && p.n_tile <= 192 ? 2 : 1;
-  p.tmem_columns = 128;
-  while (p.tmem_columns < kAColumns + p.d_buffers * p.n_tile) p.tmem_columns *= 2;
+  p.a_slots = kMaxASlots * 32 + p.d_buffers * p.n_tile <= 512 ? kMaxASlots : kGroups;
+  p.tmem_columns = 32;
+  while (p.tmem_columns < p.a_slots * 32 + p.d_buffers * p.n_tile) p.tmem_columns *= 2;
   const int x_bytes = p.n_tile * 128;
   p.w_bytes = w_bytes;
   p.x_slots = std::clamp(131072 / x_bytes, 4, 8);
@@ -455,6 +479,7 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
   p.ring_offset = kRingOffset;
   const size_t smem = kRingOffset + static_cast<size_t>(p.x_slots) * x_bytes + static_cast<size_t>(p.w_slots) * w_bytes;
 
+  const bool mbf = a.meta_dtype == DQ_BF16;
   auto run = [&](auto kernel) -> int32_t {
     DQ_CUDA(allow_shared(kernel, smem));
     cudaLaunchConfig_t cfg = {};
@@ -484,7 +509,8 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
     *taken = true;
     return DQ_OK;
   };
-  return a.x_dtype == DQ_BF16 ? run(gemm_umma_kernel<true>) : run(gemm_umma_kernel<false>);
+  if (a.x_dtype == DQ_BF16) return mbf ? run(gemm_umma_kernel<true, true>) : run(gemm_umma_kernel<true, false>);
+  return mbf ? run(gemm_umma_kernel<false, true>) : run(gemm_umma_kernel<false, false>);
 }
 
 }  // namespace dq

@@ -1,14 +1,16 @@
 // Packed codes -> 16-bit weights, one weight row per thread, natural order: the A operand of
 // tcgen05.mma as tensor memory holds it (lane = weight row, a 32-bit column = two values of K).
 //
-// A code is moved into the upper mantissa bits of 1.0f: f = 1 + q * 2^(p - 23) with its lowest bit
-// at bit p, by one shift shared by the codes of a window and one AND-OR per code.  Then
-//   w = f * (s * 2^(23 - p)) + (o - s * 2^(23 - p))
-// is ONE fp32 fma per value (two per packed instruction), with no conversion and no unbiasing:
-// the constant's own rounding is 2^(-1-p) of a scale step (p >= 14 at 2, 3 and 4 bits; p = 8 at 8
-// bits, where a step is 1/128 of the range).  One rounding to the operand type follows.  About 4
-// issue cycles per value, against 2 for the accumulator-side scaling of the mma.sync kernels --
-// but here a decoded value is multiplied with up to 256 activation rows at once.
+// ONE AND-OR puts two codes (one per 16-bit half) into the mantissa of a power of two of the
+// METADATA's type -- with the code's lowest bit at mantissa bit p and the exponent chosen so that
+// this bit is worth 1, a half is exactly M_p + q -- and ONE mixed-precision fma per value,
+//   w = (M_p + q) * s + (o - M_p * s),   16-bit factors, fp32 addend and result,
+// unbiases, scales and shifts it; the scale enters in its own type and the addend's rounding is
+// M_p * 2^-24 of a scale step (M_p <= 1024).  One conversion per pair rounds to the operand type.
+// That is about 1.1 (2, 4, 8 bits) to 1.5 (3 bits) ALU instructions per value -- logic, shifts and
+// conversions issue at half rate and bound the loop -- plus one fma at full rate; building fp32
+// values code by code (an AND-OR and half a conversion each) took 2 and ran 128 x 64 values in 680
+// cycles per SM.  8-bit codes do not fit a bf16 mantissa: with bf16 metadata they take that way.
 #pragma once
 
 #include "dq_umma.cuh"
@@ -18,95 +20,132 @@ namespace umma {
 
 #ifdef __CUDACC__
 
+// Bytes of a row of a 128-value tile are 16 * BITS: the TMA swizzle mode (log2 of the 16-byte pieces).
 template <int BITS>
-struct DecodeCfg;
-template <>
-struct DecodeCfg<2> {
-  static constexpr int kPairs = 2, kSwizzle = 1;
-};
-template <>
-struct DecodeCfg<3> {
-  static constexpr int kPairs = 3, kSwizzle = 0;
-};
-template <>
-struct DecodeCfg<4> {
-  static constexpr int kPairs = 1, kSwizzle = 2;
-};
-template <>
-struct DecodeCfg<8> {
-  static constexpr int kPairs = 1, kSwizzle = 3;
-};
+constexpr int kSwizzleBits = BITS == 2 ? 1 : BITS == 4 ? 2 : BITS == 8 ? 3 : 0;
 
-// Multiplier and addend of the two values of a register, per position pair.
-template <int BITS>
+// Scale and addends of one group.
+template <int BITS, bool MBF16>
 struct Affine {
-  float2 mul[DecodeCfg<BITS>::kPairs], add[DecodeCfg<BITS>::kPairs];
-  __device__ __forceinline__ void set(float s, float o) {
-    auto put = [&](int i, float lo, float hi) {
-      mul[i] = make_float2(s * lo, s * hi);
-      add[i] = make_float2(fmaf(-s, lo, o), fmaf(-s, hi, o));
-    };
-    if constexpr (BITS == 2) put(0, 256.0f, 64.0f), put(1, 16.0f, 4.0f);
-    if constexpr (BITS == 3) put(0, 512.0f, 64.0f), put(1, 8.0f, 512.0f), put(2, 64.0f, 8.0f);
-    if constexpr (BITS == 4) put(0, 256.0f, 16.0f);
-    if constexpr (BITS == 8) put(0, 32768.0f, 32768.0f);
+  // code positions in the mantissa (bits): at 2 bits 0 2 4 (6), at 3 bits 0 3 (6), at 4 bits 0 (4)
+  static constexpr int kWide = BITS == 8 && MBF16;  // fp32 codes
+  static constexpr int kPlaces = BITS == 2 ? (MBF16 ? 3 : 4) : BITS == 3 ? (MBF16 ? 2 : 3) : BITS == 4 ? (MBF16 ? 1 : 2) : 1;
+  static constexpr int kMantissa = MBF16 ? 7 : 10;
+  unsigned short scale;
+  float wide_mul, add[kPlaces];
+  __device__ __forceinline__ void set(unsigned short s16, float o) {
+    scale = s16;
+    const float s = MBF16 ? __uint_as_float(static_cast<uint32_t>(s16) << 16) : __half2float(__ushort_as_half(s16));
+    if constexpr (kWide) {
+      wide_mul = s * 32768.0f;
+      add[0] = fmaf(-s, 32768.0f, o);
+    } else {
+#pragma unroll
+      for (int i = 0; i < kPlaces; ++i) add[i] = fmaf(-s, static_cast<float>(1 << (kMantissa - i * BITS)), o);
+    }
+  }
+  // The magic number of place i in both halves: M = 2^(kMantissa - i * BITS).
+  static constexpr uint32_t magic(int i) {
+    const uint32_t half = MBF16 ? static_cast<uint32_t>(127 + kMantissa - i * BITS) << 7 : static_cast<uint32_t>(15 + kMantissa - i * BITS) << 10;
+    return half | (half << 16);
+  }
+  static constexpr uint32_t mask(int i) {
+    const uint32_t half = ((1u << BITS) - 1u) << (i * BITS);
+    return half | (half << 16);
   }
 };
 
 template <bool BF16>
-__device__ __forceinline__ uint32_t pack16(float2 v) {
+__device__ __forceinline__ uint32_t pack16(float lo, float hi) {
   if constexpr (BF16) {
-    const __nv_bfloat162 b = __floats2bfloat162_rn(v.x, v.y);
+    const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&b);
   } else {
-    const __half2 h = __floats2half2_rn(v.x, v.y);
+    const __half2 h = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&h);
   }
 }
 
-// 32 values (BITS words) -> 16 registers of two.
-template <int BITS, bool BF16>
-__device__ __forceinline__ void decode32(const uint32_t* w, const Affine<BITS>& c, uint32_t* out) {
-  constexpr uint32_t kOne = 0x3F800000u;
-  auto field = [&](uint32_t u, int p) -> float { return __uint_as_float((u & (((1u << BITS) - 1u) << p)) | kOne); };
-  auto emit = [&](int n, float lo, float hi, int pair) {
-    out[n] = pack16<BF16>(__ffma2_rn(make_float2(lo, hi), c.mul[pair], c.add[pair]));
-  };
-  if constexpr (BITS == 2 || BITS == 4) {
-    constexpr int kPerWord = 32 / BITS;
-#pragma unroll
-    for (int i = 0; i < BITS; ++i) {
-      const uint32_t u[4] = {w[i] << 15, w[i] << 7, w[i] >> 1, w[i] >> 9};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int n = (i * kPerWord + j * (8 / BITS)) / 2;
-        if constexpr (BITS == 4) {
-          emit(n, field(u[j], 15), field(u[j], 19), 0);
-        } else {
-          emit(n, field(u[j], 15), field(u[j], 17), 0);
-          emit(n + 1, field(u[j], 19), field(u[j], 21), 1);
-        }
-      }
-    }
-  } else if constexpr (BITS == 3) {
-    const uint32_t u[11] = {w[0] << 14, w[0] << 5, w[0] >> 4, __funnelshift_r(w[0], w[1], 13), w[1] << 10, w[1] << 1,
-                            w[1] >> 8, __funnelshift_r(w[1], w[2], 17), w[2] << 6, w[2] >> 3, w[2] >> 12};
-#pragma unroll
-    for (int n = 0; n < 16; ++n) {
-      const int a = 2 * n, b = 2 * n + 1;
-      emit(n, field(u[a / 3], 14 + 3 * (a % 3)), field(u[b / 3], 14 + 3 * (b % 3)), n % 3);
+// (16-bit half of `pair`) * scale + add, in fp32.
+template <bool MBF16>
+__device__ __forceinline__ float fma_half(uint32_t pair, bool high, unsigned short scale, float add) {
+  float d;
+  if constexpr (MBF16) {
+    if (high) {
+      asm("{\n .reg .b16 l, h;\n mov.b32 {l, h}, %1;\n fma.rn.f32.bf16 %0, h, %2, %3;\n}" : "=f"(d) : "r"(pair), "h"(scale), "f"(add));
+    } else {
+      asm("{\n .reg .b16 l, h;\n mov.b32 {l, h}, %1;\n fma.rn.f32.bf16 %0, l, %2, %3;\n}" : "=f"(d) : "r"(pair), "h"(scale), "f"(add));
     }
   } else {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const float lo = __uint_as_float(__byte_perm(w[i], kOne, 0x7604u | ((2 * j) << 4)));
-        const float hi = __uint_as_float(__byte_perm(w[i], kOne, 0x7604u | ((2 * j + 1) << 4)));
-        emit(2 * i + j, lo, hi, 0);
-      }
+    if (high) {
+      asm("{\n .reg .b16 l, h;\n mov.b32 {l, h}, %1;\n fma.rn.f32.f16 %0, h, %2, %3;\n}" : "=f"(d) : "r"(pair), "h"(scale), "f"(add));
+    } else {
+      asm("{\n .reg .b16 l, h;\n mov.b32 {l, h}, %1;\n fma.rn.f32.f16 %0, l, %2, %3;\n}" : "=f"(d) : "r"(pair), "h"(scale), "f"(add));
     }
   }
+  return d;
+}
+
+// 32 values (BITS words) -> 16 registers of two.
+template <int BITS, bool BF16, bool MBF16>
+__device__ __forceinline__ void decode32(const uint32_t* w, const Affine<BITS, MBF16>& c, uint32_t* out) {
+  using A = Affine<BITS, MBF16>;
+  float f[32];
+  // codes `lo` (low half of u) and `hi` (high half), at mantissa place i
+  auto take = [&](uint32_t u, int i, int lo, int hi) {
+    const uint32_t q = (u & A::mask(i)) | A::magic(i);
+    f[lo] = fma_half<MBF16>(q, false, c.scale, c.add[i]);
+    f[hi] = fma_half<MBF16>(q, true, c.scale, c.add[i]);
+  };
+  if constexpr (A::kWide) {
+    // 1 + q * 2^-15 in fp32: byte q under the upper half of 1.0f
+#pragma unroll
+    for (int v = 0; v < 32; ++v) {
+      f[v] = fmaf(__uint_as_float(__byte_perm(w[v / 4], 0x3F800000u, 0x7604u | ((v & 3) << 4))), c.wide_mul, c.add[0]);
+    }
+  } else if constexpr (BITS == 8) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {  // two bytes of w under the upper bytes of two 1024.0
+      const uint32_t q = __byte_perm(w[i / 2], A::magic(0), (i & 1) ? 0x7352u : 0x7150u);
+      f[2 * i] = fma_half<MBF16>(q, false, c.scale, c.add[0]);
+      f[2 * i + 1] = fma_half<MBF16>(q, true, c.scale, c.add[0]);
+    }
+  } else if constexpr (BITS == 4) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int v = 8 * i;
+      if constexpr (A::kPlaces == 2) {
+        take(w[i], 0, v, v + 4), take(w[i], 1, v + 1, v + 5);
+        take(w[i] >> 8, 0, v + 2, v + 6), take(w[i] >> 8, 1, v + 3, v + 7);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) take(w[i] >> (4 * j), 0, v + j, v + j + 4);
+      }
+    }
+  } else if constexpr (BITS == 2) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) take(w[i] >> (2 * (j - j % A::kPlaces)), j % A::kPlaces, 16 * i + j, 16 * i + j + 8);
+    }
+  } else {
+    // bits 16 t .. 16 t + 15 of the 96 below bits 48 + 16 t ..: code i in the low halves, i + 16 in the high ones
+    const uint32_t h[3] = {__byte_perm(w[0], w[1], 0x7610u), __byte_perm(w[0], w[2], 0x5432u), __byte_perm(w[1], w[2], 0x7610u)};
+    constexpr int P = A::kPlaces;
+#pragma unroll
+    for (int j = 0; j < 5; ++j) take(h[0] >> (3 * (j - j % P)), j % P, j, j + 16);               // codes 0..4 at bits 0..14
+#pragma unroll
+    for (int j = 0; j < 4; ++j) take(h[1] >> (2 + 3 * (j - j % P)), j % P, j + 6, j + 22);       // 6..9 at bits 2..13
+#pragma unroll
+    for (int j = 0; j < 5; ++j) take(h[2] >> (1 + 3 * (j - j % P)), j % P, j + 11, j + 27);      // 11..15 at bits 1..15
+    // the two codes that straddle halves
+    const uint32_t five = ((h[0] >> 15) & 0x00010001u) | ((h[1] << 1) & 0x00060006u);
+    const uint32_t ten = ((h[1] >> 14) & 0x00030003u) | ((h[2] << 2) & 0x00040004u);
+    take(five, 0, 5, 21);
+    take(ten, 0, 10, 26);
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) out[i] = pack16<BF16>(f[2 * i], f[2 * i + 1]);
 }
 
 // The 64 values (2 * BITS words) of half `half` of row `row` in a staged 128 x 128-value tile.
@@ -125,7 +164,7 @@ __device__ __forceinline__ void read_row64(const unsigned char* tile, int row, i
       w[0] = a.x, w[1] = a.y, w[2] = b.x, w[3] = b.y, w[4] = b.z, w[5] = b.w;
     }
   } else {
-    constexpr int kMask = (1 << DecodeCfg<BITS>::kSwizzle) - 1;  // 16-byte pieces are XORed with address bits 7..
+    constexpr int kMask = (1 << kSwizzleBits<BITS>) - 1;  // 16-byte pieces are XORed with address bits 7..
 #pragma unroll
     for (int i = 0; i < BITS / 2; ++i) {
       int at = row * ROW + half * (8 * BITS) + i * 16;
