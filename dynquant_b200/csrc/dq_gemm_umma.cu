@@ -39,9 +39,10 @@ using namespace umma;
 
 constexpr int kJobs = 4;
 constexpr int kDecodeWarp0 = 4;        // warps 0..3: TMA x, MMA, TMA weights, tensor memory
-constexpr int kGroups = 4;             // decoding warpgroups: 64-value stage i belongs to group i % 4
+constexpr int kGroups = 4;             // decoding warpgroups: stage (chunk of 128 values of K) i belongs to group i % 4
 constexpr int kThreads = (kDecodeWarp0 + 4 * kGroups) * 32;
-constexpr int kMaxASlots = 8;          // operand tiles of 128 x 64 in tensor memory, 32 columns each
+constexpr int kASlots = kGroups;       // operand tiles of 128 x 128 in tensor memory, 64 columns each
+constexpr int kAColumns = kASlots * 64;
 constexpr int kMaxRing = 16;
 
 struct Job {
@@ -60,7 +61,7 @@ struct Params {
   int64_t out_stride;
   int jobs, m, chunks;                 // chunks of 128 values of K
   int row_tiles, tiles;                // over all jobs; tiles = row_tiles x token tiles
-  int n_tile, d_buffers, a_slots, tmem_columns;
+  int n_tile, d_buffers, tmem_columns;
   int x_slots, w_slots, w_bytes;       // rings; bytes of a weight slot
   int slices;
   uint32_t ring_offset, barrier_offset;
@@ -82,8 +83,8 @@ struct Cursor {
   }
 };
 
-// Warpgroup `group`'s stages of the `stages` of a row tile, numbered from `stage0` on over the life of
-// the block; chunk c0 + i / 2 and half i % 2 of it are stage stage0 + i.  False once a wait has run out.
+// Warpgroup `group`'s chunks of a row tile: chunk c0 + i is stage stage0 + i, numbered over the life of
+// the block.  False once a wait has run out.
 template <int BITS, bool BF16, bool MBF16>
 __device__ bool decode_tile(const Job& job, const Params& p, int row0, int c0, int group, uint32_t stage0, int stages,
                             const unsigned char* w_ring, const Bars& bars, uint32_t tmem, Cursor& w_at, Cursor& a_at,
@@ -98,43 +99,55 @@ __device__ bool decode_tile(const Job& job, const Params& p, int row0, int c0, i
   auto widen = [&](unsigned short v) -> float {
     return MBF16 ? __uint_as_float(static_cast<uint32_t>(v) << 16) : __half2float(__ushort_as_half(v));
   };
+  const bool two_groups = job.group_shift == 0;  // 64-value groups: a chunk holds two
+  auto group_of = [&](int i, int half) -> int { return min((2 * (c0 + i) + half) >> job.group_shift, job.num_groups - 1); };
+  unsigned short s_next[2], o_next[2] = {0, 0};
+  auto fetch = [&](int i) {
+    const int g0 = group_of(i, 0);
+    s_next[0] = __ldg(s_row + g0);
+    if (o_row != nullptr) o_next[0] = __ldg(o_row + g0);
+    if (two_groups) {
+      const int g1 = group_of(i, 1);
+      s_next[1] = __ldg(s_row + g1);
+      if (o_row != nullptr) o_next[1] = __ldg(o_row + g1);
+    }
+  };
   const int first = static_cast<int>((static_cast<uint32_t>(group) - stage0) & (kGroups - 1));
-  auto group_of = [&](int i) -> int { return min((2 * c0 + i) >> job.group_shift, job.num_groups - 1); };
   if (first >= stages) return true;
-  int g = group_of(first), g_have = -1;
-  unsigned short s_next = __ldg(s_row + g), o_next = o_row != nullptr ? __ldg(o_row + g) : 0;
-  Affine<BITS, MBF16> affine;
+  fetch(first);
   for (int i = first; i < stages; i += kGroups) {
-    if (g != g_have) {
-      affine.set(s_next, o_row != nullptr ? widen(o_next) : 0.0f);
-      g_have = g;
-    }
-    // the next stage's metadata travels while this one is decoded
-    g = i + kGroups < stages ? group_of(i + kGroups) : g;
-    if (g != g_have) {
-      s_next = __ldg(s_row + g);
-      if (o_row != nullptr) o_next = __ldg(o_row + g);
-    }
+    Affine<BITS, MBF16> affine;
+    affine.set(s_next[0], o_row != nullptr ? widen(o_next[0]) : 0.0f);
+    const unsigned short s_half = s_next[1], o_half = o_next[1];
+    fetch(min(i + kGroups, stages - 1));  // the next chunk's metadata travels while this one is decoded
     const uint32_t slot = w_at.slot, a_slot = a_at.slot;
     if (!mbar_wait(bars.w_full + slot * 8, w_at.pass, failed)) return false;
-    uint32_t w[2 * BITS];
-    read_row64<BITS>(w_ring + slot * p.w_bytes, r, i & 1, w);
-    uint32_t v[16];
-    decode32<BITS, BF16, MBF16>(w, affine, v);
-    __syncwarp();
-    if (lane == 0) mbar_arrive(bars.w_empty + slot * 8);  // (the words are in registers)
-    if (!mbar_wait(bars.a_empty + a_slot * 8, a_at.pass ^ 1, failed)) return false;
-    fence_after_sync();
-    const uint32_t dst = tmem + a_slot * 32 + (static_cast<uint32_t>(warp4 * 32) << 16);
-    tmem_st16(dst, v);
-    decode32<BITS, BF16, MBF16>(w + BITS, affine, v);
-    tmem_st16(dst + 16, v);
+    const uint32_t dst = tmem + a_slot * 64 + (static_cast<uint32_t>(warp4 * 32) << 16);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      uint32_t w[2 * BITS];
+      read_row64<BITS>(w_ring + slot * p.w_bytes, r, half, w);
+      if (half == 1) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bars.w_empty + slot * 8);  // (the words are in registers)
+        if (two_groups) affine.set(s_half, o_row != nullptr ? widen(o_half) : 0.0f);
+      }
+      uint32_t v[16];
+      decode32<BITS, BF16, MBF16>(w, affine, v);
+      if (half == 0) {
+        if (!mbar_wait(bars.a_empty + a_slot * 8, a_at.pass ^ 1, failed)) return false;
+        fence_after_sync();
+      }
+      tmem_st16(dst + half * 32, v);
+      decode32<BITS, BF16, MBF16>(w + BITS, affine, v);
+      tmem_st16(dst + half * 32 + 16, v);
+    }
     tmem_wait_st();
     fence_before_sync();
     __syncwarp();
     if (lane == 0) mbar_arrive(bars.a_full + a_slot * 8);
-    w_at.advance(static_cast<uint32_t>(p.w_slots), kGroups / 2);
-    a_at.advance(static_cast<uint32_t>(p.a_slots), kGroups);
+    w_at.advance(static_cast<uint32_t>(p.w_slots), kGroups);
+    a_at.advance(kASlots, kGroups);
   }
   return true;
 }
@@ -151,11 +164,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
   bars.w_full = bars.x_empty + kMaxRing * 8;
   bars.w_empty = bars.w_full + kMaxRing * 8;
   bars.a_full = bars.w_empty + kMaxRing * 8;
-  bars.a_empty = bars.a_full + kMaxASlots * 8;
-  bars.d_full = bars.a_empty + kMaxASlots * 8;
+  bars.a_empty = bars.a_full + kASlots * 8;
+  bars.d_full = bars.a_empty + kASlots * 8;
   bars.d_empty = bars.d_full + 2 * 8;
   bars.drain = bars.d_empty + 2 * 8;
-  const int x_bytes = p.n_tile * 128;
+  const int x_bytes = p.n_tile * 256;  // two slabs of 64 values
   unsigned char* x_ring = smem + p.ring_offset;
   unsigned char* w_ring = x_ring + p.x_slots * x_bytes;
   const int warp = threadIdx.x >> 5;
@@ -164,8 +177,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
   if (threadIdx.x == 0) {
     *failed = 0;
     for (int i = 0; i < p.x_slots; ++i) mbar_init(bars.x_full + i * 8, 1), mbar_init(bars.x_empty + i * 8, 1);
-    for (int i = 0; i < p.w_slots; ++i) mbar_init(bars.w_full + i * 8, 1), mbar_init(bars.w_empty + i * 8, 8);
-    for (int i = 0; i < p.a_slots; ++i) mbar_init(bars.a_full + i * 8, 4), mbar_init(bars.a_empty + i * 8, 1);
+    for (int i = 0; i < p.w_slots; ++i) mbar_init(bars.w_full + i * 8, 1), mbar_init(bars.w_empty + i * 8, 4);
+    for (int i = 0; i < kASlots; ++i) mbar_init(bars.a_full + i * 8, 4), mbar_init(bars.a_empty + i * 8, 1);
     for (int i = 0; i < 2; ++i) mbar_init(bars.d_full + i * 8, 1), mbar_init(bars.d_empty + i * 8, 4 * kGroups);
     mbar_init(bars.drain, 1);
     fence_mbar_init();
@@ -176,7 +189,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + 4);
-  const uint32_t d_tmem = tmem + p.a_slots * 32;
+  const uint32_t d_tmem = tmem + kAColumns;
   pdl_launch_dependents();
 
   // this CTA's share of the reduction axis (slices: as equal as possible, in chunks)
@@ -204,7 +217,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
         int local;
         const Job& job = p.job[job_of(tile % p.row_tiles, local)];
         const int token0 = (tile / p.row_tiles) * p.n_tile;
-        const int count = weights ? c1 - c0 : 2 * (c1 - c0);
+        const int count = c1 - c0;
         const int bytes = weights ? 2048 * job.bits : x_bytes;
         for (int i = 0; i < count; ++i, ++issued, at.advance(slots)) {
           const uint32_t slot = at.slot;
@@ -213,7 +226,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
           if (weights) {
             tma_load_2d(smem_addr(w_ring) + slot * p.w_bytes, &job.wmap, (c0 + i) * 4 * job.bits, local * 128, full + slot * 8);
           } else {
-            tma_load_2d(smem_addr(x_ring) + slot * x_bytes, &p.xmap, c0 * 128 + i * 64, token0, full + slot * 8);
+            const uint32_t dst = smem_addr(x_ring) + slot * x_bytes;
+            tma_load_2d(dst, &p.xmap, (c0 + i) * 128, token0, full + slot * 8);
+            tma_load_2d(dst + x_bytes / 2, &p.xmap, (c0 + i) * 128 + 64, token0, full + slot * 8);
           }
         }
       }
@@ -235,19 +250,20 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
         if (!mbar_wait(bars.d_empty + buffer * 8, d_at.pass ^ 1, failed)) break;
         fence_after_sync();
         const uint32_t d = d_tmem + buffer * p.n_tile;
-        for (int i = 0; i < 2 * (c1 - c0); ++i) {
+        for (int i = 0; i < c1 - c0; ++i) {
           const uint32_t xs = x_at.slot, as = a_at.slot;
           if (!(ok = mbar_wait(bars.x_full + xs * 8, x_at.pass, failed))) break;
           if (!(ok = mbar_wait(bars.a_full + as * 8, a_at.pass, failed))) break;
           fence_after_sync();
           const uint64_t b = smem_descriptor(smem_addr(x_ring) + xs * x_bytes);
-          const uint32_t a = tmem + as * 32;
+          const uint64_t b2 = smem_descriptor(smem_addr(x_ring) + xs * x_bytes + x_bytes / 2);
+          const uint32_t a = tmem + as * 64;
 #pragma unroll
-          for (int k = 0; k < 4; ++k) mma_ts(d, a + k * 8, b + k * 2, idesc, i > 0 || k > 0);
+          for (int k = 0; k < 8; ++k) mma_ts(d, a + k * 8, (k < 4 ? b : b2) + (k & 3) * 2, idesc, i > 0 || k > 0);
           mma_commit(bars.a_empty + as * 8);
           mma_commit(bars.x_empty + xs * 8);
           x_at.advance(static_cast<uint32_t>(p.x_slots));
-          a_at.advance(static_cast<uint32_t>(p.a_slots));
+          a_at.advance(kASlots);
         }
         if (ok) mma_commit(bars.d_full + buffer * 8);
       }
@@ -262,11 +278,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
     const int group = (warp - kDecodeWarp0) >> 2;
     const int warp4 = warp & 3;
     const int r = warp4 * 32 + lane;
-    const int stages = 2 * (c1 - c0);
+    const int stages = c1 - c0;
     uint32_t stage = 0;
     Cursor w_at, a_at, d_at;
-    w_at.advance(static_cast<uint32_t>(p.w_slots), static_cast<uint32_t>(group / 2));
-    a_at.advance(static_cast<uint32_t>(p.a_slots), static_cast<uint32_t>(group));
+    w_at.advance(static_cast<uint32_t>(p.w_slots), static_cast<uint32_t>(group));
+    a_at.advance(kASlots, static_cast<uint32_t>(group));
     for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, d_at.advance(static_cast<uint32_t>(p.d_buffers)), stage += stages) {
       int local;
       const Job& job = p.job[job_of(tile % p.row_tiles, local)];
@@ -328,8 +344,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
       unsigned short* dst = static_cast<unsigned short*>(p.out) + job.col0 + row;
       const uint32_t red = base + p.ring_offset + (threadIdx.x & 127) * 4;
       for (int col = first + (threadIdx.x >> 7); col < last && token0 + col < p.m; col += kThreads / 128) {
-        float sum = 0.0f;
-        for (int s = 0; s < p.slices; ++s) sum += cluster_ld(red + col * 512, s);
+        float part[8];  // all requested, then added in slice order
+#pragma unroll
+        for (int s = 0; s < 8; ++s) part[s] = s < p.slices ? cluster_ld(red + col * 512, s) : 0.0f;
+        float sum = part[0];
+#pragma unroll
+        for (int s = 1; s < 8; ++s) sum += part[s];
         dst[static_cast<int64_t>(token0 + col) * p.out_stride] =
             static_cast<unsigned short>(round_to_16(sum + bias, BF16 ? DQ_BF16 : DQ_F16));
       }
@@ -393,8 +413,11 @@ struct Shape {
 };
 
 // Token tiles and slices of the reduction axis with the least estimated time: waves of CTAs times
-// the cycles of one (stages of 64 values, each bound by the decode or by the tensor pipe, plus a
-// start and an end per tile).
+// the cycles of one -- 128-value stages, each bound by the hand-over between the block's roles or by
+// the tensor pipe (2 n_tile cycles per 64 values), plus a start and an end.  The slices of all tiles
+// are resident at once or there are none: a second wave of clusters costs more than it gives (4096 x
+// 14336, 16 rows: 22 us with 4 slices, 38 with 8), and clusters of eight pack badly into the GPCs
+// (1152 x 7936, 128 rows: 14 us with 6 slices, 21 with 8).
 Shape pick_shape(int m, int row_tiles, int chunks, int sm_count) {
   Shape best = {};
   double best_cost = 1e30;
@@ -402,13 +425,14 @@ Shape pick_shape(int m, int row_tiles, int chunks, int sm_count) {
   for (int tt = min_tiles; tt <= min_tiles + 2; ++tt) {
     const int n = static_cast<int>(ceil_div(ceil_div(m, tt), 16) * 16);
     if (n * (tt - 1) >= m) continue;
-    for (int s = 1; s <= 8 && s <= chunks; ++s) {
-      const int resident = s == 1 ? sm_count : (s <= 2 ? sm_count : s <= 4 ? sm_count - 8 : sm_count - 20) / s * s;
-      const double ctas = static_cast<double>(row_tiles) * tt * s;
-      const double waves = std::ceil(ctas / resident);
-      const double stage = std::max(300.0, 2.0 * n);
-      const double overlap = s == 1 && n <= 192 ? 0.0 : 10.0 * n;  // an epilogue that nothing hides
-      const double cost = waves * (2.0 * static_cast<double>(ceil_div(chunks, s)) * stage + overlap + (s > 1 ? 1500.0 : 0.0)) + 10.0 * n + 3000.0;
+    const double stage = std::max(700.0, 4.0 * n + 60.0);
+    for (int s = 1; s <= 6 && s <= chunks; ++s) {
+      const int64_t ctas = static_cast<int64_t>(row_tiles) * tt * s;
+      const int resident = s <= 2 ? sm_count : s <= 4 ? sm_count - 16 : sm_count - 24;
+      if (s > 1 && ctas > resident) break;
+      const double waves = std::ceil(static_cast<double>(ctas) / sm_count);
+      const double hidden = s == 1 && n <= 128 ? 0.0 : 10.0 * n;  // an epilogue that the next tile does not cover
+      const double cost = waves * (static_cast<double>(ceil_div(chunks, s)) * stage + hidden) + (s > 1 ? 1500.0 : 0.0) + 10.0 * n + 7000.0;
       if (cost < best_cost) best_cost = cost, best = {n, tt, s};
     }
   }
@@ -464,17 +488,15 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
     return DQ_OK;
   }
   const int grid_x = p.slices > 1 ? p.tiles : std::min(p.tiles, dev->sm_count);
-  // Tensor memory: operand slots (eight where there is room: a warpgroup then works two stages
-  // ahead) and the accumulators (two where a CTA has several tiles and both fit).
-  p.d_buffers = p.slices == 1 && p.tiles > grid_x && p.n_tile <= 192 ? 2 : 1;
-  p.a_slots = kMaxASlots * 32 + p.d_buffers * p.n_tile <= 512 ? kMaxASlots : kGroups;
+  p.d_buffers = p.slices == 1 && p.tiles > grid_x && p.n_tile <= 128 ? 2 : 1;
   p.tmem_columns = 32;
-  while (p.tmem_columns < p.a_slots * 32 + p.d_buffers * p.n_tile) p.tmem_columns *= 2;
-  const int x_bytes = p.n_tile * 128;
+  while (p.tmem_columns < kAColumns + p.d_buffers * p.n_tile) p.tmem_columns *= 2;
+  // Rings: activation slots of 128 values (2..6), then weight slots (a slot per warpgroup at least)
+  const int x_bytes = p.n_tile * 256;
   p.w_bytes = w_bytes;
-  p.x_slots = std::clamp(131072 / x_bytes, 4, 8);
-  const int budget = dev->max_smem_optin - static_cast<int>(kRingOffset) - 1024;
-  p.w_slots = std::clamp((budget - p.x_slots * x_bytes) / w_bytes, 2, 12);
+  const int budget = dev->max_smem_optin - static_cast<int>(kRingOffset);
+  p.x_slots = std::clamp((budget - kGroups * w_bytes) / x_bytes, 2, 6);
+  p.w_slots = std::clamp((budget - p.x_slots * x_bytes) / w_bytes, kGroups, 12);
   p.barrier_offset = kBarrierOffset;
   p.ring_offset = kRingOffset;
   const size_t smem = kRingOffset + static_cast<size_t>(p.x_slots) * x_bytes + static_cast<size_t>(p.w_slots) * w_bytes;
