@@ -39,10 +39,16 @@ using namespace umma;
 
 constexpr int kJobs = 4;
 constexpr int kDecodeWarp0 = 4;        // warps 0..3: TMA x, MMA, TMA weights, tensor memory
-constexpr int kGroups = 4;             // decoding warpgroups: stage (chunk of 128 values of K) i belongs to group i % 4
-constexpr int kThreads = (kDecodeWarp0 + 4 * kGroups) * 32;
-constexpr int kASlots = kGroups;       // operand tiles of 128 x 128 in tensor memory, 64 columns each
-constexpr int kAColumns = kASlots * 64;
+// Decoding warpgroups and the operand tiles of 128 x 128 weights in tensor memory, one per warpgroup:
+// stage (chunk of 128 values of K) i belongs to warpgroup i % kGroups and always to its tile, so that
+// nobody can ever be two passes ahead of a tile's barrier.  Four groups and tiles of 64 columns, or
+// (every weight as two 16-bit pieces) three groups and tiles of 128.
+template <bool SPLIT>
+struct Roles {
+  static constexpr int kGroups = SPLIT ? 3 : 4, kTileColumns = SPLIT ? 128 : 64, kColumns = kGroups * kTileColumns;
+  static constexpr int kThreads = (kDecodeWarp0 + 4 * kGroups) * 32;
+};
+constexpr int kMaxGroups = 4;
 constexpr int kMaxRing = 16;
 
 struct Job {
@@ -85,10 +91,11 @@ struct Cursor {
 
 // Warpgroup `group`'s chunks of a row tile: chunk c0 + i is stage stage0 + i, numbered over the life of
 // the block.  False once a wait has run out.
-template <int BITS, bool BF16, bool MBF16>
+template <int BITS, bool BF16, bool MBF16, bool SPLIT>
 __device__ bool decode_tile(const Job& job, const Params& p, int row0, int c0, int group, uint32_t stage0, int stages,
-                            const unsigned char* w_ring, const Bars& bars, uint32_t tmem, Cursor& w_at, Cursor& a_at,
+                            const unsigned char* w_ring, const Bars& bars, uint32_t tmem, Cursor& w_at, uint32_t& a_pass,
                             volatile int* failed) {
+  constexpr int kGroups = Roles<SPLIT>::kGroups;
   const int lane = threadIdx.x & 31;
   const int warp4 = (threadIdx.x >> 5) & 3;
   const int r = warp4 * 32 + lane;
@@ -112,7 +119,7 @@ __device__ bool decode_tile(const Job& job, const Params& p, int row0, int c0, i
       if (o_row != nullptr) o_next[1] = __ldg(o_row + g1);
     }
   };
-  const int first = static_cast<int>((static_cast<uint32_t>(group) - stage0) & (kGroups - 1));
+  const int first = (group + kGroups - static_cast<int>(stage0 % kGroups)) % kGroups;
   if (first >= stages) return true;
   fetch(first);
   for (int i = first; i < stages; i += kGroups) {
@@ -120,40 +127,46 @@ __device__ bool decode_tile(const Job& job, const Params& p, int row0, int c0, i
     affine.set(s_next[0], o_row != nullptr ? widen(o_next[0]) : 0.0f);
     const unsigned short s_half = s_next[1], o_half = o_next[1];
     fetch(min(i + kGroups, stages - 1));  // the next chunk's metadata travels while this one is decoded
-    const uint32_t slot = w_at.slot, a_slot = a_at.slot;
+    const uint32_t slot = w_at.slot;
     if (!mbar_wait(bars.w_full + slot * 8, w_at.pass, failed)) return false;
-    const uint32_t dst = tmem + a_slot * 64 + (static_cast<uint32_t>(warp4 * 32) << 16);
+    const uint32_t dst = tmem + group * Roles<SPLIT>::kTileColumns + (static_cast<uint32_t>(warp4 * 32) << 16);
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-      uint32_t w[2 * BITS];
+      uint32_t w[2 * BITS], v[16], low[16];
       read_row64<BITS>(w_ring + slot * p.w_bytes, r, half, w);
       if (half == 1) {
         __syncwarp();
         if (lane == 0) mbar_arrive(bars.w_empty + slot * 8);  // (the words are in registers)
         if (two_groups) affine.set(s_half, o_row != nullptr ? widen(o_half) : 0.0f);
       }
-      uint32_t v[16];
-      decode32<BITS, BF16, MBF16>(w, affine, v);
-      if (half == 0) {
-        if (!mbar_wait(bars.a_empty + a_slot * 8, a_at.pass ^ 1, failed)) return false;
+      decode32<BITS, BF16, MBF16, SPLIT>(w, affine, v, low);
+      if (half == 0) {  // the MMAs of this group's previous chunk are done with the tile
+        if (!mbar_wait(bars.a_empty + group * 8, a_pass ^ 1, failed)) return false;
         fence_after_sync();
       }
       tmem_st16(dst + half * 32, v);
-      decode32<BITS, BF16, MBF16>(w + BITS, affine, v);
+      if constexpr (SPLIT) tmem_st16(dst + 64 + half * 32, low);
+      decode32<BITS, BF16, MBF16, SPLIT>(w + BITS, affine, v, low);
       tmem_st16(dst + half * 32 + 16, v);
+      if constexpr (SPLIT) tmem_st16(dst + 64 + half * 32 + 16, low);
     }
     tmem_wait_st();
     fence_before_sync();
     __syncwarp();
-    if (lane == 0) mbar_arrive(bars.a_full + a_slot * 8);
+    if (lane == 0) mbar_arrive(bars.a_full + group * 8);
     w_at.advance(static_cast<uint32_t>(p.w_slots), kGroups);
-    a_at.advance(kASlots, kGroups);
+    a_pass ^= 1;
   }
   return true;
 }
 
-template <bool BF16, bool MBF16>
-__global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_constant__ Params p) {
+// SPLIT: the weights enter as the sum of two 16-bit operands, so that nothing of their fp32 values is
+// lost that the sums could show.  Up to DQ_GEMV_CHUNKED_MAX_ROWS activation rows, where the mma.sync
+// kernels scale fp32 accumulators and never round a weight; above that the dense path this kernel
+// replaces rounds every weight once, and so does this kernel.
+template <bool BF16, bool MBF16, bool SPLIT>
+__global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(const __grid_constant__ Params p) {
+  constexpr int kGroups = Roles<SPLIT>::kGroups;
   extern __shared__ __align__(1024) unsigned char smem[];
   // control block at the front: failure flag, tensor memory address, barriers
   volatile int* failed = reinterpret_cast<volatile int*>(smem);
@@ -164,8 +177,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
   bars.w_full = bars.x_empty + kMaxRing * 8;
   bars.w_empty = bars.w_full + kMaxRing * 8;
   bars.a_full = bars.w_empty + kMaxRing * 8;
-  bars.a_empty = bars.a_full + kASlots * 8;
-  bars.d_full = bars.a_empty + kASlots * 8;
+  bars.a_empty = bars.a_full + kMaxGroups * 8;
+  bars.d_full = bars.a_empty + kMaxGroups * 8;
   bars.d_empty = bars.d_full + 2 * 8;
   bars.drain = bars.d_empty + 2 * 8;
   const int x_bytes = p.n_tile * 256;  // two slabs of 64 values
@@ -178,7 +191,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
     *failed = 0;
     for (int i = 0; i < p.x_slots; ++i) mbar_init(bars.x_full + i * 8, 1), mbar_init(bars.x_empty + i * 8, 1);
     for (int i = 0; i < p.w_slots; ++i) mbar_init(bars.w_full + i * 8, 1), mbar_init(bars.w_empty + i * 8, 4);
-    for (int i = 0; i < kASlots; ++i) mbar_init(bars.a_full + i * 8, 4), mbar_init(bars.a_empty + i * 8, 1);
+    for (int i = 0; i < kGroups; ++i) mbar_init(bars.a_full + i * 8, 4), mbar_init(bars.a_empty + i * 8, 1);
     for (int i = 0; i < 2; ++i) mbar_init(bars.d_full + i * 8, 1), mbar_init(bars.d_empty + i * 8, 4 * kGroups);
     mbar_init(bars.drain, 1);
     fence_mbar_init();
@@ -189,7 +202,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + 4);
-  const uint32_t d_tmem = tmem + kAColumns;
+  const uint32_t d_tmem = tmem + Roles<SPLIT>::kColumns;
   pdl_launch_dependents();
 
   // this CTA's share of the reduction axis (slices: as equal as possible, in chunks)
@@ -251,19 +264,22 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
         fence_after_sync();
         const uint32_t d = d_tmem + buffer * p.n_tile;
         for (int i = 0; i < c1 - c0; ++i) {
-          const uint32_t xs = x_at.slot, as = a_at.slot;
+          const uint32_t xs = x_at.slot;
           if (!(ok = mbar_wait(bars.x_full + xs * 8, x_at.pass, failed))) break;
-          if (!(ok = mbar_wait(bars.a_full + as * 8, a_at.pass, failed))) break;
+          const uint64_t b0 = smem_descriptor(smem_addr(x_ring) + xs * x_bytes);
+          const uint64_t b1 = smem_descriptor(smem_addr(x_ring) + xs * x_bytes + x_bytes / 2);
+          if (!(ok = mbar_wait(bars.a_full + a_at.slot * 8, a_at.pass, failed))) break;
           fence_after_sync();
-          const uint64_t b = smem_descriptor(smem_addr(x_ring) + xs * x_bytes);
-          const uint64_t b2 = smem_descriptor(smem_addr(x_ring) + xs * x_bytes + x_bytes / 2);
-          const uint32_t a = tmem + as * 64;
+          const uint32_t a = tmem + a_at.slot * Roles<SPLIT>::kTileColumns;
 #pragma unroll
-          for (int k = 0; k < 8; ++k) mma_ts(d, a + k * 8, (k < 4 ? b : b2) + (k & 3) * 2, idesc, i > 0 || k > 0);
-          mma_commit(bars.a_empty + as * 8);
+          for (int k = 0; k < 8; ++k) {
+            mma_ts(d, a + k * 8, (k < 4 ? b0 : b1) + (k & 3) * 2, idesc, i > 0 || k > 0);
+            if constexpr (SPLIT) mma_ts(d, a + 64 + k * 8, (k < 4 ? b0 : b1) + (k & 3) * 2, idesc, true);
+          }
+          mma_commit(bars.a_empty + a_at.slot * 8);
+          a_at.advance(kGroups);
           mma_commit(bars.x_empty + xs * 8);
           x_at.advance(static_cast<uint32_t>(p.x_slots));
-          a_at.advance(kASlots);
         }
         if (ok) mma_commit(bars.d_full + buffer * 8);
       }
@@ -280,14 +296,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
     const int r = warp4 * 32 + lane;
     const int stages = c1 - c0;
     uint32_t stage = 0;
-    Cursor w_at, a_at, d_at;
+    uint32_t a_pass = 0;
+    Cursor w_at, d_at;
     w_at.advance(static_cast<uint32_t>(p.w_slots), static_cast<uint32_t>(group));
-    a_at.advance(kASlots, static_cast<uint32_t>(group));
     for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, d_at.advance(static_cast<uint32_t>(p.d_buffers)), stage += stages) {
       int local;
       const Job& job = p.job[job_of(tile % p.row_tiles, local)];
       bool ok;
-#define DQ_DECODE(B) ok = decode_tile<B, BF16, MBF16>(job, p, local * 128, c0, group, stage, stages, w_ring, bars, tmem, w_at, a_at, failed)
+#define DQ_DECODE(B) ok = decode_tile<B, BF16, MBF16, SPLIT>(job, p, local * 128, c0, group, stage, stages, w_ring, bars, tmem, w_at, a_pass, failed)
       switch (job.bits) {
         case 2: DQ_DECODE(2); break;
         case 3: DQ_DECODE(3); break;
@@ -343,7 +359,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_umma_kernel(const __grid_con
       const float bias = job.bias != nullptr ? load_f32(job.bias, row, BF16 ? DQ_BF16 : DQ_F16) : 0.0f;
       unsigned short* dst = static_cast<unsigned short*>(p.out) + job.col0 + row;
       const uint32_t red = base + p.ring_offset + (threadIdx.x & 127) * 4;
-      for (int col = first + (threadIdx.x >> 7); col < last && token0 + col < p.m; col += kThreads / 128) {
+      for (int col = first + (threadIdx.x >> 7); col < last && token0 + col < p.m; col += Roles<SPLIT>::kThreads / 128) {
         float part[8];  // all requested, then added in slice order
 #pragma unroll
         for (int s = 0; s < 8; ++s) part[s] = s < p.slices ? cluster_ld(red + col * 512, s) : 0.0f;
@@ -488,15 +504,19 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
     return DQ_OK;
   }
   const int grid_x = p.slices > 1 ? p.tiles : std::min(p.tiles, dev->sm_count);
-  p.d_buffers = p.slices == 1 && p.tiles > grid_x && p.n_tile <= 128 ? 2 : 1;
+  const bool split = a.m <= DQ_GEMV_CHUNKED_MAX_ROWS;
+  const int a_columns = split ? Roles<true>::kColumns : Roles<false>::kColumns;
+  p.d_buffers = p.slices == 1 && p.tiles > grid_x && a_columns + 2 * p.n_tile <= 512 ? 2 : 1;
   p.tmem_columns = 32;
-  while (p.tmem_columns < kAColumns + p.d_buffers * p.n_tile) p.tmem_columns *= 2;
-  // Rings: activation slots of 128 values (2..6), then weight slots (a slot per warpgroup at least)
+  while (p.tmem_columns < a_columns + p.d_buffers * p.n_tile) p.tmem_columns *= 2;
+  // Rings: activation slots of 128 values (2..6), then weight slots -- a multiple of the warpgroups, so
+  // that a slot always belongs to the same one (its barrier then cannot be two passes behind).
   const int x_bytes = p.n_tile * 256;
   p.w_bytes = w_bytes;
   const int budget = dev->max_smem_optin - static_cast<int>(kRingOffset);
-  p.x_slots = std::clamp((budget - kGroups * w_bytes) / x_bytes, 2, 6);
-  p.w_slots = std::clamp((budget - p.x_slots * x_bytes) / w_bytes, kGroups, 12);
+  p.x_slots = std::clamp((budget - kMaxGroups * w_bytes) / x_bytes, 2, 6);
+  const int groups = split ? Roles<true>::kGroups : Roles<false>::kGroups;
+  p.w_slots = std::clamp((budget - p.x_slots * x_bytes) / w_bytes / groups * groups, groups, 12);
   p.barrier_offset = kBarrierOffset;
   p.ring_offset = kRingOffset;
   const size_t smem = kRingOffset + static_cast<size_t>(p.x_slots) * x_bytes + static_cast<size_t>(p.w_slots) * w_bytes;
@@ -506,7 +526,7 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
     DQ_CUDA(allow_shared(kernel, smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(grid_x), static_cast<unsigned>(p.slices));
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(static_cast<unsigned>(split ? Roles<true>::kThreads : Roles<false>::kThreads));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -531,8 +551,12 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
     *taken = true;
     return DQ_OK;
   };
-  if (a.x_dtype == DQ_BF16) return mbf ? run(gemm_umma_kernel<true, true>) : run(gemm_umma_kernel<true, false>);
-  return mbf ? run(gemm_umma_kernel<false, true>) : run(gemm_umma_kernel<false, false>);
+  if (split) {
+    if (a.x_dtype == DQ_BF16) return mbf ? run(gemm_umma_kernel<true, true, true>) : run(gemm_umma_kernel<true, false, true>);
+    return mbf ? run(gemm_umma_kernel<false, true, true>) : run(gemm_umma_kernel<false, false, true>);
+  }
+  if (a.x_dtype == DQ_BF16) return mbf ? run(gemm_umma_kernel<true, true, false>) : run(gemm_umma_kernel<true, false, false>);
+  return mbf ? run(gemm_umma_kernel<false, true, false>) : run(gemm_umma_kernel<false, false, false>);
 }
 
 }  // namespace dq

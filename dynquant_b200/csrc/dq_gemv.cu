@@ -553,6 +553,43 @@ int32_t check_activation(const void* x, int32_t x_dtype, int64_t m, void* out, i
   return DQ_OK;
 }
 
+// Whether a matmul goes to the tcgen05 kernel (dq_gemm_umma.cu) rather than to the mma.sync kernels.
+// Measured on 60 random shapes x 4 widths (rows 512..28672, K 512..18944, 1..40 activation rows); us,
+// mma.sync -> tcgen05:
+//  * above 32 rows, and several shards above 8: always (12544 x 10624 2-bit 40 rows 2150 -> 50);
+//  * 9..32 rows: except where ONE launch of the tiled or the many-rows kernel serves all rows with
+//    whole blocks of four steps -- up to 16 rows on K <= 4096 (2816 x 2048 16 rows: 7.5 -> 7.4, 1009 x
+//    1024: 3.7 -> 5.2), up to 32 on small matrices (2688 x 512 32 rows: 3.8 -> 6.5);
+//  * 1..8 rows, where the mma.sync kernels have no good shape:
+//      - 64-value groups with an odd number of 128-value steps: the SIMT kernel (1024 x 5760, 1 / 8
+//        rows: 12.8 / 132 -> 7.4 / 7.7);
+//      - few rows and long slices of the reduction axis in the tiled kernel, which halves the step
+//        count only while the halves stay even (1152 x 7936, 62 steps: 25 -> 9; 896 x 3584: 7.1 -> 5.9);
+//      - odd step counts in the register-ring kernel: 8-bit matrices of many rows (25390 x 4736: 54 ->
+//        39) and six to eight rows x a long axis (7407 x 10624 8 rows: 41 -> 29).
+bool gemm_first(int64_t m, const dq_weight* shards, int num_shards) {
+  if (m > 32 || (m > DQ_GEMV_MAX_ROWS && num_shards > 1)) return true;
+  for (int i = 0; i < num_shards; ++i) {
+    const dq_weight& w = shards[i];
+    const int64_t k = w.in_features, steps = ceil_div(k, 128);
+    if (m > DQ_GEMV_MAX_ROWS) {
+      const bool blocks = k % 512 == 0;
+      const bool one_launch = (m <= 16 && k <= 4096 && w.rows <= (w.bits == 8 ? 4096 : 16384)) || (k <= 2048 && w.rows * k <= 6000000);
+      return !(blocks && one_launch);
+    }
+    if (w.group_values == 64 && steps % 2 != 0 && m > (w.rows * k > 1000000 ? 0 : 1)) return true;
+    if (steps % 2 != 0) {
+      if (w.bits == 8 && w.rows * k >= 40000000) return true;
+      if (m >= 6 && k >= 10240) return true;
+    } else {
+      int64_t slice = steps;
+      for (int kw = 1; kw < 8 && slice % 4 == 0; kw *= 2) slice /= 2;
+      if (w.rows <= 1536 && slice >= 14) return true;
+    }
+  }
+  return false;
+}
+
 }  // namespace
 }  // namespace dq
 
@@ -756,6 +793,19 @@ int32_t dq_gemm_shards(const void* x, int32_t x_dtype, int64_t m, const dq_weigh
     }
   }
   return DQ_OK;
+}
+
+int32_t dq_matmul_shards(const void* x, int32_t x_dtype, int64_t m, const dq_weight* shards, int32_t num_shards,
+                         const void* bias, void* out, int64_t out_stride, int32_t out_dtype, void* stream) {
+  DQ_REQUIRE(shards != nullptr && num_shards > 0, "matmul_shards: need at least one shard");
+  if (out_dtype == x_dtype && dq::gemm_first(m, shards, num_shards)) {
+    const int32_t rc = dq_gemm_shards(x, x_dtype, m, shards, num_shards, bias, out, out_stride, out_dtype, stream);
+    if (rc != DQ_ERR_UNSUPPORTED) return rc;
+  }
+  if (m > DQ_GEMV_CHUNKED_MAX_ROWS) {
+    return dq::fail(DQ_ERR_UNSUPPORTED, "matmul_shards: a geometry only dequantize + dense serves above %d rows", DQ_GEMV_CHUNKED_MAX_ROWS);
+  }
+  return dq_gemv_shards_rows(x, x_dtype, m, shards, num_shards, bias, out, out_stride, out_dtype, stream);
 }
 
 int32_t dq_gemv_sequence(const dq_gemv_job* jobs, int32_t num_jobs, void* stream) {

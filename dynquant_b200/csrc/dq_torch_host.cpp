@@ -191,15 +191,10 @@ PyObject* multiply(const at::Tensor* x, const dq_weight* w, int n, const at::Ten
     sizes.back() = total;
     at::Tensor out = new_cuda(sizes, x->scalar_type(), q.device());
     const int tag = tag_of(x->scalar_type());
-    if (m > DQ_GEMV_CHUNKED_MAX_ROWS) {
-      const int32_t rc = dq_gemm_shards(flat.const_data_ptr(), tag, m, w, n, bias == nullptr ? nullptr : cast.const_data_ptr(),
+    const int32_t rc = dq_matmul_shards(flat.const_data_ptr(), tag, m, w, n, bias == nullptr ? nullptr : cast.const_data_ptr(),
                                         out.data_ptr(), total, tag, stream);
-      if (rc == DQ_ERR_UNSUPPORTED) return at::Tensor();
-      check(rc);
-      return out;
-    }
-    check(dq_gemv_shards_rows(flat.const_data_ptr(), tag, m, w, n, bias == nullptr ? nullptr : cast.const_data_ptr(),
-                              out.data_ptr(), total, tag, stream));
+    if (rc == DQ_ERR_UNSUPPORTED && m > DQ_GEMV_CHUNKED_MAX_ROWS) return at::Tensor();
+    check(rc);
     return out;
   });
 }

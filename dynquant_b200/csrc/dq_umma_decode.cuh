@@ -86,9 +86,11 @@ __device__ __forceinline__ float fma_half(uint32_t pair, bool high, unsigned sho
   return d;
 }
 
-// 32 values (BITS words) -> 16 registers of two.
-template <int BITS, bool BF16, bool MBF16>
-__device__ __forceinline__ void decode32(const uint32_t* w, const Affine<BITS, MBF16>& c, uint32_t* out) {
+// 32 values (BITS words) -> 16 registers of two; `low` (if not null): what the rounding of each value
+// to 16 bits left over, rounded the same way, so that out + low carries the value to 16 bits (bf16) or
+// 21 (fp16) -- the remainder is one exact mixed-precision fma per value.
+template <int BITS, bool BF16, bool MBF16, bool SPLIT>
+__device__ __forceinline__ void decode32(const uint32_t* w, const Affine<BITS, MBF16>& c, uint32_t* out, uint32_t* low) {
   using A = Affine<BITS, MBF16>;
   float f[32];
   // codes `lo` (low half of u) and `hi` (high half), at mantissa place i
@@ -145,7 +147,13 @@ __device__ __forceinline__ void decode32(const uint32_t* w, const Affine<BITS, M
     take(ten, 0, 10, 26);
   }
 #pragma unroll
-  for (int i = 0; i < 16; ++i) out[i] = pack16<BF16>(f[2 * i], f[2 * i + 1]);
+  for (int i = 0; i < 16; ++i) {
+    out[i] = pack16<BF16>(f[2 * i], f[2 * i + 1]);
+    if constexpr (SPLIT) {
+      constexpr unsigned short kMinusOne = BF16 ? 0xBF80 : 0xBC00;
+      low[i] = pack16<BF16>(fma_half<BF16>(out[i], false, kMinusOne, f[2 * i]), fma_half<BF16>(out[i], true, kMinusOne, f[2 * i + 1]));
+    }
+  }
 }
 
 // The 64 values (2 * BITS words) of half `half` of row `row` in a staged 128 x 128-value tile.

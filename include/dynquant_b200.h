@@ -183,6 +183,12 @@ DQ_API int32_t dq_gemv_shards_rows(const void* x, int32_t x_dtype, int64_t m, co
 DQ_API int32_t dq_gemm_shards(const void* x, int32_t x_dtype, int64_t m, const dq_weight* shards,
                               int32_t num_shards, const void* bias, void* out, int64_t out_stride,
                               int32_t out_dtype, void* stream);
+/* Any number of activation rows through whichever kernel is the fastest for the sizes: dq_gemm_shards
+ * where that pays, else dq_gemv_shards_rows; DQ_ERR_UNSUPPORTED above its 64 rows where
+ * dq_gemm_shards does not take the geometry. */
+DQ_API int32_t dq_matmul_shards(const void* x, int32_t x_dtype, int64_t m, const dq_weight* shards,
+                                int32_t num_shards, const void* bias, void* out, int64_t out_stride,
+                                int32_t out_dtype, void* stream);
 /* Synchronises `stream`; DQ_ERR_DEVICE once a bounded wait inside one of these kernels has run out
  * on the current device (its output is then incomplete; the context stays usable). */
 DQ_API int32_t dq_gemm_status(void* stream);

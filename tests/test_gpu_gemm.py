@@ -1,0 +1,72 @@
+"""The tcgen05 kernel for many activation rows (``gemm_umma_kernel``) at the edges of its tiles."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from test_gpu_parity import oracle_gemv, within_one_ulp_16
+from test_gpu_shapes import random_qt
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bits", [2, 3, 4, 8])
+@pytest.mark.parametrize(("m", "rows", "k", "group", "act", "meta", "offsets"), [
+    (9, 129, 640, 128, torch.bfloat16, torch.float16, True),     # one row past a tile, an odd number of chunks
+    (64, 257, 1152, 64, torch.float16, torch.bfloat16, False),   # the last row count with split weights
+    (65, 127, 128, 128, torch.bfloat16, torch.bfloat16, True),   # the first without, one chunk
+    (256, 640, 2048, 128, torch.float16, torch.float16, True),   # a full token tile, sliced over a cluster
+    (257, 1000, 416, 64, torch.bfloat16, torch.float16, True),   # one token past it, a ragged reduction axis
+    (700, 20000, 256, 256, torch.bfloat16, torch.bfloat16, False),  # several tiles per block
+])
+def test_many_rows_match_the_oracle(bits, m, rows, k, group, act, meta, offsets):
+    import ctypes
+
+    from dynquant_b200 import _lib, ops
+
+    qt = random_qt(rows, k, bits, group=group, meta=meta, seed=m + bits, offsets=offsets)
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(m)).to(act).cuda()
+    bias = torch.randn(rows, generator=torch.Generator().manual_seed(3)).to(act).cuda()
+    lib, tag = _lib.load(), _lib.DQ_BF16 if act == torch.bfloat16 else _lib.DQ_F16
+    w = ops.weight_descriptor("gemm", qt.packed, qt.scales, qt.offsets, bits, group, k)
+    padded = torch.full((m + 2, rows), 7.0, dtype=act, device="cuda")
+    out, stream = padded[1:-1], ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    rc = lib.dq_gemm_shards(x.data_ptr(), tag, m, ctypes.byref(w), 1, bias.data_ptr(), out.data_ptr(), rows, tag, stream)
+    if bits == 3 and group == 64 and -(-k // 64) % 2:
+        assert rc == _lib.DQ_ERR_UNSUPPORTED  # rows that are not whole 16-byte pieces
+        return
+    assert rc == _lib.DQ_OK and ops.last_kernel() == "gemm_umma_kernel"
+    assert lib.dq_gemm_status(stream) == _lib.DQ_OK
+    assert bool((padded[0] == 7.0).all()) and bool((padded[-1] == 7.0).all())
+    dense = ops.dequant(qt.packed, qt.scales, qt.offsets, bits, group, k, out_dtype=torch.float32)
+    want = x.double() @ dense.double().T + bias.double()
+    if m <= 64:  # weights enter unrounded: the fp32 result, rounded once
+        assert within_one_ulp_16(out, want.float().cpu().numpy())
+    else:        # weights rounded once to the activation type
+        error = (out.double() - want).norm() / want.norm()
+        assert error <= (4e-3 if act == torch.bfloat16 else 5e-4)
+    again = torch.empty_like(out)
+    lib.dq_gemm_shards(x.data_ptr(), tag, m, ctypes.byref(w), 1, bias.data_ptr(), again.data_ptr(), rows, tag, stream)
+    assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("m", [2, 7, 12, 40, 130])
+def test_shards_of_mixed_widths_in_one_launch(m):
+    from dynquant_b200 import ops
+    from dynquant_b200.plugin import DynQuantLinearMethod, ShardSpec
+
+    k, sizes, widths = 1408, (300, 128, 77), (8, 2, 3)  # 11 steps of 64-value groups: the tcgen05 kernel at any row count
+    method, layer = DynQuantLinearMethod(None, [ShardSpec(str(i), b, 64, n) for i, (n, b) in enumerate(zip(sizes, widths))]), torch.nn.Module()
+    method.create_weights(layer, k, list(sizes), k, sum(sizes), torch.bfloat16, device="cuda")
+    shards = [random_qt(n, k, b, group=64, meta=torch.bfloat16, seed=b) for n, b in zip(sizes, widths)]
+    for i, qt in enumerate(shards):
+        method.load_shard(layer, i, qt)
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(m)).to(torch.bfloat16).cuda()
+    bias = torch.randn(sum(sizes)).to(torch.bfloat16).cuda()
+    before = ops.launch_count()
+    got = method.apply(layer, x, bias)
+    assert ops.launch_count() - before == 1 and ops.last_kernel() == "gemm_umma_kernel"
+    want = torch.cat([torch.from_numpy(oracle_gemv(x, qt)) for qt in shards], dim=1) + bias.float().cpu()
+    error = (got.float().cpu() - want).norm() / want.norm()
+    assert error <= 4e-3
