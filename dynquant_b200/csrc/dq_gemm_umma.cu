@@ -134,11 +134,7 @@ __device__ bool decode_tile(const Job& job, const Params& p, int row0, int c0, i
     for (int half = 0; half < 2; ++half) {
       uint32_t w[2 * BITS], v[16], low[16];
       read_row64<BITS>(w_ring + slot * p.w_bytes, r, half, w);
-      if (half == 1) {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bars.w_empty + slot * 8);  // (the words are in registers)
-        if (two_groups) affine.set(s_half, o_row != nullptr ? widen(o_half) : 0.0f);
-      }
+      if (half == 1 && two_groups) affine.set(s_half, o_row != nullptr ? widen(o_half) : 0.0f);
       decode32<BITS, BF16, MBF16, SPLIT>(w, affine, v, low);
       if (half == 0) {  // the MMAs of this group's previous chunk are done with the tile
         if (!mbar_wait(bars.a_empty + group * 8, a_pass ^ 1, failed)) return false;
@@ -153,7 +149,12 @@ __device__ bool decode_tile(const Job& job, const Params& p, int row0, int c0, i
     tmem_wait_st();
     fence_before_sync();
     __syncwarp();
-    if (lane == 0) mbar_arrive(bars.a_full + group * 8);
+    if (lane == 0) {
+      mbar_arrive(bars.a_full + group * 8);
+      // Only now: an arrival may overtake shared-memory loads still in flight, and the slot is refilled
+      // at once.  By here every word has gone through the decode.
+      mbar_arrive(bars.w_empty + slot * 8);
+    }
     w_at.advance(static_cast<uint32_t>(p.w_slots), kGroups);
     a_pass ^= 1;
   }

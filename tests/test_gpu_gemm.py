@@ -19,6 +19,7 @@ pytestmark = pytest.mark.gpu
     (256, 640, 2048, 128, torch.float16, torch.float16, True),   # a full token tile, sliced over a cluster
     (257, 1000, 416, 64, torch.bfloat16, torch.float16, True),   # one token past it, a ragged reduction axis
     (700, 20000, 256, 256, torch.bfloat16, torch.bfloat16, False),  # several tiles per block
+    (206, 1536, 8192, 128, torch.bfloat16, torch.float16, True),    # the shortest rings: slots refilled at once
 ])
 def test_many_rows_match_the_oracle(bits, m, rows, k, group, act, meta, offsets):
     import ctypes
