@@ -30,7 +30,7 @@
 
 #include "dq_gemm_umma.cuh"
 #include "dq_gemv.cuh"
-#include "dq_umma_decode.cuh"
+#include "dq_umma_pipeline.cuh"
 
 namespace dq {
 namespace {
@@ -38,26 +38,12 @@ namespace {
 using namespace umma;
 
 constexpr int kJobs = 4;
-constexpr int kDecodeWarp0 = 4;        // warps 0..3: TMA x, MMA, TMA weights, tensor memory
-// Decoding warpgroups and the operand tiles of 128 x 128 weights in tensor memory, one per warpgroup:
-// stage (chunk of 128 values of K) i belongs to warpgroup i % kGroups and always to its tile, so that
-// nobody can ever be two passes ahead of a tile's barrier.  Four groups and tiles of 64 columns, or
-// (every weight as two 16-bit pieces) three groups and tiles of 128.
-template <bool SPLIT>
-struct Roles {
-  static constexpr int kGroups = SPLIT ? 3 : 4, kTileColumns = SPLIT ? 128 : 64, kColumns = kGroups * kTileColumns;
-  static constexpr int kThreads = (kDecodeWarp0 + 4 * kGroups) * 32;
-};
-constexpr int kMaxGroups = 4;
-constexpr int kMaxRing = 16;
-
 struct Job {
   CUtensorMap wmap;
-  const void* scales;
-  const void* offsets;                 // may be null
+  Meta meta;
   const void* bias;                    // may be null; element 0 belongs to output column 0 of this job
   int64_t col0;
-  int rows, row_tiles, bits, num_groups, group_shift;  // group = 64 << group_shift
+  int rows, row_tiles, bits;
 };
 
 struct Params {
@@ -75,92 +61,6 @@ struct Params {
 
 __device__ unsigned int g_gemm_failed = 0;
 
-struct Bars {
-  uint32_t x_full, x_empty, w_full, w_empty, a_full, a_empty, d_full, d_empty, drain;
-};
-
-// Where a role stands in a ring: a slot and the parity of its pass (run-time divisions would cost the
-// single-thread roles more than their work: 0.3 us per stage, measured).
-struct Cursor {
-  uint32_t slot = 0, pass = 0;
-  __device__ __forceinline__ void advance(uint32_t slots, uint32_t by = 1) {
-    slot += by;
-    if (slot >= slots) slot -= slots, pass ^= 1;  // (by <= slots)
-  }
-};
-
-// Warpgroup `group`'s chunks of a row tile: chunk c0 + i is stage stage0 + i, numbered over the life of
-// the block.  False once a wait has run out.
-template <int BITS, bool BF16, bool MBF16, bool SPLIT>
-__device__ bool decode_tile(const Job& job, const Params& p, int row0, int c0, int group, uint32_t stage0, int stages,
-                            const unsigned char* w_ring, const Bars& bars, uint32_t tmem, Cursor& w_at, uint32_t& a_pass,
-                            volatile int* failed) {
-  constexpr int kGroups = Roles<SPLIT>::kGroups;
-  const int lane = threadIdx.x & 31;
-  const int warp4 = (threadIdx.x >> 5) & 3;
-  const int r = warp4 * 32 + lane;
-  const int row = min(row0 + r, job.rows - 1);
-  const unsigned short* s_row = static_cast<const unsigned short*>(job.scales) + static_cast<int64_t>(row) * job.num_groups;
-  const unsigned short* o_row =
-      job.offsets == nullptr ? nullptr : static_cast<const unsigned short*>(job.offsets) + static_cast<int64_t>(row) * job.num_groups;
-  auto widen = [&](unsigned short v) -> float {
-    return MBF16 ? __uint_as_float(static_cast<uint32_t>(v) << 16) : __half2float(__ushort_as_half(v));
-  };
-  const bool two_groups = job.group_shift == 0;  // 64-value groups: a chunk holds two
-  auto group_of = [&](int i, int half) -> int { return min((2 * (c0 + i) + half) >> job.group_shift, job.num_groups - 1); };
-  unsigned short s_next[2], o_next[2] = {0, 0};
-  auto fetch = [&](int i) {
-    const int g0 = group_of(i, 0);
-    s_next[0] = __ldg(s_row + g0);
-    if (o_row != nullptr) o_next[0] = __ldg(o_row + g0);
-    if (two_groups) {
-      const int g1 = group_of(i, 1);
-      s_next[1] = __ldg(s_row + g1);
-      if (o_row != nullptr) o_next[1] = __ldg(o_row + g1);
-    }
-  };
-  const int first = (group + kGroups - static_cast<int>(stage0 % kGroups)) % kGroups;
-  if (first >= stages) return true;
-  fetch(first);
-  for (int i = first; i < stages; i += kGroups) {
-    Affine<BITS, MBF16> affine;
-    affine.set(s_next[0], o_row != nullptr ? widen(o_next[0]) : 0.0f);
-    const unsigned short s_half = s_next[1], o_half = o_next[1];
-    fetch(min(i + kGroups, stages - 1));  // the next chunk's metadata travels while this one is decoded
-    const uint32_t slot = w_at.slot;
-    if (!mbar_wait(bars.w_full + slot * 8, w_at.pass, failed)) return false;
-    const uint32_t dst = tmem + group * Roles<SPLIT>::kTileColumns + (static_cast<uint32_t>(warp4 * 32) << 16);
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      uint32_t w[2 * BITS], v[16], low[16];
-      read_row64<BITS>(w_ring + slot * p.w_bytes, r, half, w);
-      if (half == 1 && two_groups) affine.set(s_half, o_row != nullptr ? widen(o_half) : 0.0f);
-      decode32<BITS, BF16, MBF16, SPLIT>(w, affine, v, low);
-      if (half == 0) {  // the MMAs of this group's previous chunk are done with the tile
-        if (!mbar_wait(bars.a_empty + group * 8, a_pass ^ 1, failed)) return false;
-        fence_after_sync();
-      }
-      tmem_st16(dst + half * 32, v);
-      if constexpr (SPLIT) tmem_st16(dst + 64 + half * 32, low);
-      decode32<BITS, BF16, MBF16, SPLIT>(w + BITS, affine, v, low);
-      tmem_st16(dst + half * 32 + 16, v);
-      if constexpr (SPLIT) tmem_st16(dst + 64 + half * 32 + 16, low);
-    }
-    tmem_wait_st();
-    fence_before_sync();
-    __syncwarp();
-    if (lane == 0) {
-      mbar_arrive(bars.a_full + group * 8);
-      // Only now: an arrival may overtake shared-memory loads still in flight, and the slot is refilled
-      // at once.  By here every word has gone through the decode.
-      mbar_arrive(bars.w_empty + slot * 8);
-    }
-    w_at.advance(static_cast<uint32_t>(p.w_slots), kGroups);
-    a_pass ^= 1;
-  }
-  return true;
-}
-
 // SPLIT: the weights enter as the sum of two 16-bit operands, so that nothing of their fp32 values is
 // lost that the sums could show.  Up to DQ_GEMV_CHUNKED_MAX_ROWS activation rows, where the mma.sync
 // kernels scale fp32 accumulators and never round a weight; above that the dense path this kernel
@@ -172,16 +72,7 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
   // control block at the front: failure flag, tensor memory address, barriers
   volatile int* failed = reinterpret_cast<volatile int*>(smem);
   const uint32_t base = smem_addr(smem);
-  Bars bars;
-  bars.x_full = base + p.barrier_offset;
-  bars.x_empty = bars.x_full + kMaxRing * 8;
-  bars.w_full = bars.x_empty + kMaxRing * 8;
-  bars.w_empty = bars.w_full + kMaxRing * 8;
-  bars.a_full = bars.w_empty + kMaxRing * 8;
-  bars.a_empty = bars.a_full + kMaxGroups * 8;
-  bars.d_full = bars.a_empty + kMaxGroups * 8;
-  bars.d_empty = bars.d_full + 2 * 8;
-  bars.drain = bars.d_empty + 2 * 8;
+  const Bars bars = bars_at(base + p.barrier_offset);
   const int x_bytes = p.n_tile * 256;  // two slabs of 64 values
   unsigned char* x_ring = smem + p.ring_offset;
   unsigned char* w_ring = x_ring + p.x_slots * x_bytes;
@@ -190,12 +81,7 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
 
   if (threadIdx.x == 0) {
     *failed = 0;
-    for (int i = 0; i < p.x_slots; ++i) mbar_init(bars.x_full + i * 8, 1), mbar_init(bars.x_empty + i * 8, 1);
-    for (int i = 0; i < p.w_slots; ++i) mbar_init(bars.w_full + i * 8, 1), mbar_init(bars.w_empty + i * 8, 4);
-    for (int i = 0; i < kGroups; ++i) mbar_init(bars.a_full + i * 8, 4), mbar_init(bars.a_empty + i * 8, 1);
-    for (int i = 0; i < 2; ++i) mbar_init(bars.d_full + i * 8, 1), mbar_init(bars.d_empty + i * 8, 4 * kGroups);
-    mbar_init(bars.drain, 1);
-    fence_mbar_init();
+    init_bars(bars, p.x_slots, p.w_slots, kGroups);
     tma_prefetch_map(&p.xmap);
   }
   if (warp == 3) tmem_alloc(base + 4, static_cast<uint32_t>(p.tmem_columns));
@@ -246,12 +132,7 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
           }
         }
       }
-      if (!ok || *failed != 0) {  // wait for the copies in flight
-        for (uint32_t k = issued > slots ? issued - slots : 0; k < issued; ++k) {
-          for (int i = 0; i < kSpins && !mbar_try(full + (k % slots) * 8, (k / slots) & 1); ++i) {
-          }
-        }
-      }
+      if (!ok || *failed != 0) drain_copies(full, issued, slots);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -272,11 +153,7 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
           if (!(ok = mbar_wait(bars.a_full + a_at.slot * 8, a_at.pass, failed))) break;
           fence_after_sync();
           const uint32_t a = tmem + a_at.slot * Roles<SPLIT>::kTileColumns;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            mma_ts(d, a + k * 8, (k < 4 ? b0 : b1) + (k & 3) * 2, idesc, i > 0 || k > 0);
-            if constexpr (SPLIT) mma_ts(d, a + 64 + k * 8, (k < 4 ? b0 : b1) + (k & 3) * 2, idesc, true);
-          }
+          mma_chunk<SPLIT>(d, a, b0, b1, idesc, i > 0);
           mma_commit(bars.a_empty + a_at.slot * 8);
           a_at.advance(kGroups);
           mma_commit(bars.x_empty + xs * 8);
@@ -284,11 +161,7 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
         }
         if (ok) mma_commit(bars.d_full + buffer * 8);
       }
-      if (*failed != 0) {  // MMAs in flight read and write tensor memory: it is freed after them
-        mma_commit(bars.drain);
-        for (int i = 0; i < kSpins && !mbar_try(bars.drain, 0); ++i) {
-        }
-      }
+      if (*failed != 0) drain_mma(bars);
     }
     __syncwarp();
   } else if (warp >= kDecodeWarp0) {
@@ -296,6 +169,7 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
     const int warp4 = warp & 3;
     const int r = warp4 * 32 + lane;
     const int stages = c1 - c0;
+    const WeightRing ring = {w_ring, p.w_slots, p.w_bytes};
     uint32_t stage = 0;
     uint32_t a_pass = 0;
     Cursor w_at, d_at;
@@ -304,7 +178,7 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
       int local;
       const Job& job = p.job[job_of(tile % p.row_tiles, local)];
       bool ok;
-#define DQ_DECODE(B) ok = decode_tile<B, BF16, MBF16, SPLIT>(job, p, local * 128, c0, group, stage, stages, w_ring, bars, tmem, w_at, a_pass, failed)
+#define DQ_DECODE(B) ok = decode_tile<B, BF16, MBF16, SPLIT>(job.meta, min(local * 128 + r, job.rows - 1), r, c0, group, stage, stages, ring, bars, tmem, w_at, a_pass, failed)
       switch (job.bits) {
         case 2: DQ_DECODE(2); break;
         case 3: DQ_DECODE(3); break;
@@ -385,39 +259,6 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
 constexpr uint32_t kBarrierOffset = 64;
 constexpr uint32_t kRingOffset = 1024;
 
-bool encode_map(CUtensorMap* map, CUtensorMapDataType type, const void* base, int64_t inner, int64_t outer, int64_t row_bytes,
-                int box_inner, int box_outer, CUtensorMapSwizzle swizzle) {
-  static const auto encode = [] {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult found;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) != cudaSuccess ||
-        found != cudaDriverEntryPointSuccess) {
-      fn = nullptr;
-    }
-    return reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(fn);
-  }();
-  if (encode == nullptr) return false;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(inner), static_cast<cuuint64_t>(outer)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_bytes)};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_inner), static_cast<cuuint32_t>(box_outer)};
-  const cuuint32_t step[2] = {1, 1};
-  return encode(map, type, 2, const_cast<void*>(base), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
-                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-CUtensorMapSwizzle weight_swizzle(int bits) {
-  return bits == 2 ? CU_TENSOR_MAP_SWIZZLE_32B : bits == 3 ? CU_TENSOR_MAP_SWIZZLE_NONE : bits == 4 ? CU_TENSOR_MAP_SWIZZLE_64B
-                                                                                                     : CU_TENSOR_MAP_SWIZZLE_128B;
-}
-
-// 64 << shift values per group, or -1.
-int group_shift_of(int group_values) {
-  for (int s = 0; s < 16; ++s) {
-    if (group_values == (64 << s)) return s;
-  }
-  return -1;
-}
-
 bool geometry_ok(const GemvArgs& a, int bits) {
   const bool x16 = a.x_dtype == DQ_BF16 || a.x_dtype == DQ_F16, meta16 = a.meta_dtype == DQ_BF16 || a.meta_dtype == DQ_F16;
   if (!x16 || !meta16 || a.out_dtype != a.x_dtype || a.in_features % 8 != 0 || group_shift_of(a.group_values) < 0) return false;
@@ -477,15 +318,12 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
                     4 * bits[i], 128, weight_swizzle(bits[i]))) {
       return DQ_OK;
     }
-    job.scales = b.scales;
-    job.offsets = b.offsets;
+    job.meta = {b.scales, b.offsets, b.num_groups, group_shift_of(b.group_values)};
     job.col0 = b.out_col0;
     job.bias = b.bias == nullptr ? nullptr : static_cast<const unsigned short*>(b.bias) + b.out_col0;
     job.rows = b.rows;
     job.row_tiles = static_cast<int>(ceil_div(b.rows, 128));
     job.bits = bits[i];
-    job.num_groups = b.num_groups;
-    job.group_shift = group_shift_of(b.group_values);
     p.row_tiles += job.row_tiles;
     w_bytes = std::max(w_bytes, 2048 * bits[i]);
   }
@@ -564,9 +402,10 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
 
 extern "C" int32_t dq_gemm_status(void* stream) {
   auto s = static_cast<cudaStream_t>(stream);
-  unsigned int word = 0;
+  unsigned int word = 0, moe = 0;
+  DQ_CUDA(dq::moe_gemm_failed(&moe, s));
   DQ_CUDA(cudaMemcpyFromSymbolAsync(&word, dq::g_gemm_failed, sizeof(word), 0, cudaMemcpyDeviceToHost, s));
   DQ_CUDA(cudaStreamSynchronize(s));
-  if (word != 0u) return dq::fail(DQ_ERR_DEVICE, "gemm: a wait inside a block ran out; an output of this device is incomplete");
+  if ((word | moe) != 0u) return dq::fail(DQ_ERR_DEVICE, "gemm: a wait inside a block ran out; an output of this device is incomplete");
   return DQ_OK;
 }

@@ -233,6 +233,79 @@ PyObject* py_fused(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return multiply(x, w.data(), count, *q, args[5]);
 }
 
+// A bank of packed rows, 2-D or [experts, rows, cols].
+bool bank_of(PyObject* const* args, int64_t bits, int64_t group_size, int64_t k, int64_t rows, const at::Tensor** q, dq_weight* w) {
+  *q = tensor(args[0]);
+  const at::Tensor *s = tensor(args[1]), *o = nullptr;
+  if (!packed_buffers(*q, s, args[2], &o)) return false;
+  Shard p = {};
+  p.bits = bits, p.in_features = k, p.rows = rows;
+  if (!row_shape(bits, group_size, k, &p.group_values, &p.num_groups, &p.words_per_row)) return false;
+  if ((*q)->numel() != rows * p.words_per_row || s->numel() != rows * p.num_groups || (*q)->size(-1) != p.words_per_row) return false;
+  *w = weight_of(**q, *s, o, p);
+  return true;
+}
+
+// moe(x, ids, weights, w13 packed, scales, offsets, w2 packed, scales, offsets, (experts, hidden, inter), bits13, bits2, group_size)
+PyObject* py_moe(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  constexpr int64_t kMaxChunk = 4096;  // tokens per call: bounds the scratch
+  if (n != 13 || !plain_context() || !PyTuple_Check(args[9]) || PyTuple_GET_SIZE(args[9]) != 3) return unhandled();
+  const at::Tensor *x = activation(args[0]), *ids = tensor(args[1]), *weights = tensor(args[2]);
+  if (x == nullptr || ids == nullptr || weights == nullptr || x->scalar_type() == at::kFloat || x->numel() == 0) return unhandled();
+  const int64_t experts = PyLong_AsLongLong(PyTuple_GET_ITEM(args[9], 0)), hidden = PyLong_AsLongLong(PyTuple_GET_ITEM(args[9], 1)),
+                inter = PyLong_AsLongLong(PyTuple_GET_ITEM(args[9], 2)), bits13 = PyLong_AsLongLong(args[10]),
+                bits2 = PyLong_AsLongLong(args[11]), group_size = PyLong_AsLongLong(args[12]);
+  if (PyErr_Occurred()) {
+    PyErr_Clear();
+    return unhandled();
+  }
+  const at::Tensor *q13, *q2;
+  dq_weight w13, w2;
+  if (!bank_of(args + 3, bits13, group_size, hidden, experts * 2 * inter, &q13, &w13) ||
+      !bank_of(args + 6, bits2, group_size, inter, experts * hidden, &q2, &w2)) {
+    return unhandled();
+  }
+  const at::Device device = q13->device();
+  const int64_t tokens = x->size(-1) == hidden ? x->numel() / hidden : 0;
+  if (tokens == 0 || ids->numel() % tokens != 0 || ids->numel() == 0 || weights->numel() != ids->numel() || x->device() != device ||
+      q2->device() != device || ids->device() != device || weights->device() != device) {
+    return unhandled();
+  }
+  const int64_t topk = ids->numel() / tokens;
+  const int tag = tag_of(x->scalar_type());
+  return on_device(device, [&](cudaStream_t stream) {
+    const at::Tensor flat = x->is_contiguous() ? *x : x->contiguous();
+    at::Tensor id = ids->scalar_type() == at::kInt ? *ids : ids->to(at::kInt);
+    at::Tensor p = weights->scalar_type() == at::kFloat ? *weights : weights->to(at::kFloat);
+    if (!id.is_contiguous()) id = id.contiguous();
+    if (!p.is_contiguous()) p = p.contiguous();
+    at::Tensor out = new_cuda(x->sizes(), x->scalar_type(), device);
+    const int64_t row = hidden * x->element_size();
+    const int64_t small = dq_moe_max_tokens();
+    bool wide = tokens > small;
+    at::Tensor scratch;
+    for (int64_t at = 0; at < tokens;) {
+      const int64_t count = std::min<int64_t>(tokens - at, wide ? kMaxChunk : small);
+      int64_t need = 0;
+      check(wide ? dq_moe_gemm_scratch_bytes(count, topk, hidden, inter, experts, tag, &need)
+                 : dq_moe_scratch_bytes(count, topk, hidden, inter, experts, tag, &need));
+      if (!scratch.defined() || scratch.numel() < need) scratch = new_cuda({need}, at::kByte, device);
+      const auto call = wide ? dq_moe_gemm : dq_moe_gemv_shard;
+      const int32_t rc = call(static_cast<const char*>(flat.const_data_ptr()) + at * row, tag, count,
+                              static_cast<const int32_t*>(id.const_data_ptr()) + at * topk, static_cast<const float*>(p.const_data_ptr()) + at * topk,
+                              topk, 0, experts, &w13, &w2, hidden, inter, static_cast<char*>(out.data_ptr()) + at * row, tag, scratch.data_ptr(),
+                              scratch.numel(), stream);
+      if (rc == DQ_ERR_UNSUPPORTED && wide) {
+        wide = false;
+        continue;
+      }
+      check(rc);
+      at += count;
+    }
+    return out;
+  });
+}
+
 // embedding(ids, packed, scales, offsets, bits, group_size, in_features)
 PyObject* py_embedding(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 7 || !plain_context()) return unhandled();
@@ -305,6 +378,7 @@ PyObject* py_encode(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyMethodDef kMethods[] = {
     {"matmul", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_matmul)), METH_FASTCALL, nullptr},
     {"fused", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_fused)), METH_FASTCALL, nullptr},
+    {"moe", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_moe)), METH_FASTCALL, nullptr},
     {"embedding", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_embedding)), METH_FASTCALL, nullptr},
     {"dequant", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_dequant)), METH_FASTCALL, nullptr},
     {"encode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_encode)), METH_FASTCALL, nullptr},

@@ -1,0 +1,211 @@
+// The pipeline that the tcgen05 kernels share: who does what in a block, the barriers between the
+// roles, the decoding warpgroups.
+//
+// Warp 0 brings activations (TMA), warp 2 packed weights (TMA), warp 1 issues the MMAs, warp 3 owns the
+// tensor memory, the warps from 4 on decode in warpgroups of four.  A weight tile is 128 rows x 128
+// values; a thread of a warpgroup owns one of its rows (the tensor memory lane that it may write).
+#pragma once
+
+#include "dq_umma_decode.cuh"
+
+namespace dq {
+namespace umma {
+
+#ifdef __CUDACC__
+
+constexpr int kDecodeWarp0 = 4;        // warps 0..3: TMA x, MMA, TMA weights, tensor memory
+// Decoding warpgroups and the operand tiles of 128 x 128 weights in tensor memory, one per warpgroup:
+// stage (chunk of 128 values of K) i belongs to warpgroup i % kGroups and always to its tile, so that
+// nobody can ever be two passes ahead of a tile's barrier.  Four groups and tiles of 64 columns, or
+// (every weight as two 16-bit pieces) three groups and tiles of 128.
+template <bool SPLIT>
+struct Roles {
+  static constexpr int kGroups = SPLIT ? 3 : 4, kTileColumns = SPLIT ? 128 : 64, kColumns = kGroups * kTileColumns;
+  static constexpr int kThreads = (kDecodeWarp0 + 4 * kGroups) * 32;
+};
+constexpr int kMaxGroups = 4;
+constexpr int kMaxRing = 16;
+
+
+struct Bars {
+  uint32_t x_full, x_empty, w_full, w_empty, a_full, a_empty, d_full, d_empty, drain;
+};
+
+// Where a role stands in a ring: a slot and the parity of its pass (run-time divisions would cost the
+// single-thread roles more than their work: 0.3 us per stage, measured).
+struct Cursor {
+  uint32_t slot = 0, pass = 0;
+  __device__ __forceinline__ void advance(uint32_t slots, uint32_t by = 1) {
+    slot += by;
+    if (slot >= slots) slot -= slots, pass ^= 1;  // (by <= slots)
+  }
+};
+
+// The metadata of a packed matrix, and the weight ring that its tiles pass through.
+struct Meta {
+  const void* scales;
+  const void* offsets;                 // may be null
+  int num_groups, group_shift;         // group = 64 << group_shift
+};
+struct WeightRing {
+  const unsigned char* tiles;
+  int slots, bytes;
+};
+
+// Warpgroup `group`'s chunks of a tile of 128 weight rows, `row` the one of this thread and `tile_row` its
+// place in the staged tile: chunk c0 + i is stage stage0 + i, numbered over the life of the block.  False
+// once a wait has run out.
+template <int BITS, bool BF16, bool MBF16, bool SPLIT>
+__device__ bool decode_tile(const Meta& meta, int64_t row, int tile_row, int c0, int group, uint32_t stage0, int stages, const WeightRing& ring,
+                            const Bars& bars, uint32_t tmem, Cursor& w_at, uint32_t& a_pass, volatile int* failed) {
+  constexpr int kGroups = Roles<SPLIT>::kGroups;
+  const int lane = threadIdx.x & 31;
+  const int warp4 = (threadIdx.x >> 5) & 3;
+  const unsigned short* s_row = static_cast<const unsigned short*>(meta.scales) + row * meta.num_groups;
+  const unsigned short* o_row =
+      meta.offsets == nullptr ? nullptr : static_cast<const unsigned short*>(meta.offsets) + row * meta.num_groups;
+  auto widen = [&](unsigned short v) -> float {
+    return MBF16 ? __uint_as_float(static_cast<uint32_t>(v) << 16) : __half2float(__ushort_as_half(v));
+  };
+  const bool two_groups = meta.group_shift == 0;  // 64-value groups: a chunk holds two
+  auto group_of = [&](int i, int half) -> int { return min((2 * (c0 + i) + half) >> meta.group_shift, meta.num_groups - 1); };
+  unsigned short s_next[2], o_next[2] = {0, 0};
+  auto fetch = [&](int i) {
+    const int g0 = group_of(i, 0);
+    s_next[0] = __ldg(s_row + g0);
+    if (o_row != nullptr) o_next[0] = __ldg(o_row + g0);
+    if (two_groups) {
+      const int g1 = group_of(i, 1);
+      s_next[1] = __ldg(s_row + g1);
+      if (o_row != nullptr) o_next[1] = __ldg(o_row + g1);
+    }
+  };
+  const int first = (group + kGroups - static_cast<int>(stage0 % kGroups)) % kGroups;
+  if (first >= stages) return true;
+  fetch(first);
+  for (int i = first; i < stages; i += kGroups) {
+    Affine<BITS, MBF16> affine;
+    affine.set(s_next[0], o_row != nullptr ? widen(o_next[0]) : 0.0f);
+    const unsigned short s_half = s_next[1], o_half = o_next[1];
+    fetch(min(i + kGroups, stages - 1));  // the next chunk's metadata travels while this one is decoded
+    const uint32_t slot = w_at.slot;
+    if (!mbar_wait(bars.w_full + slot * 8, w_at.pass, failed)) return false;
+    const uint32_t dst = tmem + group * Roles<SPLIT>::kTileColumns + (static_cast<uint32_t>(warp4 * 32) << 16);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      uint32_t w[2 * BITS], v[16], low[16];
+      read_row64<BITS>(ring.tiles + slot * ring.bytes, tile_row, half, w);
+      if (half == 1 && two_groups) affine.set(s_half, o_row != nullptr ? widen(o_half) : 0.0f);
+      decode32<BITS, BF16, MBF16, SPLIT>(w, affine, v, low);
+      if (half == 0) {  // the MMAs of this group's previous chunk are done with the tile
+        if (!mbar_wait(bars.a_empty + group * 8, a_pass ^ 1, failed)) return false;
+        fence_after_sync();
+      }
+      tmem_st16(dst + half * 32, v);
+      if constexpr (SPLIT) tmem_st16(dst + 64 + half * 32, low);
+      decode32<BITS, BF16, MBF16, SPLIT>(w + BITS, affine, v, low);
+      tmem_st16(dst + half * 32 + 16, v);
+      if constexpr (SPLIT) tmem_st16(dst + 64 + half * 32 + 16, low);
+    }
+    tmem_wait_st();
+    fence_before_sync();
+    __syncwarp();
+    if (lane == 0) {
+      mbar_arrive(bars.a_full + group * 8);
+      // Only now: an arrival may overtake shared-memory loads still in flight, and the slot is refilled
+      // at once.  By here every word has gone through the decode.
+      mbar_arrive(bars.w_empty + slot * 8);
+    }
+    w_at.advance(static_cast<uint32_t>(ring.slots), kGroups);
+    a_pass ^= 1;
+  }
+  return true;
+}
+
+// Barriers from `at` on (shared memory).
+constexpr uint32_t kBarrierBytes = (4 * kMaxRing + 2 * kMaxGroups + 5) * 8;
+__device__ __forceinline__ Bars bars_at(uint32_t at) {
+  Bars b;
+  b.x_full = at;
+  b.x_empty = b.x_full + kMaxRing * 8;
+  b.w_full = b.x_empty + kMaxRing * 8;
+  b.w_empty = b.w_full + kMaxRing * 8;
+  b.a_full = b.w_empty + kMaxRing * 8;
+  b.a_empty = b.a_full + kMaxGroups * 8;
+  b.d_full = b.a_empty + kMaxGroups * 8;
+  b.d_empty = b.d_full + 2 * 8;
+  b.drain = b.d_empty + 2 * 8;
+  return b;
+}
+__device__ __forceinline__ void init_bars(const Bars& b, int x_slots, int w_slots, int groups) {
+  for (int i = 0; i < x_slots; ++i) mbar_init(b.x_full + i * 8, 1), mbar_init(b.x_empty + i * 8, 1);
+  for (int i = 0; i < w_slots; ++i) mbar_init(b.w_full + i * 8, 1), mbar_init(b.w_empty + i * 8, 4);
+  for (int i = 0; i < groups; ++i) mbar_init(b.a_full + i * 8, 4), mbar_init(b.a_empty + i * 8, 1);
+  for (int i = 0; i < 2; ++i) mbar_init(b.d_full + i * 8, 1), mbar_init(b.d_empty + i * 8, 4 * static_cast<uint32_t>(groups));
+  mbar_init(b.drain, 1);
+  fence_mbar_init();
+}
+
+// One chunk's MMAs: eight steps of 16 values, the operand tile at `a`, the two activation slabs of 64
+// values at b0 and b1.
+template <bool SPLIT>
+__device__ __forceinline__ void mma_chunk(uint32_t d, uint32_t a, uint64_t b0, uint64_t b1, uint32_t idesc, bool accumulate) {
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    mma_ts(d, a + k * 8, (k < 4 ? b0 : b1) + (k & 3) * 2, idesc, accumulate || k > 0);
+    if constexpr (SPLIT) mma_ts(d, a + 64 + k * 8, (k < 4 ? b0 : b1) + (k & 3) * 2, idesc, true);
+  }
+}
+
+// A producer that gives up waits for its copies in flight ...
+__device__ __forceinline__ void drain_copies(uint32_t full, uint32_t issued, uint32_t slots) {
+  for (uint32_t k = issued > slots ? issued - slots : 0; k < issued; ++k) {
+    for (int i = 0; i < kSpins && !mbar_try(full + (k % slots) * 8, (k / slots) & 1); ++i) {
+    }
+  }
+}
+// ... and the MMA warp for its MMAs, which read and write tensor memory that is about to be freed.
+__device__ __forceinline__ void drain_mma(const Bars& bars) {
+  mma_commit(bars.drain);
+  for (int i = 0; i < kSpins && !mbar_try(bars.drain, 0); ++i) {
+  }
+}
+
+#endif  // __CUDACC__
+
+// ---- host -------------------------------------------------------------------
+inline bool encode_map(CUtensorMap* map, CUtensorMapDataType type, const void* base, int64_t inner, int64_t outer, int64_t row_bytes,
+                int box_inner, int box_outer, CUtensorMapSwizzle swizzle) {
+  static const auto encode = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      fn = nullptr;
+    }
+    return reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(fn);
+  }();
+  if (encode == nullptr) return false;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(inner), static_cast<cuuint64_t>(outer)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_bytes)};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_inner), static_cast<cuuint32_t>(box_outer)};
+  const cuuint32_t step[2] = {1, 1};
+  return encode(map, type, 2, const_cast<void*>(base), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+inline CUtensorMapSwizzle weight_swizzle(int bits) {
+  return bits == 2 ? CU_TENSOR_MAP_SWIZZLE_32B : bits == 3 ? CU_TENSOR_MAP_SWIZZLE_NONE : bits == 4 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                                                                                     : CU_TENSOR_MAP_SWIZZLE_128B;
+}
+
+// 64 << shift values per group, or -1.
+inline int group_shift_of(int group_values) {
+  for (int s = 0; s < 16; ++s) {
+    if (group_values == (64 << s)) return s;
+  }
+  return -1;
+}
+
+}  // namespace umma
+}  // namespace dq

@@ -339,6 +339,14 @@ class DynQuantMoEMethod:
               topk_ids: torch.Tensor, **_: Any) -> torch.Tensor:
         """``topk_weights`` are used as given (renormalise in the router if the model does)."""
         num_experts, hidden, inter = layer.dynquant_moe
+        if ops._host is not None and not torch.compiler.is_compiling():
+            params = getattr(layer, "_layer", layer)._parameters  # (a wrapped layer's banks may be 3-D: the same rows)
+            get = params.get
+            out = ops._host.moe(x, topk_ids, topk_weights, get("w13_qweight"), get("w13_scales"), get("w13_offsets"),
+                                get("w2_qweight"), get("w2_scales"), get("w2_offsets"), layer.dynquant_moe, self.bits_gate_up,
+                                self.bits_down, self.group_size)
+            if out is not None:
+                return out
         gate_up = self._bank(layer, "w13", self.bits_gate_up, hidden)
         down = self._bank(layer, "w2", self.bits_down, inter)
         lead = x.shape[:-1]

@@ -104,7 +104,7 @@ DQ_API int64_t dq_launch_count(void);
  * ("gemv_mma_stream_kernel", "gemv_mma_stream_multi_kernel", "gemv_mma_stream_sliced_kernel", "gemv_mma_tile_kernel",
  * "gemv_mma_kernel", "gemv_fast_kernel",
  * "gemv_general_kernel", "gemv_plan_kernel", "gemv_rows_kernel", "moe_grouped_kernel", "moe_combine_kernel",
- * "moe_down_token_kernel", "gemm_umma_kernel"; "" before the first launch).  No reference
+ * "moe_down_token_kernel", "gemm_umma_kernel", "moe_umma_kernel"; "" before the first launch).  No reference
  * counterpart: the reference has two kernels and a documented rule between them
  * (csrc/gemv/gemv.cu:566-598); here a test uses this to prove which kernel it exercised. */
 DQ_API const char* dq_last_kernel(void);
@@ -317,6 +317,16 @@ DQ_API int32_t dq_moe_gemv_shard(const void* x, int32_t x_dtype, int64_t tokens,
                                  int64_t num_experts, const dq_weight* gate_up, const dq_weight* down,
                                  int64_t hidden, int64_t inter, void* y, int32_t y_dtype, void* scratch,
                                  int64_t scratch_bytes, void* stream);
+/* The same layer for any number of tokens (prefill), on the tcgen05 tensor cores: the assignments
+ * sorted by expert on the device, every active expert's weights decoded once per 128 of its tokens,
+ * unrounded as in dq_moe_gemv.  Sizes and alignment as there, plus hidden % 8 == 0, inter % 8 == 0, at
+ * most 1024 experts and 16-byte aligned x and y (else DQ_ERR_UNSUPPORTED, nothing launched). */
+DQ_API int32_t dq_moe_gemm_scratch_bytes(int64_t tokens, int64_t topk, int64_t hidden, int64_t inter,
+                                         int64_t num_experts, int32_t act_dtype, int64_t* bytes);
+DQ_API int32_t dq_moe_gemm(const void* x, int32_t x_dtype, int64_t tokens, const int32_t* topk_ids,
+                           const float* topk_w, int64_t topk, int64_t first_expert, int64_t num_experts,
+                           const dq_weight* gate_up, const dq_weight* down, int64_t hidden, int64_t inter,
+                           void* y, int32_t y_dtype, void* scratch, int64_t scratch_bytes, void* stream);
 /* dq_moe_gemv without a scratch argument and without any allocation.  This entry point has
  * no counterpart in the reference.
  *
