@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
 
   if (threadIdx.x == 0) {
     *failed = 0;
-    init_bars(bars, p.x_slots, p.w_slots, kGroups);
+    init_bars(bars, p.x_slots, p.w_slots, kGroups, 4 * kGroups);
     tma_prefetch_map(&p.xmap);
   }
   if (warp == 3) tmem_alloc(base + 4, static_cast<uint32_t>(p.tmem_columns));

@@ -33,7 +33,15 @@ using namespace umma;
 constexpr int kRouteThreads = 1024;
 constexpr int kMaxExperts = 1024;
 constexpr int kGroups = Roles<true>::kGroups;
-constexpr int kThreads = Roles<true>::kThreads;
+// Four warps more than the dense kernel: a tile is only 6 to 16 chunks long, so warps of their own finish
+// it while the decoding warps work on the next (down, 6 chunks of 0.5 us per tile: 143 us per layer of
+// 1000 tokens with the decoding warps doing it).
+constexpr int kEpilogueWarp0 = kDecodeWarp0 + 4 * kGroups;
+constexpr int kThreads = (kEpilogueWarp0 + 4) * 32;
+// Activations come in boxes of 32 rows, as many as a tile has tokens for: 128 rows for every tile of 62
+// tokens were 4.5 TB/s out of L2 (1000 tokens: gate_up 168 us).
+constexpr int kBoxRows = 32;
+constexpr int kColumns = 128;          // accumulator columns: one tile of up to 128 tokens, or two of up to 64
 
 __device__ unsigned int g_moe_failed = 0;
 
@@ -117,11 +125,31 @@ struct Params {
   int rows;                  // output rows per expert (inter, or hidden)
   int row_blocks;            // of 64 (gate_up) or 128 (down) rows per expert
   int chunks, bits;
-  int n_cap, d_buffers, tmem_columns;
+  int n_cap;
   int x_slots, w_slots, w_bytes;
 };
 
-constexpr uint32_t kBarrierOffset = 64, kRingOffset = 1024;
+constexpr uint32_t kBarrierOffset = 64, kOrderOffset = 1024, kRingOffset = 3072;
+static_assert(kBarrierOffset + kBarrierBytes <= kOrderOffset, "");
+
+// Where a tile's accumulator lies.  Tiles of up to 64 tokens take the two halves of the columns in turn
+// (the MMAs of one run under the epilogue of the other), a larger one takes both; every role walks the
+// same sequence.
+struct Halves {
+  uint32_t at = 0, passes = 0;  // passes: a parity bit per half
+  bool both = false;
+  __device__ __forceinline__ void take(int tokens) {
+    both = tokens > 64;
+    if (both) at = 0;
+  }
+  __device__ __forceinline__ bool wait(uint32_t bars, uint32_t flip, volatile int* failed) const {
+    return mbar_wait(bars + at * 8, ((passes >> at) & 1) ^ flip, failed) && (!both || mbar_wait(bars + 8, (passes >> 1) ^ flip, failed));
+  }
+  __device__ __forceinline__ void done() {
+    passes ^= both ? 3u : 1u << at;
+    if (!both) at ^= 1;
+  }
+};
 
 template <bool BF16, bool MBF16, bool GATE_UP>
 __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_constant__ Params p) {
@@ -136,11 +164,11 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
 
   if (threadIdx.x == 0) {
     *failed = 0;
-    init_bars(bars, p.x_slots, p.w_slots, kGroups);
+    init_bars(bars, p.x_slots, p.w_slots, kGroups, 4);
     tma_prefetch_map(&p.xmap);
     tma_prefetch_map(&p.wmap);
   }
-  if (warp == 3) tmem_alloc(base + 4, static_cast<uint32_t>(p.tmem_columns));
+  if (warp == 3) tmem_alloc(base + 4, 512);
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
@@ -158,7 +186,6 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
       const bool weights = warp == 2;
       const uint32_t full = weights ? bars.w_full : bars.x_full, empty = weights ? bars.w_empty : bars.x_empty;
       const uint32_t slots = static_cast<uint32_t>(weights ? p.w_slots : p.x_slots);
-      const uint32_t bytes = static_cast<uint32_t>(weights ? 2048 * p.bits : x_bytes);
       Cursor at;
       uint32_t issued = 0;
       bool ok = true;
@@ -167,6 +194,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
         const int4 e = next;
         next = entry(tile + gridDim.x);
         const int block = tile % p.row_blocks;
+        const int boxes = (e.z + kBoxRows - 1) / kBoxRows;  // of activation rows, per slab of 64 values
+        const uint32_t bytes = static_cast<uint32_t>(weights ? 2048 * p.bits : boxes * kBoxRows * 256);
         const int w_row = GATE_UP ? e.x * 2 * p.rows + block * 64 : e.x * p.rows + block * 128;
         for (int i = 0; i < p.chunks; ++i, ++issued, at.advance(slots)) {
           const uint32_t slot = at.slot;
@@ -178,8 +207,10 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
             if (GATE_UP) tma_load_2d(dst + 1024 * p.bits, &p.wmap, i * 4 * p.bits, w_row + p.rows, full + slot * 8);
           } else {
             const uint32_t dst = smem_addr(x_ring) + slot * x_bytes;
-            tma_load_2d(dst, &p.xmap, i * 128, e.y, full + slot * 8);
-            tma_load_2d(dst + x_bytes / 2, &p.xmap, i * 128 + 64, e.y, full + slot * 8);
+            for (int b = 0; b < boxes; ++b) {
+              tma_load_2d(dst + b * (kBoxRows * 128), &p.xmap, i * 128, e.y + b * kBoxRows, full + slot * 8);
+              tma_load_2d(dst + x_bytes / 2 + b * (kBoxRows * 128), &p.xmap, i * 128 + 64, e.y + b * kBoxRows, full + slot * 8);
+            }
           }
         }
       }
@@ -188,16 +219,18 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
     __syncwarp();
   } else if (warp == 1) {
     if (elect_one()) {
-      Cursor x_at, a_at, d_at;
+      Cursor x_at, a_at;
+      Halves halves;
       bool ok = true;
       int4 next = entry(blockIdx.x);
-      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, d_at.advance(static_cast<uint32_t>(p.d_buffers))) {
+      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, halves.done()) {
         const int4 e = next;
         next = entry(tile + gridDim.x);
         const uint32_t idesc = mma_descriptor(BF16, (e.z + 15) / 16 * 16);
-        if (!mbar_wait(bars.d_empty + d_at.slot * 8, d_at.pass ^ 1, failed)) break;
+        halves.take(e.z);
+        if (!halves.wait(bars.d_empty, 1, failed)) break;
         fence_after_sync();
-        const uint32_t d = d_tmem + d_at.slot * p.n_cap;
+        const uint32_t d = d_tmem + halves.at * 64;
         for (int i = 0; i < p.chunks; ++i) {
           const uint32_t xs = x_at.slot;
           if (!(ok = mbar_wait(bars.x_full + xs * 8, x_at.pass, failed))) break;
@@ -210,76 +243,99 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
           x_at.advance(static_cast<uint32_t>(p.x_slots));
           a_at.advance(kGroups);
         }
-        if (ok) mma_commit(bars.d_full + d_at.slot * 8);
+        if (ok) {
+          mma_commit(bars.d_full + halves.at * 8);
+          if (halves.both) mma_commit(bars.d_full + 8);
+        }
       }
       if (*failed != 0) drain_mma(bars);
     }
     __syncwarp();
   } else if (warp >= kDecodeWarp0) {
-    const int group = (warp - kDecodeWarp0) >> 2, warp4 = warp & 3;
-    const int r = warp4 * 32 + lane;
-    const WeightRing ring = {w_ring, p.w_slots, p.w_bytes};
-    uint32_t stage = 0, a_pass = 0;
-    Cursor w_at, d_at;
-    w_at.advance(static_cast<uint32_t>(p.w_slots), static_cast<uint32_t>(group));
+    // The rows of a warp's 32 lanes: for gate_up 16 gate rows and the matching 16 up rows.
+    const int warp4 = warp & 3, pair = warp4 * 16 + (lane & 15);
+    const int tile_row = GATE_UP ? (lane < 16 ? 0 : 64) + pair : warp4 * 32 + lane;
     int4 next = entry(blockIdx.x);
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, d_at.advance(static_cast<uint32_t>(p.d_buffers)), stage += p.chunks) {
-      const int4 e = next;
-      next = entry(tile + gridDim.x);
-      const int block = tile % p.row_blocks;
-      const int pair = warp4 * 16 + (lane & 15);
-      const int row = GATE_UP ? block * 64 + pair : block * 128 + r;  // of the expert's (gate, up or down) rows
-      const int64_t bank = GATE_UP ? static_cast<int64_t>(e.x) * 2 * p.rows + (lane < 16 ? 0 : p.rows) + row : static_cast<int64_t>(e.x) * p.rows + row;
-      const int tile_row = GATE_UP ? (lane < 16 ? 0 : 64) + pair : r;
-      const int64_t bank_row = bank < p.bank_rows ? bank : p.bank_rows - 1;
-      bool ok;
-#define DQ_DECODE(B) ok = decode_tile<B, BF16, MBF16, true>(p.meta, bank_row, tile_row, 0, group, stage, p.chunks, ring, bars, tmem, w_at, a_pass, failed)
-      switch (p.bits) {
-        case 2: DQ_DECODE(2); break;
-        case 3: DQ_DECODE(3); break;
-        case 4: DQ_DECODE(4); break;
-        default: DQ_DECODE(8); break;
-      }
+    if (warp < kEpilogueWarp0) {
+      const int group = (warp - kDecodeWarp0) >> 2;
+      const WeightRing ring = {w_ring, p.w_slots, p.w_bytes};
+      uint32_t stage = 0, a_pass = 0;
+      Cursor w_at;
+      w_at.advance(static_cast<uint32_t>(p.w_slots), static_cast<uint32_t>(group));
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, stage += p.chunks) {
+        const int4 e = next;
+        next = entry(tile + gridDim.x);
+        const int block = tile % p.row_blocks;
+        const int64_t bank = GATE_UP ? static_cast<int64_t>(e.x) * 2 * p.rows + (lane < 16 ? 0 : p.rows) + block * 64 + pair
+                                     : static_cast<int64_t>(e.x) * p.rows + block * 128 + tile_row;
+        const int64_t bank_row = bank < p.bank_rows ? bank : p.bank_rows - 1;
+#define DQ_DECODE(B) \
+  ok = decode_tile<B, BF16, MBF16, true>(p.meta, bank_row, tile_row, 0, group, stage, p.chunks, ring, bars, tmem, w_at, a_pass, failed)
+        switch (p.bits) {
+          case 2: DQ_DECODE(2); break;
+          case 3: DQ_DECODE(3); break;
+          case 4: DQ_DECODE(4); break;
+          default: DQ_DECODE(8); break;
+        }
 #undef DQ_DECODE
-      if (!ok) break;
-      if (!mbar_wait(bars.d_full + d_at.slot * 8, d_at.pass, failed)) break;
-      fence_after_sync();
-      const uint32_t src = d_tmem + d_at.slot * p.n_cap + (static_cast<uint32_t>(warp4 * 32) << 16);
-      for (int col = group * 16; col < e.z; col += kGroups * 16) {  // the warpgroups share the columns
-        uint32_t v[16];
-        tmem_ld16(src + col, v);
-        tmem_wait_ld();
-        if constexpr (GATE_UP) {
-          // lane l < 16 has gate row l, lane l + 16 the matching up row: each finishes eight of the columns
-          const int first = col + (lane < 16 ? 0 : 8);
-          unsigned short* dst = static_cast<unsigned short*>(p.out) + static_cast<int64_t>(e.y + first) * p.rows + row;
+      }
+    } else {
+      int* places = reinterpret_cast<int*>(smem + kOrderOffset) + warp4 * kColumns;  // this warp's copy of the tile's assignments
+      Halves halves;
+      for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, halves.done()) {
+        const int4 e = next;
+        next = entry(tile + gridDim.x);
+        const int block = tile % p.row_blocks;
+        const int row = GATE_UP ? block * 64 + pair : block * 128 + tile_row;  // of the expert's output rows
+        if (!GATE_UP) {
+          __syncwarp();
+          for (int c = lane; c < e.z; c += 32) places[c] = __ldcg(p.order + e.y + c);
+          __syncwarp();
+        }
+        halves.take(e.z);
+        if (!halves.wait(bars.d_full, 0, failed)) break;
+        fence_after_sync();
+        const uint32_t src = d_tmem + halves.at * 64 + (static_cast<uint32_t>(warp4 * 32) << 16);
+        for (int col = 0; col < e.z; col += 16) {
+          uint32_t v[16];
+          tmem_ld16(src + col, v);
+          tmem_wait_ld();
+          if constexpr (GATE_UP) {
+            // lane l < 16 has gate row l, lane l + 16 the matching up row: each finishes eight of the columns
+            const int first = col + (lane < 16 ? 0 : 8);
+            unsigned short* dst = static_cast<unsigned short*>(p.out) + static_cast<int64_t>(e.y + first) * p.rows + row;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float other = __uint_as_float(__shfl_xor_sync(0xffffffffu, lane < 16 ? v[i + 8] : v[i], 16));
-            const float g = lane < 16 ? __uint_as_float(v[i]) : other, u = lane < 16 ? other : __uint_as_float(v[i + 8]);
-            if (row < p.rows && first + i < e.z) {
-              dst[static_cast<int64_t>(i) * p.rows] =
-                  static_cast<unsigned short>(round_to_16((g / (1.0f + __expf(-g))) * u, BF16 ? DQ_BF16 : DQ_F16));
+            for (int i = 0; i < 8; ++i) {
+              const float other = __uint_as_float(__shfl_xor_sync(0xffffffffu, lane < 16 ? v[i + 8] : v[i], 16));
+              const float g = lane < 16 ? __uint_as_float(v[i]) : other, u = lane < 16 ? other : __uint_as_float(v[i + 8]);
+              if (row < p.rows && first + i < e.z) {
+                dst[static_cast<int64_t>(i) * p.rows] =
+                    static_cast<unsigned short>(round_to_16((g / (1.0f + __expf(-g))) * u, BF16 ? DQ_BF16 : DQ_F16));
+              }
+            }
+          } else if (row < p.rows) {
+            float* dst = static_cast<float*>(p.out) + row;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              if (col + i < e.z) dst[static_cast<int64_t>(places[col + i]) * p.rows] = __uint_as_float(v[i]);
             }
           }
-        } else if (row < p.rows) {
-          float* dst = static_cast<float*>(p.out) + row;
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            if (col + i < e.z) dst[static_cast<int64_t>(__ldcg(p.order + e.y + col + i)) * p.rows] = __uint_as_float(v[i]);
-          }
+        }
+        fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(bars.d_empty + halves.at * 8);
+          if (halves.both) mbar_arrive(bars.d_empty + 8);
         }
       }
-      fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bars.d_empty + d_at.slot * 8);
     }
   }
 
   __syncthreads();
   if (threadIdx.x == 0 && *failed != 0) atomicOr(&g_moe_failed, 1u);
   fence_after_sync();
-  if (warp == 3) tmem_free(tmem, static_cast<uint32_t>(p.tmem_columns));
+  if (warp == 3) tmem_free(tmem, 512);
 }
 
 __global__ void __launch_bounds__(256) moe_combine_rows_kernel(const float4* d, const float* w, const int32_t* ids, int first_expert,
@@ -358,12 +414,9 @@ int32_t launch_bank(const dq_weight& w, const dq_geometry& g, const void* act, i
   if (!encode_map(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_INT32, w.packed, g.words_per_row, w.rows, static_cast<int64_t>(g.words_per_row) * 4, 4 * w.bits,
                   GATE_UP ? 64 : 128, weight_swizzle(w.bits)) ||
       !encode_map(&p.xmap, act_dtype == DQ_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, act, g.in_features, act_rows,
-                  static_cast<int64_t>(g.in_features) * 2, 64, p.n_cap, CU_TENSOR_MAP_SWIZZLE_128B)) {
+                  static_cast<int64_t>(g.in_features) * 2, 64, kBoxRows, CU_TENSOR_MAP_SWIZZLE_128B)) {
     return fail(DQ_ERR_CUDA, "moe_gemm: a tensor map could not be encoded");
   }
-  // tensor memory: the operand tiles, then one accumulator tile of n_cap columns, or two where they fit
-  p.d_buffers = Roles<true>::kColumns + 2 * p.n_cap <= 512 ? 2 : 1;
-  p.tmem_columns = 512;
   const int x_bytes = p.n_cap * 256, budget = dev.max_smem_optin - static_cast<int>(kRingOffset);
   p.x_slots = std::clamp((budget - kGroups * p.w_bytes) / x_bytes, 2, 4);
   p.w_slots = std::clamp((budget - p.x_slots * x_bytes) / p.w_bytes / kGroups * kGroups, kGroups, 12);
@@ -432,10 +485,10 @@ int32_t dq_moe_gemm(const void* x, int32_t x_dtype, int64_t tokens, const int32_
   auto* table = reinterpret_cast<dq::RouteTable*>(base + lay.table);
   auto* tiles = reinterpret_cast<int4*>(base + lay.tiles);
   auto* order = reinterpret_cast<int32_t*>(base + lay.order);
-  // Columns of a tile: 64 (two accumulator tiles then fit) where hardly an expert has more tokens than
+  // Columns of a tile (and rows of an activation slot): 64 where hardly an expert has more tokens than
   // that, else 128, so that an expert's weights are decoded once.
   const double mean = static_cast<double>(assignments) / experts;
-  const int n_cap = mean + 3.0 * std::sqrt(mean) <= 64.0 ? 64 : 128;
+  const int n_cap = mean + 3.0 * std::sqrt(mean) <= 64.0 ? 64 : dq::kColumns;
   if (const int32_t rc = dq::launch(dq::moe_route_kernel, dim3(1), dq::kRouteThreads, 0, s, "moe_gemm(route)", topk_ids, first, experts,
                                     assignments, n_cap, table, tiles, order)) {
     return rc;

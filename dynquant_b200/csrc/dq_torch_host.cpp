@@ -21,7 +21,10 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 
+#include <algorithm>
 #include <array>
+#include <cmath>
+#include <cstring>
 #include <optional>
 
 #include "dynquant_b200.h"
@@ -246,6 +249,19 @@ bool bank_of(PyObject* const* args, int64_t bits, int64_t group_size, int64_t k,
   return true;
 }
 
+// Whether `tokens` go through dq_moe_gemm: when dq_moe_gemv, which reads an expert's weights once per eight
+// of its tokens and call of at most `small` tokens, would make two mean passes over the experts or more --
+// one pass of dq_moe_gemm costs about as much (128 experts, top-8: 100 / 128 / 256 tokens 198 / 217 / 437 us
+// against 200 / 200 / 205; 8 experts, top-4: 16 / 32 tokens 32 / 50 us against 33 / 34).
+bool moe_is_wide(int64_t tokens, int64_t topk, int64_t experts, int64_t small) {
+  double passes = 0.0;
+  for (int64_t at = 0; at < tokens && passes < 2.0; at += small) {
+    const double mean = static_cast<double>(std::min(tokens - at, small) * topk) / static_cast<double>(experts);
+    passes += std::max(1.0 - std::exp(-mean), mean > 1.0 ? mean / 8.0 + 0.5 : 0.0);  // (the experts with a token at least)
+  }
+  return passes >= 1.95;
+}
+
 // moe(x, ids, weights, w13 packed, scales, offsets, w2 packed, scales, offsets, (experts, hidden, inter), bits13, bits2, group_size)
 PyObject* py_moe(PyObject*, PyObject* const* args, Py_ssize_t n) {
   constexpr int64_t kMaxChunk = 4096;  // tokens per call: bounds the scratch
@@ -282,7 +298,7 @@ PyObject* py_moe(PyObject*, PyObject* const* args, Py_ssize_t n) {
     at::Tensor out = new_cuda(x->sizes(), x->scalar_type(), device);
     const int64_t row = hidden * x->element_size();
     const int64_t small = dq_moe_max_tokens();
-    bool wide = tokens > small;
+    bool wide = moe_is_wide(tokens, topk, experts, small);
     at::Tensor scratch;
     for (int64_t at = 0; at < tokens;) {
       const int64_t count = std::min<int64_t>(tokens - at, wide ? kMaxChunk : small);

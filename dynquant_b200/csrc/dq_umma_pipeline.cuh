@@ -137,11 +137,11 @@ __device__ __forceinline__ Bars bars_at(uint32_t at) {
   b.drain = b.d_empty + 2 * 8;
   return b;
 }
-__device__ __forceinline__ void init_bars(const Bars& b, int x_slots, int w_slots, int groups) {
+__device__ __forceinline__ void init_bars(const Bars& b, int x_slots, int w_slots, int groups, int epilogue_warps) {
   for (int i = 0; i < x_slots; ++i) mbar_init(b.x_full + i * 8, 1), mbar_init(b.x_empty + i * 8, 1);
   for (int i = 0; i < w_slots; ++i) mbar_init(b.w_full + i * 8, 1), mbar_init(b.w_empty + i * 8, 4);
   for (int i = 0; i < groups; ++i) mbar_init(b.a_full + i * 8, 4), mbar_init(b.a_empty + i * 8, 1);
-  for (int i = 0; i < 2; ++i) mbar_init(b.d_full + i * 8, 1), mbar_init(b.d_empty + i * 8, 4 * static_cast<uint32_t>(groups));
+  for (int i = 0; i < 2; ++i) mbar_init(b.d_full + i * 8, 1), mbar_init(b.d_empty + i * 8, static_cast<uint32_t>(epilogue_warps));
   mbar_init(b.drain, 1);
   fence_mbar_init();
 }

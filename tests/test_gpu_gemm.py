@@ -71,3 +71,40 @@ def test_shards_of_mixed_widths_in_one_launch(m):
     want = torch.cat([torch.from_numpy(oracle_gemv(x, qt)) for qt in shards], dim=1) + bias.float().cpu()
     error = (got.float().cpu() - want).norm() / want.norm()
     assert error <= 4e-3
+
+
+@pytest.mark.parametrize(("tokens", "experts", "topk", "hidden", "inter", "widths", "act", "meta"), [
+    (1, 8, 2, 256, 192, (4, 3), torch.bfloat16, torch.float16),      # one token; 64-row blocks that end inside a tile
+    (64, 4, 2, 512, 128, (2, 8), torch.float16, torch.float16),      # tiles of 64 columns and fewer
+    (130, 2, 2, 384, 320, (8, 2), torch.bfloat16, torch.bfloat16),   # every expert has every token: 128 + 2 columns
+    (700, 16, 4, 1024, 512, (3, 4), torch.bfloat16, torch.float16),  # several tiles per block, small and large in turn
+])
+def test_an_expert_layer_over_many_tokens_matches_its_small_calls(tokens, experts, topk, hidden, inter, widths, act, meta):
+    import ctypes
+
+    from dynquant_b200 import _lib, ops
+    from dynquant_b200.workloads import random_quant_tensor, seeded_routing
+
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    gate_up = random_quant_tensor(experts * 2 * inter, hidden, widths[0], meta_dtype=meta, device="cuda", generator=gen)
+    down = random_quant_tensor(experts * hidden, inter, widths[1], meta_dtype=meta, device="cuda", generator=gen)
+    ids, weights = seeded_routing(tokens, experts, topk, seed=tokens, device="cuda")
+    ids[0, 0] = -1  # an assignment that belongs to nobody here
+    x = torch.randn(tokens, hidden, device="cuda", generator=gen).to(act)
+    want = torch.cat([ops.moe_gemv(x[i:i + 64].contiguous(), ids[i:i + 64].contiguous(), weights[i:i + 64].contiguous(), gate_up, down,
+                                   num_experts=experts, out_dtype=torch.float32) for i in range(0, tokens, 64)])
+    lib, tag, need = _lib.load(), _lib.DQ_BF16 if act == torch.bfloat16 else _lib.DQ_F16, ctypes.c_int64()
+    _lib.check(lib.dq_moe_gemm_scratch_bytes(tokens, topk, hidden, inter, experts, tag, ctypes.byref(need)))
+    scratch = torch.empty(need.value, dtype=torch.uint8, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    banks = [ops.weight_descriptor("moe", q.packed, q.scales, q.offsets, q.bits, 128, q.in_features) for q in (gate_up, down)]
+    outs = []
+    for _ in range(2):
+        y = torch.full((tokens + 2, hidden), 7.0, device="cuda")
+        _lib.check(lib.dq_moe_gemm(x.data_ptr(), tag, tokens, ids.data_ptr(), weights.data_ptr(), topk, 0, experts, ctypes.byref(banks[0]),
+                                   ctypes.byref(banks[1]), hidden, inter, y[1:-1].data_ptr(), _lib.DQ_F32, scratch.data_ptr(), need.value, stream))
+        outs.append(y)
+    assert ops.last_kernel() == "moe_umma_kernel" and lib.dq_gemm_status(stream) == _lib.DQ_OK
+    assert torch.equal(outs[0], outs[1]) and bool((outs[0][0] == 7.0).all()) and bool((outs[0][-1] == 7.0).all())
+    # the intermediate is rounded on both sides: flips of its last bit are what differs
+    assert (outs[0][1:-1] - want).norm() / want.norm() <= (1e-3 if act == torch.bfloat16 else 2e-4)
