@@ -871,6 +871,31 @@ bool mma_path_supports(const GemvArgs& a, int bits) {
   return device_info() != nullptr;
 }
 
+namespace {
+
+// Where several matrices that share an activation (gate / up, q / k / v) take the cluster-sliced
+// streaming body rather than the tiled kernel, which has a third of its resident warps.  Measured, us,
+// tiled -> sliced, gate / up pairs and q / k / v at 2 / 3 / 4 / 8 bits:
+//  * from 90 M values on: 2 x 17408 x 5120 at one row 23.8 / 30.3 / 26.7 / 54.1 -> 18.6 / 27.9 / 20.9 / 29.6,
+//    at four rows 26.9 / 33.2 / 35.6 / 56.9 -> 20.9 / 30.1 / 24.6 / 36.4; 2 x 14336 x 4096 at one row 17.9 /
+//    22.2 / 19.1 / 34.6 -> 15.8 / 22.8 / 17.2 / 23.7;
+//  * mostly 8-bit codes, from 20 M on: 6144 x 4096 as q / k / v 10.5 -> 9.1, 2 x 3072 x 8192 16.7 -> 14.0;
+//  * four rows and more, from 20 M on, where the slices come out even (step counts that are multiples of
+//    16): 6144 x 4096 10.1 / 9.5 / 8.9 -> 7.5 / 9.1 / 8.0; but 7168 x 5120, ten blocks over four slices,
+//    10.6 / 11.8 / 10.5 -> 11.1 / 13.7 / 12.1.
+bool stream_sliced_fused_first(const GemvArgs* jobs, const int* bits, int n) {
+  int64_t values = 0, code_bits = 0;
+  for (int i = 0; i < n; ++i) {
+    const int64_t v = static_cast<int64_t>(jobs[i].rows) * jobs[i].in_features;
+    values += v, code_bits += v * bits[i];
+  }
+  if (n < 2 || values < 20000000) return false;
+  if (values >= 90000000 || code_bits * 2 >= values * 11) return true;
+  return jobs[0].m >= 4 && jobs[0].in_features >= 4096 && jobs[0].in_features % 2048 == 0;
+}
+
+}  // namespace
+
 int32_t launch_gemv_mma_fused(const GemvArgs* jobs, const int* bits, int n, cudaStream_t stream, bool* taken,
                               const peerpush::Push* push) {
   *taken = false;
@@ -882,6 +907,10 @@ int32_t launch_gemv_mma_fused(const GemvArgs* jobs, const int* bits, int n, cuda
   if (push == nullptr && tuning_int("DQ_B200_NO_STREAM_MULTI") == 0) {
     // matrices long enough to be streamed: the streaming body, a range of CTAs per matrix
     if (const int32_t rc = launch_gemv_stream_fused(jobs, bits, n, stream, taken)) return rc;
+    if (*taken) return DQ_OK;
+  }
+  if (push == nullptr && stream_sliced_fused_first(jobs, bits, n)) {
+    if (const int32_t rc = launch_gemv_stream_sliced_fused(jobs, bits, n, stream, taken)) return rc;
     if (*taken) return DQ_OK;
   }
   return try_tile(jobs, bits, n, *dev, stream, taken, push);
@@ -910,7 +939,9 @@ bool rows_kernel_first(const GemvArgs& a, int bits) {
   // many-rows kernel does that once per eight row tiles and reads ahead meanwhile (4096 x 14336,
   // eight rows, 2 / 3 / 4 / 8 bits: 21 / 28 / 16 / 30 us against 27 / 30 / 37 / 53).
   const int64_t frag_bytes = static_cast<int64_t>(a.m) * steps * (bits == 8 ? 32 : 16) * 16;
-  return frag_bytes > (144 << 10);
+  // (from 96 KB on where the matrix is small: 2048 x 6144, eight rows, 2 / 3 / 4 bits 7.4 / 7.7 / 6.3 against
+  // 8.5 / 9.0 / 8.4)
+  return frag_bytes > (144 << 10) || (a.m >= 6 && frag_bytes >= (96 << 10) && static_cast<int64_t>(a.rows) * a.in_features < 16000000);
 }
 
 // Where the streaming body with the reduction axis sliced over a cluster (dq_gemv_stream_sliced.cu)
@@ -925,6 +956,9 @@ bool rows_kernel_first(const GemvArgs& a, int bits) {
 //    per SM, from 20 MB on (10240 x 5120 at one row, 4 / 8 bits: 12.0 / 15.5 against 14.7 / 22.5;
 //    but 7168 x 5120 at 4 bits, 18 MB, 10.8 against 9.0, and 17408 x 5120, 544 CTAs, 14.0 / 19.5 /
 //    17.0 at 2 / 3 / 4 bits against 13.0 / 17.0 / 15.7);
+//  * it cannot slice the reduction axis eight ways and has about a CTA per SM or fewer, from 20 M values
+//    on (5120 x 5120 at 2 / 3 / 4 / 8 bits: at one row 6.5 / 8.4 / 7.4 / 8.7 against 7.8 / 8.8 / 8.2 / 15.3, at
+//    four 7.2 / 8.9 / 7.9 / 9.2 against 10.1 / 11.0 / 10.1 / 17.8);
 //  * seven or eight activation rows (8192 x 8192 13.7 / 16.9 / 16.8 / 22.9 against 18.5 / 20.7 / 20.6
 //    / 32; 11008 x 4096 11.1 / 13.7 / 11.7 / 14.1 against 13.9 / 14.5 / 13.7 / 21.1);
 //  * up to 8192 weight rows: four and more activation rows from 20 MB on (4096 x 14336 at 3 / 4 bits
@@ -942,12 +976,13 @@ bool stream_sliced_first(const GemvArgs& a, int bits, bool rows_first) {
   const DeviceInfo* dev = device_info();
   if (dev == nullptr || a.group_values != kStepValues || a.words_per_row % (4 * bits) != 0) return false;
   const int64_t bytes = static_cast<int64_t>(a.rows) * a.words_per_row * 4;
-  if (bytes < (16 << 20)) return false;
-  if (rows_first || a.m >= 7) return true;
   const int steps = a.words_per_row / (4 * bits);
   int kw = 8;
   while (kw > 1 && (steps % kw != 0 || (steps / kw) % 2 != 0)) kw /= 2;
   const int64_t ctas = ceil_div(ceil_div(a.rows, 16) * kw, 8);
+  if (kw < 8 && ctas * 4 < static_cast<int64_t>(dev->sm_count) * 5 && static_cast<int64_t>(a.rows) * a.in_features >= 20000000) return true;
+  if (bytes < (16 << 20)) return false;
+  if (rows_first || a.m >= 7) return true;
   // (a CTA per SM AND a long chain per warp: 2048 x 16384 has 128 CTAs there but slices of 16 steps,
   // and runs 9.0 us at 4 bits against 14.1 here, whose 16 row groups x 8 slices cannot fill the SMs)
   if (ctas * 4 < static_cast<int64_t>(dev->sm_count) * 5 && steps / kw >= 24) return true;

@@ -431,9 +431,12 @@ __global__ void __launch_bounds__(kThreads, 3) gemv_mma_stream_kernel(const Gemv
 // -- staging only its part of the activation -- and the sums meet in the cluster's first CTA
 // through distributed shared memory, added in slice order (a fixed summation order), which stores.
 // p.steps is the whole row's step count here; the slices are whole blocks, equal to within one.
-template <int BITS, bool XBF16, bool MBF16, bool P16 = false>
-__global__ void __launch_bounds__(kThreads, 3) gemv_mma_stream_sliced_kernel(const GemvArgs a, const Params p) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+//
+// A device function of (row group, row groups of the matrix) so that one launch can also run several
+// matrices side by side (dq_gemv_stream_sliced.cu); outside a cluster there is one slice.
+template <int BITS, bool XBF16, bool MBF16, bool P16>
+__device__ __forceinline__ void sliced_body(const GemvArgs& a, const Params& p, const unsigned int group, const unsigned int groups,
+                                            unsigned char* smem_raw) {
   constexpr int P = Cfg<BITS>::P;
   constexpr int NA = P16 ? 16 : MmaPlan<BITS>::kARegs;
   uint32_t slice, slices;
@@ -453,7 +456,7 @@ __global__ void __launch_bounds__(kThreads, 3) gemv_mma_stream_sliced_kernel(con
   sa.offsets = a.offsets != nullptr ? static_cast<const unsigned short*>(a.offsets) + s0 : nullptr;
   sa.x = static_cast<const unsigned short*>(a.x) + s0 * 128;  // (the row pitch stays a.in_features)
   float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  stream_body<BITS, XBF16, MBF16, P16, false, true>(sa, sp, blockIdx.x, gridDim.x, smem_raw, acc);
+  stream_body<BITS, XBF16, MBF16, P16, false, true>(sa, sp, group, groups, smem_raw, acc);
 
   // Both cluster barriers are reached by every thread of every CTA; the second keeps a CTA's shared
   // memory alive until the first CTA has read it.
@@ -474,7 +477,7 @@ __global__ void __launch_bounds__(kThreads, 3) gemv_mma_stream_sliced_kernel(con
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (slice != 0) return;
   const int lane = tid & (kWarp - 1), warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int tile = static_cast<int>(blockIdx.x) * kWarps + warp;
+  const int tile = static_cast<int>(group) * kWarps + warp;
   if (tile >= p.tiles) return;
   const int row_a = tile * 16 + g, row_b = row_a + 8;
   const int m0 = 2 * t;
@@ -486,6 +489,13 @@ __global__ void __launch_bounds__(kThreads, 3) gemv_mma_stream_sliced_kernel(con
     if (row_a < a.rows) store_out(a, m0 + 1, row_a, acc[1]);
     if (row_b < a.rows) store_out(a, m0 + 1, row_b, acc[3]);
   }
+}
+
+// (Built for the two CTAs per SM that it is held to: with the third one's registers 4 % faster.)
+template <int BITS, bool XBF16, bool MBF16, bool P16 = false>
+__global__ void __launch_bounds__(kThreads, 2) gemv_mma_stream_sliced_kernel(const GemvArgs a, const Params p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  sliced_body<BITS, XBF16, MBF16, P16>(a, p, blockIdx.x, gridDim.x, smem_raw);
 }
 
 }  // namespace stream

@@ -104,7 +104,8 @@ DQ_API int64_t dq_launch_count(void);
  * ("gemv_mma_stream_kernel", "gemv_mma_stream_multi_kernel", "gemv_mma_stream_sliced_kernel", "gemv_mma_tile_kernel",
  * "gemv_mma_kernel", "gemv_fast_kernel",
  * "gemv_general_kernel", "gemv_plan_kernel", "gemv_rows_kernel", "moe_grouped_kernel", "moe_combine_kernel",
- * "moe_down_token_kernel", "gemm_umma_kernel", "moe_umma_kernel"; "" before the first launch).  No reference
+ * "moe_down_token_kernel", "gemm_umma_kernel", "moe_umma_kernel",
+ * "gemv_mma_stream_sliced_multi_kernel"; "" before the first launch).  No reference
  * counterpart: the reference has two kernels and a documented rule between them
  * (csrc/gemv/gemv.cu:566-598); here a test uses this to prove which kernel it exercised. */
 DQ_API const char* dq_last_kernel(void);
