@@ -438,7 +438,8 @@ def dequantize(qt: QuantTensor, *, dtype: torch.dtype | None = None) -> torch.Te
         dense = _host.dequant(qt.packed, qt.scales, qt.offsets, qt.bits, qt.group_size, qt.in_features)
     if dense is None:
         dense = dequant(*_kernel_args(qt))
-    dense = dense.reshape(qt.logical_shape)
+    if dense.shape != qt.logical_shape:
+        dense = dense.reshape(qt.logical_shape)
     return dense if dtype is None else dense.to(dtype)
 
 

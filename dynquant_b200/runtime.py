@@ -66,7 +66,15 @@ class _PackedModule(nn.Module):
         self.__dict__["_view"] = None       # (data_ptr of packed, QuantTensor)
         if tied_to is None:
             for name, tensor in zip(BUFFER_NAMES, (weight.packed, weight.scales, weight.offsets)):
-                self.register_buffer(name, tensor)
+                self._own(name, tensor)
+
+    def _own(self, name: str, tensor: torch.Tensor | None) -> None:
+        """``register_buffer`` without its checks (2 us a buffer, half of packing a small layer), which
+        can find nothing here; the global registration hooks, where there are any, still run."""
+        if getattr(nn.modules.module, "_global_buffer_registration_hooks", True):
+            self.register_buffer(name, tensor)
+        else:
+            self._buffers[name] = tensor
 
     # -- the attributes callers of the reference module read --
     bits = property(lambda self: self.spec.bits)
@@ -107,11 +115,11 @@ def _encode(weight: torch.Tensor, bits: int, group_size: int, symmetric: bool) -
     """Min/max encoding of a dense weight: ``dq_encode`` where the weight is on the GPU and of a
     shape that kernel takes, else on the host (no clip search: the reference's encoder search is
     outside this package)."""
-    w = weight.detach()
-    if w.is_cuda and ops._host is not None:
-        parts = ops._host.encode(w, bits, group_size, symmetric)  # the same bits, on the GPU
+    if weight.is_cuda and ops._host is not None:
+        parts = ops._host.encode(weight, bits, group_size, symmetric)  # the same bits, on the GPU
         if parts is not None:
-            return QuantTensor(*parts, bits, group_size, w.shape[-1], tuple(w.shape), symmetric=symmetric)
+            return QuantTensor(*parts, bits, group_size, weight.shape[-1], tuple(weight.shape), symmetric=symmetric)
+    w = weight.detach()
     meta = w.dtype if w.dtype in (torch.float16, torch.bfloat16) else torch.float16
     qt = QuantTensor.from_dense(w.cpu(), bits=bits, group_size=group_size, symmetric=symmetric, compute_dtype=meta)
     return qt.to(w.device)
@@ -123,7 +131,7 @@ class DynQuantLinear(_PackedModule):
     def __init__(self, weight: QuantTensor, bias: torch.Tensor | None = None, *,
                  tied_to: _PackedModule | None = None) -> None:
         super().__init__(weight, tied_to=tied_to)
-        self.register_buffer("bias", bias.detach().clone() if bias is not None else None)
+        self._own("bias", bias.detach().clone() if bias is not None else None)
 
     @classmethod
     def from_linear(cls, linear: nn.Linear, bits: int, *, group_size: int = DEFAULT_GROUP_SIZE,
