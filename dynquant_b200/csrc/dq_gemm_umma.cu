@@ -38,6 +38,7 @@ namespace {
 using namespace umma;
 
 constexpr int kJobs = 4;
+constexpr int kMaxSlices = 6;
 struct Job {
   CUtensorMap wmap;
   Meta meta;
@@ -221,28 +222,59 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
   }
 
   __syncthreads();
-  if (p.slices > 1) {  // one tile per cluster: add the slices' columns, a share of them per CTA
+  if (p.slices > 1) {
+    // One tile per cluster: add the slices' columns, a share of them per CTA.  A warp takes a column, a
+    // lane four of its rows, all slices' loads of two columns requested before the first is used (one
+    // row and column at a time, slice after slice, two slices took 3 us at 64 columns and 5.6 at 128).
     cluster_sync();
     const int tile = blockIdx.x;
     int local;
     const Job& job = p.job[job_of(tile % p.row_tiles, local)];
     const int per = (p.n_tile + p.slices - 1) / p.slices;
-    const int first = slice * per, last = min(first + per, p.n_tile);
-    const int row = local * 128 + (threadIdx.x & 127);
     const int token0 = (tile / p.row_tiles) * p.n_tile;
+    const int first = slice * per, last = min(min(first + per, p.n_tile), p.m - token0);
+    const int row = local * 128 + lane * 4;
     if (*failed == 0 && row < job.rows) {
-      const float bias = job.bias != nullptr ? load_f32(job.bias, row, BF16 ? DQ_BF16 : DQ_F16) : 0.0f;
-      unsigned short* dst = static_cast<unsigned short*>(p.out) + job.col0 + row;
-      const uint32_t red = base + p.ring_offset + (threadIdx.x & 127) * 4;
-      for (int col = first + (threadIdx.x >> 7); col < last && token0 + col < p.m; col += Roles<SPLIT>::kThreads / 128) {
-        float part[8];  // all requested, then added in slice order
+      constexpr int kType = BF16 ? DQ_BF16 : DQ_F16, kWarps = Roles<SPLIT>::kThreads / 32;
+      float bias[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      if (job.bias != nullptr) {
 #pragma unroll
-        for (int s = 0; s < 8; ++s) part[s] = s < p.slices ? cluster_ld(red + col * 512, s) : 0.0f;
-        float sum = part[0];
+        for (int i = 0; i < 4; ++i) bias[i] = load_f32(job.bias, min(row + i, job.rows - 1), kType);
+      }
+      const uint32_t red = base + p.ring_offset + lane * 16;
+      for (int col0 = first + warp; col0 < last; col0 += 2 * kWarps) {
+        float4 part[2][kMaxSlices];
 #pragma unroll
-        for (int s = 1; s < 8; ++s) sum += part[s];
-        dst[static_cast<int64_t>(token0 + col) * p.out_stride] =
-            static_cast<unsigned short>(round_to_16(sum + bias, BF16 ? DQ_BF16 : DQ_F16));
+        for (int c = 0; c < 2; ++c) {
+          const int col = min(col0 + c * kWarps, last - 1);
+#pragma unroll
+          for (int s = 0; s < kMaxSlices; ++s) {
+            part[c][s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (s < p.slices) part[c][s] = cluster_ld4(red + col * 512, s);
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int col = col0 + c * kWarps;
+          if (col >= last) break;
+          float4 sum = part[c][0];
+#pragma unroll
+          for (int s = 1; s < kMaxSlices; ++s) {  // in slice order
+            sum.x += part[c][s].x, sum.y += part[c][s].y, sum.z += part[c][s].z, sum.w += part[c][s].w;
+          }
+          unsigned short* dst = static_cast<unsigned short*>(p.out) + static_cast<int64_t>(token0 + col) * p.out_stride + job.col0 + row;
+          const uint2 packed = make_uint2(round_pair_to_16(sum.x + bias[0], sum.y + bias[1], kType),
+                                          round_pair_to_16(sum.z + bias[2], sum.w + bias[3], kType));
+          if (row + 3 < job.rows && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
+            *reinterpret_cast<uint2*>(dst) = packed;
+          } else {
+            const uint32_t half[4] = {packed.x & 0xFFFFu, packed.x >> 16, packed.y & 0xFFFFu, packed.y >> 16};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              if (row + i < job.rows) dst[i] = static_cast<unsigned short>(half[i]);
+            }
+          }
+        }
       }
     }
     cluster_sync();  // nobody leaves while its sums are being read
@@ -270,27 +302,30 @@ struct Shape {
   int n_tile, token_tiles, slices;
 };
 
-// Token tiles and slices of the reduction axis with the least estimated time: waves of CTAs times
-// the cycles of one -- 128-value stages, each bound by the hand-over between the block's roles or by
-// the tensor pipe (2 n_tile cycles per 64 values), plus a start and an end.  The slices of all tiles
-// are resident at once or there are none: a second wave of clusters costs more than it gives (4096 x
-// 14336, 16 rows: 22 us with 4 slices, 38 with 8), and clusters of eight pack badly into the GPCs
-// (1152 x 7936, 128 rows: 14 us with 6 slices, 21 with 8).
-Shape pick_shape(int m, int row_tiles, int chunks, int sm_count) {
+// Token tiles and slices of the reduction axis with the least estimated time (us, fitted to measurements
+// at 16..1024 rows on matrices of 128 x 128 to 14336 x 4096): waves of CTAs times the chunks of one, each
+// bound by the decode or by the tensor pipe, a start and an end, and what a cluster costs -- the sums
+// that cross it and, the more of the chip it fills, its launch.  The slices of all tiles are resident at
+// once or there are none: a second wave of clusters costs more than it gives (4096 x 14336, 16 rows: 22
+// us with 4 slices, 38 with 8), and clusters of eight pack badly into the GPCs (1152 x 7936, 128 rows: 14
+// us with 6 slices, 21 with 8).
+Shape pick_shape(int m, int row_tiles, int chunks, bool split, int sm_count) {
   Shape best = {};
   double best_cost = 1e30;
   const int min_tiles = static_cast<int>(ceil_div(m, 256));
-  for (int tt = min_tiles; tt <= min_tiles + 2; ++tt) {
+  for (int tt = min_tiles; tt <= min_tiles + (m > 256 ? 2 : 0); ++tt) {  // (up to 256 rows a second tile only decodes twice)
     const int n = static_cast<int>(ceil_div(ceil_div(m, tt), 16) * 16);
     if (n * (tt - 1) >= m) continue;
-    const double stage = std::max(700.0, 4.0 * n + 60.0);
-    for (int s = 1; s <= 6 && s <= chunks; ++s) {
+    const double again = 1.0 + 0.08 * (tt - min_tiles);
+    const double chunk = (split ? 0.49 + 0.001 * n : std::max(0.42, 0.22 + 0.0022 * n)) * again;
+    for (int s = 1; s <= kMaxSlices && s <= chunks; ++s) {
       const int64_t ctas = static_cast<int64_t>(row_tiles) * tt * s;
       const int resident = s <= 2 ? sm_count : s <= 4 ? sm_count - 16 : sm_count - 24;
       if (s > 1 && ctas > resident) break;
       const double waves = std::ceil(static_cast<double>(ctas) / sm_count);
-      const double hidden = s == 1 && n <= 128 ? 0.0 : 10.0 * n;  // an epilogue that the next tile does not cover
-      const double cost = waves * (static_cast<double>(ceil_div(chunks, s)) * stage + hidden) + (s > 1 ? 1500.0 : 0.0) + 10.0 * n + 7000.0;
+      const double hidden = s == 1 && n <= 128 ? 0.0 : 0.005 * n;  // an epilogue that the next tile does not cover
+      const double cluster = s > 1 ? 1.0 + 0.004 * n * s + 1.1 * (s - 1) * static_cast<double>(ctas) / sm_count : 0.0;
+      const double cost = waves * (static_cast<double>(ceil_div(chunks, s)) * chunk + hidden) + cluster + 2.2 + 0.01 * n;
       if (cost < best_cost) best_cost = cost, best = {n, tt, s};
     }
   }
@@ -332,7 +367,7 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
   p.out = a.out;
   p.out_stride = a.out_stride;
   p.chunks = static_cast<int>(ceil_div(a.in_features, 128));
-  Shape shape = pick_shape(a.m, p.row_tiles, p.chunks, dev->sm_count);
+  Shape shape = pick_shape(a.m, p.row_tiles, p.chunks, a.m <= DQ_GEMV_CHUNKED_MAX_ROWS, dev->sm_count);
   if (const int n = tuning_int("DQ_B200_UMMA_N", 0)) shape.n_tile = n, shape.token_tiles = static_cast<int>(ceil_div(a.m, n));
   if (const int s = tuning_int("DQ_B200_UMMA_SLICES", 0)) shape.slices = s;
   p.n_tile = shape.n_tile;

@@ -118,9 +118,11 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ float cluster_ld(uint32_t addr, int rank) {
-  float v;
-  asm volatile("{\n .reg .b32 a;\n mapa.shared::cluster.u32 a, %1, %2;\n ld.shared::cluster.f32 %0, [a];\n}" : "=f"(v) : "r"(addr), "r"(rank));
+__device__ __forceinline__ float4 cluster_ld4(uint32_t addr, int rank) {
+  float4 v;
+  asm volatile("{\n .reg .b32 a;\n mapa.shared::cluster.u32 a, %4, %5;\n ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n}"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr), "r"(rank));
   return v;
 }
 
