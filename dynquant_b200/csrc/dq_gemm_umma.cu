@@ -8,15 +8,18 @@
 //   * warp 2 streams packed 128 x 128-value tiles into shared memory by TMA (they are 4..16 KB, so
 //     a ring of them keeps HBM busy), warp 0 the activation in 64-value slabs with the 128-byte
 //     swizzle, both zero-filled past the edges of their tensors;
-//   * four warpgroups (warps 4..19) decode, 64 values of K in turn: a thread owns one weight row, so
-//     its scale and offset are two registers and its packed words one contiguous piece of shared
-//     memory; the 16-bit weights go straight to TENSOR MEMORY (tcgen05.st) in the
-//     natural order -- not to shared memory, whose bandwidth the activation needs;
+//   * four warpgroups (three where weights are split in two operands) decode, 128 values of K in turn:
+//     a thread owns one weight row, so its scale and offset are two registers and its packed words one
+//     contiguous piece of shared memory; the 16-bit weights go straight to TENSOR MEMORY (tcgen05.st)
+//     in the natural order -- not to shared memory, whose bandwidth the activation needs;
 //   * warp 1 issues the MMAs (A from tensor memory, B from shared memory), accumulating in tensor
-//     memory; two accumulator tiles where they fit (n_tile <= 192), so that the decode of the next
-//     tile runs under the epilogue of this one.
-// What bounds it: with n_tile >= 144 the tensor pipe (128 x n_tile x 64 take 2 n_tile cycles), below
-// that the decode (about 290 cycles per 128 x 64 values on the SM's four schedulers).
+//     memory; two accumulator tiles where they fit, so that the decode of the next tile runs under the
+//     epilogue of this one.
+// What bounds it: for wide tiles the tensor pipe -- an MMA whose A is in tensor memory takes about
+// 60 + 0.47 n_tile cycles per 16 values of K -- below that the decode's issue slots (14336 x 4096,
+// 4-bit: issue 55 %, integer pipe 54 %, tensor 31 % at 65 rows; 0.5 us per 128 x 128 values and SM
+// split in two operands).  14336 x 4096, 4-bit, at 16 / 128 / 512 / 4096 rows: 21 / 22 / 53 / 370 us (1.30
+// PFLOP/s) where dequantize + dense took 215 us at the first two and 521 at the last.
 //
 // Small matrices: the reduction axis is sliced over a thread-block cluster (grid.y), each CTA leaves
 // its fp32 tile in its own shared memory and the CTAs of the cluster add a share of the columns

@@ -17,9 +17,9 @@ Two layers:
 And the dispatch layer of the reference runtime
 (``packages/dynquant-core/src/dynquant/runtime/ops.py:163-260``):
 ``dequantize``, ``quantized_matmul`` and ``embedding_lookup`` with the same
-signatures and the same rule -- at most ``gemv_max_rows()`` activation rows go
-to the packed GEMV, more go to dequant + a dense matmul.  There is no torch or
-CPU fallback here: a tensor that is not on a CUDA device raises.
+signatures; any number of activation rows goes to the packed kernels, and
+dequant + a dense matmul serves what they refuse above 64 rows.  There is no
+torch or CPU fallback here: a tensor that is not on a CUDA device raises.
 """
 
 from __future__ import annotations
@@ -470,8 +470,8 @@ def quantized_matmul(x: torch.Tensor, qt: QuantTensor, bias: torch.Tensor | None
     elif flat.shape[0] <= GEMV_CHUNKED_MAX_ROWS and flat.is_cuda:
         out = gemv_row_chunks(flat.contiguous(), [qt], None if bias is None else bias.contiguous())
     else:
-        weight = dequant(*args)
-        out = torch.nn.functional.linear(flat, weight.to(x.dtype), bias)
+        # what the tensor-core kernel refuses; rounded once, to the type the dense matmul reads
+        out = torch.nn.functional.linear(flat, dequant(*args, out_dtype=x.dtype), bias)
     return out.reshape(*lead, qt.num_rows)
 
 

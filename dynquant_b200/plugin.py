@@ -289,7 +289,7 @@ class DynQuantLinearMethod:
             out = ops.gemv_row_chunks(flat.contiguous(), shards, None if bias is None else bias.contiguous())
         else:
             parts = [
-                torch.nn.functional.linear(flat, ops.dequant(*ops._kernel_args(qt)).to(flat.dtype)) for qt in shards
+                torch.nn.functional.linear(flat, ops.dequant(*ops._kernel_args(qt), out_dtype=flat.dtype)) for qt in shards
             ]
             out = parts[0] if len(parts) == 1 else torch.cat(parts, dim=-1)
             if bias is not None:
