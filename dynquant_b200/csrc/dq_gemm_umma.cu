@@ -15,10 +15,10 @@
 //   * warp 1 issues the MMAs (A from tensor memory, B from shared memory), accumulating in tensor
 //     memory; two accumulator tiles where they fit, so that the decode of the next tile runs under the
 //     epilogue of this one.
-// What bounds it: for wide tiles the tensor pipe -- an MMA whose A is in tensor memory takes about
-// 60 + 0.47 n_tile cycles per 16 values of K -- below that the decode's issue slots (14336 x 4096,
-// 4-bit: issue 55 %, integer pipe 54 %, tensor 31 % at 65 rows; 0.5 us per 128 x 128 values and SM
-// split in two operands).  14336 x 4096, 4-bit, at 16 / 128 / 512 / 4096 rows: 21 / 22 / 53 / 370 us (1.30
+// What bounds it: for wide tiles the tensor pipe (n_tile / 2 cycles per 16 values of K) at the clock that
+// the power cap leaves, below that the decode's issue slots (14336 x 4096, 4-bit: issue 55 %, integer
+// pipe 54 %, tensor 31 % at 65 rows, with 112 of 148 SMs at work; 0.5 us per 128 x 128 values and SM split
+// in two operands).  14336 x 4096, 4-bit, at 16 / 128 / 512 / 4096 rows: 21 / 22 / 53 / 366 us (1.31
 // PFLOP/s) where dequantize + dense took 215 us at the first two and 521 at the last.
 //
 // Small matrices: the reduction axis is sliced over a thread-block cluster (grid.y), each CTA leaves
@@ -59,6 +59,7 @@ struct Params {
   int row_tiles, tiles;                // over all jobs; tiles = row_tiles x token tiles
   int n_tile, d_buffers, tmem_columns;
   int x_slots, w_slots, w_bytes;       // rings; bytes of a weight slot
+  int x_slabs;                         // slabs of 64 values in an activation slot: 2 (a chunk) or 1
   int slices;
   uint32_t ring_offset, barrier_offset;
 };
@@ -77,7 +78,8 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
   volatile int* failed = reinterpret_cast<volatile int*>(smem);
   const uint32_t base = smem_addr(smem);
   const Bars bars = bars_at(base + p.barrier_offset);
-  const int x_bytes = p.n_tile * 256;  // two slabs of 64 values
+  const int x_slabs = SPLIT ? 2 : p.x_slabs;
+  const int slab_bytes = p.n_tile * 128, x_bytes = slab_bytes * x_slabs;
   unsigned char* x_ring = smem + p.ring_offset;
   unsigned char* w_ring = x_ring + p.x_slots * x_bytes;
   const int warp = threadIdx.x >> 5;
@@ -121,7 +123,7 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
         int local;
         const Job& job = p.job[job_of(tile % p.row_tiles, local)];
         const int token0 = (tile / p.row_tiles) * p.n_tile;
-        const int count = c1 - c0;
+        const int count = weights || x_slabs == 2 ? c1 - c0 : (c1 - c0) * 2;
         const int bytes = weights ? 2048 * job.bits : x_bytes;
         for (int i = 0; i < count; ++i, ++issued, at.advance(slots)) {
           const uint32_t slot = at.slot;
@@ -131,8 +133,9 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
             tma_load_2d(smem_addr(w_ring) + slot * p.w_bytes, &job.wmap, (c0 + i) * 4 * job.bits, local * 128, full + slot * 8);
           } else {
             const uint32_t dst = smem_addr(x_ring) + slot * x_bytes;
-            tma_load_2d(dst, &p.xmap, (c0 + i) * 128, token0, full + slot * 8);
-            tma_load_2d(dst + x_bytes / 2, &p.xmap, (c0 + i) * 128 + 64, token0, full + slot * 8);
+            const int x0 = c0 * 128 + i * 64 * x_slabs;
+            tma_load_2d(dst, &p.xmap, x0, token0, full + slot * 8);
+            if (x_slabs == 2) tma_load_2d(dst + slab_bytes, &p.xmap, x0 + 64, token0, full + slot * 8);
           }
         }
       }
@@ -150,14 +153,23 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
         fence_after_sync();
         const uint32_t d = d_tmem + buffer * p.n_tile;
         for (int i = 0; i < c1 - c0; ++i) {
-          const uint32_t xs = x_at.slot;
+          uint32_t xs = x_at.slot;
           if (!(ok = mbar_wait(bars.x_full + xs * 8, x_at.pass, failed))) break;
-          const uint64_t b0 = smem_descriptor(smem_addr(x_ring) + xs * x_bytes);
-          const uint64_t b1 = smem_descriptor(smem_addr(x_ring) + xs * x_bytes + x_bytes / 2);
           if (!(ok = mbar_wait(bars.a_full + a_at.slot * 8, a_at.pass, failed))) break;
           fence_after_sync();
           const uint32_t a = tmem + a_at.slot * Roles<SPLIT>::kTileColumns;
-          mma_chunk<SPLIT>(d, a, b0, b1, idesc, i > 0);
+          uint32_t slab = smem_addr(x_ring) + xs * x_bytes;
+          mma_slab<SPLIT>(d, a, smem_descriptor(slab), idesc, i > 0);
+          if (x_slabs == 1) {
+            mma_commit(bars.x_empty + xs * 8);
+            x_at.advance(static_cast<uint32_t>(p.x_slots));
+            xs = x_at.slot;
+            if (!(ok = mbar_wait(bars.x_full + xs * 8, x_at.pass, failed))) break;
+            slab = smem_addr(x_ring) + xs * x_bytes;
+          } else {
+            slab += slab_bytes;
+          }
+          mma_slab<SPLIT>(d, a + 32, smem_descriptor(slab), idesc, true);
           mma_commit(bars.a_empty + a_at.slot * 8);
           a_at.advance(kGroups);
           mma_commit(bars.x_empty + xs * 8);
@@ -386,12 +398,18 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
   p.d_buffers = p.slices == 1 && p.tiles > grid_x && a_columns + 2 * p.n_tile <= 512 ? 2 : 1;
   p.tmem_columns = 32;
   while (p.tmem_columns < a_columns + p.d_buffers * p.n_tile) p.tmem_columns *= 2;
-  // Rings: activation slots of 128 values (2..6), then weight slots -- a multiple of the warpgroups, so
-  // that a slot always belongs to the same one (its barrier then cannot be two passes behind).
-  const int x_bytes = p.n_tile * 256;
+  // Rings: activation slots of 128 values (up to 6), then weight slots -- a multiple of the warpgroups, so
+  // that a slot always belongs to the same one (its barrier then cannot be two passes behind).  Where the
+  // activation of three chunks does not fit (8 bits, from 224 columns on) the slots are of 64 values: two
+  // of 128 leave a copy only one chunk's time (8-bit 17280 x 1152 at 512 / 4096 rows 26.8 / 186 us against
+  // 25.7 / 175, 4096 x 4096 at 4096 rows 128 against 111).  Elsewhere the second wait per chunk only
+  // costs (14336 x 4096, 4-bit, 65 rows: 19.4 us against 17.4).
   p.w_bytes = w_bytes;
   const int budget = dev->max_smem_optin - static_cast<int>(kRingOffset);
-  p.x_slots = std::clamp((budget - kMaxGroups * w_bytes) / x_bytes, 2, 6);
+  const int x_room = (budget - kMaxGroups * w_bytes) / (p.n_tile * 128);  // slabs of 64 values
+  p.x_slabs = x_room < 6 ? 1 : 2;
+  p.x_slots = std::min(x_room / p.x_slabs, 6);
+  const int x_bytes = p.n_tile * 128 * p.x_slabs;
   const int groups = split ? Roles<true>::kGroups : Roles<false>::kGroups;
   p.w_slots = std::clamp((budget - p.x_slots * x_bytes) / w_bytes / groups * groups, groups, 12);
   p.barrier_offset = kBarrierOffset;

@@ -146,15 +146,21 @@ __device__ __forceinline__ void init_bars(const Bars& b, int x_slots, int w_slot
   fence_mbar_init();
 }
 
-// One chunk's MMAs: eight steps of 16 values, the operand tile at `a`, the two activation slabs of 64
-// values at b0 and b1.
+// The MMAs of 64 values of K, four steps of 16: a piece of the operand tile at `a`, a slab of activations
+// at `b`.
+template <bool SPLIT>
+__device__ __forceinline__ void mma_slab(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, bool accumulate) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    mma_ts(d, a + k * 8, b + k * 2, idesc, accumulate || k > 0);
+    if constexpr (SPLIT) mma_ts(d, a + 64 + k * 8, b + k * 2, idesc, true);
+  }
+}
+// One chunk's: an operand tile, two slabs.
 template <bool SPLIT>
 __device__ __forceinline__ void mma_chunk(uint32_t d, uint32_t a, uint64_t b0, uint64_t b1, uint32_t idesc, bool accumulate) {
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    mma_ts(d, a + k * 8, (k < 4 ? b0 : b1) + (k & 3) * 2, idesc, accumulate || k > 0);
-    if constexpr (SPLIT) mma_ts(d, a + 64 + k * 8, (k < 4 ? b0 : b1) + (k & 3) * 2, idesc, true);
-  }
+  mma_slab<SPLIT>(d, a, b0, idesc, accumulate);
+  mma_slab<SPLIT>(d, a + 32, b1, idesc, true);
 }
 
 // A producer that gives up waits for its copies in flight ...
