@@ -17,6 +17,7 @@ prints {"kind", "cores", "seconds", "bytes", "gbps", "modules"} as one JSON line
 
 from __future__ import annotations
 
+import importlib.util
 import json
 import os
 import sys
@@ -57,8 +58,11 @@ def main() -> None:
             # reference operator: x dtype must equal the scales dtype (bf16 here)
             return torch.ops.dynquant.gemv(x, packed, scales, offsets, bits, group, k)
     else:
-        sys.path.insert(0, str(HERE.parent))
-        from oracle import oracle as O
+        # by its path: run as a script, this directory is sys.path[0] and "oracle" would be the module in it
+        place = importlib.util.spec_from_file_location("dq_oracle_py", HERE / "oracle.py")
+        O = importlib.util.module_from_spec(place)
+        sys.modules[place.name] = O  # (its dataclasses look their module up)
+        place.loader.exec_module(O)
 
         kind, cores = "port", 1
 

@@ -211,3 +211,16 @@ print('ok')
 """
     res = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=300)
     assert res.returncode == 0 and "ok" in res.stdout, res.stderr[-2000:]
+
+
+def test_the_cpu_timing_script_runs_as_a_script():
+    """What ``bench.py`` starts for its reference arm, without the reference's compiled operators."""
+    import json
+    import os
+
+    spec = {"modules": [[64, 256, 3], [32, 128, 8]], "m": 1, "repeat": 2, "threads": 1}
+    run = subprocess.run([sys.executable, str(ROOT / "oracle" / "cpu_baseline.py"), json.dumps(spec)], capture_output=True,
+                         text=True, timeout=600, env={**os.environ, "DQ_BASELINE_FORCE_PORT": "1"})
+    assert run.returncode == 0, run.stderr[-500:]
+    line = json.loads(run.stdout.strip().splitlines()[-1])
+    assert line["kind"] == "port" and line["modules"] == 4 and line["seconds"] > 0
