@@ -14,6 +14,11 @@
 // shares 32 values exchanges its 24-bit pieces and three of its lanes store a word each).
 // 2048 x 6144 at 4 bits: 37 ms through the host's tensor operations and two copies over PCIe; here
 // the launch is a few microseconds.
+//
+// The kernels that multiply by packed weights request them BEFORE their griddepcontrol.wait, as data
+// that no kernel in flight writes.  Launched right behind this one they would have a programmatic edge
+// to it, which an ordinary kernel releases when its blocks exit and not when its stores are visible.
+// So a memset follows: an ordinary edge on both sides, behind which the words are complete.
 #include <algorithm>
 
 #include "dq_common.cuh"
@@ -22,6 +27,8 @@ namespace dq {
 namespace {
 
 constexpr int kEncodeThreads = 256;
+
+__device__ unsigned int g_after_encode;  // what the memset behind the kernel writes; nobody reads it
 
 struct EncodeArgs {
   const void* w;
@@ -193,5 +200,8 @@ extern "C" int32_t dq_encode(const void* w, int32_t w_dtype, int64_t rows, int64
     default: dq::launch_encode<8>(a, lanes, grid, s); break;
   }
   DQ_CHECK_LAUNCH("encode");
+  void* word = nullptr;
+  DQ_CUDA(cudaGetSymbolAddress(&word, dq::g_after_encode));
+  DQ_CUDA(cudaMemsetAsync(word, 0, sizeof(unsigned int), s));
   return DQ_OK;
 }

@@ -131,7 +131,10 @@ DQ_API int32_t dq_dequant_rows(const dq_weight* w, const void* ids, int32_t ids_
  * Min/max group quantization of a dense [rows, in_features] matrix into packed words
  * [rows, groups * group_values * bits / 32] and scales / offsets [rows, groups] of meta_dtype;
  * rows are padded with zeros to whole groups.  Bit-identical to the host encoder.  Groups of 32,
- * 64, 128 or 256 values and in_features % 8 == 0, else DQ_ERR_UNSUPPORTED (nothing launched). */
+ * 64, 128 or 256 values and in_features % 8 == 0, else DQ_ERR_UNSUPPORTED (nothing launched).
+ * Ordered before everything that follows on the stream.  (The multiplying entry points read packed
+ * words, scales and offsets ahead of their programmatic dependency: a caller whose OWN kernel writes
+ * them must put a copy, a memset or an event wait between that kernel and the first of those calls.) */
 DQ_API int32_t dq_encode(const void* w, int32_t w_dtype, int64_t rows, int64_t in_features, int32_t bits,
                          int64_t group_values, int32_t symmetric, void* packed, void* scales, void* offsets,
                          int32_t meta_dtype, void* stream);

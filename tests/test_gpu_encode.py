@@ -46,3 +46,44 @@ def test_embedding_rows_equal_the_rows_of_the_dense_table(k, group, bits, ids_dt
     got = DynQuantEmbedding(table)(ids)
     assert got.shape == (3, 41, k)
     assert torch.equal(got, table.dequantize()[ids.long()])
+
+
+@pytest.mark.parametrize("m", [1, 24, 100])
+def test_a_call_right_behind_the_encoder_waits_for_its_words(m):
+    """The multiplying kernels request weights before their programmatic dependency resolves: the
+    edge that leaves the encoder must be an ordinary one."""
+    from cuda.bindings import runtime as cudart
+
+    from dynquant_b200.runtime import DynQuantLinear
+
+    rows, k = 640, 1024
+    linear = torch.nn.Linear(k, rows, bias=False, device="cuda", dtype=torch.bfloat16)
+    x = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+    want = DynQuantLinear.from_linear(linear, 4)
+    torch.cuda.synchronize()
+    want = want(x)
+    torch.cuda.synchronize()
+    for _ in range(20):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            got = DynQuantLinear.from_linear(linear, 4)(x)
+        stream.synchronize()
+        assert torch.equal(got, want)
+
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        layer = DynQuantLinear.from_linear(linear, 4)
+        got = layer(x)
+    raw = cudart.cudaGraph_t(graph.raw_cuda_graph())
+    err, _, _, _, count = cudart.cudaGraphGetEdges_v2(raw)
+    assert err == cudart.cudaError_t.cudaSuccess and count >= 2
+    err, sources, targets, _, _ = cudart.cudaGraphGetEdges_v2(raw, count)
+    err, roots, _ = cudart.cudaGraphGetRootNodes(raw, 1)
+    kind = lambda node: cudart.cudaGraphNodeGetType(node)[1]  # noqa: E731
+    assert kind(roots[0]) == cudart.cudaGraphNodeType.cudaGraphNodeTypeKernel
+    behind = [t for s, t in zip(sources, targets) if int(s) == int(roots[0])]
+    # (a programmatic edge joins two kernels: none leaves the encoder)
+    assert behind and all(kind(t) == cudart.cudaGraphNodeType.cudaGraphNodeTypeMemset for t in behind)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
