@@ -338,25 +338,29 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
   if (warp == 3) tmem_free(tmem, 512);
 }
 
+// A quad of columns per thread, the tokens over the grid's y axis (which ends at 65535) and round it.
+constexpr int64_t kMaxGridY = 65535;
 __global__ void __launch_bounds__(256) moe_combine_rows_kernel(const float4* d, const float* w, const int32_t* ids, int first_expert,
-                                                               int topk, int quads, int num_experts, void* y, int y_dtype) {
+                                                               int tokens, int topk, int quads, int num_experts, void* y, int y_dtype) {
   pdl_launch_dependents();
   pdl_wait_prior_grid();
-  const int q = blockIdx.x * 256 + threadIdx.x, token = blockIdx.y;
+  const int q = blockIdx.x * 256 + threadIdx.x;
   if (q >= quads) return;
-  float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  for (int k = 0; k < topk; ++k) {
-    const int a = token * topk + k, e = __ldcg(ids + a) - first_expert;
-    if (e < 0 || e >= num_experts) continue;
-    const float p = __ldcg(w + a);
-    const float4 v = __ldcg(d + static_cast<int64_t>(a) * quads + q);
-    acc.x = fmaf(p, v.x, acc.x), acc.y = fmaf(p, v.y, acc.y), acc.z = fmaf(p, v.z, acc.z), acc.w = fmaf(p, v.w, acc.w);
-  }
-  const int64_t at = static_cast<int64_t>(token) * quads + q;
-  if (y_dtype == DQ_F32) {
-    static_cast<float4*>(y)[at] = acc;
-  } else {
-    static_cast<uint2*>(y)[at] = make_uint2(round_pair_to_16(acc.x, acc.y, y_dtype), round_pair_to_16(acc.z, acc.w, y_dtype));
+  for (int token = blockIdx.y; token < tokens; token += gridDim.y) {
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int k = 0; k < topk; ++k) {
+      const int a = token * topk + k, e = __ldcg(ids + a) - first_expert;
+      if (e < 0 || e >= num_experts) continue;
+      const float p = __ldcg(w + a);
+      const float4 v = __ldcg(d + static_cast<int64_t>(a) * quads + q);
+      acc.x = fmaf(p, v.x, acc.x), acc.y = fmaf(p, v.y, acc.y), acc.z = fmaf(p, v.z, acc.z), acc.w = fmaf(p, v.w, acc.w);
+    }
+    const int64_t at = static_cast<int64_t>(token) * quads + q;
+    if (y_dtype == DQ_F32) {
+      static_cast<float4*>(y)[at] = acc;
+    } else {
+      static_cast<uint2*>(y)[at] = make_uint2(round_pair_to_16(acc.x, acc.y, y_dtype), round_pair_to_16(acc.z, acc.w, y_dtype));
+    }
   }
 }
 
@@ -509,8 +513,9 @@ int32_t dq_moe_gemm(const void* x, int32_t x_dtype, int64_t tokens, const int32_
   p.out = base + lay.d;
   if (const int32_t rc = dq::launch_bank<false>(*down, g_dn, base + lay.h, x_dtype, assignments, static_cast<int>(hidden), p, *dev, s)) return rc;
   const int quads = static_cast<int>(hidden / 4);
-  if (const int32_t rc = dq::launch(dq::moe_combine_rows_kernel, dim3(static_cast<unsigned>(dq::ceil_div(quads, 256)), static_cast<unsigned>(tokens)),
-                                    256, 0, s, "moe_gemm(combine)", reinterpret_cast<const float4*>(base + lay.d), topk_w, topk_ids, first,
+  const dim3 combine(static_cast<unsigned>(dq::ceil_div(quads, 256)), static_cast<unsigned>(std::min(tokens, dq::kMaxGridY)));
+  if (const int32_t rc = dq::launch(dq::moe_combine_rows_kernel, combine, 256, 0, s, "moe_gemm(combine)",
+                                    reinterpret_cast<const float4*>(base + lay.d), topk_w, topk_ids, first, static_cast<int>(tokens),
                                     static_cast<int>(topk), quads, experts, y, y_dtype)) {
     return rc;
   }

@@ -108,3 +108,36 @@ def test_an_expert_layer_over_many_tokens_matches_its_small_calls(tokens, expert
     assert torch.equal(outs[0], outs[1]) and bool((outs[0][0] == 7.0).all()) and bool((outs[0][-1] == 7.0).all())
     # the intermediate is rounded on both sides: flips of its last bit are what differs
     assert (outs[0][1:-1] - want).norm() / want.norm() <= (1e-3 if act == torch.bfloat16 else 2e-4)
+
+
+def moe_gemm(x, ids, weights, gate_up, down, experts, *, first_expert=0):
+    """``dq_moe_gemm`` with fp32 results."""
+    import ctypes
+
+    from dynquant_b200 import _lib, ops
+
+    lib, tag, need = _lib.load(), _lib.DQ_BF16 if x.dtype == torch.bfloat16 else _lib.DQ_F16, ctypes.c_int64()
+    (tokens, hidden), topk, inter = x.shape, ids.shape[1], down.in_features
+    _lib.check(lib.dq_moe_gemm_scratch_bytes(tokens, topk, hidden, inter, experts, tag, ctypes.byref(need)))
+    scratch = torch.empty(need.value, dtype=torch.uint8, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    banks = [ops.weight_descriptor("moe", q.packed, q.scales, q.offsets, q.bits, 128, q.in_features) for q in (gate_up, down)]
+    y = torch.empty(tokens, hidden, device="cuda")
+    _lib.check(lib.dq_moe_gemm(x.data_ptr(), tag, tokens, ids.data_ptr(), weights.data_ptr(), topk, first_expert, experts, ctypes.byref(banks[0]),
+                               ctypes.byref(banks[1]), hidden, inter, y.data_ptr(), _lib.DQ_F32, scratch.data_ptr(), need.value, stream))
+    assert lib.dq_gemm_status(stream) == _lib.DQ_OK
+    return y
+
+
+def test_an_expert_layer_over_more_tokens_than_a_grid_has_rows():
+    from dynquant_b200.workloads import random_quant_tensor, seeded_routing
+
+    tokens, experts, hidden, inter = 70000, 8, 256, 128  # a grid's y axis ends at 65535
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    gate_up = random_quant_tensor(experts * 2 * inter, hidden, 4, meta_dtype=torch.float16, device="cuda", generator=gen)
+    down = random_quant_tensor(experts * hidden, inter, 3, meta_dtype=torch.float16, device="cuda", generator=gen)
+    ids, weights = seeded_routing(tokens, experts, 2, seed=1, device="cuda")
+    x = torch.randn(tokens, hidden, device="cuda", generator=gen).to(torch.bfloat16)
+    whole = moe_gemm(x, ids, weights, gate_up, down, experts)
+    parts = [moe_gemm(x[i:i + 30000], ids[i:i + 30000], weights[i:i + 30000], gate_up, down, experts) for i in range(0, tokens, 30000)]
+    assert torch.equal(whole, torch.cat(parts))
