@@ -25,9 +25,9 @@
 // its fp32 tile in its own shared memory and the CTAs of the cluster add a share of the columns
 // each, in slice order, over distributed shared memory -- deterministic.
 //
-// Every wait is bounded (dq_umma.cuh): when one runs out the block stops issuing, drains its own
-// copies, frees its tensor memory, leaves its output unwritten and raises the device's error word
-// (dq_gemm_status).
+// Every wait is bounded (dq_umma.cuh): when one runs out the block's roles stop one after the other, its
+// copies and MMAs in flight are drained, its tensor memory is freed, its output is left incomplete and
+// the device's error word is raised (dq_gemm_status).
 #include <algorithm>
 #include <cmath>
 
@@ -61,6 +61,7 @@ struct Params {
   int x_slots, w_slots, w_bytes;       // rings; bytes of a weight slot
   int x_slabs;                         // slabs of 64 values in an activation slot: 2 (a chunk) or 1
   int slices;
+  int give_up;                         // dq_gemm_fail_next
   uint32_t ring_offset, barrier_offset;
 };
 
@@ -76,6 +77,7 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
   extern __shared__ __align__(1024) unsigned char smem[];
   // control block at the front: failure flag, tensor memory address, barriers
   volatile int* failed = reinterpret_cast<volatile int*>(smem);
+  InFlight* left = reinterpret_cast<InFlight*>(smem + 8);
   const uint32_t base = smem_addr(smem);
   const Bars bars = bars_at(base + p.barrier_offset);
   const int x_slabs = SPLIT ? 2 : p.x_slabs;
@@ -86,7 +88,7 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    *failed = 0;
+    *failed = p.give_up;
     init_bars(bars, p.x_slots, p.w_slots, kGroups, 4 * kGroups);
     tma_prefetch_map(&p.xmap);
   }
@@ -139,7 +141,7 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
           }
         }
       }
-      if (!ok || *failed != 0) drain_copies(full, issued, slots);
+      left->issued[warp] = issued;
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -177,7 +179,7 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
         }
         if (ok) mma_commit(bars.d_full + buffer * 8);
       }
-      if (*failed != 0) drain_mma(bars);
+      left->mma_lane = lane;
     }
     __syncwarp();
   } else if (warp >= kDecodeWarp0) {
@@ -237,6 +239,10 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
   }
 
   __syncthreads();
+  if (*failed != 0) {  // (the same for all: every role has stopped)
+    drain(*left, bars, p.x_slots, p.w_slots);
+    __syncthreads();
+  }
   if (p.slices > 1) {
     // One tile per cluster: add the slices' columns, a share of them per CTA.  A warp takes a column, a
     // lane four of its rows, all slices' loads of two columns requested before the first is used (one
@@ -412,6 +418,7 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
   const int x_bytes = p.n_tile * 128 * p.x_slabs;
   const int groups = split ? Roles<true>::kGroups : Roles<false>::kGroups;
   p.w_slots = std::clamp((budget - p.x_slots * x_bytes) / w_bytes / groups * groups, groups, 12);
+  p.give_up = take_fail_next();
   p.barrier_offset = kBarrierOffset;
   p.ring_offset = kRingOffset;
   const size_t smem = kRingOffset + static_cast<size_t>(p.x_slots) * x_bytes + static_cast<size_t>(p.w_slots) * w_bytes;
@@ -455,6 +462,18 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
 }
 
 }  // namespace dq
+
+namespace dq {
+namespace {
+thread_local int t_fail_next = 0;
+}
+int take_fail_next() { return t_fail_next > 0 ? (--t_fail_next, 1) : 0; }
+}  // namespace dq
+
+extern "C" int32_t dq_gemm_fail_next(int32_t calls) {
+  dq::t_fail_next = std::max(calls, 0);
+  return DQ_OK;
+}
 
 extern "C" int32_t dq_gemm_status(void* stream) {
   auto s = static_cast<cudaStream_t>(stream);

@@ -10,6 +10,9 @@ namespace dq {
 // that are not 64 * 2^n values, rows or pointers that TMA cannot address (16-byte multiples).
 int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaStream_t stream, bool* taken);
 
+// 1 if this call is one of those that dq_gemm_fail_next lets fail, else 0.
+int take_fail_next();
+
 // The failure word of the expert kernels (dq_moe_umma.cu), copied to the host.
 cudaError_t moe_gemm_failed(unsigned int* word, cudaStream_t stream);
 

@@ -127,6 +127,7 @@ struct Params {
   int chunks, bits;
   int n_cap;
   int x_slots, w_slots, w_bytes;
+  int give_up;               // dq_gemm_fail_next
 };
 
 constexpr uint32_t kBarrierOffset = 64, kOrderOffset = 1024, kRingOffset = 3072;
@@ -155,6 +156,7 @@ template <bool BF16, bool MBF16, bool GATE_UP>
 __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   volatile int* failed = reinterpret_cast<volatile int*>(smem);
+  InFlight* left = reinterpret_cast<InFlight*>(smem + 8);
   const uint32_t base = smem_addr(smem);
   const Bars bars = bars_at(base + kBarrierOffset);
   const int x_bytes = p.n_cap * 256;
@@ -163,7 +165,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    *failed = 0;
+    *failed = p.give_up;
     init_bars(bars, p.x_slots, p.w_slots, kGroups, 4);
     tma_prefetch_map(&p.xmap);
     tma_prefetch_map(&p.wmap);
@@ -214,7 +216,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
           }
         }
       }
-      if (!ok || *failed != 0) drain_copies(full, issued, slots);
+      left->issued[warp] = issued;
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -248,7 +250,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
           if (halves.both) mma_commit(bars.d_full + 8);
         }
       }
-      if (*failed != 0) drain_mma(bars);
+      left->mma_lane = lane;
     }
     __syncwarp();
   } else if (warp >= kDecodeWarp0) {
@@ -333,6 +335,10 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
   }
 
   __syncthreads();
+  if (*failed != 0) {  // (the same for all: every role has stopped)
+    drain(*left, bars, p.x_slots, p.w_slots);
+    __syncthreads();
+  }
   if (threadIdx.x == 0 && *failed != 0) atomicOr(&g_moe_failed, 1u);
   fence_after_sync();
   if (warp == 3) tmem_free(tmem, 512);
@@ -508,6 +514,7 @@ int32_t dq_moe_gemm(const void* x, int32_t x_dtype, int64_t tokens, const int32_
   p.tiles = tiles;
   p.order = order;
   p.n_cap = n_cap;
+  p.give_up = dq::take_fail_next();
   p.out = base + lay.h;
   if (const int32_t rc = dq::launch_bank<true>(*gate_up, g_gu, base + lay.xs, x_dtype, assignments, static_cast<int>(inter), p, *dev, s)) return rc;
   p.out = base + lay.d;

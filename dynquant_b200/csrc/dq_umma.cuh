@@ -45,7 +45,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   if (mbar_try(bar, parity)) return true;
   for (int i = 0; i < kSpins; ++i) {
     if (mbar_try(bar, parity)) return true;
-    if ((i & 255) == 255 && *failed != 0) return false;
+    if ((i & 255) == 7 && *failed != 0) return false;
   }
   *failed = 1;
   return false;

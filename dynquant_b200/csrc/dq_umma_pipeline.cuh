@@ -163,17 +163,27 @@ __device__ __forceinline__ void mma_chunk(uint32_t d, uint32_t a, uint64_t b0, u
   mma_slab<SPLIT>(d, a + 32, b1, idesc, true);
 }
 
-// A producer that gives up waits for its copies in flight ...
-__device__ __forceinline__ void drain_copies(uint32_t full, uint32_t issued, uint32_t slots) {
-  for (uint32_t k = issued > slots ? issued - slots : 0; k < issued; ++k) {
-    for (int i = 0; i < kSpins && !mbar_try(full + (k % slots) * 8, (k / slots) & 1); ++i) {
+// What the roles of a block leave in flight when they stop; only a block that gives up looks at it.
+struct InFlight {
+  uint32_t issued[3];  // copies, by the warp that issues them (0 and 2)
+  int mma_lane;        // of warp 1: the thread whose MMAs a commit waits for
+};
+// Called by all threads once every role has stopped -- a producer may have issued its last copy long before
+// another role's wait runs out, so a role cannot do it for itself: waits (bounded) until the copies and the
+// MMAs are through with the memory that is about to change hands.
+__device__ __forceinline__ void drain(const InFlight& left, const Bars& bars, int x_slots, int w_slots) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 1 && lane == left.mma_lane) {
+    mma_commit(bars.drain);
+    for (int i = 0; i < kSpins && !mbar_try(bars.drain, 0); ++i) {
     }
   }
-}
-// ... and the MMA warp for its MMAs, which read and write tensor memory that is about to be freed.
-__device__ __forceinline__ void drain_mma(const Bars& bars) {
-  mma_commit(bars.drain);
-  for (int i = 0; i < kSpins && !mbar_try(bars.drain, 0); ++i) {
+  if ((warp == 0 || warp == 2) && lane == 0) {
+    const uint32_t issued = left.issued[warp], slots = static_cast<uint32_t>(warp == 2 ? w_slots : x_slots);
+    for (uint32_t k = issued > slots ? issued - slots : 0; k < issued; ++k) {
+      for (int i = 0; i < kSpins && !mbar_try((warp == 2 ? bars.w_full : bars.x_full) + (k % slots) * 8, (k / slots) & 1); ++i) {
+      }
+    }
   }
 }
 

@@ -196,6 +196,10 @@ DQ_API int32_t dq_matmul_shards(const void* x, int32_t x_dtype, int64_t m, const
 /* Synchronises `stream`; DQ_ERR_DEVICE once a bounded wait inside one of these kernels has run out
  * on the current device (its output is then incomplete; the context stays usable). */
 DQ_API int32_t dq_gemm_status(void* stream);
+/* Failure-handling hook: the calling thread's next `calls` launches of the tcgen05 kernels start as if a
+ * wait in every block had just run out -- they stop, leave their outputs incomplete and report it, the
+ * way the tests exercise that path without hanging anything. */
+DQ_API int32_t dq_gemm_fail_next(int32_t calls);
 
 /* One GEMV of a sequence; see dq_gemv_sequence. */
 typedef struct dq_gemv_job {

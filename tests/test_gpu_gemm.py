@@ -110,6 +110,20 @@ def test_an_expert_layer_over_many_tokens_matches_its_small_calls(tokens, expert
     assert (outs[0][1:-1] - want).norm() / want.norm() <= (1e-3 if act == torch.bfloat16 else 2e-4)
 
 
+def gemm(x, qt):
+    """``dq_gemm_shards`` of one matrix."""
+    import ctypes
+
+    from dynquant_b200 import _lib, ops
+
+    lib, tag = _lib.load(), _lib.DQ_BF16 if x.dtype == torch.bfloat16 else _lib.DQ_F16
+    w = ops.weight_descriptor("gemm", qt.packed, qt.scales, qt.offsets, qt.bits, qt.geometry.effective_group, qt.in_features)
+    out = torch.empty(x.shape[0], qt.num_rows, dtype=x.dtype, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    _lib.check(lib.dq_gemm_shards(x.data_ptr(), tag, x.shape[0], ctypes.byref(w), 1, None, out.data_ptr(), qt.num_rows, tag, stream))
+    return out
+
+
 def moe_gemm(x, ids, weights, gate_up, down, experts, *, first_expert=0):
     """``dq_moe_gemm`` with fp32 results."""
     import ctypes
@@ -125,7 +139,6 @@ def moe_gemm(x, ids, weights, gate_up, down, experts, *, first_expert=0):
     y = torch.empty(tokens, hidden, device="cuda")
     _lib.check(lib.dq_moe_gemm(x.data_ptr(), tag, tokens, ids.data_ptr(), weights.data_ptr(), topk, first_expert, experts, ctypes.byref(banks[0]),
                                ctypes.byref(banks[1]), hidden, inter, y.data_ptr(), _lib.DQ_F32, scratch.data_ptr(), need.value, stream))
-    assert lib.dq_gemm_status(stream) == _lib.DQ_OK
     return y
 
 
@@ -141,3 +154,36 @@ def test_an_expert_layer_over_more_tokens_than_a_grid_has_rows():
     whole = moe_gemm(x, ids, weights, gate_up, down, experts)
     parts = [moe_gemm(x[i:i + 30000], ids[i:i + 30000], weights[i:i + 30000], gate_up, down, experts) for i in range(0, tokens, 30000)]
     assert torch.equal(whole, torch.cat(parts))
+
+
+def _give_up_and_recover() -> None:
+    """In a process of its own: the word that the kernels raise stays."""
+    from dynquant_b200 import _lib
+    from dynquant_b200.workloads import random_quant_tensor, seeded_routing
+
+    lib, gen = _lib.load(), torch.Generator(device="cuda").manual_seed(1)
+    for m, rows, k in ((24, 1000, 4096), (40, 20000, 512), (300, 1000, 2048), (4096, 4096, 512)):  # sliced and not, split and not
+        qt = random_quant_tensor(rows, k, 4, meta_dtype=torch.float16, device="cuda", generator=gen)
+        x = torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16)
+        want = gemm(x, qt)
+        for _ in range(3):
+            lib.dq_gemm_fail_next(1)
+            gemm(x, qt)
+        assert lib.dq_gemm_status(None) == _lib.DQ_ERR_DEVICE
+        assert torch.equal(gemm(x, qt), want)
+    bank = [random_quant_tensor(n, k, 3, meta_dtype=torch.float16, device="cuda", generator=gen) for n, k in ((8 * 512, 512), (8 * 512, 256))]
+    ids, weights = seeded_routing(200, 8, 2, seed=1, device="cuda")
+    x = torch.randn(200, 512, device="cuda", generator=gen).to(torch.bfloat16)
+    want = moe_gemm(x, ids, weights, *bank, 8)
+    lib.dq_gemm_fail_next(1)
+    moe_gemm(x, ids, weights, *bank, 8)
+    assert torch.equal(moe_gemm(x, ids, weights, *bank, 8), want)
+
+
+def test_a_block_that_gives_up_leaves_the_device_usable():
+    import multiprocessing
+
+    child = multiprocessing.get_context("spawn").Process(target=_give_up_and_recover)
+    child.start()
+    child.join(300)
+    assert child.exitcode == 0
