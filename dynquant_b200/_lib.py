@@ -137,6 +137,7 @@ SIGNATURES = {
     "dq_gemv_shards_rows": (_I32, [_P, _I32, _I64, _WP, _I32, _P, _P, _I64, _I32, _P]),
     "dq_gemm_shards": (_I32, [_P, _I32, _I64, _WP, _I32, _P, _P, _I64, _I32, _P]),
     "dq_matmul_shards": (_I32, [_P, _I32, _I64, _WP, _I32, _P, _P, _I64, _I32, _P]),
+    "dq_poll_status": (_I32, [_I32]),
     "dq_gemm_status": (_I32, [_P]),
     "dq_gemm_fail_next": (_I32, [_I32]),
     "dq_gemv_sequence": (_I32, [ctypes.POINTER(GemvJob), _I32, _P]),

@@ -29,11 +29,14 @@ void note_kernel(const char* name) { t_last_kernel = name; }
 const char* last_kernel() { return t_last_kernel; }
 int64_t launches_so_far() { return g_launches.load(std::memory_order_relaxed); }
 
+namespace {
+constexpr int kMaxDevices = 64;
+DeviceInfo cache[kMaxDevices];
+std::atomic<bool> ready[kMaxDevices];
+std::mutex mu;
+}  // namespace
+
 const DeviceInfo* device_info() {
-  constexpr int kMaxDevices = 64;
-  static DeviceInfo cache[kMaxDevices];
-  static std::atomic<bool> ready[kMaxDevices];
-  static std::mutex mu;
   int device = 0;
   cudaError_t err = cudaGetDevice(&device);
   if (err != cudaSuccess || device < 0 || device >= kMaxDevices) {
@@ -54,10 +57,37 @@ const DeviceInfo* device_info() {
       fail(DQ_ERR_CUDA, "cudaDeviceGetAttribute failed: %s", cudaGetErrorString(err));
       return nullptr;
     }
+    // Once per device and process; a call that is the first one inside a stream capture may do this too.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    void *host = nullptr, *mapped = nullptr;
+    err = cudaThreadExchangeStreamCaptureMode(&mode);
+    if (err == cudaSuccess) {
+      err = cudaHostAlloc(&host, kReportWords * sizeof(unsigned int), cudaHostAllocPortable | cudaHostAllocMapped);
+      if (err == cudaSuccess) err = cudaHostGetDevicePointer(&mapped, host, 0);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    if (err != cudaSuccess || mapped != host) {  // (one address space: the kernels' address is the host's)
+      fail(DQ_ERR_CUDA, "no host memory for the kernels' reports: %s", cudaGetErrorString(err));
+      return nullptr;
+    }
+    info.report = static_cast<unsigned int*>(host);
+    for (int i = 0; i < kReportWords; ++i) info.report[i] = 0u;
     cache[device] = info;
     ready[device].store(true, std::memory_order_release);
   }
   return &cache[device];
+}
+
+int32_t take_report(int device) {
+  if (device < 0 || device >= kMaxDevices || !ready[device].load(std::memory_order_acquire)) return DQ_OK;  // (nothing has run there)
+  unsigned int* report = cache[device].report;
+  const auto taken = [&](Report what) {
+    return __atomic_load_n(report + what, __ATOMIC_RELAXED) != 0u && __atomic_exchange_n(report + what, 0u, __ATOMIC_RELAXED) != 0u;
+  };
+  if (taken(kReportWait)) {
+    return fail(DQ_ERR_DEVICE, "gemm: a wait inside a block ran out; an output of an earlier call on this device is incomplete");
+  }
+  return DQ_OK;
 }
 
 namespace {
@@ -115,6 +145,15 @@ extern "C" {
 int64_t dq_launch_count(void) { return dq::launches_so_far(); }
 const char* dq_last_kernel(void) { return dq::last_kernel(); }
 
+
+int32_t dq_poll_status(int32_t device) { return dq::take_report(device); }
+
+int32_t dq_gemm_status(void* stream) {
+  int device = 0;
+  DQ_CUDA(cudaGetDevice(&device));
+  DQ_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
+  return dq::take_report(device);
+}
 
 int32_t dq_abi_version(void) { return DQ_ABI_VERSION; }
 int32_t dq_built_with_cuda(void) { return 1; }

@@ -100,9 +100,17 @@ struct DeviceInfo {
   int device;
   int sm_count;
   int max_smem_optin;  // bytes per CTA
+  unsigned int* report;  // what kernels report (Report), in host memory that the device maps
 };
 // Cached per device; returns nullptr and sets the error on failure.
 const DeviceInfo* device_info();
+
+// Words that a kernel sets to 1 to report something to the host, which sees them without a
+// synchronisation of its own once the kernel has run.
+enum Report { kReportWait = 0, kReportWords };
+// DQ_ERR_DEVICE and a message if a kernel on `device` has reported something since the last call that
+// said so, else DQ_OK.  Reads host memory only.
+int32_t take_report(int device);
 
 // What a launch asks the runtime about its kernel, remembered per (kernel, device) on the calling
 // thread: the attribute call costs 0.4 us and the occupancy query 1 us of host time, every launch
@@ -154,6 +162,11 @@ __device__ __forceinline__ float load_f32(const void* __restrict__ p, int64_t i,
     return __uint_as_float(static_cast<uint32_t>(raw) << 16);
   }
   return __ldg(reinterpret_cast<const float*>(p) + i);
+}
+
+// Sets a word of DeviceInfo::report.  (Plain stores of one value: any number of threads may.)
+__device__ __forceinline__ void report_to_host(unsigned int* report, Report what) {
+  *reinterpret_cast<volatile unsigned int*>(report + what) = 1u;
 }
 
 // One rounding (nearest-even) to the tagged dtype.

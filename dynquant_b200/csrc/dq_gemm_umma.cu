@@ -27,7 +27,7 @@
 //
 // Every wait is bounded (dq_umma.cuh): when one runs out the block's roles stop one after the other, its
 // copies and MMAs in flight are drained, its tensor memory is freed, its output is left incomplete and
-// the device's error word is raised (dq_gemm_status).
+// the host is told (DeviceInfo::report).
 #include <algorithm>
 #include <cmath>
 
@@ -62,10 +62,9 @@ struct Params {
   int x_slabs;                         // slabs of 64 values in an activation slot: 2 (a chunk) or 1
   int slices;
   int give_up;                         // dq_gemm_fail_next
+  unsigned int* report;
   uint32_t ring_offset, barrier_offset;
 };
-
-__device__ unsigned int g_gemm_failed = 0;
 
 // SPLIT: the weights enter as the sum of two 16-bit operands, so that nothing of their fp32 values is
 // lost that the sums could show.  Up to DQ_GEMV_CHUNKED_MAX_ROWS activation rows, where the mma.sync
@@ -300,7 +299,7 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
     }
     cluster_sync();  // nobody leaves while its sums are being read
   }
-  if (threadIdx.x == 0 && *failed != 0) atomicOr(&g_gemm_failed, 1u);
+  if (threadIdx.x == 0 && *failed != 0) report_to_host(p.report, kReportWait);
   fence_after_sync();
   if (warp == 3) tmem_free(tmem, static_cast<uint32_t>(p.tmem_columns));
 }
@@ -419,6 +418,7 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
   const int groups = split ? Roles<true>::kGroups : Roles<false>::kGroups;
   p.w_slots = std::clamp((budget - p.x_slots * x_bytes) / w_bytes / groups * groups, groups, 12);
   p.give_up = take_fail_next();
+  p.report = dev->report;
   p.barrier_offset = kBarrierOffset;
   p.ring_offset = kRingOffset;
   const size_t smem = kRingOffset + static_cast<size_t>(p.x_slots) * x_bytes + static_cast<size_t>(p.w_slots) * w_bytes;
@@ -472,15 +472,5 @@ int take_fail_next() { return t_fail_next > 0 ? (--t_fail_next, 1) : 0; }
 
 extern "C" int32_t dq_gemm_fail_next(int32_t calls) {
   dq::t_fail_next = std::max(calls, 0);
-  return DQ_OK;
-}
-
-extern "C" int32_t dq_gemm_status(void* stream) {
-  auto s = static_cast<cudaStream_t>(stream);
-  unsigned int word = 0, moe = 0;
-  DQ_CUDA(dq::moe_gemm_failed(&moe, s));
-  DQ_CUDA(cudaMemcpyFromSymbolAsync(&word, dq::g_gemm_failed, sizeof(word), 0, cudaMemcpyDeviceToHost, s));
-  DQ_CUDA(cudaStreamSynchronize(s));
-  if ((word | moe) != 0u) return dq::fail(DQ_ERR_DEVICE, "gemm: a wait inside a block ran out; an output of this device is incomplete");
   return DQ_OK;
 }

@@ -13,7 +13,4 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
 // 1 if this call is one of those that dq_gemm_fail_next lets fail, else 0.
 int take_fail_next();
 
-// The failure word of the expert kernels (dq_moe_umma.cu), copied to the host.
-cudaError_t moe_gemm_failed(unsigned int* word, cudaStream_t stream);
-
 }  // namespace dq

@@ -43,8 +43,6 @@ constexpr int kThreads = (kEpilogueWarp0 + 4) * 32;
 constexpr int kBoxRows = 32;
 constexpr int kColumns = 128;          // accumulator columns: one tile of up to 128 tokens, or two of up to 64
 
-__device__ unsigned int g_moe_failed = 0;
-
 struct RouteTable {
   int num_tiles, num_rows, pad[2];  // column tiles; assignments that belong to a local expert
 };
@@ -128,6 +126,7 @@ struct Params {
   int n_cap;
   int x_slots, w_slots, w_bytes;
   int give_up;               // dq_gemm_fail_next
+  unsigned int* report;
 };
 
 constexpr uint32_t kBarrierOffset = 64, kOrderOffset = 1024, kRingOffset = 3072;
@@ -339,7 +338,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
     drain(*left, bars, p.x_slots, p.w_slots);
     __syncthreads();
   }
-  if (threadIdx.x == 0 && *failed != 0) atomicOr(&g_moe_failed, 1u);
+  if (threadIdx.x == 0 && *failed != 0) report_to_host(p.report, kReportWait);
   fence_after_sync();
   if (warp == 3) tmem_free(tmem, 512);
 }
@@ -439,10 +438,6 @@ int32_t launch_bank(const dq_weight& w, const dq_geometry& g, const void* act, i
 
 }  // namespace
 
-cudaError_t moe_gemm_failed(unsigned int* word, cudaStream_t stream) {
-  return cudaMemcpyFromSymbolAsync(word, g_moe_failed, sizeof(*word), 0, cudaMemcpyDeviceToHost, stream);
-}
-
 }  // namespace dq
 
 extern "C" {
@@ -515,6 +510,7 @@ int32_t dq_moe_gemm(const void* x, int32_t x_dtype, int64_t tokens, const int32_
   p.order = order;
   p.n_cap = n_cap;
   p.give_up = dq::take_fail_next();
+  p.report = dev->report;
   p.out = base + lay.h;
   if (const int32_t rc = dq::launch_bank<true>(*gate_up, g_gu, base + lay.xs, x_dtype, assignments, static_cast<int>(inter), p, *dev, s)) return rc;
   p.out = base + lay.d;

@@ -138,7 +138,15 @@ at::Tensor new_cuda(at::IntArrayRef sizes, at::ScalarType dtype, at::Device devi
   return at::Tensor(at::detail::empty_cuda(sizes, dtype, device, std::nullopt));
 }
 
-// Runs `body` without the GIL on `device`; wraps the tensor it returns (undefined: not handled).
+struct LibraryError : std::runtime_error {
+  using std::runtime_error::runtime_error;
+};
+void check(int32_t rc) {
+  if (rc != DQ_OK) throw LibraryError(dq_last_error());
+}
+
+// Runs `body` without the GIL on `device`; wraps the tensor it returns (undefined: not handled).  What
+// the kernels of earlier calls on the device have reported by now is raised first.
 template <typename Body>
 PyObject* on_device(at::Device device, Body body) {
   try {
@@ -149,6 +157,7 @@ PyObject* on_device(at::Device device, Body body) {
         ~Release() { PyEval_RestoreThread(state); }
       } release;
       const c10::cuda::CUDAGuard guard(device);
+      check(dq_poll_status(device.index()));
       out = body(at::cuda::getCurrentCUDAStream().stream());
     }
     return out.defined() ? THPVariable_Wrap(std::move(out)) : unhandled();
@@ -158,13 +167,6 @@ PyObject* on_device(at::Device device, Body body) {
     PyErr_SetString(PyExc_RuntimeError, e.what());
   }
   return nullptr;
-}
-
-struct LibraryError : std::runtime_error {
-  using std::runtime_error::runtime_error;
-};
-void check(int32_t rc) {
-  if (rc != DQ_OK) throw LibraryError(dq_last_error());
 }
 
 // x [.., K] against n shards side by side.

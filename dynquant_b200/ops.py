@@ -343,6 +343,15 @@ def gemv_max_rows() -> int:
     return int(_lib.load().dq_gemv_max_rows())
 
 
+def check_status(device: torch.device | None = None) -> None:
+    """Waits for the current stream of ``device`` and raises what the kernels of earlier calls there have
+    reported (``dq_gemm_status``).  Every call through the compiled host path raises the same, without the
+    wait, for what had been reported when it was made; a report is raised once."""
+    device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
+    with torch.cuda.device(device):
+        _lib.check(_lib.load().dq_gemm_status(_stream(device)))
+
+
 def launch_count() -> int:
     """Kernels the library has launched in this process so far (``dq_launch_count``)."""
     return int(_lib.load().dq_launch_count())

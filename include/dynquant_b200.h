@@ -193,8 +193,11 @@ DQ_API int32_t dq_gemm_shards(const void* x, int32_t x_dtype, int64_t m, const d
 DQ_API int32_t dq_matmul_shards(const void* x, int32_t x_dtype, int64_t m, const dq_weight* shards,
                                 int32_t num_shards, const void* bias, void* out, int64_t out_stride,
                                 int32_t out_dtype, void* stream);
-/* Synchronises `stream`; DQ_ERR_DEVICE once a bounded wait inside one of these kernels has run out
- * on the current device (its output is then incomplete; the context stays usable). */
+/* What the kernels of earlier calls have reported: DQ_ERR_DEVICE, once, after a bounded wait inside one
+ * of the tcgen05 kernels has run out (an output is then incomplete; the context stays usable), else
+ * DQ_OK.  dq_poll_status reads host memory only: it sees what kernels on `device` (its number) that have
+ * run by now reported.  dq_gemm_status synchronises `stream` first and asks for the current device. */
+DQ_API int32_t dq_poll_status(int32_t device);
 DQ_API int32_t dq_gemm_status(void* stream);
 /* Failure-handling hook: the calling thread's next `calls` launches of the tcgen05 kernels start as if a
  * wait in every block had just run out -- they stop, leave their outputs incomplete and report it, the

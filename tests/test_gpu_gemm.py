@@ -156,9 +156,8 @@ def test_an_expert_layer_over_more_tokens_than_a_grid_has_rows():
     assert torch.equal(whole, torch.cat(parts))
 
 
-def _give_up_and_recover() -> None:
-    """In a process of its own: the word that the kernels raise stays."""
-    from dynquant_b200 import _lib
+def test_a_block_that_gives_up_reports_it_and_leaves_the_device_usable():
+    from dynquant_b200 import _lib, ops
     from dynquant_b200.workloads import random_quant_tensor, seeded_routing
 
     lib, gen = _lib.load(), torch.Generator(device="cuda").manual_seed(1)
@@ -169,7 +168,9 @@ def _give_up_and_recover() -> None:
         for _ in range(3):
             lib.dq_gemm_fail_next(1)
             gemm(x, qt)
-        assert lib.dq_gemm_status(None) == _lib.DQ_ERR_DEVICE
+        with pytest.raises(RuntimeError, match="ran out"):
+            ops.check_status()
+        ops.check_status()  # once
         assert torch.equal(gemm(x, qt), want)
     bank = [random_quant_tensor(n, k, 3, meta_dtype=torch.float16, device="cuda", generator=gen) for n, k in ((8 * 512, 512), (8 * 512, 256))]
     ids, weights = seeded_routing(200, 8, 2, seed=1, device="cuda")
@@ -177,13 +178,21 @@ def _give_up_and_recover() -> None:
     want = moe_gemm(x, ids, weights, *bank, 8)
     lib.dq_gemm_fail_next(1)
     moe_gemm(x, ids, weights, *bank, 8)
+    torch.cuda.synchronize()
+    assert lib.dq_poll_status(0) == _lib.DQ_ERR_DEVICE and lib.dq_poll_status(0) == _lib.DQ_OK
     assert torch.equal(moe_gemm(x, ids, weights, *bank, 8), want)
 
 
-def test_a_block_that_gives_up_leaves_the_device_usable():
-    import multiprocessing
+def test_a_module_raises_what_its_last_call_reported():
+    from dynquant_b200 import _lib
+    from dynquant_b200.runtime import DynQuantLinear
 
-    child = multiprocessing.get_context("spawn").Process(target=_give_up_and_recover)
-    child.start()
-    child.join(300)
-    assert child.exitcode == 0
+    layer = DynQuantLinear(random_qt(512, 1024, 3, meta=torch.bfloat16, seed=1))
+    x = torch.randn(100, 1024, device="cuda").to(torch.bfloat16)
+    want = layer(x)
+    _lib.load().dq_gemm_fail_next(1)
+    layer(x)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="ran out"):
+        layer(x)
+    assert torch.equal(layer(x), want)
