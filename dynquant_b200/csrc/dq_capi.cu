@@ -87,6 +87,9 @@ int32_t take_report(int device) {
   if (taken(kReportWait)) {
     return fail(DQ_ERR_DEVICE, "gemm: a wait inside a block ran out; an output of an earlier call on this device is incomplete");
   }
+  if (taken(kReportId)) {
+    return fail(DQ_ERR_DEVICE, "embedding lookup: an earlier call on this device was given an id outside its table (its row is NaN)");
+  }
   return DQ_OK;
 }
 

@@ -107,7 +107,7 @@ const DeviceInfo* device_info();
 
 // Words that a kernel sets to 1 to report something to the host, which sees them without a
 // synchronisation of its own once the kernel has run.
-enum Report { kReportWait = 0, kReportWords };
+enum Report { kReportWait = 0, kReportId, kReportWords };
 // DQ_ERR_DEVICE and a message if a kernel on `device` has reported something since the last call that
 // said so, else DQ_OK.  Reads host memory only.
 int32_t take_report(int device);

@@ -21,6 +21,7 @@
 // contiguous LSB-first bit string: groups are whole numbers of 32-value blocks).  dequant_kernel
 // is the general one: one thread per block of 16/32/8/4 values at 2/3/4/8-bit, any tail.
 #include <algorithm>
+#include <type_traits>
 
 #include "dq_decode.cuh"
 
@@ -37,16 +38,17 @@ struct DequantArgs {
   const void* ids;       // null, or the packed row of every output row
   int ids_are_32;        // int32 ids (else int64)
   int table_rows;        // rows of the packed tensor (ids lie below it)
+  unsigned int* report;  // an id that does not is reported
   int meta_dtype, out_dtype;
   int rows;              // output rows
   int words_per_row, num_groups, words_per_group, group_values, in_features;
   int blocks_per_group, blocks_per_row;
 };
 
-// Which packed row an output row comes from: itself, or (an embedding lookup) the id at its place.
-// An id outside the table gives -1.
+// Which packed row an output row of an embedding lookup comes from: the id at its place.
+// An id outside the table gives -1 -- the kernels then write a row of NaN and report it, which the host
+// raises: the gather that this replaces failed a device assertion, which costs the caller the context.
 __device__ __forceinline__ int source_row(const DequantArgs& a, int row) {
-  if (a.ids == nullptr) return row;
   const int64_t id = a.ids_are_32 ? static_cast<int64_t>(__ldg(static_cast<const int*>(a.ids) + row))
                                   : static_cast<int64_t>(__ldg(static_cast<const long long*>(a.ids) + row));
   return id >= 0 && id < a.table_rows ? static_cast<int>(id) : -1;
@@ -58,10 +60,10 @@ __device__ __forceinline__ int source_row(const DequantArgs& a, int row) {
 // the high half of its product with an octet's number is the octet's row (exact below 2^32).
 //
 // Bound by the stores (2 bytes written per value, bits/8 read): 14336 x 4096 at 3 / 4 / 8 bits takes
-// 39 / 37 / 37 us where filling the output with zeros takes 33.  (Octets over blockIdx.x and rows
+// 38 / 37 / 37 us where filling the output with zeros takes 33.  (Octets over blockIdx.x and rows
 // over blockIdx.y, one octet per thread: 52 / 44 / 44 -- and 14 us against 10 on 14080 x 768, whose
 // rows left most threads of a CTA idle.)  256 threads and 4 octets: 43; 2 octets: 39 to 41.
-template <int BITS, int U>
+template <int BITS, int U, bool IDS>
 __global__ void __launch_bounds__(kDequantThreads) dequant_octet_kernel(const DequantArgs a, unsigned octets_per_row,
                                                                         unsigned long long per_row_magic, unsigned total,
                                                                         int group_shift) {
@@ -79,9 +81,9 @@ __global__ void __launch_bounds__(kDequantThreads) dequant_octet_kernel(const De
     if (at < total) {
       const int row = static_cast<int>(__umul64hi(at, per_row_magic));
       const int o = static_cast<int>(at - row * octets_per_row);
-      const int from = source_row(a, row);
-      known[u] = from >= 0;
-      if (from >= 0) {
+      const int from = IDS ? source_row(a, row) : row;
+      if constexpr (IDS) known[u] = from >= 0;
+      if (!IDS || from >= 0) {
         const int bit = o * 8 * BITS;
         const int word = bit >> 5;
         const uint32_t* src = a.packed + static_cast<int64_t>(from) * a.words_per_row;
@@ -124,8 +126,9 @@ __global__ void __launch_bounds__(kDequantThreads) dequant_octet_kernel(const De
         vals[i] = __fmul_rn(qf, scale[u]);
         if (has_offsets) vals[i] = __fadd_rn(vals[i], offset[u]);
       }
-      if (!known[u]) vals[i] = __int_as_float(0x7FC00000);
+      if (IDS && !known[u]) vals[i] = __int_as_float(0x7FC00000);
     }
+    if (IDS && !known[u]) report_to_host(a.report, kReportId);
     // rows are whole octets, so octet `at` of the output starts at value 8 * at
     if (a.out_dtype == DQ_F32) {
       float4* dst = reinterpret_cast<float4*>(a.out) + static_cast<size_t>(at) * 2;
@@ -166,8 +169,9 @@ __global__ void __launch_bounds__(kDequantThreads) dequant_kernel(const DequantA
       continue;
     }
     const int64_t out_base = static_cast<int64_t>(row) * a.in_features + value_base;
-    const int from = source_row(a, row);
+    const int from = a.ids == nullptr ? row : source_row(a, row);
     if (from < 0) {
+      report_to_host(a.report, kReportId);
       for (int j = 0; j < live; ++j) store_f32(a.out, out_base + j, a.out_dtype, __int_as_float(0x7FC00000));
       continue;
     }
@@ -277,6 +281,7 @@ int32_t launch_dequant(const dq_weight* w, const dq_geometry& g, const void* ids
 
   const DeviceInfo* dev = device_info();
   if (dev == nullptr) return DQ_ERR_CUDA;
+  a.report = dev->report;
   // The octet kernel: whole octets per row and per group, 16-byte aligned output rows, and
   // (8-bit) 8-byte aligned packed rows.
   const size_t out_elem = static_cast<size_t>(dtype_size(out_dtype));
@@ -297,19 +302,20 @@ int32_t launch_dequant(const dq_weight* w, const dq_geometry& g, const void* ids
     // than loads in flight (6912 x 1024, 0.9 M octets: 7.1 us with one, 8.3 with four).
     const bool four = num_octets >= static_cast<int64_t>(dev->sm_count) * 2048 * 4;
     const unsigned grid = static_cast<unsigned>(ceil_div(num_octets, kDequantThreads * (four ? 4 : 1)));
-    switch (w->bits) {
-      case 2:
-        (four ? dequant_octet_kernel<2, 4> : dequant_octet_kernel<2, 1>)<<<grid, kDequantThreads, 0, s>>>(a, per_row, magic, total, shift);
-        break;
-      case 3:
-        (four ? dequant_octet_kernel<3, 4> : dequant_octet_kernel<3, 1>)<<<grid, kDequantThreads, 0, s>>>(a, per_row, magic, total, shift);
-        break;
-      case 4:
-        (four ? dequant_octet_kernel<4, 4> : dequant_octet_kernel<4, 1>)<<<grid, kDequantThreads, 0, s>>>(a, per_row, magic, total, shift);
-        break;
-      default:
-        (four ? dequant_octet_kernel<8, 4> : dequant_octet_kernel<8, 1>)<<<grid, kDequantThreads, 0, s>>>(a, per_row, magic, total, shift);
-        break;
+    const auto run = [&](auto ids) {
+      constexpr bool IDS = decltype(ids)::value;
+      const auto pick = [&](auto one, auto many) { (four ? many : one)<<<grid, kDequantThreads, 0, s>>>(a, per_row, magic, total, shift); };
+      switch (w->bits) {
+        case 2: pick(dequant_octet_kernel<2, 1, IDS>, dequant_octet_kernel<2, 4, IDS>); break;
+        case 3: pick(dequant_octet_kernel<3, 1, IDS>, dequant_octet_kernel<3, 4, IDS>); break;
+        case 4: pick(dequant_octet_kernel<4, 1, IDS>, dequant_octet_kernel<4, 4, IDS>); break;
+        default: pick(dequant_octet_kernel<8, 1, IDS>, dequant_octet_kernel<8, 4, IDS>); break;
+      }
+    };
+    if (a.ids != nullptr) {
+      run(std::true_type{});
+    } else {
+      run(std::false_type{});
     }
     DQ_CHECK_LAUNCH("dequant");
     return DQ_OK;

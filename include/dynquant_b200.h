@@ -123,7 +123,8 @@ DQ_API int32_t dq_resolve_geometry(const char* op, const dq_weight* w, dq_geomet
 DQ_API int32_t dq_dequant(const dq_weight* w, void* out, int32_t out_dtype, void* stream);
 /* Embedding lookup (reference: embedding_lookup, runtime/ops.py:234-260, three gathers and a
  * dequant): out [count, in_features] = the dense rows `ids` (device array of int64, or int32) of
- * the table, in one launch.  An id outside the table gives a row of NaN. */
+ * the table, in one launch.  An id outside the table gives a row of NaN and is reported
+ * (dq_poll_status). */
 DQ_API int32_t dq_dequant_rows(const dq_weight* w, const void* ids, int32_t ids_are_int32, int64_t count,
                                void* out, int32_t out_dtype, void* stream);
 
@@ -194,8 +195,8 @@ DQ_API int32_t dq_matmul_shards(const void* x, int32_t x_dtype, int64_t m, const
                                 int32_t num_shards, const void* bias, void* out, int64_t out_stride,
                                 int32_t out_dtype, void* stream);
 /* What the kernels of earlier calls have reported: DQ_ERR_DEVICE, once, after a bounded wait inside one
- * of the tcgen05 kernels has run out (an output is then incomplete; the context stays usable), else
- * DQ_OK.  dq_poll_status reads host memory only: it sees what kernels on `device` (its number) that have
+ * of the tcgen05 kernels has run out (an output is then incomplete; the context stays usable), or after
+ * an embedding lookup with an id outside its table; else DQ_OK.  dq_poll_status reads host memory only: it sees what kernels on `device` (its number) that have
  * run by now reported.  dq_gemm_status synchronises `stream` first and asks for the current device. */
 DQ_API int32_t dq_poll_status(int32_t device);
 DQ_API int32_t dq_gemm_status(void* stream);

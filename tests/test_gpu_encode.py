@@ -87,3 +87,25 @@ def test_a_call_right_behind_the_encoder_waits_for_its_words(m):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("bad", [300, -1, 2**40])
+@pytest.mark.parametrize("k", [512, 100])
+def test_an_id_outside_the_table_is_raised_by_the_next_call(k, bad):
+    from dynquant_b200 import QuantTensor, ops
+    from dynquant_b200.runtime import DynQuantEmbedding
+
+    table = DynQuantEmbedding(QuantTensor.from_dense(torch.randn(300, k), bits=4, group_size=-1, compute_dtype=torch.bfloat16).to("cuda"))
+    good = torch.tensor([0, 299, 7], device="cuda")
+    want = table(good)
+    ids = torch.tensor([0, bad, 7], device="cuda")
+    rows = table(ids)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="id outside"):
+        table(good)
+    assert torch.equal(table(good), want)  # raised once
+    assert torch.equal(rows[::2], want[::2]) and bool(rows[1].isnan().all())
+    table(ids)
+    with pytest.raises(RuntimeError, match="id outside"):
+        ops.check_status()
+    ops.check_status()
