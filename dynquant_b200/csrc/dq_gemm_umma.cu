@@ -66,6 +66,9 @@ struct Params {
   uint32_t ring_offset, barrier_offset;
 };
 
+constexpr uint32_t kBarrierOffset = 64, kRingOffset = 1024;
+static_assert(kBarrierOffset + kBarrierBytes <= kRingOffset, "");
+
 // SPLIT: the weights enter as the sum of two 16-bit operands, so that nothing of their fp32 values is
 // lost that the sums could show.  Up to DQ_GEMV_CHUNKED_MAX_ROWS activation rows, where the mma.sync
 // kernels scale fp32 accumulators and never round a weight; above that the dense path this kernel
@@ -86,6 +89,24 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
+  // this CTA's share of the reduction axis (slices: as equal as possible, in chunks)
+  const int slice = static_cast<int>(blockIdx.y);
+  const int c0 = static_cast<int>(static_cast<int64_t>(p.chunks) * slice / p.slices);
+  const int c1 = static_cast<int>(static_cast<int64_t>(p.chunks) * (slice + 1) / p.slices);
+
+  auto job_of = [&](int row_tile, int& local) -> int {
+    int j = 0;
+    local = row_tile;
+    while (j + 1 < p.jobs && local >= p.job[j].row_tiles) local -= p.job[j++].row_tiles;
+    return j;
+  };
+
+  // groups [g0, g0 + groups_of(job)) hold the values of this share
+  const auto first_group = [&](const Job& job) -> int { return (2 * c0) >> job.meta.group_shift; };
+  const auto groups_of = [&](const Job& job) -> int {
+    return min((2 * c1 - 1) >> job.meta.group_shift, job.meta.num_groups - 1) - first_group(job) + 1;
+  };
+
   if (threadIdx.x == 0) {
     *failed = p.give_up;
     init_bars(bars, p.x_slots, p.w_slots, kGroups, 4 * kGroups);
@@ -98,18 +119,6 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + 4);
   const uint32_t d_tmem = tmem + Roles<SPLIT>::kColumns;
   pdl_launch_dependents();
-
-  // this CTA's share of the reduction axis (slices: as equal as possible, in chunks)
-  const int slice = static_cast<int>(blockIdx.y);
-  const int c0 = static_cast<int>(static_cast<int64_t>(p.chunks) * slice / p.slices);
-  const int c1 = static_cast<int>(static_cast<int64_t>(p.chunks) * (slice + 1) / p.slices);
-
-  auto job_of = [&](int row_tile, int& local) -> int {
-    int j = 0;
-    local = row_tile;
-    while (j + 1 < p.jobs && local >= p.job[j].row_tiles) local -= p.job[j++].row_tiles;
-    return j;
-  };
 
   if (warp == 0 || warp == 2) {
     if (elect_one()) {
@@ -194,8 +203,13 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
     for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, d_at.advance(static_cast<uint32_t>(p.d_buffers)), stage += stages) {
       int local;
       const Job& job = p.job[job_of(tile % p.row_tiles, local)];
+      float power = 1.0f, back = 1.0f;
+      if constexpr (kScaledRows<BF16, SPLIT>) {
+        const int k = row_power<MBF16>(job.meta, job.bits, min(local * 128 + r, job.rows - 1), first_group(job), groups_of(job));
+        power = power_of_two(k), back = power_of_two(-k);
+      }
       bool ok;
-#define DQ_DECODE(B) ok = decode_tile<B, BF16, MBF16, SPLIT>(job.meta, min(local * 128 + r, job.rows - 1), r, c0, group, stage, stages, ring, bars, tmem, w_at, a_pass, failed)
+#define DQ_DECODE(B) ok = decode_tile<B, BF16, MBF16, SPLIT>(job.meta, min(local * 128 + r, job.rows - 1), r, power, c0, group, stage, stages, ring, bars, tmem, w_at, a_pass, failed)
       switch (job.bits) {
         case 2: DQ_DECODE(2); break;
         case 3: DQ_DECODE(3); break;
@@ -217,6 +231,10 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
         uint32_t v[16];
         tmem_ld16(src + col, v);
         tmem_wait_ld();
+        if constexpr (kScaledRows<BF16, SPLIT>) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * back);
+        }
         if (p.slices > 1) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) red[(col + i) * 128 + r] = __uint_as_float(v[i]);
@@ -307,9 +325,6 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
 // ---------------------------------------------------------------------------
 // Host
 // ---------------------------------------------------------------------------
-
-constexpr uint32_t kBarrierOffset = 64;
-constexpr uint32_t kRingOffset = 1024;
 
 bool geometry_ok(const GemvArgs& a, int bits) {
   const bool x16 = a.x_dtype == DQ_BF16 || a.x_dtype == DQ_F16, meta16 = a.meta_dtype == DQ_BF16 || a.meta_dtype == DQ_F16;

@@ -129,7 +129,8 @@ struct Params {
   unsigned int* report;
 };
 
-constexpr uint32_t kBarrierOffset = 64, kOrderOffset = 1024, kRingOffset = 3072;
+constexpr uint32_t kBarrierOffset = 64, kOrderOffset = 1024, kPowersOffset = 3072;
+constexpr uint32_t ring_offset(bool scaled_rows) { return scaled_rows ? 4096 : kPowersOffset; }
 static_assert(kBarrierOffset + kBarrierBytes <= kOrderOffset, "");
 
 // Where a tile's accumulator lies.  Tiles of up to 64 tokens take the two halves of the columns in turn
@@ -159,13 +160,14 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
   const uint32_t base = smem_addr(smem);
   const Bars bars = bars_at(base + kBarrierOffset);
   const int x_bytes = p.n_cap * 256;
-  unsigned char* x_ring = smem + kRingOffset;
+  unsigned char* x_ring = smem + ring_offset(kScaledRows<BF16, true>);
+  signed char* powers = reinterpret_cast<signed char*>(smem + kPowersOffset);  // of a tile's rows, by slot
   unsigned char* w_ring = x_ring + p.x_slots * x_bytes;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     *failed = p.give_up;
-    init_bars(bars, p.x_slots, p.w_slots, kGroups, 4);
+    init_bars(bars, p.x_slots, p.w_slots, kGroups, 4, 4, 4 * kGroups + 4);
     tma_prefetch_map(&p.xmap);
     tma_prefetch_map(&p.wmap);
   }
@@ -181,6 +183,13 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
   const int tiles = __ldcg(&p.table->num_tiles) * p.row_blocks;
   // (column tile, row block) of a tile; the next one's entry is requested while this one is worked on
   auto entry = [&](int tile) -> int4 { return tile < tiles ? __ldcg(p.tiles + tile / p.row_blocks) : make_int4(0, 0, 0, 0); };
+
+  // The bank's row at `place` of a tile's 128.
+  const auto row_of = [&](int4 e, int block, int place) -> int64_t {
+    const int64_t row = GATE_UP ? static_cast<int64_t>(e.x) * 2 * p.rows + block * 64 + (place < 64 ? place : p.rows + place - 64)
+                                : static_cast<int64_t>(e.x) * p.rows + block * 128 + place;
+    return row < p.bank_rows ? row : p.bank_rows - 1;
+  };
 
   if (warp == 0 || warp == 2) {
     if (elect_one()) {
@@ -257,6 +266,15 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
     const int warp4 = warp & 3, pair = warp4 * 16 + (lane & 15);
     const int tile_row = GATE_UP ? (lane < 16 ? 0 : 64) + pair : warp4 * 32 + lane;
     int4 next = entry(blockIdx.x);
+    Cursor p_at;  // (kScaledRows) where this warp reads the rows' powers
+    const auto read_power = [&](int& k) -> bool {
+      if (!mbar_wait(bars.p_full + p_at.slot * 8, p_at.pass, failed)) return false;
+      k = powers[p_at.slot * 128 + tile_row];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bars.p_empty + p_at.slot * 8);
+      p_at.advance(kPowerSlots);
+      return true;
+    };
     if (warp < kEpilogueWarp0) {
       const int group = (warp - kDecodeWarp0) >> 2;
       const WeightRing ring = {w_ring, p.w_slots, p.w_bytes};
@@ -268,11 +286,13 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
         const int4 e = next;
         next = entry(tile + gridDim.x);
         const int block = tile % p.row_blocks;
-        const int64_t bank = GATE_UP ? static_cast<int64_t>(e.x) * 2 * p.rows + (lane < 16 ? 0 : p.rows) + block * 64 + pair
-                                     : static_cast<int64_t>(e.x) * p.rows + block * 128 + tile_row;
-        const int64_t bank_row = bank < p.bank_rows ? bank : p.bank_rows - 1;
+        const int64_t bank_row = row_of(e, block, tile_row);
+        int k = 0;  // what the row is multiplied by: 2^k
+        if constexpr (kScaledRows<BF16, true>) {
+          if (!read_power(k)) break;
+        }
 #define DQ_DECODE(B) \
-  ok = decode_tile<B, BF16, MBF16, true>(p.meta, bank_row, tile_row, 0, group, stage, p.chunks, ring, bars, tmem, w_at, a_pass, failed)
+  ok = decode_tile<B, BF16, MBF16, true>(p.meta, bank_row, tile_row, power_of_two(k), 0, group, stage, p.chunks, ring, bars, tmem, w_at, a_pass, failed)
         switch (p.bits) {
           case 2: DQ_DECODE(2); break;
           case 3: DQ_DECODE(3); break;
@@ -284,7 +304,25 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
     } else {
       int* places = reinterpret_cast<int*>(smem + kOrderOffset) + warp4 * kColumns;  // this warp's copy of the tile's assignments
       Halves halves;
-      for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, halves.done()) {
+      // The rows' powers (kScaledRows) for the decoding warps too, two tiles ahead of them: a scan of their own
+      // would hold the decode up, and one warp for all four takes longer than a tile of the down projection.
+      Cursor found;
+      int4 ahead = entry(blockIdx.x);
+      const auto find_power = [&](int tile) -> bool {
+        if (tile >= tiles) return true;
+        if (!mbar_wait(bars.p_empty + found.slot * 8, found.pass ^ 1, failed)) return false;
+        const int4 e = ahead;
+        ahead = entry(tile + gridDim.x);
+        powers[found.slot * 128 + tile_row] =
+            static_cast<signed char>(row_power<MBF16>(p.meta, p.bits, row_of(e, tile % p.row_blocks, tile_row), 0, p.meta.num_groups));
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bars.p_full + found.slot * 8);
+        found.advance(kPowerSlots);
+        return true;
+      };
+      bool ok = true;
+      if constexpr (kScaledRows<BF16, true>) ok = find_power(blockIdx.x) && find_power(blockIdx.x + gridDim.x);
+      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, halves.done()) {
         const int4 e = next;
         next = entry(tile + gridDim.x);
         const int block = tile % p.row_blocks;
@@ -294,6 +332,10 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
           for (int c = lane; c < e.z; c += 32) places[c] = __ldcg(p.order + e.y + c);
           __syncwarp();
         }
+        int k = 0;
+        if constexpr (kScaledRows<BF16, true>) {
+          if (!read_power(k)) break;
+        }
         halves.take(e.z);
         if (!halves.wait(bars.d_full, 0, failed)) break;
         fence_after_sync();
@@ -302,6 +344,10 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
           uint32_t v[16];
           tmem_ld16(src + col, v);
           tmem_wait_ld();
+          if constexpr (kScaledRows<BF16, true>) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * power_of_two(-k));
+          }
           if constexpr (GATE_UP) {
             // lane l < 16 has gate row l, lane l + 16 the matching up row: each finishes eight of the columns
             const int first = col + (lane < 16 ? 0 : 8);
@@ -329,6 +375,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
           mbar_arrive(bars.d_empty + halves.at * 8);
           if (halves.both) mbar_arrive(bars.d_empty + 8);
         }
+        if constexpr (kScaledRows<BF16, true>) ok = find_power(tile + 2 * gridDim.x);
       }
     }
   }
@@ -426,11 +473,12 @@ int32_t launch_bank(const dq_weight& w, const dq_geometry& g, const void* act, i
                   static_cast<int64_t>(g.in_features) * 2, 64, kBoxRows, CU_TENSOR_MAP_SWIZZLE_128B)) {
     return fail(DQ_ERR_CUDA, "moe_gemm: a tensor map could not be encoded");
   }
-  const int x_bytes = p.n_cap * 256, budget = dev.max_smem_optin - static_cast<int>(kRingOffset);
+  const bool bf = act_dtype == DQ_BF16, mbf = w.meta_dtype == DQ_BF16;
+  const uint32_t front = ring_offset(!bf);
+  const int x_bytes = p.n_cap * 256, budget = dev.max_smem_optin - static_cast<int>(front);
   p.x_slots = std::clamp((budget - kGroups * p.w_bytes) / x_bytes, 2, 4);
   p.w_slots = std::clamp((budget - p.x_slots * x_bytes) / p.w_bytes / kGroups * kGroups, kGroups, 12);
-  const size_t smem = kRingOffset + static_cast<size_t>(p.x_slots) * x_bytes + static_cast<size_t>(p.w_slots) * p.w_bytes;
-  const bool bf = act_dtype == DQ_BF16, mbf = w.meta_dtype == DQ_BF16;
+  const size_t smem = front + static_cast<size_t>(p.x_slots) * x_bytes + static_cast<size_t>(p.w_slots) * p.w_bytes;
   const auto kernel = bf ? (mbf ? moe_umma_kernel<true, true, GATE_UP> : moe_umma_kernel<true, false, GATE_UP>)
                          : (mbf ? moe_umma_kernel<false, true, GATE_UP> : moe_umma_kernel<false, false, GATE_UP>);
   return launch(kernel, dim3(static_cast<unsigned>(dev.sm_count)), kThreads, smem, stream, "moe_gemm", p);

@@ -196,3 +196,54 @@ def test_a_module_raises_what_its_last_call_reported():
     with pytest.raises(RuntimeError, match="ran out"):
         layer(x)
     assert torch.equal(layer(x), want)
+
+
+def scaled_rows(qt, exponents):
+    """Row i times 2^exponents[i % len]."""
+    factor = 2.0 ** torch.tensor(exponents, dtype=torch.float32, device="cuda").repeat(-(-qt.num_rows // len(exponents)))[:qt.num_rows, None]
+    qt.scales, qt.offsets = ((t.float() * factor).to(t.dtype) for t in (qt.scales, qt.offsets))
+    return qt
+
+
+@pytest.mark.parametrize("bits", [2, 3, 4, 8])
+@pytest.mark.parametrize(("m", "rows", "k", "group", "meta", "x_exponent", "exponents"), [
+    (24, 300, 4224, 64, torch.bfloat16, 4, range(-18, 2)),      # sliced; weights down to where fp16 has none
+    (24, 300, 4096, 128, torch.bfloat16, -13, range(0, 22)),    # ... and past 65504
+    (64, 20000, 512, 128, torch.float16, 4, range(-12, 6)),     # several tiles per block
+    (17, 129, 12288, 128, torch.float16, -6, range(-3, 12)),    # more groups than a warp has lanes
+])
+def test_fp16_weights_of_any_size_enter_unrounded(bits, m, rows, k, group, meta, x_exponent, exponents):
+    from dynquant_b200 import ops
+
+    exponents = list(exponents)
+    qt = scaled_rows(random_qt(rows, k, bits, group=group, meta=meta, seed=bits), exponents)
+    x = (torch.randn(m, k, generator=torch.Generator().manual_seed(m)) * 2.0 ** x_exponent).to(torch.float16).cuda()
+    got = gemm(x, qt)
+    assert ops.last_kernel() == "gemm_umma_kernel"
+    want = x.double() @ ops.dequant(qt.packed, qt.scales, qt.offsets, bits, group, k, out_dtype=torch.float32).double().T
+    for i in range(len(exponents)):  # each size against its own largest result
+        part = want[:, i::len(exponents)]
+        assert float(part.abs().max()) < 65504
+        assert within_one_ulp_16(got[:, i::len(exponents)], part.float().cpu().numpy())
+
+
+@pytest.mark.parametrize("meta", [torch.float16, torch.bfloat16])
+def test_fp16_expert_weights_of_any_size_enter_unrounded(meta):
+    from dynquant_b200 import ops
+    from dynquant_b200.workloads import random_quant_tensor, seeded_routing
+
+    tokens, experts, topk, hidden, inter = 300, 8, 2, 1024, 384
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    gate_up = random_quant_tensor(experts * 2 * inter, hidden, 3, meta_dtype=meta, device="cuda", generator=gen)
+    down = random_quant_tensor(experts * hidden, inter, 4, meta_dtype=meta, device="cuda", generator=gen)
+    small = -14 if meta == torch.bfloat16 else -6
+    exponents = list(range(-16, 16)) if meta == torch.bfloat16 else list(range(-6, 10))
+    gate_up, down = scaled_rows(gate_up, [small]), scaled_rows(down, exponents)
+    ids, weights = seeded_routing(tokens, experts, topk, seed=1, device="cuda")
+    x = (torch.randn(tokens, hidden, device="cuda", generator=gen) * 2.0 ** -small).clamp(-65504, 65504).to(torch.float16)
+    got = moe_gemm(x, ids, weights, gate_up, down, experts)
+    want = torch.cat([ops.moe_gemv(x[i:i + 64].contiguous(), ids[i:i + 64].contiguous(), weights[i:i + 64].contiguous(), gate_up, down,
+                                   num_experts=experts, out_dtype=torch.float32) for i in range(0, tokens, 64)])
+    for i in range(len(exponents)):  # (flips of the rounded intermediate's last bit are what differs)
+        a, b = got[:, i::len(exponents)], want[:, i::len(exponents)]
+        assert (a - b).norm() <= 2e-4 * b.norm()
