@@ -70,7 +70,7 @@ constexpr uint32_t kBarrierOffset = 64, kRingOffset = 1024;
 static_assert(kBarrierOffset + kBarrierBytes <= kRingOffset, "");
 
 // SPLIT: the weights enter as the sum of two 16-bit operands, so that nothing of their fp32 values is
-// lost that the sums could show.  Up to DQ_GEMV_CHUNKED_MAX_ROWS activation rows, where the mma.sync
+// lost that a 16-bit output could show (figures: dq_umma_decode.cuh).  Up to DQ_GEMV_CHUNKED_MAX_ROWS activation rows, where the mma.sync
 // kernels scale fp32 accumulators and never round a weight; above that the dense path this kernel
 // replaces rounds every weight once, and so does this kernel.
 template <bool BF16, bool MBF16, bool SPLIT>

@@ -13,7 +13,7 @@
 //   4. down     the same over (column tile, 128 rows of the down bank) with h as the activation; fp32
 //               results go back to assignment order.
 //   5. combine  y[t] = sum_k p[t,k] * d[t,k] in slot order.
-// Weights enter as two 16-bit operands (see SPLIT, dq_gemm_umma.cu): as unrounded as in dq_moe.cu.  The
+// Weights enter as two 16-bit operands (see SPLIT, dq_gemm_umma.cu), 16 (bf16) or 21 bits of each.  The
 // order inside an expert is left to atomics: a column's result does not depend on its place, so the
 // layer is bit-identical run to run all the same.
 //

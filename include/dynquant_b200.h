@@ -330,8 +330,8 @@ DQ_API int32_t dq_moe_gemv_shard(const void* x, int32_t x_dtype, int64_t tokens,
                                  int64_t hidden, int64_t inter, void* y, int32_t y_dtype, void* scratch,
                                  int64_t scratch_bytes, void* stream);
 /* The same layer for any number of tokens (prefill), on the tcgen05 tensor cores: the assignments
- * sorted by expert on the device, every active expert's weights decoded once per 128 of its tokens,
- * unrounded as in dq_moe_gemv.  Sizes and alignment as there, plus hidden % 8 == 0, inter % 8 == 0, at
+ * sorted by expert on the device, every active expert's weights decoded once per 128 of its tokens, each
+ * as two 16-bit pieces (16 bits of it with bf16 activations, 21 with fp16).  Sizes and alignment as there, plus hidden % 8 == 0, inter % 8 == 0, at
  * most 1024 experts and 16-byte aligned x and y (else DQ_ERR_UNSUPPORTED, nothing launched). */
 DQ_API int32_t dq_moe_gemm_scratch_bytes(int64_t tokens, int64_t topk, int64_t hidden, int64_t inter,
                                          int64_t num_experts, int32_t act_dtype, int64_t* bytes);
