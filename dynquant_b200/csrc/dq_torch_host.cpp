@@ -6,7 +6,7 @@
 // dequant).  Here the tensors' pointers and sizes go straight into the C ABI's descriptors.
 //
 // Every function returns None for whatever it does not take -- odd shapes or types, tensor
-// subclasses, tracing, dispatch modes, autograd -- and the Python code that calls it then goes its
+// subclasses, tracing, dispatch modes, autograd in either direction -- and the Python code that calls it then goes its
 // long way, where all checks and messages live.  Called through the vectorcall protocol
 // (METH_FASTCALL); the GIL is released around the allocation and the launch.
 #include <Python.h>
@@ -58,6 +58,7 @@ const at::Tensor* tensor(PyObject* o) {
   if (!THPVariable_Check(o)) return nullptr;
   const at::Tensor& t = THPVariable_Unpack(o);
   if (!t.defined() || !t.is_cuda() || t.unsafeGetTensorImpl()->is_python_dispatch() || !t.has_storage()) return nullptr;
+  if (t.is_neg() || t._fw_grad(0).defined()) return nullptr;  // (a lazy negation; a forward-mode tangent)
   return &t;
 }
 

@@ -248,3 +248,19 @@ def test_vllm_adapter_layer_loads_through_the_placement_hooks_and_runs_one_launc
     assert ops.launch_count() - before == 1
     want = torch.cat([dense_ref(x, qt) for qt in parts], dim=-1) + bias.float().cpu()
     torch.testing.assert_close(got.float().cpu(), want, rtol=2e-2, atol=5e-3 * float(want.abs().max()))
+
+
+def test_forward_mode_tangents_and_lazy_negations_take_the_dense_path():
+    """Above 64 rows a call is dequantize + dense matmul to anything that differentiates it."""
+    from torch.autograd import forward_ad
+
+    from dynquant_b200.runtime import DynQuantLinear
+
+    qt = make_quant(96, 512, 128, 4, torch.float16).to("cuda")
+    layer, dense = DynQuantLinear(qt), qt.dequantize()
+    x, t = (torch.randn(100, 512, dtype=torch.float16, device="cuda") for _ in range(2))
+    want = torch.nn.functional.linear(t, dense)
+    with forward_ad.dual_level():
+        tangent = forward_ad.unpack_dual(layer(forward_ad.make_dual(x, t))).tangent
+    assert tangent is not None and torch.equal(tangent, want)
+    torch.testing.assert_close(layer(torch._neg_view(x)), -layer(x), rtol=2e-2, atol=0.1)
