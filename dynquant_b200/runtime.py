@@ -8,9 +8,8 @@ padding_idx=None, tied_to=None)`` (:215-260), state-dict keys ``qweight`` / ``sc
 
 What is different underneath: the reference rebuilds a ``QuantTensor`` view of the buffers on
 every forward call (``runtime/linear.py:128-143``) and pays for it in host time per module.
-Here the view is built once and kept until the storage under it moves (``.to()``,
-``load_state_dict`` with ``assign=True``): a forward is one comparison of a data pointer and
-one library call.
+Here a forward on the GPU is one library call on the buffers themselves; where a view is needed it is
+built once and kept until a buffer is replaced (``.to()``, ``load_state_dict`` with ``assign=True``).
 """
 
 from __future__ import annotations
@@ -63,7 +62,7 @@ class _PackedModule(nn.Module):
         super().__init__()
         self.spec = PackedSpec.of(weight)
         self.__dict__["_lender"] = tied_to  # bypasses nn.Module.__setattr__: not a child module
-        self.__dict__["_view"] = None       # (data_ptr of packed, QuantTensor)
+        self.__dict__["_view"] = None       # QuantTensor of the holder's buffers
         if tied_to is None:
             for name, tensor in zip(BUFFER_NAMES, (weight.packed, weight.scales, weight.offsets)):
                 self._own(name, tensor)
@@ -91,14 +90,13 @@ class _PackedModule(nn.Module):
 
     @property
     def weight_qt(self) -> QuantTensor:
-        """The buffers as a ``QuantTensor`` (no copy); rebuilt only when the storage moved."""
-        buffers = self.holder._buffers
-        packed = buffers[BUFFER_NAMES[0]]
-        cached = self.__dict__["_view"]
-        if cached is None or cached[0] != packed.data_ptr():
-            cached = (packed.data_ptr(), self.spec.view(packed, buffers[BUFFER_NAMES[1]], buffers[BUFFER_NAMES[2]]))
-            self.__dict__["_view"] = cached
-        return cached[1]
+        """The buffers as a ``QuantTensor`` (no copy); rebuilt only when one of them is another tensor
+        (``.half()`` replaces the scales alone)."""
+        packed, scales, offsets = (self.holder._buffers[name] for name in BUFFER_NAMES)
+        view = self.__dict__["_view"]
+        if view is None or view.packed is not packed or view.scales is not scales or view.offsets is not offsets:
+            view = self.__dict__["_view"] = self.spec.view(packed, scales, offsets)
+        return view
 
     @property
     def nbytes(self) -> int:

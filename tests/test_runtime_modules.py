@@ -45,6 +45,18 @@ def test_tied_table_is_held_once_and_followed_when_the_storage_moves():
     assert torch.equal(after.packed, qt.packed) and torch.equal(after.scales, qt.scales)
 
 
+def test_a_view_follows_scales_that_change_alone():
+    from dynquant_b200.runtime import DynQuantLinear
+
+    module = DynQuantLinear(make_quant(64, 128, -1, 4, torch.bfloat16))
+    before = module.weight_qt
+    module.half()  # the packed words stay the same tensor
+    assert module.weight_qt is not before and module.weight_qt.scales.dtype == torch.float16
+    assert module.weight_qt.scales is module.scales and module.weight_qt.offsets is module.offsets
+    module.offsets.data = module.offsets.data + 1.0
+    assert torch.equal(module.weight_qt.offsets, module.offsets)
+
+
 def test_only_matrices_in_the_linear_layout_are_accepted():
     from dataclasses import replace
 
