@@ -554,37 +554,51 @@ int32_t check_activation(const void* x, int32_t x_dtype, int64_t m, void* out, i
 }
 
 // Whether a matmul goes to the tcgen05 kernel (dq_gemm_umma.cu) rather than to the mma.sync kernels.
-// Measured on 60 random shapes x 4 widths (rows 512..28672, K 512..18944, 1..40 activation rows); us,
-// mma.sync -> tcgen05:
+// Figures, us, mma.sync -> tcgen05; every line was measured on both sides of its thresholds
+// (benchmarks/dispatch_regression.py --rule gemm, --force for the kernel everywhere: 28 shapes at 9..48 rows,
+// 50 at 1..8, four widths):
 //  * above 32 rows, and several shards above 8: always (12544 x 10624 2-bit 40 rows 2150 -> 50);
 //  * 9..32 rows: except where ONE launch of the tiled or the many-rows kernel serves all rows with
-//    whole blocks of four steps -- up to 16 rows on K <= 4096 (2816 x 2048 16 rows: 7.5 -> 7.4, 1009 x
-//    1024: 3.7 -> 5.2), up to 32 on small matrices (2688 x 512 32 rows: 3.8 -> 6.5);
+//    whole blocks of four steps -- up to 16 rows on K <= 4096 (1009 x 1024: 3.7 -> 5.2), at 2 and 4 bits with
+//    1536 rows or more on any K (8192 x 8192 9 rows 20.9 -> 23.7, 2048 x 8192 a fifth, 5120 x 17408 a tenth), at 3
+//    up to 36 M values (4096 x 8192 14.1 -> 15.5; 8192 x 8192 24.4 -> 24.2), up to 32 on small matrices (2688 x 512 32 rows: 3.8 -> 6.5);
 //  * 1..8 rows, where the mma.sync kernels have no good shape:
 //      - 64-value groups with an odd number of 128-value steps: the SIMT kernel (1024 x 5760, 1 / 8
-//        rows: 12.8 / 132 -> 7.4 / 7.7);
-//      - few rows and long slices of the reduction axis in the tiled kernel, which halves the step
-//        count only while the halves stay even (1152 x 7936, 62 steps: 25 -> 9; 896 x 3584: 7.1 -> 5.9);
-//      - odd step counts in the register-ring kernel: 8-bit matrices of many rows (25390 x 4736: 54 ->
-//        39) and six to eight rows x a long axis (7407 x 10624 8 rows: 41 -> 29).
+//        rows: 11.8 / 126 -> 7.8 / 8.0);
+//      - few rows and a reduction axis that the tiled kernel slices four ways or fewer, because it halves the
+//        step count only while the halves stay even (1152 x 7936, 62 steps: 20 -> 8.3; 896 x 3584 at eight rows
+//        8.5 -> 6.3; 1536 x 4608 level at one row).  From about 1280 rows on a long axis goes to the many-rows or
+//        the sliced streaming kernel (1536 x 8960 9.2 -> 10.5, 1536 x 13824 half as long again), and so do 8
+//        bits from 16 MB on (1024 x 18944 10.6 -> 14.8);
+//      - sliced eight ways, six rows and more (8 bits: four) x 14 steps a slice or more: the staged activation
+//        does not fit (512 x 14336 at six rows 18.8 -> 12.6, at four 10.8 -> 12.5, at one 6.8 -> 12.3);
+//      - odd step counts in the register-ring kernel: 8-bit matrices of many rows (25390 x 4736: 55 ->
+//        42) and six to eight rows x a long axis (7407 x 10624 6 rows: 38 -> 27; but 2048 x 10624 at 2..4 bits a
+//        fifth slower, 2048 x 12672 at six rows 12.3 -> 14.1).
 bool gemm_first(int64_t m, const dq_weight* shards, int num_shards) {
+  const int forced = m <= DQ_GEMV_CHUNKED_MAX_ROWS ? tuning_int("DQ_B200_GEMM_FIRST", -1) : -1;  // 0: never, 1: always
+  if (forced >= 0) return forced != 0;
   if (m > 32 || (m > DQ_GEMV_MAX_ROWS && num_shards > 1)) return true;
   for (int i = 0; i < num_shards; ++i) {
     const dq_weight& w = shards[i];
     const int64_t k = w.in_features, steps = ceil_div(k, 128);
     if (m > DQ_GEMV_MAX_ROWS) {
       const bool blocks = k % 512 == 0;
-      const bool one_launch = (m <= 16 && k <= 4096 && w.rows <= (w.bits == 8 ? 4096 : 16384)) || (k <= 2048 && w.rows * k <= 6000000);
+      const bool one_launch = (m <= 16 && k <= 4096 && w.rows <= (w.bits == 8 ? 4096 : 16384)) ||
+                              (m <= 16 && w.rows >= 1536 && (w.bits == 2 || w.bits == 4 || (w.bits == 3 && w.rows * k <= 36000000))) ||
+                              (k <= 2048 && w.rows * k <= 6000000);
       return !(blocks && one_launch);
     }
     if (w.group_values == 64 && steps % 2 != 0 && m > (w.rows * k > 1000000 ? 0 : 1)) return true;
     if (steps % 2 != 0) {
       if (w.bits == 8 && w.rows * k >= 40000000) return true;
-      if (m >= 6 && k >= 10240) return true;
+      if (m >= 6 && k >= 10240 && (w.bits == 8 || w.rows >= 3072)) return true;
     } else {
-      int64_t slice = steps;
-      for (int kw = 1; kw < 8 && slice % 4 == 0; kw *= 2) slice /= 2;
-      if (w.rows <= 1536 && slice >= 14) return true;
+      int64_t slice = steps, slices = 1;
+      for (; slices < 8 && slice % 4 == 0; slices *= 2) slice /= 2;
+      const bool streamed = w.bits == 8 && w.rows * k >= (16 << 20);
+      if (slices < 8 && slice >= 14 && !streamed && w.rows <= (slice <= 26 ? 1536 : 1280)) return true;
+      if (slices == 8 && slice >= 14 && !streamed && w.rows <= 1280 && m >= (w.bits == 8 ? 4 : 6)) return true;
     }
   }
   return false;
