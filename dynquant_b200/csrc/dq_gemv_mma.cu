@@ -874,32 +874,24 @@ bool mma_path_supports(const GemvArgs& a, int bits) {
 namespace {
 
 // Where several matrices that share an activation (gate / up, q / k / v) take the cluster-sliced
-// streaming body rather than the tiled kernel, which has a third of its resident warps: the CTAs of the
-// sliced launch that it takes (0: any number), or -1.  Measured (benchmarks/dispatch_regression.py --rule fused
-// --force, 39 sets of matrices), us, tiled -> sliced, at 2 / 3 / 4 / 8 bits:
-//  * from 90 M values on, where the launch fills the two CTAs that an SM holds to two thirds, or to three
-//    quarters with 3-bit codes among them, whose decode is the longest: 2 x 17408 x 5120 at one row 25.0 / 31.2 /
-//    28.4 / 56.0 -> 20.0 / 29.2 / 22.8 / 31.7, 2 x 14336 x 4096 (224 CTAs) 17.9 / 22.9 / 20.3 / 36.8 -> 16.0 / 23.1 /
-//    18.8 / 25.5; but 2 x 12288 x 4096 (192) 3-bit 20.0 -> 22.6, 2 x 13824 x 5120 (216) 3-bit 25.1 -> 28.8, 2 x 11008
-//    x 4096 (172) 13.6 / 17.2 / 15.4 -> 15.5 / 22.4 / 17.6;
-//  * mostly 8-bit codes, from 20 M on: 6144 x 4096 as q / k / v 10.8 -> 9.1, 2 x 3072 x 8192 17.5 -> 14.4;
+// streaming body rather than the tiled kernel, which has a third of its resident warps.  Measured, us,
+// tiled -> sliced, gate / up pairs and q / k / v at 2 / 3 / 4 / 8 bits:
+//  * from 90 M values on: 2 x 17408 x 5120 at one row 23.8 / 30.3 / 26.7 / 54.1 -> 18.6 / 27.9 / 20.9 / 29.6,
+//    at four rows 26.9 / 33.2 / 35.6 / 56.9 -> 20.9 / 30.1 / 24.6 / 36.4; 2 x 14336 x 4096 at one row 17.9 /
+//    22.2 / 19.1 / 34.6 -> 15.8 / 22.8 / 17.2 / 23.7;
+//  * mostly 8-bit codes, from 20 M on: 6144 x 4096 as q / k / v 10.5 -> 9.1, 2 x 3072 x 8192 16.7 -> 14.0;
 //  * four rows and more, from 20 M on, where the slices come out even (step counts that are multiples of
-//    16): 6144 x 4096 9.4 / 9.1 / 9.2 -> 7.4 / 8.9 / 7.8, 2 x 8192 x 6144 19.6 / 24.2 / 23.0 -> 15.3 / 21.0 / 17.3; but 7168
-//    x 5120, ten blocks over four slices, 10.5 / 11.7 / 11.0 -> 11.1 / 13.5 / 12.1, 2 x 8960 x 1536 a tenth and more.
-int stream_sliced_fused_ctas(const GemvArgs* jobs, const int* bits, int n, int sm_count) {
+//    16): 6144 x 4096 10.1 / 9.5 / 8.9 -> 7.5 / 9.1 / 8.0; but 7168 x 5120, ten blocks over four slices,
+//    10.6 / 11.8 / 10.5 -> 11.1 / 13.7 / 12.1.
+bool stream_sliced_fused_first(const GemvArgs* jobs, const int* bits, int n) {
   int64_t values = 0, code_bits = 0;
-  bool three = false;
   for (int i = 0; i < n; ++i) {
     const int64_t v = static_cast<int64_t>(jobs[i].rows) * jobs[i].in_features;
     values += v, code_bits += v * bits[i];
-    three = three || bits[i] == 3;
   }
-  const int forced = tuning_int("DQ_B200_FUSED_SLICED", -1);  // 0: never, 1: wherever it qualifies
-  if (forced >= 0) return forced - 1;
-  if (n < 2 || values < 20000000) return -1;
-  if (code_bits * 2 >= values * 11) return 0;
-  if (values >= 90000000) return three ? sm_count * 3 / 2 : sm_count * 4 / 3;
-  return jobs[0].m >= 4 && jobs[0].in_features >= 4096 && jobs[0].in_features % 2048 == 0 ? 0 : -1;
+  if (n < 2 || values < 20000000) return false;
+  if (values >= 90000000 || code_bits * 2 >= values * 11) return true;
+  return jobs[0].m >= 4 && jobs[0].in_features >= 4096 && jobs[0].in_features % 2048 == 0;
 }
 
 }  // namespace
@@ -917,8 +909,8 @@ int32_t launch_gemv_mma_fused(const GemvArgs* jobs, const int* bits, int n, cuda
     if (const int32_t rc = launch_gemv_stream_fused(jobs, bits, n, stream, taken)) return rc;
     if (*taken) return DQ_OK;
   }
-  if (const int least = push == nullptr ? stream_sliced_fused_ctas(jobs, bits, n, dev->sm_count) : -1; least >= 0) {
-    if (const int32_t rc = launch_gemv_stream_sliced_fused(jobs, bits, n, least, stream, taken)) return rc;
+  if (push == nullptr && stream_sliced_fused_first(jobs, bits, n)) {
+    if (const int32_t rc = launch_gemv_stream_sliced_fused(jobs, bits, n, stream, taken)) return rc;
     if (*taken) return DQ_OK;
   }
   return try_tile(jobs, bits, n, *dev, stream, taken, push);
@@ -948,8 +940,7 @@ bool rows_kernel_first(const GemvArgs& a, int bits) {
   // eight rows, 2 / 3 / 4 / 8 bits: 21 / 28 / 16 / 30 us against 27 / 30 / 37 / 53).
   const int64_t frag_bytes = static_cast<int64_t>(a.m) * steps * (bits == 8 ? 32 : 16) * 16;
   // (from 96 KB on where the matrix is small: 2048 x 6144, eight rows, 2 / 3 / 4 bits 7.4 / 7.7 / 6.3 against
-  // 8.5 / 9.0 / 8.4; 23 shapes of 512 .. 5120 rows x 3072 .. 12288, six to eight rows: none slower)
-  if (tuning_int("DQ_B200_ROWS_96K", -1) == 0) return frag_bytes > (144 << 10);
+  // 8.5 / 9.0 / 8.4)
   return frag_bytes > (144 << 10) || (a.m >= 6 && frag_bytes >= (96 << 10) && static_cast<int64_t>(a.rows) * a.in_features < 16000000);
 }
 
@@ -965,13 +956,9 @@ bool rows_kernel_first(const GemvArgs& a, int bits) {
 //    per SM, from 20 MB on (10240 x 5120 at one row, 4 / 8 bits: 12.0 / 15.5 against 14.7 / 22.5;
 //    but 7168 x 5120 at 4 bits, 18 MB, 10.8 against 9.0, and 17408 x 5120, 544 CTAs, 14.0 / 19.5 /
 //    17.0 at 2 / 3 / 4 bits against 13.0 / 17.0 / 15.7);
-//  * it cannot slice the reduction axis eight ways and has about a CTA per SM or fewer, from 20 M values and K
-//    = 4608 on (5120 x 5120 at 2 / 3 / 4 bits: at one row 6.5 / 8.3 / 7.3 against 7.3 / 8.7 / 8.7, at four 7.1 / 8.7 / 7.8
-//    against 10.1 / 10.9 / 10.3; 4608 x 8704 8.7 / 11.5 against 13.9 / 18.6), shorter axes only where it has more CTAs
-//    than SMs (10240 x 3584, 160 CTAs, 8.4 / 10.8 / 9.1 against 9.2 / 11.5 / 10.7; but 8192 x 3584, 128, 8.3 / 10.5 / 9.0
-//    against 8.0 / 8.4 / 8.1; 10240 x 2560 7.8 / 10.6 / 8.9 against 7.2 / 8.6 / 8.4).  Not below 26 M values at 3 bits and one
-//    row (4096 x 5120 8.2 against 7.1, 3072 x 7168 8.9 against 8.2; two rows and K = 4608 9.1 .. 10.3 against 10.8),
-//    nor for 4 bits where the many-rows kernel has the matrix (2816 x 8704 8.8 against 8.4);
+//  * it cannot slice the reduction axis eight ways and has about a CTA per SM or fewer, from 20 M values
+//    on (5120 x 5120 at 2 / 3 / 4 / 8 bits: at one row 6.5 / 8.4 / 7.4 / 8.7 against 7.8 / 8.8 / 8.2 / 15.3, at
+//    four 7.2 / 8.9 / 7.9 / 9.2 against 10.1 / 11.0 / 10.1 / 17.8);
 //  * seven or eight activation rows (8192 x 8192 13.7 / 16.9 / 16.8 / 22.9 against 18.5 / 20.7 / 20.6
 //    / 32; 11008 x 4096 11.1 / 13.7 / 11.7 / 14.1 against 13.9 / 14.5 / 13.7 / 21.1);
 //  * up to 8192 weight rows: four and more activation rows from 20 MB on (4096 x 14336 at 3 / 4 bits
@@ -993,14 +980,7 @@ bool stream_sliced_first(const GemvArgs& a, int bits, bool rows_first) {
   int kw = 8;
   while (kw > 1 && (steps % kw != 0 || (steps / kw) % 2 != 0)) kw /= 2;
   const int64_t ctas = ceil_div(ceil_div(a.rows, 16) * kw, 8);
-  const int64_t values = static_cast<int64_t>(a.rows) * a.in_features;
-  const int forced = tuning_int("DQ_B200_SLICED_20M", -1);  // 0: without the next term, 1: for all that it could be about
-  if (forced == 1 && kw < 8) return true;
-  if (forced != 0 && kw < 8 && ctas * 4 < static_cast<int64_t>(dev->sm_count) * 5 && values >= 20000000 &&
-      (a.in_features >= 4608 || (a.in_features >= 3584 && ctas > dev->sm_count)) &&
-      !(bits == 3 && values < 26000000 && a.m <= (a.in_features < 5120 ? 2 : 1)) && !(bits == 4 && rows_first)) {
-    return true;
-  }
+  if (kw < 8 && ctas * 4 < static_cast<int64_t>(dev->sm_count) * 5 && static_cast<int64_t>(a.rows) * a.in_features >= 20000000) return true;
   if (bytes < (16 << 20)) return false;
   if (rows_first || a.m >= 7) return true;
   // (a CTA per SM AND a long chain per warp: 2048 x 16384 has 128 CTAs there but slices of 16 steps,
