@@ -940,7 +940,8 @@ bool rows_kernel_first(const GemvArgs& a, int bits) {
   // eight rows, 2 / 3 / 4 / 8 bits: 21 / 28 / 16 / 30 us against 27 / 30 / 37 / 53).
   const int64_t frag_bytes = static_cast<int64_t>(a.m) * steps * (bits == 8 ? 32 : 16) * 16;
   // (from 96 KB on where the matrix is small: 2048 x 6144, eight rows, 2 / 3 / 4 bits 7.4 / 7.7 / 6.3 against
-  // 8.5 / 9.0 / 8.4)
+  // 8.5 / 9.0 / 8.4; 23 shapes of 512 .. 5120 rows x 3072 .. 12288, six to eight rows: none slower)
+  if (tuning_int("DQ_B200_ROWS_96K", -1) == 0) return frag_bytes > (144 << 10);
   return frag_bytes > (144 << 10) || (a.m >= 6 && frag_bytes >= (96 << 10) && static_cast<int64_t>(a.rows) * a.in_features < 16000000);
 }
 
@@ -956,9 +957,13 @@ bool rows_kernel_first(const GemvArgs& a, int bits) {
 //    per SM, from 20 MB on (10240 x 5120 at one row, 4 / 8 bits: 12.0 / 15.5 against 14.7 / 22.5;
 //    but 7168 x 5120 at 4 bits, 18 MB, 10.8 against 9.0, and 17408 x 5120, 544 CTAs, 14.0 / 19.5 /
 //    17.0 at 2 / 3 / 4 bits against 13.0 / 17.0 / 15.7);
-//  * it cannot slice the reduction axis eight ways and has about a CTA per SM or fewer, from 20 M values
-//    on (5120 x 5120 at 2 / 3 / 4 / 8 bits: at one row 6.5 / 8.4 / 7.4 / 8.7 against 7.8 / 8.8 / 8.2 / 15.3, at
-//    four 7.2 / 8.9 / 7.9 / 9.2 against 10.1 / 11.0 / 10.1 / 17.8);
+//  * it cannot slice the reduction axis eight ways and has about a CTA per SM or fewer, from 20 M values and K
+//    = 4608 on (5120 x 5120 at 2 / 3 / 4 bits: at one row 6.5 / 8.3 / 7.3 against 7.3 / 8.7 / 8.7, at four 7.1 / 8.7 / 7.8
+//    against 10.1 / 10.9 / 10.3; 4608 x 8704 8.7 / 11.5 against 13.9 / 18.6), shorter axes only where it has more CTAs
+//    than SMs (10240 x 3584, 160 CTAs, 8.4 / 10.8 / 9.1 against 9.2 / 11.5 / 10.7; but 8192 x 3584, 128, 8.3 / 10.5 / 9.0
+//    against 8.0 / 8.4 / 8.1; 10240 x 2560 7.8 / 10.6 / 8.9 against 7.2 / 8.6 / 8.4).  Not below 26 M values at 3 bits and one
+//    row (4096 x 5120 8.2 against 7.1, 3072 x 7168 8.9 against 8.2; two rows and K = 4608 9.1 .. 10.3 against 10.8),
+//    nor for 4 bits where the many-rows kernel has the matrix (2816 x 8704 8.8 against 8.4);
 //  * seven or eight activation rows (8192 x 8192 13.7 / 16.9 / 16.8 / 22.9 against 18.5 / 20.7 / 20.6
 //    / 32; 11008 x 4096 11.1 / 13.7 / 11.7 / 14.1 against 13.9 / 14.5 / 13.7 / 21.1);
 //  * up to 8192 weight rows: four and more activation rows from 20 MB on (4096 x 14336 at 3 / 4 bits
@@ -980,7 +985,14 @@ bool stream_sliced_first(const GemvArgs& a, int bits, bool rows_first) {
   int kw = 8;
   while (kw > 1 && (steps % kw != 0 || (steps / kw) % 2 != 0)) kw /= 2;
   const int64_t ctas = ceil_div(ceil_div(a.rows, 16) * kw, 8);
-  if (kw < 8 && ctas * 4 < static_cast<int64_t>(dev->sm_count) * 5 && static_cast<int64_t>(a.rows) * a.in_features >= 20000000) return true;
+  const int64_t values = static_cast<int64_t>(a.rows) * a.in_features;
+  const int forced = tuning_int("DQ_B200_SLICED_20M", -1);  // 0: without the next term, 1: for all that it could be about
+  if (forced == 1 && kw < 8) return true;
+  if (forced != 0 && kw < 8 && ctas * 4 < static_cast<int64_t>(dev->sm_count) * 5 && values >= 20000000 &&
+      (a.in_features >= 4608 || (a.in_features >= 3584 && ctas > dev->sm_count)) &&
+      !(bits == 3 && values < 26000000 && a.m <= (a.in_features < 5120 ? 2 : 1)) && !(bits == 4 && rows_first)) {
+    return true;
+  }
   if (bytes < (16 << 20)) return false;
   if (rows_first || a.m >= 7) return true;
   // (a CTA per SM AND a long chain per warp: 2048 x 16384 has 128 CTAs there but slices of 16 steps,
