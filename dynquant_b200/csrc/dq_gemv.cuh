@@ -45,7 +45,7 @@ int32_t launch_gemv_stream_fused(const GemvArgs* jobs, const int* bits, int n, c
 // body with the reduction axis sliced over a thread-block cluster (dq_gemv_stream_sliced.cu).
 int32_t launch_gemv_stream_sliced(const GemvArgs& a, int bits, cudaStream_t stream, bool* taken);
 // The same for one to four matrices that share an activation, in one launch.
-int32_t launch_gemv_stream_sliced_fused(const GemvArgs* jobs, const int* bits, int n, cudaStream_t stream, bool* taken);
+int32_t launch_gemv_stream_sliced_fused(const GemvArgs* jobs, const int* bits, int n, int least_ctas, cudaStream_t stream, bool* taken);
 // min_rows..64 activation rows against one matrix in one pass over the weights (dq_gemv_rows.cu).
 // *taken stays false, nothing launched, when the matrix or the activation does not qualify.
 int32_t launch_gemv_rows(const GemvArgs& a, int bits, cudaStream_t stream, bool* taken, int min_rows = 9);

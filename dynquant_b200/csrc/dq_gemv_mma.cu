@@ -874,24 +874,32 @@ bool mma_path_supports(const GemvArgs& a, int bits) {
 namespace {
 
 // Where several matrices that share an activation (gate / up, q / k / v) take the cluster-sliced
-// streaming body rather than the tiled kernel, which has a third of its resident warps.  Measured, us,
-// tiled -> sliced, gate / up pairs and q / k / v at 2 / 3 / 4 / 8 bits:
-//  * from 90 M values on: 2 x 17408 x 5120 at one row 23.8 / 30.3 / 26.7 / 54.1 -> 18.6 / 27.9 / 20.9 / 29.6,
-//    at four rows 26.9 / 33.2 / 35.6 / 56.9 -> 20.9 / 30.1 / 24.6 / 36.4; 2 x 14336 x 4096 at one row 17.9 /
-//    22.2 / 19.1 / 34.6 -> 15.8 / 22.8 / 17.2 / 23.7;
-//  * mostly 8-bit codes, from 20 M on: 6144 x 4096 as q / k / v 10.5 -> 9.1, 2 x 3072 x 8192 16.7 -> 14.0;
+// streaming body rather than the tiled kernel, which has a third of its resident warps: the CTAs of the
+// sliced launch that it takes (0: any number), or -1.  Measured (benchmarks/dispatch_regression.py --rule fused
+// --force, 39 sets of matrices), us, tiled -> sliced, at 2 / 3 / 4 / 8 bits:
+//  * from 90 M values on, where the launch fills the two CTAs that an SM holds to two thirds, or to three
+//    quarters with 3-bit codes among them, whose decode is the longest: 2 x 17408 x 5120 at one row 25.0 / 31.2 /
+//    28.4 / 56.0 -> 20.0 / 29.2 / 22.8 / 31.7, 2 x 14336 x 4096 (224 CTAs) 17.9 / 22.9 / 20.3 / 36.8 -> 16.0 / 23.1 /
+//    18.8 / 25.5; but 2 x 12288 x 4096 (192) 3-bit 20.0 -> 22.6, 2 x 13824 x 5120 (216) 3-bit 25.1 -> 28.8, 2 x 11008
+//    x 4096 (172) 13.6 / 17.2 / 15.4 -> 15.5 / 22.4 / 17.6;
+//  * mostly 8-bit codes, from 20 M on: 6144 x 4096 as q / k / v 10.8 -> 9.1, 2 x 3072 x 8192 17.5 -> 14.4;
 //  * four rows and more, from 20 M on, where the slices come out even (step counts that are multiples of
-//    16): 6144 x 4096 10.1 / 9.5 / 8.9 -> 7.5 / 9.1 / 8.0; but 7168 x 5120, ten blocks over four slices,
-//    10.6 / 11.8 / 10.5 -> 11.1 / 13.7 / 12.1.
-bool stream_sliced_fused_first(const GemvArgs* jobs, const int* bits, int n) {
+//    16): 6144 x 4096 9.4 / 9.1 / 9.2 -> 7.4 / 8.9 / 7.8, 2 x 8192 x 6144 19.6 / 24.2 / 23.0 -> 15.3 / 21.0 / 17.3; but 7168
+//    x 5120, ten blocks over four slices, 10.5 / 11.7 / 11.0 -> 11.1 / 13.5 / 12.1, 2 x 8960 x 1536 a tenth and more.
+int stream_sliced_fused_ctas(const GemvArgs* jobs, const int* bits, int n, int sm_count) {
   int64_t values = 0, code_bits = 0;
+  bool three = false;
   for (int i = 0; i < n; ++i) {
     const int64_t v = static_cast<int64_t>(jobs[i].rows) * jobs[i].in_features;
     values += v, code_bits += v * bits[i];
+    three = three || bits[i] == 3;
   }
-  if (n < 2 || values < 20000000) return false;
-  if (values >= 90000000 || code_bits * 2 >= values * 11) return true;
-  return jobs[0].m >= 4 && jobs[0].in_features >= 4096 && jobs[0].in_features % 2048 == 0;
+  const int forced = tuning_int("DQ_B200_FUSED_SLICED", -1);  // 0: never, 1: wherever it qualifies
+  if (forced >= 0) return forced - 1;
+  if (n < 2 || values < 20000000) return -1;
+  if (code_bits * 2 >= values * 11) return 0;
+  if (values >= 90000000) return three ? sm_count * 3 / 2 : sm_count * 4 / 3;
+  return jobs[0].m >= 4 && jobs[0].in_features >= 4096 && jobs[0].in_features % 2048 == 0 ? 0 : -1;
 }
 
 }  // namespace
@@ -909,8 +917,8 @@ int32_t launch_gemv_mma_fused(const GemvArgs* jobs, const int* bits, int n, cuda
     if (const int32_t rc = launch_gemv_stream_fused(jobs, bits, n, stream, taken)) return rc;
     if (*taken) return DQ_OK;
   }
-  if (push == nullptr && stream_sliced_fused_first(jobs, bits, n)) {
-    if (const int32_t rc = launch_gemv_stream_sliced_fused(jobs, bits, n, stream, taken)) return rc;
+  if (const int least = push == nullptr ? stream_sliced_fused_ctas(jobs, bits, n, dev->sm_count) : -1; least >= 0) {
+    if (const int32_t rc = launch_gemv_stream_sliced_fused(jobs, bits, n, least, stream, taken)) return rc;
     if (*taken) return DQ_OK;
   }
   return try_tile(jobs, bits, n, *dev, stream, taken, push);

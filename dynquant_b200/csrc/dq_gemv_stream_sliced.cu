@@ -212,7 +212,7 @@ size_t job_smem(const GemvArgs& a, int slices) {
 
 }  // namespace
 
-int32_t launch_gemv_stream_sliced_fused(const GemvArgs* jobs, const int* bits, int n, cudaStream_t stream_h, bool* taken) {
+int32_t launch_gemv_stream_sliced_fused(const GemvArgs* jobs, const int* bits, int n, int least_ctas, cudaStream_t stream_h, bool* taken) {
   *taken = false;
   const DeviceInfo* dev = device_info();
   if (dev == nullptr) return DQ_ERR_CUDA;
@@ -267,6 +267,7 @@ int32_t launch_gemv_stream_sliced_fused(const GemvArgs* jobs, const int* bits, i
       if (static_cast<int64_t>(per_sm) * dev->sm_count < groups) return DQ_OK;
       slices = 1;
     }
+    if (groups * slices < least_ctas) return DQ_OK;
     const size_t smem = smem_for(slices);
     DQ_CUDA(allow_shared(kernel, smem));
     cudaLaunchConfig_t cfg = {};
