@@ -52,7 +52,8 @@ RULES = {
         (4096, 5120), (5120, 5120), (5632, 5120), (3072, 7168), (4096, 7168), (5120, 7168), (2560, 9216), (4096, 9216), (5632, 9216),
         (6144, 3584), (8192, 3584), (11264, 3584), (8192, 2560), (10240, 2560), (8192, 2816), (16384, 2816), (2048, 11008), (4096, 11008),
         (8192, 11008), (2560, 13824), (5120, 4608), (5632, 3840), (7168, 4608), (8704, 4608), (4608, 4608), (9472, 3584), (10240, 3584),
-        (5632, 4352), (3840, 5632), (4096, 6656), (3328, 6144), (2816, 8704), (4608, 8704), (5120, 6656)], (1, 2, 4, 8))),
+        (5632, 4352), (3840, 5632), (4096, 6656), (3328, 6144), (2816, 8704), (4608, 8704), (5120, 6656),
+        (1536, 13824), (1536, 18944), (2304, 9728), (3072, 8960), (3328, 7936)], (1, 2, 4, 8))),
     "fused": (("DQ_B200_FUSED_SLICED",), [(rows, k, 128, (1, 2, 4, 8)) for rows, k in [
         ((12800, 12800), 4096), ((13312, 13312), 4096), ((16384, 16384), 4096), ((9216, 9216), 5120), ((7168, 7168), 8192),
         ((9472, 9472), 8192), ((5504, 5504), 8192), ((4096, 4096), 12288), ((8704, 8704), 6144), ((15360, 15360), 3072),
