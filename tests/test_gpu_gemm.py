@@ -247,3 +247,79 @@ def test_fp16_expert_weights_of_any_size_enter_unrounded(meta):
     for i in range(len(exponents)):  # (flips of the rounded intermediate's last bit are what differs)
         a, b = got[:, i::len(exponents)], want[:, i::len(exponents)]
         assert (a - b).norm() <= 2e-4 * b.norm()
+
+
+def small_moe(experts, hidden, inter, seed=1):
+    from dynquant_b200.workloads import random_quant_tensor
+
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    return (random_quant_tensor(experts * 2 * inter, hidden, 3, meta_dtype=torch.bfloat16, device="cuda", generator=gen),
+            random_quant_tensor(experts * hidden, inter, 4, meta_dtype=torch.bfloat16, device="cuda", generator=gen), gen)
+
+
+@pytest.mark.parametrize("first_expert", [0, 24])
+def test_skewed_routing_over_a_rank_of_experts(first_expert):
+    """A few experts take nearly all tokens, many take one or none; a rank's ids carry global numbers."""
+    from dynquant_b200 import ops
+
+    tokens, experts, hidden, inter = 600, 40, 512, 256
+    gate_up, down, gen = small_moe(experts, hidden, inter)
+    hot = torch.tensor([[0, 1], [1, 2], [2, 0]], device="cuda").repeat(tokens // 3, 1)  # 400 tokens each: four tiles
+    ids = hot.to(torch.int32)
+    ids[:20, 0] = torch.arange(10, 30, device="cuda", dtype=torch.int32)                # twenty experts with one token
+    ids[::7, 1] = 60                                                                    # nobody's
+    ids = (ids + first_expert).contiguous()
+    weights = torch.rand(tokens, 2, device="cuda", generator=gen)
+    x = torch.randn(tokens, hidden, device="cuda", generator=gen).to(torch.bfloat16)
+    got = moe_gemm(x, ids, weights, gate_up, down, experts, first_expert=first_expert)
+    want = torch.cat([ops.moe_gemv(x[i:i + 60].contiguous(), ids[i:i + 60].contiguous(), weights[i:i + 60].contiguous(), gate_up, down,
+                                   num_experts=experts, first_expert=first_expert, out_dtype=torch.float32) for i in range(0, tokens, 60)])
+    assert (got - want).norm() <= 1e-3 * want.norm()  # flips of the rounded intermediate's last bit
+    for token in (0, 19, 21, 599):  # one-token experts and hot ones alike, row by row
+        assert (got[token] - want[token]).norm() <= 4e-3 * want[token].norm()
+
+
+@pytest.mark.parametrize("tokens", [200, 4097, 9000])
+def test_plugin_expert_layer_over_many_tokens(tokens):
+    """Through the plugin's method: the tcgen05 kernels, 4096 tokens a call at most."""
+    from dynquant_b200 import ops
+    from dynquant_b200.plugin import DynQuantMoEMethod
+    from dynquant_b200.workloads import seeded_routing
+
+    experts, hidden, inter = 8, 256, 128
+    gate_up, down, gen = small_moe(experts, hidden, inter)
+    method, layer = DynQuantMoEMethod(None, bits_gate_up=3, bits_down=4), torch.nn.Module()
+    method.create_weights(layer, experts, hidden, inter, torch.bfloat16, device="cuda")
+    method.load_banks(layer, gate_up, down)
+    ids, weights = seeded_routing(tokens, experts, 2, seed=2, device="cuda")
+    x = torch.randn(tokens, hidden, device="cuda", generator=gen).to(torch.bfloat16)
+    got = method.apply(layer, x, weights, ids)
+    assert ops.last_kernel() == "moe_umma_kernel"
+    assert torch.equal(got, moe_gemm(x, ids, weights, gate_up, down, experts).to(torch.bfloat16))
+    assert torch.equal(method.apply(layer, x, weights, ids.long()), got)
+    want = torch.cat([ops.moe_gemv(x[i:i + 64].contiguous(), ids[i:i + 64].contiguous(), weights[i:i + 64].contiguous(), gate_up, down,
+                                   num_experts=experts, out_dtype=torch.float32) for i in range(0, min(tokens, 4160), 64)])
+    # one rounding of the output (2^-9) and flips of the intermediate's last bit
+    assert (got[:len(want)].float() - want).norm() <= 4e-3 * want.norm()
+
+
+@pytest.mark.parametrize(("m", "rows", "k", "bits", "kernel"), [
+    (1, (1536,), 14336, 4, "gemv_mma_tile_kernel"),          # sliced eight ways: not few slices
+    (1, (1536,), 13824, 3, "gemv_mma_stream_sliced_kernel"),  # a long axis of more than 1280 rows
+    (1, (1152,), 13824, 4, "gemm_umma_kernel"),
+    (6, (512,), 14336, 4, "gemm_umma_kernel"),
+    (9, (2048,), 8192, 4, "gemv_rows_kernel"),
+    (1, (8192,), 2560, 3, "gemv_mma_tile_kernel"),           # 20 M values on a short axis
+    (1, (5120,), 5120, 3, "gemv_mma_stream_sliced_kernel"),
+    (2, (11008, 11008), 4096, 3, "gemv_mma_tile_kernel"),    # 172 CTAs of 296
+    (2, (14336, 14336), 4096, 3, "gemv_mma_stream_sliced_multi_kernel"),  # 224
+])
+def test_lines_between_the_kernels(m, rows, k, bits, kernel):
+    from dynquant_b200 import ops
+
+    shards = [random_qt(n, k, bits, meta=torch.bfloat16, seed=i) for i, n in enumerate(rows)]
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(m)).to(torch.bfloat16).cuda()
+    got = ops.quantized_matmul(x, shards[0]) if len(shards) == 1 else ops.gemv_shards(x, shards)
+    assert ops.last_kernel() == kernel
+    dense = torch.cat([ops.dequant(q.packed, q.scales, q.offsets, bits, 128, k, out_dtype=torch.float32) for q in shards])
+    assert within_one_ulp_16(got, (x.double() @ dense.double().T).float().cpu().numpy())

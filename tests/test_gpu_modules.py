@@ -264,3 +264,54 @@ def test_forward_mode_tangents_and_lazy_negations_take_the_dense_path():
         tangent = forward_ad.unpack_dual(layer(forward_ad.make_dual(x, t))).tangent
     assert tangent is not None and torch.equal(tangent, want)
     torch.testing.assert_close(layer(torch._neg_view(x)), -layer(x), rtol=2e-2, atol=0.1)
+
+
+def test_calls_follow_the_current_stream_of_their_thread():
+    """Every entry point of the host path on streams of its own: behind what the stream still has to do, in
+    several threads at once."""
+    import threading
+
+    from dynquant_b200.plugin import DynQuantLinearMethod, DynQuantMoEMethod, ShardSpec
+    from dynquant_b200.runtime import DynQuantEmbedding, DynQuantLinear
+    from dynquant_b200.workloads import random_quant_tensor, seeded_routing
+
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    qt = random_quant_tensor(700, 1024, 3, meta_dtype=torch.bfloat16, device="cuda", generator=gen)
+    linear, table = DynQuantLinear(qt), DynQuantEmbedding(qt)
+    fused, fused_layer = DynQuantLinearMethod(None, [ShardSpec("a", 3, 128, 700), ShardSpec("b", 3, 128, 700)]), torch.nn.Module()
+    fused.create_weights(fused_layer, 1024, [700, 700], 1024, 1400, torch.bfloat16, device="cuda")
+    for i in range(2):
+        fused.load_shard(fused_layer, i, qt)
+    moe, moe_layer = DynQuantMoEMethod(None, bits_gate_up=3, bits_down=4), torch.nn.Module()
+    moe.create_weights(moe_layer, 4, 1024, 256, torch.bfloat16, device="cuda")
+    moe.load_banks(moe_layer, random_quant_tensor(4 * 512, 1024, 3, meta_dtype=torch.bfloat16, device="cuda", generator=gen),
+                   random_quant_tensor(4 * 1024, 256, 4, meta_dtype=torch.bfloat16, device="cuda", generator=gen))
+    routing = {m: seeded_routing(m, 4, 2, seed=m, device="cuda") for m in (1, 24, 300)}
+
+    def calls(m, x, ids):
+        experts, weights = routing[m]
+        return [linear(x), fused.apply(fused_layer, x), moe.apply(moe_layer, x, weights, experts), table(ids), qt.dequantize()]
+
+    inputs = {m: (torch.randn(m, 1024, device="cuda", generator=gen).to(torch.bfloat16), torch.randint(700, (m,), device="cuda"))
+              for m in (1, 24, 300)}
+    want = {m: calls(m, *inputs[m]) for m in inputs}
+    torch.cuda.synchronize()
+    failures = []
+
+    def worker(m):
+        stream, (x, ids) = torch.cuda.Stream(), inputs[m]
+        with torch.cuda.stream(stream):
+            for _ in range(10):
+                torch.cuda._sleep(2_000_000)  # the inputs come late: a call on another stream would read zeros
+                late_x, late_ids = torch.zeros_like(x).add_(x), torch.zeros_like(ids).add_(ids)
+                got = calls(m, late_x, late_ids)
+                stream.synchronize()
+                if not all(torch.equal(a, b) for a, b in zip(got, want[m])):
+                    failures.append(m)
+
+    threads = [threading.Thread(target=worker, args=(m,)) for m in inputs for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures
