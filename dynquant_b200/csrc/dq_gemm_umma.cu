@@ -18,8 +18,9 @@
 // What bounds it: for wide tiles the tensor pipe (n_tile / 2 cycles per 16 values of K) at the clock that
 // the power cap leaves, below that the decode's issue slots (14336 x 4096, 4-bit: issue 55 %, integer
 // pipe 54 %, tensor 31 % at 65 rows, with 112 of 148 SMs at work; 0.5 us per 128 x 128 values and SM split
-// in two operands).  14336 x 4096, 4-bit, at 16 / 128 / 512 / 4096 rows: 21 / 22 / 53 / 366 us (1.31
-// PFLOP/s) where dequantize + dense took 215 us at the first two and 521 at the last.
+// in two operands).  14336 x 4096, 4-bit, at 16 / 128 / 512 / 4096 rows: 21 / 22 / 53 / 427 us (1.13
+// PFLOP/s, 79 % of the sustained dense peak; 366 us in bursts too short for the power cap) where dequantize +
+// dense took 215 us at the first two and 558 at the last.
 //
 // Small matrices: the reduction axis is sliced over a thread-block cluster (grid.y), each CTA leaves
 // its fp32 tile in its own shared memory and the CTAs of the cluster add a share of the columns

@@ -971,7 +971,7 @@ bool rows_kernel_first(const GemvArgs& a, int bits) {
 //    than SMs (10240 x 3584, 160 CTAs, 8.4 / 10.8 / 9.1 against 9.2 / 11.5 / 10.7; but 8192 x 3584, 128, 8.3 / 10.5 / 9.0
 //    against 8.0 / 8.4 / 8.1; 10240 x 2560 7.8 / 10.6 / 8.9 against 7.2 / 8.6 / 8.4).  Not below 26 M values at 3 bits and one
 //    row where the tiled kernel has the matrix (4096 x 5120 8.2 against 7.1, 3072 x 7168 8.9 against 8.2; with K =
-//    4608 at two rows either: 10.8 against 9.9), nor at 4 bits where the many-rows kernel has it (six shapes: 2816 x
+//    4608 at two rows either: 10.8 against 9.9), nor at 4 bits where the many-rows kernel has it (2816 x
 //    8704 8.8 against 8.4, 1536 x 18944 12.3 against 11.2, at eight rows 16 against 12);
 //  * seven or eight activation rows (8192 x 8192 13.7 / 16.9 / 16.8 / 22.9 against 18.5 / 20.7 / 20.6
 //    / 32; 11008 x 4096 11.1 / 13.7 / 11.7 / 14.1 against 13.9 / 14.5 / 13.7 / 21.1);
