@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(Roles<SPLIT>::kThreads, 1) gemm_umma_kernel(co
       const Job& job = p.job[job_of(tile % p.row_tiles, local)];
       float power = 1.0f, back = 1.0f;
       if constexpr (kScaledRows<BF16, SPLIT>) {
-        const int k = row_power<MBF16>(job.meta, job.bits, min(local * 128 + r, job.rows - 1), first_group(job), groups_of(job));
+        const int k = row_power<MBF16>(job.meta, job.bits, job.rows, min(local * 128 + r, job.rows - 1), first_group(job), groups_of(job));
         power = power_of_two(k), back = power_of_two(-k);
       }
       bool ok;

@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_umma_kernel(const __grid_cons
         const int4 e = ahead;
         ahead = entry(tile + gridDim.x);
         powers[found.slot * 128 + tile_row] =
-            static_cast<signed char>(row_power<MBF16>(p.meta, p.bits, row_of(e, tile % p.row_blocks, tile_row), 0, p.meta.num_groups));
+            static_cast<signed char>(row_power<MBF16>(p.meta, p.bits, p.bank_rows, row_of(e, tile % p.row_blocks, tile_row), 0, p.meta.num_groups));
         __syncwarp();
         if (lane == 0) mbar_arrive(bars.p_full + found.slot * 8);
         found.advance(kPowerSlots);

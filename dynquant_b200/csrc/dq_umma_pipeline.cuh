@@ -77,17 +77,20 @@ __device__ __forceinline__ unsigned short scaled16(unsigned short s, float power
 // A row's power k: its weights in groups [g0, g0 + count) of that row, all below max|s| * (2^bits - 1) +
 // max|o|, times 2^k stay below 2^15.  A thread takes a row, in 16-byte pieces that start on a 16-byte
 // boundary (what they hold of the row's other groups may count; what belongs to its neighbours is masked),
-// up to four of each array in flight.
+// up to four of each array in flight; where a piece would reach past the arrays of `rows` rows, value by value.
 template <bool MBF16>
-__device__ __forceinline__ int row_power(const Meta& meta, int bits, int64_t row, int g0, int count) {
+__device__ __forceinline__ int row_power(const Meta& meta, int bits, int64_t rows, int64_t row, int g0, int count) {
   struct Pieces {
     uintptr_t row0, row1, at;  // bytes: the row's, and the next piece's
     int last;                  // pieces - 1
+    bool inside;               // all of them in the array
   };
   const auto pieces = [&](const void* p) -> Pieces {
     const uintptr_t row0 = reinterpret_cast<uintptr_t>(p) + static_cast<uintptr_t>(row * meta.num_groups) * 2, from = row0 + static_cast<uintptr_t>(g0) * 2;
-    const uintptr_t at = from & ~uintptr_t{15};
-    return {row0, row0 + static_cast<uintptr_t>(meta.num_groups) * 2, at, static_cast<int>((from + static_cast<uintptr_t>(count) * 2 - 1 - at) >> 4)};
+    const uintptr_t at = from & ~uintptr_t{15}, base = reinterpret_cast<uintptr_t>(p);
+    const int last = static_cast<int>((from + static_cast<uintptr_t>(count) * 2 - 1 - at) >> 4);
+    return {row0, row0 + static_cast<uintptr_t>(meta.num_groups) * 2, at, last,
+            at >= base && at + (static_cast<uintptr_t>(last) + 1) * 16 <= base + static_cast<uintptr_t>(rows * meta.num_groups) * 2};
   };
   const auto fold = [](uint32_t most, uint4 v, const Pieces& p, int i) -> uint32_t {  // |.| as its bits: ordered like the values
     uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -107,7 +110,13 @@ __device__ __forceinline__ int row_power(const Meta& meta, int bits, int64_t row
   const bool has_offsets = meta.offsets != nullptr;
   const Pieces s = pieces(meta.scales), o = has_offsets ? pieces(meta.offsets) : s;
   uint32_t s_most = 0, o_most = 0;
-  for (int i0 = 0; i0 <= s.last || i0 <= o.last; i0 += kBatch) {
+  const bool inside = s.inside && o.inside;
+  for (int g = 0; g < count && !inside; ++g) {
+    const int64_t at = row * meta.num_groups + g0 + g;
+    s_most = max(s_most, __ldg(static_cast<const unsigned short*>(meta.scales) + at) & 0x7FFFu);
+    if (has_offsets) o_most = max(o_most, __ldg(static_cast<const unsigned short*>(meta.offsets) + at) & 0x7FFFu);
+  }
+  for (int i0 = 0; inside && (i0 <= s.last || i0 <= o.last); i0 += kBatch) {
     uint4 sv[kBatch], ov[kBatch];
 #pragma unroll
     for (int i = 0; i < kBatch; ++i) sv[i] = load(s, min(i0 + i, s.last)), ov[i] = load(o, min(i0 + i, o.last));

@@ -323,3 +323,28 @@ def test_lines_between_the_kernels(m, rows, k, bits, kernel):
     assert ops.last_kernel() == kernel
     dense = torch.cat([ops.dequant(q.packed, q.scales, q.offsets, bits, 128, k, out_dtype=torch.float32) for q in shards])
     assert within_one_ulp_16(got, (x.double() @ dense.double().T).float().cpu().numpy())
+
+
+@pytest.mark.parametrize("m", [2, 40])
+def test_fp16_shards_whose_metadata_start_anywhere(m):
+    """Eleven or 22 groups a row and odd row counts: rows of scales that start on no 16-byte boundary, the last
+    ones at the end of the buffer."""
+    from dynquant_b200 import ops
+    from dynquant_b200.plugin import DynQuantLinearMethod, ShardSpec
+
+    k, sizes, widths = 1408, (301, 127, 77), (8, 2, 4)
+    method, layer = DynQuantLinearMethod(None, [ShardSpec(str(i), b, 64, n) for i, (n, b) in enumerate(zip(sizes, widths))]), torch.nn.Module()
+    method.create_weights(layer, k, list(sizes), k, sum(sizes), torch.float16, device="cuda")
+    shards = [scaled_rows(random_qt(n, k, b, group=64, seed=b), list(range(-9, 3))) for n, b in zip(sizes, widths)]
+    for i, qt in enumerate(shards):
+        method.load_shard(layer, i, qt)
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(m)).to(torch.float16).cuda()
+    got = method.apply(layer, x)
+    assert ops.last_kernel() == "gemm_umma_kernel"
+    start = 0
+    for qt in shards:
+        dense = ops.dequant(qt.packed, qt.scales, qt.offsets, qt.bits, 64, k, out_dtype=torch.float32)
+        part, want = got[:, start:start + qt.num_rows], x.double() @ dense.double().T
+        start += qt.num_rows
+        for i in range(12):
+            assert within_one_ulp_16(part[:, i::12], want[:, i::12].float().cpu().numpy())
