@@ -14,8 +14,9 @@
 // fmaf as well; with fp32 scales it follows the torch definition.  An absent
 // offsets tensor means "no add", not "+0".
 //
-// Two kernels.  dequant_octet_kernel is the one nearly every tensor takes (in_features and
-// the group size multiples of 8): a thread produces 8 consecutive values -- one 16-byte
+// Three kernels.  dequant_pairs_kernel takes what models have: 16-bit metadata and output, in_features and
+// the group size multiples of 16.  dequant_octet_kernel takes the rest of the regular tensors (in_features and
+// the group size multiples of 8, any types): a thread produces 8 consecutive values -- one 16-byte
 // store for a 16-bit output, so a warp writes 512 contiguous bytes per store instruction --
 // from the 8 * BITS bits at bit 8 * BITS * octet of its row (the packed row is one
 // contiguous LSB-first bit string: groups are whole numbers of 32-value blocks).  dequant_kernel
@@ -24,6 +25,7 @@
 #include <type_traits>
 
 #include "dq_decode.cuh"
+#include "dq_umma_decode.cuh"
 
 namespace dq {
 namespace {
@@ -59,8 +61,8 @@ __device__ __forceinline__ int source_row(const DequantArgs& a, int row) {
 // `group_shift` >= 0: the group size is 2^shift.  `per_row_magic` = ceil(2^64 / octets_per_row):
 // the high half of its product with an octet's number is the octet's row (exact below 2^32).
 //
-// Bound by the stores (2 bytes written per value, bits/8 read): 14336 x 4096 at 3 / 4 / 8 bits takes
-// 38 / 37 / 37 us where filling the output with zeros takes 33.  (Octets over blockIdx.x and rows
+// Bound by its instructions: 14336 x 4096 at 3 / 4 / 8 bits takes 36 / 33 / 36 us in a graph, filling its
+// output 18.6.  (Octets over blockIdx.x and rows
 // over blockIdx.y, one octet per thread: 52 / 44 / 44 -- and 14 us against 10 on 14080 x 768, whose
 // rows left most threads of a CTA idle.)  256 threads and 4 octets: 43; 2 octets: 39 to 41.
 template <int BITS, int U, bool IDS>
@@ -142,6 +144,139 @@ __global__ void __launch_bounds__(kDequantThreads) dequant_octet_kernel(const De
       }
       reinterpret_cast<uint4*>(a.out)[at] = make_uint4(p16[0], p16[1], p16[2], p16[3]);
     }
+  }
+}
+
+// 16 codes -> eight registers of two, each as an exact 16-bit number of the METADATA's type: codes `first` and
+// `second` of register j.  ONE AND-OR puts two codes into the mantissas of a power of two, one packed subtraction
+// takes that off again.
+template <int BITS, bool MBF16>
+struct Codes16 {
+  static constexpr int kMantissa = MBF16 ? 7 : 10;
+  static constexpr int first(int j) { return BITS == 8 ? 2 * j : BITS == 4 ? j / 4 * 8 + j % 4 : j; }
+  static constexpr int second(int j) { return BITS == 8 ? 2 * j + 1 : BITS == 4 ? j / 4 * 8 + j % 4 + 4 : j + 8; }
+  static __device__ __forceinline__ uint32_t minus(uint32_t a, uint32_t b) {
+    if constexpr (MBF16) {
+      const __nv_bfloat162 d = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+      return *reinterpret_cast<const uint32_t*>(&d);
+    } else {
+      const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+      return *reinterpret_cast<const uint32_t*>(&d);
+    }
+  }
+  // The codes at bit `place` of both halves; place + BITS <= kMantissa.
+  static __device__ __forceinline__ uint32_t take(uint32_t u, int place) {
+    const uint32_t mask = ((1u << BITS) - 1u) << place, magic = static_cast<uint32_t>((MBF16 ? 127 : 15) + kMantissa - place) << kMantissa;
+    return minus((u & (mask | (mask << 16))) | (magic | (magic << 16)), magic | (magic << 16));
+  }
+  // `w`: the words that hold the codes, from bit `shift` on (3 bits: 0 or 16; else 0)
+  static __device__ __forceinline__ void get(const uint32_t* w, int shift, uint32_t* q) {
+    if constexpr (BITS == 8) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if constexpr (MBF16) {
+          // Seven bits fit the mantissa: 128 + low bits; the top bit toggles -256 / -128.  Their sum is code - 128.
+          const uint32_t p = __byte_perm(w[j / 2], 0u, (j & 1) ? 0x4342u : 0x4140u);
+          q[j] = minus((p & 0x007F007Fu) | 0x43004300u, (p & 0x00800080u) ^ 0x43804380u);
+          q[j] = minus(q[j], 0xC300C300u);
+        } else {
+          q[j] = minus(__byte_perm(w[j / 2], 0x64006400u, (j & 1) ? 0x7372u : 0x7170u), 0x64006400u);
+        }
+      }
+    } else if constexpr (BITS == 3) {
+      // Codes 0..7 and 8..15 are 24 bits each: their lower and upper 16 bits side by side.
+      const unsigned long long v = ((static_cast<unsigned long long>(w[1]) << 32) | w[0]) >> shift;
+      const uint32_t a = static_cast<uint32_t>(v), b = static_cast<uint32_t>(v >> 24);
+      const uint32_t low = __byte_perm(a, b, 0x5410u), high = __byte_perm(a, b, 0x6521u);
+      constexpr int kPlaces = kMantissa / 3;
+#pragma unroll
+      for (int j = 0; j < 5; ++j) q[j] = take(low >> (3 * (j - j % kPlaces)), 3 * (j % kPlaces));
+#pragma unroll
+      for (int j = 0; j < 3; ++j) q[5 + j] = take(high >> (7 + 3 * (j - j % kPlaces)), 3 * (j % kPlaces));
+    } else {
+      constexpr int kPlaces = kMantissa / BITS, kOfWord = 16 / BITS;  // registers of a word: 8 or 4
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int i = j % kOfWord;
+        q[j] = take(w[j / kOfWord] >> (BITS * (i - i % kPlaces)), BITS * (i % kPlaces));
+      }
+    }
+  }
+};
+
+// U runs of 16 consecutive values per thread, one 32-byte store each, kDequantThreads runs apart (as
+// dequant_octet_kernel; `runs_per_row`, `per_row_magic`, `total` count runs).  A code is an exact number of the
+// metadata's type, so that ONE mixed-precision fma, q * s + o with 16-bit factors and an fp32 addend, is the
+// exact product and the one rounding of the sum that the format asks for.  No offsets: the addend is -0, which
+// changes no sum, not even a zero's sign.
+//
+// Bound by memory: bits / 8 bytes read and 2 written per value.  14336 x 4096 at 2 / 3 / 4 / 8 bits: 22.7 / 24.4 /
+// 24.9 / 28.9 us (5.9 to 6.2 TB/s; filling such an output takes 18.6) where dequant_octet_kernel takes 36.4 /
+// 36.5 / 33.0 / 35.7: that one spends 4.5 instructions a value on the decode and reads scale and offset for every
+// eight values, this one 2.9 and for every 16.
+template <int BITS, bool MBF16, int U, bool IDS>
+__global__ void __launch_bounds__(kDequantThreads) dequant_pairs_kernel(const DequantArgs a, unsigned runs_per_row, unsigned long long per_row_magic,
+                                                                        unsigned total, int group_shift) {
+  constexpr int kWords = BITS == 3 ? 2 : BITS / 2;
+  const unsigned first = blockIdx.x * (kDequantThreads * U) + threadIdx.x;
+  uint32_t w[U][kWords];
+  unsigned short scale[U], offset[U];
+  int shift[U];
+  bool known[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const unsigned at = min(first + u * kDequantThreads, total - 1);
+    const int row = static_cast<int>(__umul64hi(at, per_row_magic)), run = static_cast<int>(at - row * runs_per_row);
+    int from = row;
+    known[u] = true;
+    if constexpr (IDS) {
+      from = source_row(a, row);
+      known[u] = from >= 0;
+      from = max(from, 0);
+    }
+    const uint32_t* src = a.packed + static_cast<int64_t>(from) * a.words_per_row + run * BITS / 2;
+    shift[u] = 0;
+    if constexpr (BITS == 2) {
+      w[u][0] = __ldg(src);
+    } else if constexpr (BITS == 3) {
+      shift[u] = (run & 1) * 16;
+      w[u][0] = __ldg(src), w[u][1] = __ldg(src + 1);
+    } else if constexpr (BITS == 4) {
+      const uint2 v = __ldg(reinterpret_cast<const uint2*>(src));
+      w[u][0] = v.x, w[u][1] = v.y;
+    } else {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
+      w[u][0] = v.x, w[u][1] = v.y, w[u][2] = v.z, w[u][3] = v.w;
+    }
+    const int64_t meta = static_cast<int64_t>(from) * a.num_groups + (group_shift >= 0 ? (run * 16) >> group_shift : (run * 16) / a.group_values);
+    scale[u] = __ldg(static_cast<const unsigned short*>(a.scales) + meta);
+    offset[u] = a.offsets != nullptr ? __ldg(static_cast<const unsigned short*>(a.offsets) + meta) : 0x8000;
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const unsigned at = first + u * kDequantThreads;
+    if (at >= total) break;
+    float o = MBF16 ? __uint_as_float(static_cast<uint32_t>(offset[u]) << 16) : __half2float(__ushort_as_half(offset[u]));
+    if constexpr (IDS) {
+      if (!known[u]) {
+        o = __int_as_float(0x7FC00000);
+        report_to_host(a.report, kReportId);
+      }
+    }
+    using C = Codes16<BITS, MBF16>;
+    uint32_t q[8], out[8];
+    float f[16];
+    C::get(w[u], shift[u], q);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      f[C::first(j)] = umma::fma_half<MBF16>(q[j], false, scale[u], o);
+      f[C::second(j)] = umma::fma_half<MBF16>(q[j], true, scale[u], o);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) out[j] = round_pair_to_16(f[2 * j], f[2 * j + 1], a.out_dtype);
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(static_cast<unsigned char*>(a.out) + static_cast<size_t>(at) * 32), "r"(out[0]),
+                 "r"(out[1]), "r"(out[2]), "r"(out[3]), "r"(out[4]), "r"(out[5]), "r"(out[6]), "r"(out[7])
+                 : "memory");
   }
 }
 
@@ -288,15 +423,47 @@ int32_t launch_dequant(const dq_weight* w, const dq_geometry& g, const void* ids
   const bool octets = a.in_features % 8 == 0 && a.group_values % 8 == 0 &&
                       reinterpret_cast<uintptr_t>(out) % 16 == 0 && (a.in_features * out_elem) % 16 == 0 &&
                       (w->bits != 8 || (reinterpret_cast<uintptr_t>(a.packed) % 8 == 0 && a.words_per_row % 2 == 0));
+  int shift = -1;
+  if ((a.group_values & (a.group_values - 1)) == 0) {
+    shift = 0;
+    while ((1 << shift) < a.group_values) ++shift;
+  }
+  // The pairs kernel: whole runs of 16 values per row and per group, 32-byte aligned output rows, and packed rows that
+  // a run's words can be read from at once.
+  const int run_bytes = w->bits == 3 ? 4 : 2 * w->bits;
+  const bool pairs = out_dtype != DQ_F32 && a.meta_dtype != DQ_F32 && a.in_features % 16 == 0 && a.in_features > 16 && a.group_values % 16 == 0 &&
+                     reinterpret_cast<uintptr_t>(out) % 32 == 0 && reinterpret_cast<uintptr_t>(a.packed) % run_bytes == 0 && a.words_per_row * 4 % run_bytes == 0;
+  const int64_t num_runs = static_cast<int64_t>(a.rows) * (a.in_features / 16);
+  if (pairs && num_runs < (int64_t{1} << 31)) {
+    const unsigned per_row = static_cast<unsigned>(a.in_features / 16);
+    const unsigned long long magic = ~0ull / per_row + 1;  // ceil(2^64 / per_row)
+    const unsigned total = static_cast<unsigned>(num_runs);
+    // Two runs per thread from a full wave of such threads on (4096 x 4096, 3-bit: 8.2 us, 9.0 with one, 9.6 with four;
+    // 2048 x 2048 is level, 512 x 1024 takes 1.83 us with one, 1.95 with two).
+    const bool two = num_runs >= static_cast<int64_t>(dev->sm_count) * 2048 * 2;
+    const unsigned grid = static_cast<unsigned>(ceil_div(num_runs, kDequantThreads * (two ? 2 : 1)));
+    const auto run = [&](auto bits, auto bf16, auto ids) {
+      constexpr int B = decltype(bits)::value;
+      constexpr bool M = decltype(bf16)::value, IDS = decltype(ids)::value;
+      (two ? dequant_pairs_kernel<B, M, 2, IDS> : dequant_pairs_kernel<B, M, 1, IDS>)<<<grid, kDequantThreads, 0, s>>>(a, per_row, magic, total, shift);
+    };
+    const auto with_bits = [&](auto bf16, auto ids) {
+      switch (w->bits) {
+        case 2: run(std::integral_constant<int, 2>{}, bf16, ids); break;
+        case 3: run(std::integral_constant<int, 3>{}, bf16, ids); break;
+        case 4: run(std::integral_constant<int, 4>{}, bf16, ids); break;
+        default: run(std::integral_constant<int, 8>{}, bf16, ids); break;
+      }
+    };
+    const auto with_meta = [&](auto ids) { a.meta_dtype == DQ_BF16 ? with_bits(std::true_type{}, ids) : with_bits(std::false_type{}, ids); };
+    a.ids != nullptr ? with_meta(std::true_type{}) : with_meta(std::false_type{});
+    DQ_CHECK_LAUNCH("dequant");
+    return DQ_OK;
+  }
   const int64_t num_octets = static_cast<int64_t>(a.rows) * (a.in_features / 8);
   if (octets && a.in_features > 8 && num_octets < (int64_t{1} << 32)) {
     const unsigned per_row = static_cast<unsigned>(a.in_features / 8);
     const unsigned long long magic = ~0ull / per_row + 1;  // ceil(2^64 / per_row)
-    int shift = -1;
-    if ((a.group_values & (a.group_values - 1)) == 0) {
-      shift = 0;
-      while ((1 << shift) < a.group_values) ++shift;
-    }
     const unsigned total = static_cast<unsigned>(num_octets);
     // Four octets per thread from a full wave of such threads on; below it more CTAs are worth more
     // than loads in flight (6912 x 1024, 0.9 M octets: 7.1 us with one, 8.3 with four).

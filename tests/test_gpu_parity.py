@@ -109,6 +109,38 @@ def test_dequant_without_offsets(bits):
     assert bits_equal(got, oracle_dequant(qt))
 
 
+@pytest.mark.parametrize("bits", BITS)
+@pytest.mark.parametrize("meta", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize(("rows", "k", "group", "offsets"), [
+    (3, 32, 32, True),          # two runs of 16 a row, less than a warp
+    (129, 4128, 96, True),      # a group size that is no power of two, an odd number of runs in the last block
+    (5000, 2080, 64, False),    # several blocks, no offsets
+    (19001, 1056, 32, True),    # two runs per thread
+])
+def test_dequant_in_runs_of_16_equals_runs_of_8(bits, meta, rows, k, group, offsets):
+    """The kernel for 32-byte aligned outputs against the one that any 16-byte aligned output takes, over codes, scales
+    and offsets of any bits: subnormal, infinite and not-a-number ones too."""
+    import ctypes
+
+    from dynquant_b200 import _lib, ops
+    from dynquant_b200.format import row_geometry
+
+    geo, gen = row_geometry(bits, group, k), torch.Generator(device="cuda").manual_seed(rows + bits)
+    packed = torch.randint(-2**31, 2**31, (rows, geo.words_per_row), device="cuda", generator=gen, dtype=torch.int64).to(torch.int32)
+    scales, off = (torch.randint(-2**15, 2**15, (rows, geo.num_groups), device="cuda", generator=gen).to(torch.int16).view(meta) for _ in range(2))
+    w = ops.weight_descriptor("dequant", packed, scales, off if offsets else None, bits, group, k)
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for dtype, tag in ((torch.bfloat16, _lib.DQ_BF16), (torch.float16, _lib.DQ_F16)):
+        outs = []
+        for skip in (16, 8):  # values: the first output lies on a 32-byte boundary, the second does not
+            buffer = torch.full((rows * k + 32,), 7.0, dtype=dtype, device="cuda")
+            assert buffer.data_ptr() % 32 == 0
+            _lib.check(_lib.load().dq_dequant(ctypes.byref(w), buffer[skip:].data_ptr(), tag, stream))
+            assert bool((buffer[:skip] == 7.0).all()) and bool((buffer[skip + rows * k:] == 7.0).all())
+            outs.append(buffer[skip:skip + rows * k].view(torch.int16))
+        assert torch.equal(*outs)
+
+
 @pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 8])
 @pytest.mark.parametrize("bits", BITS)
 @pytest.mark.parametrize(("rows", "k", "group"), GEOMETRIES)
