@@ -784,6 +784,17 @@ int32_t launch_pdl(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStrea
   return DQ_OK;
 }
 
+// Experts that a call is expected to activate: E * (1 - (1 - 1/E)^A) under uniform routing; with a slot per
+// assignment, the assignments.
+double expected_active(const MoeArgs& a) {
+  if (a.by_assignment) return a.assignments;
+  const double e_count = a.num_experts;
+  return std::max(1.0, e_count * (1.0 - std::pow(1.0 - 1.0 / e_count, a.assignments)));
+}
+
+// Warps that a launch has work for if none slices the reduction axis.
+double moe_warps(const MoeArgs& a) { return expected_active(a) * static_cast<double>(ceil_div(a.rows, 16)); }
+
 template <int BITS, int CH, bool GATE_UP>
 int32_t launch_grouped(MoeArgs a, int slots, cudaStream_t stream) {
   const DeviceInfo* dev = device_info();
@@ -797,11 +808,14 @@ int32_t launch_grouped(MoeArgs a, int slots, cudaStream_t stream) {
   const size_t one = moe_smem<BITS, CH>(a, GATE_UP).total;
   const size_t stage = static_cast<size_t>(CH) * 2 * kMoeThreads * (4 * BITS) + static_cast<size_t>(CH) * 2 * kMoeThreads;
   const size_t fixed = one - stage;
-  // Two register builds, like the tiled dense kernel: three CTAs per SM (80 registers) when a
-  // ring of two stages still fits beside the staged activation, else two (128 registers).
+  // Two register builds, like the tiled dense kernel: two CTAs per SM (128 registers), or three (80 registers) where
+  // a ring of two stages still fits beside the staged activation and two per SM do not hold all warps at once: up
+  // to four tokens (128 experts, top-8, hidden 2048, intermediate 768, 3 / 4 bits: 36.2 -> 32.1 us at four) and from 32
+  // tokens on.  In between a third CTA costs up to 10 % (16 experts, top-8, 4096 / 768, 8 tokens: 42 us, 38 with two).
   DQ_MOE_KNOB(force_ctas, "DQ_B200_MOE_CTAS");
   const size_t per_sm = 228 * 1024, reserve = 1024;
-  int ctas = force_ctas == 2 || force_ctas == 3 ? force_ctas : (a.tokens >= 32 ? 3 : 2);
+  const bool crowded = moe_warps(a) * a.kw > 2.0 * kMoeWarps * dev->sm_count;
+  int ctas = force_ctas == 2 || force_ctas == 3 ? force_ctas : crowded && (a.by_assignment || a.tokens >= 32) ? 3 : 2;
   if (ctas == 3 && fixed + 2 * stage > per_sm / 3 - reserve) ctas = 2;
   size_t budget = per_sm / ctas - reserve;
   if (fixed + 2 * stage > budget) budget = static_cast<size_t>(dev->max_smem_optin);
@@ -819,13 +833,10 @@ int32_t launch_grouped(MoeArgs a, int slots, cudaStream_t stream) {
   // for routing and for staging the activation rows of its expert, so a CTA gets at least
   // about a dozen steps per warp to do; beyond that, more and smaller CTAs even out the
   // experts' different loads.  With so few tokens that this leaves SMs idle, the grid is
-  // widened to one full wave over the experts expected to be active
-  // (E * (1 - (1 - 1/E)^A) under uniform routing).
+  // widened to one full wave over the experts expected to be active.
   const int tiles = (a.rows + 15) / 16;
   const int items = static_cast<int>(ceil_div(tiles, a.rw));
-  const double e_count = a.num_experts;
-  const double active = a.by_assignment ? static_cast<double>(a.assignments)
-                                        : std::max(1.0, e_count * (1.0 - std::pow(1.0 - 1.0 / e_count, a.assignments)));
+  const double active = expected_active(a);
   const int steps_per_item = (GATE_UP ? 2 : 1) * a.spw;
   const int items_per_cta = std::max(1, static_cast<int>(ceil_div(12, steps_per_item)));
   const int one_wave = static_cast<int>(std::ceil(static_cast<double>(ctas) * dev->sm_count / active));
@@ -842,6 +853,18 @@ int32_t launch_grouped(MoeArgs a, int slots, cudaStream_t stream) {
                    : launch_pdl(moe_grouped_kernel<BITS, false, CH, GATE_UP, 2>, grid, kMoeThreads, smem, stream, a, what);
 }
 
+// Shared memory of a launch that slices the reduction axis, with the ring of two stages.
+template <bool GATE_UP>
+size_t sliced_smem(MoeArgs a, int bits) {
+  a.kw = 2, a.nb = 2;
+  switch (bits) {
+    case 2: return moe_smem<2, 2>(a, GATE_UP).total;
+    case 3: return moe_smem<3, 2>(a, GATE_UP).total;
+    case 4: return moe_smem<4, 2>(a, GATE_UP).total;
+    default: return moe_smem<8, 2>(a, GATE_UP).total;
+  }
+}
+
 template <bool GATE_UP>
 int32_t launch_bank(const dq_weight& w, const dq_geometry& g, MoeArgs a, int slots, cudaStream_t stream) {
   a.packed = static_cast<const uint32_t*>(w.packed);
@@ -852,16 +875,29 @@ int32_t launch_bank(const dq_weight& w, const dq_geometry& g, MoeArgs a, int slo
   a.num_groups = g.num_groups;
   a.in_features = g.in_features;
   a.steps = g.words_per_row / (4 * w.bits);
-  // 8 warps: kw slices of the reduction axis (each an even number of steps), the other
-  // warps take neighbouring row tiles.
+  a.m_stride_u4 = a.steps * (w.bits == 8 ? 32 : 16) + 4;
+  // 8 warps: kw slices of the reduction axis, the other warps take neighbouring row tiles.
   DQ_MOE_KNOB(force_kw, "DQ_B200_MOE_KW");
-  // Measured on B200 (Qwen3-30B-A3B shape): up to three tokens a layer is a chain of
-  // latencies and four slices are fastest (18.4 us against 22.2 with two at one token); from
-  // four tokens on, whole rows per warp and no cross-warp sum at all (16 tokens: 68 us
-  // against 78 with two slices; 64 tokens: 107 against 124).
-  const int want_kw = a.tokens <= 3 ? 4 : 1;
+  // As many slices as still leave every (expert, row tile, slice) a resident warp.  With few of them a layer is a chain
+  // of latencies, and a warp's share of the axis is its longest link; a second round of warps costs more than
+  // shorter shares give.  Measured over 23 layer shapes at 1..32 tokens: 8 experts, top-4, hidden 4096, intermediate
+  // 768, 3 / 2 bits, 8 tokens: one / two / four / eight slices 52 / 36 / 26 / 27 us; 128 experts, top-8, 2048 / 768, 16 tokens:
+  // 68 / 78 with one / two.  The staged activation decides how many CTAs an SM holds: 16 experts, top-8, 4096 / 512,
+  // 8-bit gate_up, three tokens (one CTA): 50 us, 56 with two slices, at two tokens (two CTAs) 69 and 32.
+  // A slice may also be an odd number of steps, in ring stages of one step, if it stays long and leaves warps to
+  // spare: 60 experts, top-2, 2816 / 1408, four tokens: 41 -> 32 us with two slices of 11; 8 experts, top-4, 2816 / 1536,
+  // one token: slices of three in the down projection 29 us, 26 with slices of six.
+  const DeviceInfo* dev = device_info();
+  if (dev == nullptr) return DQ_ERR_CUDA;
+  const size_t smem = sliced_smem<GATE_UP>(a, w.bits);
+  const int64_t ctas = std::clamp<int64_t>((228 << 10) / static_cast<int64_t>(smem + 1024), 1, a.by_assignment ? 3 : 2);
+  const double room = 1.05 * kMoeWarps * static_cast<double>(ctas * dev->sm_count);
+  const auto fits = [&](int slices) {
+    const double warps = slices * moe_warps(a);
+    return a.steps % slices == 0 && ((a.steps / slices) % 2 == 0 ? warps <= room : a.steps / slices >= 8 && warps <= (a.by_assignment ? 0.7 : 0.8) * room);
+  };
   int kw = 1;
-  while (kw < want_kw && a.steps % (kw * 2) == 0 && (a.steps / (kw * 2)) % 2 == 0) kw *= 2;
+  while (kw < kMoeWarps && smem <= static_cast<size_t>(dev->max_smem_optin) && fits(2 * kw)) kw *= 2;  // (partial sums need room)
   if (force_kw > 0 && a.steps % force_kw == 0) kw = force_kw;
   a.kw = kw;
   a.rw = kMoeWarps / kw;
@@ -869,8 +905,6 @@ int32_t launch_bank(const dq_weight& w, const dq_geometry& g, MoeArgs a, int slo
   const bool meta_words = a.num_groups % 2 == 0 && reinterpret_cast<uintptr_t>(a.scales) % 4 == 0 &&
                           reinterpret_cast<uintptr_t>(a.offsets) % 4 == 0;
   const bool pairs = a.spw % 2 == 0 && meta_words;  // stages of two steps; else single steps
-  const int aregs = w.bits == 8 ? 32 : 16;
-  a.m_stride_u4 = a.steps * aregs + 4;
   a.magic = a.act_dtype == DQ_BF16 ? 0x43004300u : 0x64006400u;
   switch (w.bits) {
     case 2:

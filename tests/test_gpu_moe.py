@@ -49,6 +49,18 @@ def test_moe_matches_the_composition_oracle(tokens, bits_gu, bits_dn):
     assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 2e-3
 
 
+@pytest.mark.parametrize(("tokens", "experts", "hidden", "inter", "topk", "widths"), [
+    (1, 4, 4096, 128, 2, (3, 4)),    # eight slices of four steps
+    (6, 4, 2048, 512, 2, (2, 2)),    # slices with the routing worked out, several tokens per expert
+    (4, 6, 2816, 256, 2, (4, 3)),    # an odd number of steps per slice: ring stages of one step
+    (9, 4, 2816, 1408, 2, (3, 8)),   # ... past eight tokens of an expert; 11 steps that no slice divides
+    (3, 8, 4096, 256, 8, (8, 4)),    # a staged activation that leaves one CTA per SM
+])
+def test_moe_with_the_reduction_axis_sliced(tokens, experts, hidden, inter, topk, widths):
+    got, want, *_ = run_case(tokens, experts, hidden, inter, topk, *widths)
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 2e-3
+
+
 def test_moe_qwen3_shape_fp16_and_determinism():
     from dynquant_b200 import ops
 
