@@ -336,6 +336,7 @@ bool geometry_ok(const GemvArgs& a, int bits) {
 
 struct Shape {
   int n_tile, token_tiles, slices;
+  double cost;                         // us, estimated
 };
 
 // Token tiles and slices of the reduction axis with the least estimated time (us, fitted to measurements
@@ -347,7 +348,7 @@ struct Shape {
 // us with 6 slices, 21 with 8).
 Shape pick_shape(int m, int row_tiles, int chunks, bool split, int sm_count) {
   Shape best = {};
-  double best_cost = 1e30;
+  best.cost = 1e30;
   const int min_tiles = static_cast<int>(ceil_div(m, 256));
   for (int tt = min_tiles; tt <= min_tiles + (m > 256 ? 2 : 0); ++tt) {  // (up to 256 rows a second tile only decodes twice)
     const int n = static_cast<int>(ceil_div(ceil_div(m, tt), 16) * 16);
@@ -362,11 +363,28 @@ Shape pick_shape(int m, int row_tiles, int chunks, bool split, int sm_count) {
       const double hidden = s == 1 && n <= 128 ? 0.0 : 0.005 * n;  // an epilogue that the next tile does not cover
       const double cluster = s > 1 ? 1.0 + 0.004 * n * s + 1.1 * (s - 1) * static_cast<double>(ctas) / sm_count : 0.0;
       const double cost = waves * (static_cast<double>(ceil_div(chunks, s)) * chunk + hidden) + cluster + 2.2 + 0.01 * n;
-      if (cost < best_cost) best_cost = cost, best = {n, tt, s};
+      if (cost < best.cost) best = {n, tt, s, cost};
     }
   }
   return best;
 }
+
+// The row tiles that a launch of its own should have, the rest in a second one; all of them: one launch.
+//
+// Up to 256 activation rows a wave is bound by the decode, and a last wave of a few tiles costs as much as a full
+// one.  So the first launch gets whole waves and the second, whose tiles are few, slices the reduction axis over
+// clusters: 4-bit 20480 x 4096 (160 row tiles) at 16 / 64 / 128 rows 37.2 / 41.8 / 41.9 -> 29.9 / 34.7 / 34.0 us; of 60
+// matrices of 149 to 300 row tiles 12 change and gain 2 to 31 %, none loses.  With more token tiles the waves run into
+// one another and the second launch, which waits for the first to end, loses up to 7 % (1500 rows, 5120 x 5120:
+// 61 -> 65 us).
+int first_launch_tiles(int m, int row_tiles, int chunks, bool split, int sm_count) {
+  const int tiles = row_tiles / sm_count * sm_count;
+  if (m > 256 || tiles == 0 || tiles == row_tiles) return row_tiles;
+  const auto cost = [&](int t) -> double { return pick_shape(m, t, chunks, split, sm_count).cost; };
+  return cost(tiles) + cost(row_tiles - tiles) < 0.95 * cost(row_tiles) ? tiles : row_tiles;
+}
+
+int32_t launch_jobs(const GemvArgs* args, const int* bits, int count, const DeviceInfo* dev, cudaStream_t stream, bool* taken);
 
 }  // namespace
 
@@ -375,6 +393,41 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
   const DeviceInfo* dev = device_info();
   if (dev == nullptr) return DQ_ERR_CUDA;
   if (count < 1 || count > kJobs) return DQ_OK;
+  int row_tiles = 0;
+  for (int i = 0; i < count; ++i) row_tiles += static_cast<int>(ceil_div(args[i].rows, 128));
+  const int first = tuning_int("DQ_B200_UMMA_SPLIT", 1) == 0
+                        ? row_tiles
+                        : first_launch_tiles(args[0].m, row_tiles, static_cast<int>(ceil_div(args[0].in_features, 128)), args[0].m <= DQ_GEMV_CHUNKED_MAX_ROWS, dev->sm_count);
+  if (first >= row_tiles) return launch_jobs(args, bits, count, dev, stream, taken);
+  GemvArgs part[2][kJobs];
+  int part_bits[2][kJobs], parts[2] = {0, 0}, tile0 = 0;
+  for (int i = 0; i < count; ++i) {
+    const int tiles = static_cast<int>(ceil_div(args[i].rows, 128)), cut = std::clamp(first - tile0, 0, tiles) * 128;  // rows of the first part
+    tile0 += tiles;
+    for (int k = 0; k < 2; ++k) {
+      const int64_t row0 = k == 0 ? 0 : cut;
+      const int rows = k == 0 ? std::min(cut, args[i].rows) : args[i].rows - cut;
+      if (rows <= 0) continue;
+      GemvArgs& b = part[k][parts[k]];
+      b = args[i];
+      b.rows = rows;
+      b.packed += row0 * b.words_per_row;
+      b.scales = static_cast<const unsigned short*>(b.scales) + row0 * b.num_groups;
+      if (b.offsets != nullptr) b.offsets = static_cast<const unsigned short*>(b.offsets) + row0 * b.num_groups;
+      b.out_col0 += row0;
+      part_bits[k][parts[k]++] = bits[i];
+    }
+  }
+  if (const int32_t rc = launch_jobs(part[0], part_bits[0], parts[0], dev, stream, taken)) return rc;
+  if (!*taken) return DQ_OK;
+  if (const int32_t rc = launch_jobs(part[1], part_bits[1], parts[1], dev, stream, taken)) return rc;
+  return *taken ? DQ_OK : fail(DQ_ERR_CUDA, "gemm: the second launch of a matrix was refused");
+}
+
+namespace {
+
+int32_t launch_jobs(const GemvArgs* args, const int* bits, int count, const DeviceInfo* dev, cudaStream_t stream, bool* taken) {
+  *taken = false;
   Params p = {};
   const GemvArgs& a = args[0];
   int w_bytes = 0;
@@ -477,6 +530,7 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
   return mbf ? run(gemm_umma_kernel<false, true, false>) : run(gemm_umma_kernel<false, false, false>);
 }
 
+}  // namespace
 }  // namespace dq
 
 namespace dq {

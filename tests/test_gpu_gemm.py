@@ -73,6 +73,36 @@ def test_shards_of_mixed_widths_in_one_launch(m):
     assert error <= 4e-3
 
 
+@pytest.mark.parametrize(("m", "k", "sizes", "widths", "group"), [
+    (9, 4096, (19000,), (3,), 128),               # 149 row tiles, the last one ragged: a whole wave and one tile
+    (64, 4096, (12000, 7101, 300), (4, 2, 8), 64),  # the cut falls into the second shard
+    (200, 4096, (12001, 7000), (4, 4), 128),      # an odd row count before the cut: output columns that start anywhere
+])
+def test_a_last_wave_of_few_tiles_is_a_launch_of_its_own(m, k, sizes, widths, group):
+    from dynquant_b200 import ops
+    from dynquant_b200.plugin import DynQuantLinearMethod, ShardSpec
+
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the sizes are chosen for 148 SMs")
+    method, layer = DynQuantLinearMethod(None, [ShardSpec(str(i), b, group, n) for i, (n, b) in enumerate(zip(sizes, widths))]), torch.nn.Module()
+    method.create_weights(layer, k, list(sizes), k, sum(sizes), torch.bfloat16, device="cuda")
+    shards = [random_qt(n, k, b, group=group, meta=torch.bfloat16, seed=b) for n, b in zip(sizes, widths)]
+    for i, qt in enumerate(shards):
+        method.load_shard(layer, i, qt)
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(m)).to(torch.bfloat16).cuda()
+    bias = torch.randn(sum(sizes), generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+    before = ops.launch_count()
+    got = method.apply(layer, x, bias)
+    assert ops.launch_count() - before == 2 and ops.last_kernel() == "gemm_umma_kernel"
+    dense = torch.cat([ops.dequant(q.packed, q.scales, q.offsets, q.bits, group, k, out_dtype=torch.float32) for q in shards])
+    want = x.double() @ dense.double().T + bias.double()
+    if m <= 64:
+        assert within_one_ulp_16(got, want.float().cpu().numpy())
+    else:
+        assert (got.double() - want).norm() / want.norm() <= 4e-3
+    assert torch.equal(got, method.apply(layer, x, bias))
+
+
 @pytest.mark.parametrize(("tokens", "experts", "topk", "hidden", "inter", "widths", "act", "meta"), [
     (1, 8, 2, 256, 192, (4, 3), torch.bfloat16, torch.float16),      # one token; 64-row blocks that end inside a tile
     (64, 4, 2, 512, 128, (2, 8), torch.float16, torch.float16),      # tiles of 64 columns and fewer
