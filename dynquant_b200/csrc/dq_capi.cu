@@ -53,6 +53,9 @@ const DeviceInfo* device_info() {
       err = cudaDeviceGetAttribute(&info.max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin,
                                    device);
     }
+    int window = 0;
+    if (err == cudaSuccess) err = cudaDeviceGetAttribute(&window, cudaDevAttrMaxAccessPolicyWindowSize, device);
+    info.max_window = window;
     if (err != cudaSuccess) {
       fail(DQ_ERR_CUDA, "cudaDeviceGetAttribute failed: %s", cudaGetErrorString(err));
       return nullptr;

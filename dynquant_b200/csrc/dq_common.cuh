@@ -100,6 +100,7 @@ struct DeviceInfo {
   int device;
   int sm_count;
   int max_smem_optin;  // bytes per CTA
+  int64_t max_window;  // bytes of an L2 access policy window
   unsigned int* report;  // what kernels report (Report), in host memory that the device maps
 };
 // Cached per device; returns nullptr and sets the error on failure.

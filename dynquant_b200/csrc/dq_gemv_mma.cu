@@ -575,11 +575,12 @@ int32_t launch_stream(const GemvArgs& a, const DeviceInfo& dev, int tiles, int s
     cfg.blockDim = dim3(stream::kThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream_h;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    weights_leave_first(&attr[0], dev, &a, 1);
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
     DQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, q));
     DQ_CHECK_LAUNCH("gemv");
     note_kernel("gemv_mma_stream_kernel");
@@ -822,11 +823,12 @@ int32_t try_tile(const GemvArgs* jobs, const int* bits, int n, const DeviceInfo&
     cfg.blockDim = dim3(tilek::kThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream_h;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    weights_leave_first(&attr[0], dev, jobs, n);
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
     DQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, L));
     DQ_CHECK_LAUNCH("gemv");
     note_kernel("gemv_mma_tile_kernel");

@@ -110,15 +110,16 @@ int32_t launch_sliced(const GemvArgs& a, const DeviceInfo& dev, cudaStream_t str
     cfg.blockDim = dim3(stream::kThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream_h;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[3];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1;
     attr[0].val.clusterDim.y = static_cast<unsigned>(slices);
     attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    weights_leave_first(&attr[1], dev, &a, 1);
+    attr[2].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[2].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled_for_rows() ? 2 : 1;
+    cfg.numAttrs = pdl_enabled_for_rows() ? 3 : 2;
     DQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, p));
     DQ_CHECK_LAUNCH("gemv");
     note_kernel("gemv_mma_stream_sliced_kernel");
@@ -275,8 +276,9 @@ int32_t launch_gemv_stream_sliced_fused(const GemvArgs* jobs, const int* bits, i
     cfg.blockDim = dim3(stream::kThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream_h;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[3];
     int na = 0;
+    weights_leave_first(&attr[na++], *dev, jobs, n);
     if (slices > 1) {
       attr[na].id = cudaLaunchAttributeClusterDimension;
       attr[na].val.clusterDim.x = 1;
