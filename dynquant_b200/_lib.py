@@ -144,6 +144,7 @@ SIGNATURES = {
     "dq_moe_scratch_bytes": (_I32, [_I64, _I64, _I64, _I64, _I64, _I32, ctypes.POINTER(ctypes.c_int64)]),
     "dq_moe_gemv": (_I32, [_P, _I32, _I64, _P, _P, _I64, _I64, _WP, _WP, _I64, _I64, _P, _I32, _P, _I64, _P]),
     "dq_moe_gemv_shard": (_I32, [_P, _I32, _I64, _P, _P, _I64, _I64, _I64, _WP, _WP, _I64, _I64, _P, _I32, _P, _I64, _P]),
+    "dq_moe_gemv_shard_of": (_I32, [_P, _I32, _I64, _P, _P, _I64, _I64, _I64, _I64, _WP, _WP, _I64, _I64, _P, _I32, _P, _I64, _P]),
     "dq_moe_gemm_scratch_bytes": (_I32, [_I64, _I64, _I64, _I64, _I64, _I32, ctypes.POINTER(ctypes.c_int64)]),
     "dq_moe_gemm": (_I32, [_P, _I32, _I64, _P, _P, _I64, _I64, _I64, _WP, _WP, _I64, _I64, _P, _I32, _P, _I64, _P]),
     "dq_moe_gemv_static": (_I32, [_P, _I32, _I64, _P, _P, _I64, _I64, _WP, _WP, _I64, _I64, _P, _I32, _P]),

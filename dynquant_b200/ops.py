@@ -290,12 +290,14 @@ def moe_gemv(
     out_dtype: torch.dtype | None = None,
     scratch: torch.Tensor | None = None,
     first_expert: int = 0,
+    total_experts: int | None = None,
 ) -> torch.Tensor:
     """Expert layer over packed banks: ``sum_k w[t,k] * down_e(silu(gate_e(x_t)) * up_e(x_t))``.
 
     ``first_expert``: the banks hold experts ``[first_expert, first_expert + num_experts)`` of a
     larger layer and ``topk_ids`` carry the layer's global numbers (one rank of an
-    expert-parallel layer); ids outside that range are skipped.
+    expert-parallel layer); ids outside that range are skipped.  ``total_experts``: of that larger
+    layer (default: no more than these), from which the launch takes how many tokens come here.
 
     ``gate_up`` is the bank ``[E, 2*inter, hidden]`` folded to rows (gate rows of an expert
     first), ``down`` is ``[E, hidden, inter]`` folded to rows; ``topk_ids`` int32
@@ -326,9 +328,10 @@ def moe_gemv(
     y = torch.empty((tokens, hidden), dtype=out_dtype, device=x.device)
     with torch.cuda.device(x.device):
         _lib.check(
-            lib.dq_moe_gemv_shard(
+            lib.dq_moe_gemv_shard_of(
                 x.data_ptr(), _tag(x.dtype, "moe_gemv: x"), tokens, topk_ids.data_ptr(), topk_weights.data_ptr(),
-                topk, first_expert, num_experts, ctypes.byref(wgu), ctypes.byref(wdn), hidden, inter, y.data_ptr(),
+                topk, first_expert, num_experts, first_expert + num_experts if total_experts is None else total_experts,
+                ctypes.byref(wgu), ctypes.byref(wdn), hidden, inter, y.data_ptr(),
                 _tag(out_dtype, "moe_gemv: out"), scratch.data_ptr(), scratch.numel(), _stream(x.device),
             )
         )

@@ -170,7 +170,7 @@ class ExpertParallelMoE:
 
             def compute(x, ids, w, gate_up, down, num_experts, first_expert=0):
                 return ops.moe_gemv(x, ids, w, gate_up, down, num_experts=num_experts, out_dtype=torch.float32,
-                                    first_expert=first_expert)
+                                    first_expert=first_expert, total_experts=self.num_experts)
 
             self._takes_global_ids = True  # the kernels renumber the ids themselves
         self.compute = compute

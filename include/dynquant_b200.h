@@ -329,6 +329,14 @@ DQ_API int32_t dq_moe_gemv_shard(const void* x, int32_t x_dtype, int64_t tokens,
                                  int64_t num_experts, const dq_weight* gate_up, const dq_weight* down,
                                  int64_t hidden, int64_t inter, void* y, int32_t y_dtype, void* scratch,
                                  int64_t scratch_bytes, void* stream);
+/* The same with the number of experts of the whole layer, at least first_expert + num_experts (what
+ * dq_moe_gemv_shard takes it to be): the launch shape then counts the share of the assignments that comes
+ * to this rank.  Results do not depend on it beyond the order of fp32 sums. */
+DQ_API int32_t dq_moe_gemv_shard_of(const void* x, int32_t x_dtype, int64_t tokens, const int32_t* topk_ids,
+                                    const float* topk_w, int64_t topk, int64_t first_expert, int64_t num_experts,
+                                    int64_t total_experts, const dq_weight* gate_up, const dq_weight* down,
+                                    int64_t hidden, int64_t inter, void* y, int32_t y_dtype, void* scratch,
+                                    int64_t scratch_bytes, void* stream);
 /* The same layer for any number of tokens (prefill), on the tcgen05 tensor cores: the assignments
  * sorted by expert on the device, every active expert's weights decoded once per 128 of its tokens, each
  * as two 16-bit pieces (16 bits of it with bf16 activations, 21 with fp16).  Sizes and alignment as there, plus hidden % 8 == 0, inter % 8 == 0, at

@@ -95,6 +95,15 @@ def test_gemv_row_limit_is_checked_before_any_device_work():
     assert rc == _lib.DQ_ERR_INVALID and "exceeds the kernel's limit" in _lib.last_error()
 
 
+@pytest.mark.parametrize(("first", "experts", "total"), [(0, 4, 3), (4, 4, 7), (8, 4, 4), (0, 4, 1 << 31)])
+def test_a_rank_holds_experts_of_its_layer_only(first, experts, total):
+    p = ctypes.c_void_p(256)
+    w = _weight()
+    rc = _lib.load().dq_moe_gemv_shard_of(p, 1, 1, p, p, 2, first, experts, total, ctypes.byref(w), ctypes.byref(w), 128, 128,
+                                          p, 1, p, 1 << 20, None)
+    assert rc == _lib.DQ_ERR_INVALID and f"of a layer of {total}" in _lib.last_error()
+
+
 def test_torch_ops_are_registered_with_reference_schemas_and_have_fakes():
     import torch
 
