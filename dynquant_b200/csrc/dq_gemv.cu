@@ -500,6 +500,7 @@ int32_t gemv_args(GemvArgs a, const dq_weight& w, const dq_geometry& g, cudaStre
     // mostly from L2, but stay on the tensor-core path.
     if (a.m > 1 && mma_path_supports(activation_rows(a, 0, 1), w.bits)) {
       const int half = (a.m + 1) / 2;
+      a.read_again = 1;
       if (const int32_t rc = gemv_args(activation_rows(a, 0, half), w, g, stream)) return rc;
       return gemv_args(activation_rows(a, half, a.m - half), w, g, stream);
     }
@@ -754,6 +755,7 @@ int32_t dq_gemv_shards_rows(const void* x, int32_t x_dtype, int64_t m, const dq_
         dq_resolve_geometry("gemv_shards_rows", &shards[i], &geo[live]);
         args[live] = dq::make_args(static_cast<const unsigned char*>(x) + row0 * x_row, x_dtype, rows_here, shards[i], geo[live],
                                    bias, static_cast<unsigned char*>(out) + row0 * out_row, out_stride, col0, out_dtype);
+        args[live].read_again = chunks > 1 ? 1 : 0;
         bits[live] = shards[i].bits;
         which[live] = &shards[i];
         ++live;

@@ -19,10 +19,14 @@ struct GemvArgs {
   int rows;  // output features of this weight
   int words_per_row, num_groups, words_per_group, group_values, in_features;
   int chunks_per_row, chunks_per_group;  // fast path only
+  int read_again;  // 1: another launch of this call reads the same weights (row chunks, passes over half the rows)
 };
 
 // A launch attribute that lets the packed words of `jobs` leave L2 before anything else: an access policy window
-// over all of them where they lie close together (a layer loaded in one go), else over the largest.
+// over all of them where they lie close together (a layer loaded in one go; up to a third of the window may be what lies
+// between them, but nothing that this launch reads or writes besides weights), else over the largest, or over the first
+// part of it if it is longer than a window can be (128 MB here, as against an lm_head of 500).  False: the launch goes
+// without, because its weights are read again in this call, or because the stream has a window of its own, which a launch's would replace.
 //
 // Weights are read once per launch and are nine tenths of all traffic.  What they push out otherwise are the
 // activations and above all the INSTRUCTIONS of the kernels that take turns in a decode step, whose first fetches
@@ -30,19 +34,38 @@ struct GemvArgs {
 // 1059 us, of a 2B model with its head (one row, launches of 2 to 11 MB) 464 -> 458; a launch whose kernel ran just before
 // takes the same time as without (2 x 17408 x 5120, 4-bit, four rows 25.7 -> 25.2 us, 5120 x 5120, 3-bit, one row 8.3).
 // (The same by cp.async with an L2 cache hint costs registers and up to 3 % at 2 bits.)
-inline void weights_leave_first(cudaLaunchAttribute* attr, const DeviceInfo& dev, const GemvArgs* jobs, int n) {
+inline bool weights_leave_first(cudaLaunchAttribute* attr, const DeviceInfo& dev, cudaStream_t stream, const GemvArgs* jobs, int n) {
   const auto bytes = [](const GemvArgs& a) { return static_cast<int64_t>(a.rows) * a.words_per_row * 4; };
   uintptr_t low = ~uintptr_t{0}, high = 0;
   int64_t sum = 0;
   int most = 0;
   for (int i = 0; i < n; ++i) {
+    if (jobs[i].read_again != 0) return false;
+    for (int j = 0; j < i; ++j) {
+      if (jobs[j].packed == jobs[i].packed) return false;
+    }
     const auto at = reinterpret_cast<uintptr_t>(jobs[i].packed);
     low = at < low ? at : low, high = at + bytes(jobs[i]) > high ? at + bytes(jobs[i]) : high;
     sum += bytes(jobs[i]);
     if (bytes(jobs[i]) > bytes(jobs[most])) most = i;
   }
+  cudaLaunchAttributeValue own = {};
+  if (cudaStreamGetAttribute(stream, cudaLaunchAttributeAccessPolicyWindow, &own) != cudaSuccess) {
+    cudaGetLastError();
+  } else if (own.accessPolicyWindow.num_bytes != 0) {
+    return false;
+  }
   const int64_t span = static_cast<int64_t>(high - low);
-  const bool together = span <= dev.max_window && span <= sum + sum / 2;
+  bool together = span <= dev.max_window && span <= sum + sum / 2;
+  for (int i = 0; i < n && together; ++i) {
+    const GemvArgs& a = jobs[i];
+    const auto apart = [&](const void* p, int64_t elems, int dtype) {
+      const auto at = reinterpret_cast<uintptr_t>(p);
+      return at >= high || at + static_cast<uintptr_t>(elems) * dtype_size(dtype) <= low;
+    };
+    together = apart(a.x, static_cast<int64_t>(a.m) * a.in_features, a.x_dtype) && apart(a.out, a.m * a.out_stride, a.out_dtype) &&
+               (a.bias == nullptr || apart(a.bias, a.out_col0 + a.rows, a.out_dtype));
+  }
   attr->id = cudaLaunchAttributeAccessPolicyWindow;
   cudaAccessPolicyWindow& w = attr->val.accessPolicyWindow;
   w.base_ptr = together ? reinterpret_cast<void*>(low) : const_cast<uint32_t*>(jobs[most].packed);
@@ -50,6 +73,7 @@ inline void weights_leave_first(cudaLaunchAttribute* attr, const DeviceInfo& dev
   w.hitRatio = 1.0f;
   w.hitProp = cudaAccessPropertyStreaming;
   w.missProp = cudaAccessPropertyStreaming;
+  return true;
 }
 
 namespace peerpush {

@@ -576,11 +576,13 @@ int32_t launch_stream(const GemvArgs& a, const DeviceInfo& dev, int tiles, int s
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream_h;
     cudaLaunchAttribute attr[2];
-    weights_leave_first(&attr[0], dev, &a, 1);
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    unsigned count = weights_leave_first(&attr[0], dev, stream_h, &a, 1) ? 1 : 0;
+    if (pdl_enabled()) {
+      attr[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[count++].val.programmaticStreamSerializationAllowed = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    cfg.numAttrs = count;
     DQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, q));
     DQ_CHECK_LAUNCH("gemv");
     note_kernel("gemv_mma_stream_kernel");
@@ -824,11 +826,13 @@ int32_t try_tile(const GemvArgs* jobs, const int* bits, int n, const DeviceInfo&
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream_h;
     cudaLaunchAttribute attr[2];
-    weights_leave_first(&attr[0], dev, jobs, n);
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    unsigned count = weights_leave_first(&attr[0], dev, stream_h, jobs, n) ? 1 : 0;
+    if (pdl_enabled()) {
+      attr[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[count++].val.programmaticStreamSerializationAllowed = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    cfg.numAttrs = count;
     DQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, L));
     DQ_CHECK_LAUNCH("gemv");
     note_kernel("gemv_mma_tile_kernel");

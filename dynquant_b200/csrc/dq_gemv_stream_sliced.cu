@@ -115,11 +115,13 @@ int32_t launch_sliced(const GemvArgs& a, const DeviceInfo& dev, cudaStream_t str
     attr[0].val.clusterDim.x = 1;
     attr[0].val.clusterDim.y = static_cast<unsigned>(slices);
     attr[0].val.clusterDim.z = 1;
-    weights_leave_first(&attr[1], dev, &a, 1);
-    attr[2].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[2].val.programmaticStreamSerializationAllowed = 1;
+    unsigned count = weights_leave_first(&attr[1], dev, stream_h, &a, 1) ? 2 : 1;
+    if (pdl_enabled_for_rows()) {
+      attr[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[count++].val.programmaticStreamSerializationAllowed = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled_for_rows() ? 3 : 2;
+    cfg.numAttrs = count;
     DQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, p));
     DQ_CHECK_LAUNCH("gemv");
     note_kernel("gemv_mma_stream_sliced_kernel");
@@ -278,7 +280,7 @@ int32_t launch_gemv_stream_sliced_fused(const GemvArgs* jobs, const int* bits, i
     cfg.stream = stream_h;
     cudaLaunchAttribute attr[3];
     int na = 0;
-    weights_leave_first(&attr[na++], *dev, jobs, n);
+    if (weights_leave_first(&attr[na], *dev, stream_h, jobs, n)) ++na;
     if (slices > 1) {
       attr[na].id = cudaLaunchAttributeClusterDimension;
       attr[na].val.clusterDim.x = 1;
