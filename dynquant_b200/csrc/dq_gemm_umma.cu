@@ -334,6 +334,21 @@ bool geometry_ok(const GemvArgs& a, int bits) {
   return reinterpret_cast<uintptr_t>(a.x) % 16 == 0 && reinterpret_cast<uintptr_t>(a.packed) % 16 == 0;
 }
 
+// Whether this kernel takes ALL the matrices at once.  Asked before anything is launched: the caller's other paths
+// compute every one of them, and a second launch (first_launch_tiles) has to be one that is taken.
+bool jobs_ok(const GemvArgs* args, const int* bits, int count) {
+  if (count < 1 || count > kJobs) return false;
+  const GemvArgs& a = args[0];
+  for (int i = 0; i < count; ++i) {
+    const GemvArgs& b = args[i];
+    if (!geometry_ok(b, bits[i]) || b.x != a.x || b.m != a.m || b.out != a.out || b.out_stride != a.out_stride ||
+        b.in_features != a.in_features || b.meta_dtype != a.meta_dtype || b.rows < 1) {
+      return false;
+    }
+  }
+  return true;
+}
+
 struct Shape {
   int n_tile, token_tiles, slices;
   double cost;                         // us, estimated
@@ -392,7 +407,7 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
   *taken = false;
   const DeviceInfo* dev = device_info();
   if (dev == nullptr) return DQ_ERR_CUDA;
-  if (count < 1 || count > kJobs) return DQ_OK;
+  if (!jobs_ok(args, bits, count)) return DQ_OK;
   int row_tiles = 0;
   for (int i = 0; i < count; ++i) row_tiles += static_cast<int>(ceil_div(args[i].rows, 128));
   const int first = tuning_int("DQ_B200_UMMA_SPLIT", 1) == 0
@@ -433,10 +448,6 @@ int32_t launch_jobs(const GemvArgs* args, const int* bits, int count, const Devi
   int w_bytes = 0;
   for (int i = 0; i < count; ++i) {
     const GemvArgs& b = args[i];
-    if (!geometry_ok(b, bits[i]) || b.x != a.x || b.m != a.m || b.out != a.out || b.out_stride != a.out_stride ||
-        b.in_features != a.in_features || b.meta_dtype != a.meta_dtype || b.rows < 1) {
-      return DQ_OK;
-    }
     Job& job = p.job[i];
     if (!encode_map(&job.wmap, CU_TENSOR_MAP_DATA_TYPE_INT32, b.packed, b.words_per_row, b.rows, static_cast<int64_t>(b.words_per_row) * 4,
                     4 * bits[i], 128, weight_swizzle(bits[i]))) {

@@ -103,6 +103,26 @@ def test_a_last_wave_of_few_tiles_is_a_launch_of_its_own(m, k, sizes, widths, gr
     assert torch.equal(got, method.apply(layer, x, bias))
 
 
+@pytest.mark.parametrize("m", [40, 200])
+def test_a_shard_that_the_kernel_does_not_take_behind_a_whole_wave(m):
+    """148 row tiles that could be a launch of their own, and behind them a matrix of a group size that is no power of
+    two: another path computes all of it."""
+    from dynquant_b200 import ops
+    from dynquant_b200.plugin import DynQuantLinearMethod, ShardSpec
+
+    k, sizes, groups = 6144, (148 * 128, 300), (128, 96)
+    method, layer = DynQuantLinearMethod(None, [ShardSpec(str(i), 4, g, n) for i, (n, g) in enumerate(zip(sizes, groups))]), torch.nn.Module()
+    method.create_weights(layer, k, list(sizes), k, sum(sizes), torch.bfloat16, device="cuda")
+    shards = [random_qt(n, k, 4, group=g, meta=torch.bfloat16, seed=n) for n, g in zip(sizes, groups)]
+    for i, qt in enumerate(shards):
+        method.load_shard(layer, i, qt)
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(m)).to(torch.bfloat16).cuda()
+    dense = torch.cat([ops.dequant(q.packed, q.scales, q.offsets, q.bits, g, k, out_dtype=torch.float32) for q, g in zip(shards, groups)])
+    want = x.double() @ dense.double().T
+    # bf16 outputs, and above 64 rows bf16 weights: 2 ** -9 each at most
+    assert (method.apply(layer, x, None).double() - want).norm() / want.norm() <= 4e-3
+
+
 @pytest.mark.parametrize(("tokens", "experts", "topk", "hidden", "inter", "widths", "act", "meta"), [
     (1, 8, 2, 256, 192, (4, 3), torch.bfloat16, torch.float16),      # one token; 64-row blocks that end inside a tile
     (64, 4, 2, 512, 128, (2, 8), torch.float16, torch.float16),      # tiles of 64 columns and fewer
