@@ -811,13 +811,19 @@ int32_t launch_grouped(MoeArgs a, int slots, cudaStream_t stream) {
   const size_t stage = static_cast<size_t>(CH) * 2 * kMoeThreads * (4 * BITS) + static_cast<size_t>(CH) * 2 * kMoeThreads;
   const size_t fixed = one - stage;
   // Two register builds, like the tiled dense kernel: two CTAs per SM (128 registers), or three (80 registers) where
-  // a ring of two stages still fits beside the staged activation and two per SM do not hold all warps at once: up
-  // to four tokens (128 experts, top-8, hidden 2048, intermediate 768, 3 / 4 bits: 36.2 -> 32.1 us at four) and from 32
-  // tokens on.  In between a third CTA costs up to 10 % (16 experts, top-8, 4096 / 768, 8 tokens: 42 us, 38 with two).
-  DQ_MOE_KNOB(force_ctas, "DQ_B200_MOE_CTAS");
+  // a ring of two stages still fits beside the staged activation and a third CTA saves work a second round.  gate_up
+  // with a slot per assignment (up to four tokens): only if three per SM hold all warps at once and two do not (128
+  // experts, top-8, hidden 2048, intermediate 768, 3 / 4 bits, four tokens: two slices 33.9 -> 32.1 us; but 8 experts,
+  // top-2, 4096 / 14336, 4 bits, four tokens, 2.9 rounds of two: 199 -> 228, and 64 experts, top-8, 2048 / 1024, one token, where
+  // two hold all: 16.9 -> 19.1).  Any bank from 32 tokens on; in between it costs up to 10 % (16 experts, top-8, 4096 / 768,
+  // 8 tokens: 42 us, 38 with two), and so it would in the down projection of fewer.
+  DQ_MOE_KNOB(force_ctas_both, "DQ_B200_MOE_CTAS");
+  DQ_MOE_KNOB(force_ctas_one, GATE_UP ? "DQ_B200_MOE_CTAS_UP" : "DQ_B200_MOE_CTAS_DOWN");
+  const int force_ctas = force_ctas_one > 0 ? force_ctas_one : force_ctas_both;
   const size_t per_sm = 228 * 1024, reserve = 1024;
-  const bool crowded = moe_warps(a) * a.kw > 2.0 * kMoeWarps * dev->sm_count;
-  int ctas = force_ctas == 2 || force_ctas == 3 ? force_ctas : crowded && (a.by_assignment || a.tokens >= 32) ? 3 : 2;
+  const double rounds = moe_warps(a) * a.kw / (2.0 * kMoeWarps * dev->sm_count);  // of two CTAs per SM
+  const bool third = rounds > 1.0 && (a.by_assignment ? rounds <= 1.5 : a.tokens >= 32);
+  int ctas = force_ctas == 2 || force_ctas == 3 ? force_ctas : third ? 3 : 2;
   if (ctas == 3 && fixed + 2 * stage > per_sm / 3 - reserve) ctas = 2;
   size_t budget = per_sm / ctas - reserve;
   if (fixed + 2 * stage > budget) budget = static_cast<size_t>(dev->max_smem_optin);
@@ -879,24 +885,46 @@ int32_t launch_bank(const dq_weight& w, const dq_geometry& g, MoeArgs a, int slo
   a.steps = g.words_per_row / (4 * w.bits);
   a.m_stride_u4 = a.steps * (w.bits == 8 ? 32 : 16) + 4;
   // 8 warps: kw slices of the reduction axis, the other warps take neighbouring row tiles.
-  DQ_MOE_KNOB(force_kw, "DQ_B200_MOE_KW");
+  DQ_MOE_KNOB(force_kw_both, "DQ_B200_MOE_KW");
+  DQ_MOE_KNOB(force_kw_one, GATE_UP ? "DQ_B200_MOE_KW_UP" : "DQ_B200_MOE_KW_DOWN");
+  const int force_kw = force_kw_one > 0 ? force_kw_one : force_kw_both;
   // As many slices as still leave every (expert, row tile, slice) a resident warp.  With few of them a layer is a chain
   // of latencies, and a warp's share of the axis is its longest link; a second round of warps costs more than
-  // shorter shares give.  Measured over 23 layer shapes at 1..32 tokens: 8 experts, top-4, hidden 4096, intermediate
-  // 768, 3 / 2 bits, 8 tokens: one / two / four / eight slices 52 / 36 / 26 / 27 us; 128 experts, top-8, 2048 / 768, 16 tokens:
-  // 68 / 78 with one / two.  The staged activation decides how many CTAs an SM holds: 16 experts, top-8, 4096 / 512,
-  // 8-bit gate_up, three tokens (one CTA): 50 us, 56 with two slices, at two tokens (two CTAs) 69 and 32.
-  // A slice may also be an odd number of steps, in ring stages of one step, if it stays long and leaves warps to
-  // spare: 60 experts, top-2, 2816 / 1408, four tokens: 41 -> 32 us with two slices of 11; 8 experts, top-4, 2816 / 1536,
-  // one token: slices of three in the down projection 29 us, 26 with slices of six.
+  // shorter shares give.  Measured over 44 layer shapes at 1..32 tokens, every number of slices in turn: 8 experts, top-4,
+  // hidden 4096, intermediate 768, 3 / 2 bits, 8 tokens: one / two / four / eight slices 52 / 36 / 26 / 26 us; 128 experts, top-8,
+  // 2048 / 768, 16 tokens: 75 / 79 with one / two.  The staged activation decides how many CTAs an SM holds.  The limits,
+  // in warps over that room:
+  //  * eight slices of two steps: 0.6, since a CTA then sums eight partial results for two steps of each (32 of 128 experts,
+  //    top-8, 2048 / 768, two / three tokens, 0.41 / 0.62: 12.2 / 15.9 -> 11.1 / 17.4; 128 experts at one token, 0.8, 2 bits 13.6 -> 14.4);
+  //  * slices of an odd number of steps, whose ring stages are single steps: 0.8, if seven steps or longer (60 experts,
+  //    top-2, 2816 / 1408, four tokens, two of 11: 41 -> 32; 8 experts, top-2, 1024 / 3584 8-bit, one token, four of seven in the
+  //    down projection: 24 -> 16);
+  //  * long slices of 2 to 4 bits, up to four tokens, may go on in a second round, as they even out the last one: gate_up from
+  //    16 steps on 1.5, with room for two CTAs per SM (8 experts, top-1, 8192 / 10240, two tokens, two of 32: 100 -> 86; 64 experts, top-8,
+  //    7168 / 1024, three: 110 -> 96; 8 bits, 8 experts, top-2, 4096 / 14336, one: 85 -> 90), down from 24 steps on 3 (8 experts,
+  //    top-2, 4096 / 14336, two / four tokens: 124 / 224 -> 112 / 200; at six tokens 6 experts, top-3, 2048 / 8192 59 -> 63).
+  // Against four slices up to three tokens and none above, 54 shapes: 1.07 / 1.08 / 1.08 / 1.13 / 1.09 / 1.09 / 1.08 / 1.09 / 1.10
+  // in the geometric mean at 1 / 2 / 3 / 4 / 5 / 6 / 8 / 16 / 32 tokens.  Of the 486 points eight are slower there by more than 4 %, all where
+  // tiles and CTAs come out unevenly: 8 experts, 4096 / 14336, 3 / 8 bits, three tokens 0.92; 8 of 8192 / 10240, two, 0.94; 8 of 4096 / 4096
+  // 8-bit, two, 32 of 7168 / 2048, five, and 8 of 2816 / 1536, eight, 0.95; the same at one, 64 of 4096 / 1280, four, and 10 of 7680 / 1280,
+  // four, 0.96.
   const DeviceInfo* dev = device_info();
   if (dev == nullptr) return DQ_ERR_CUDA;
   const size_t smem = sliced_smem<GATE_UP>(a, w.bits);
   const int64_t ctas = std::clamp<int64_t>((228 << 10) / static_cast<int64_t>(smem + 1024), 1, a.by_assignment ? 3 : 2);
   const double room = 1.05 * kMoeWarps * static_cast<double>(ctas * dev->sm_count);
   const auto fits = [&](int slices) {
-    const double warps = slices * moe_warps(a);
-    return a.steps % slices == 0 && ((a.steps / slices) % 2 == 0 ? warps <= room : a.steps / slices >= 8 && warps <= (a.by_assignment ? 0.7 : 0.8) * room);
+    if (a.steps % slices != 0) return false;
+    const int share = a.steps / slices;
+    double limit = 1.0;
+    if (share % 2 != 0) {
+      limit = share >= 7 ? 0.8 : 0.0;
+    } else if (share == 2 && slices == kMoeWarps) {
+      limit = 0.6;
+    } else if (w.bits != 8 && a.tokens <= 4) {
+      limit = GATE_UP ? (share >= 16 && ctas >= 2 ? 1.5 : 1.0) : (share >= 24 ? 3.0 : 1.0);
+    }
+    return slices * moe_warps(a) <= limit * room;
   };
   int kw = 1;
   while (kw < kMoeWarps && smem <= static_cast<size_t>(dev->max_smem_optin) && fits(2 * kw)) kw *= 2;  // (partial sums need room)

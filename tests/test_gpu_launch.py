@@ -1,6 +1,8 @@
-"""What a call launches, read from the kernel nodes of a captured graph: grids and launch attributes."""
+"""What a call launches, read from the kernel nodes of a captured graph: grids, arguments and launch attributes."""
 
 from __future__ import annotations
+
+import ctypes
 
 import pytest
 import torch
@@ -54,6 +56,24 @@ def test_a_rank_of_an_expert_layer_is_launched_for_its_share_of_the_assignments(
     assert "moe_grouped_kernel" in of_share[0][0] and of_share[0][1][1] == of_whole[0][1][1]
     if rank == 0:  # (without the total, the experts below the first are all that is known of the others)
         assert of_share[0][1][0] > of_whole[0][1][0]
+
+
+def slices_of(call):
+    """Slices of the reduction axis of every moe_grouped_kernel that ``call`` launches, from the kernel's argument: its
+    integers after six pointers hold the steps of the axis, slices, row tiles and steps per slice, in this order."""
+    from cuda.bindings import driver
+
+    graph, nodes = kernel_nodes(call)
+    out = []
+    for name, _, node in nodes:
+        if "moe_grouped_kernel" in name:
+            arrays = done(driver.cuGraphKernelNodeGetParams(node)).kernelParams
+            argument = ctypes.cast(arrays, ctypes.POINTER(ctypes.c_void_p))[0]
+            numbers = (ctypes.c_int32 * 16).from_address(argument + 6 * 8)
+            in_features, steps, slices, tiles, share = numbers[11:16]
+            assert steps == -(-in_features // 128) and slices * share == steps and slices * tiles == 8
+            out.append(slices)
+    return out
 
 
 def window_of(call, stream=None):

@@ -8,6 +8,7 @@ import pytest
 import torch
 
 from conftest import TAG, raw
+from test_gpu_launch import slices_of
 from test_gpu_parity import within_one_ulp_16
 
 pytestmark = pytest.mark.gpu
@@ -49,16 +50,25 @@ def test_moe_matches_the_composition_oracle(tokens, bits_gu, bits_dn):
     assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 2e-3
 
 
-@pytest.mark.parametrize(("tokens", "experts", "hidden", "inter", "topk", "widths"), [
-    (1, 4, 4096, 128, 2, (3, 4)),    # eight slices of four steps
-    (6, 4, 2048, 512, 2, (2, 2)),    # slices with the routing worked out, several tokens per expert
-    (4, 6, 2816, 256, 2, (4, 3)),    # an odd number of steps per slice: ring stages of one step
-    (9, 4, 2816, 1408, 2, (3, 8)),   # ... past eight tokens of an expert; 11 steps that no slice divides
-    (3, 8, 4096, 256, 8, (8, 4)),    # a staged activation that leaves one CTA per SM
+@pytest.mark.parametrize(("tokens", "experts", "hidden", "inter", "topk", "widths", "slices"), [
+    (1, 4, 4096, 128, 2, (3, 4), [8, 1]),     # eight slices of four steps; an axis of one step
+    (6, 4, 2048, 512, 2, (2, 2), [8, 2]),     # slices with the routing worked out, several tokens per expert
+    (4, 6, 2816, 256, 2, (4, 3), [2]),        # an odd number of steps per slice: ring stages of one step
+    (24, 4, 2816, 1408, 2, (3, 8), [2, 1]),   # ... past eight tokens of an expert; 11 steps that no slice divides
+    (3, 8, 4096, 256, 8, (8, 4), [2]),        # a staged activation that leaves one CTA per SM
+    (1, 16, 2048, 1408, 4, (4, 4), [4, 1]),   # eight slices of two steps would fill more than 0.6 of the chip
+    (4, 8, 4096, 7168, 2, (2, 2), [1, 2]),    # long slices of the down projection in a second round
 ])
-def test_moe_with_the_reduction_axis_sliced(tokens, experts, hidden, inter, topk, widths):
-    got, want, *_ = run_case(tokens, experts, hidden, inter, topk, *widths)
+def test_moe_with_the_reduction_axis_sliced(tokens, experts, hidden, inter, topk, widths, slices):
+    """``slices``: of each launch of the grouped kernel (up to four tokens the down projection may be another's)."""
+    from dynquant_b200 import ops
+
+    got, want, layer, ids, w, x = run_case(tokens, experts, hidden, inter, topk, *widths)
     assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 2e-3
+    if tokens == 24:
+        assert int(torch.bincount(ids.flatten()).max()) > 8
+    x, ids, w = x.cuda(), ids.cuda(), w.cuda()
+    assert slices_of(lambda: ops.moe_gemv(x, ids, w, layer.gate_up, layer.down, num_experts=experts, out_dtype=torch.float32)) == slices
 
 
 def test_moe_qwen3_shape_fp16_and_determinism():
