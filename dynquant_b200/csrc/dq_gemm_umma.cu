@@ -410,7 +410,7 @@ int32_t launch_gemm_umma(const GemvArgs* args, const int* bits, int count, cudaS
   if (!jobs_ok(args, bits, count)) return DQ_OK;
   int row_tiles = 0;
   for (int i = 0; i < count; ++i) row_tiles += static_cast<int>(ceil_div(args[i].rows, 128));
-  const int first = tuning_int("DQ_B200_UMMA_SPLIT", 1) == 0
+  const int first = tuning_int("DQ_B200_UMMA_LAST_WAVE", 1) == 0
                         ? row_tiles
                         : first_launch_tiles(args[0].m, row_tiles, static_cast<int>(ceil_div(args[0].in_features, 128)), args[0].m <= DQ_GEMV_CHUNKED_MAX_ROWS, dev->sm_count);
   if (first >= row_tiles) return launch_jobs(args, bits, count, dev, stream, taken);

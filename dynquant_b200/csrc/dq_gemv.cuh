@@ -30,10 +30,12 @@ struct GemvArgs {
 //
 // Weights are read once per launch and are nine tenths of all traffic.  What they push out otherwise are the
 // activations and above all the INSTRUCTIONS of the kernels that take turns in a decode step, whose first fetches
-// then come from memory, launch after launch: the captured step of a 14B model's layers (15 layers, four rows) 1149 ->
-// 1059 us, of a 2B model with its head (one row, launches of 2 to 11 MB) 464 -> 458; a launch whose kernel ran just before
-// takes the same time as without (2 x 17408 x 5120, 4-bit, four rows 25.7 -> 25.2 us, 5120 x 5120, 3-bit, one row 8.3).
-// (The same by cp.async with an L2 cache hint costs registers and up to 3 % at 2 bits.)
+// then come from memory, launch after launch: the captured step of a 14B model's layers (15 layers, four rows) 1144 ->
+// 1050 us, of a 2B model with its head (one row, launches of 2 to 11 MB) 465 -> 461, without it 381 -> 357; a launch whose
+// kernel ran just before takes the same time as without (2 x 17408 x 5120, 4-bit, four rows 25.7 -> 25.2 us, 5120 x 5120, 3-bit,
+// one row 8.3), and so does a step whose weights all stay in L2 (two layers of the 2B model, 38 MB: 50.1 -> 49.9).
+// (The same by cp.async with an L2 cache hint costs registers and up to 3 % at 2 bits.  The many-rows kernel, the
+// streaming launch of several matrices and the expert layers have not been measured with a window and go without.)
 inline bool weights_leave_first(cudaLaunchAttribute* attr, const DeviceInfo& dev, cudaStream_t stream, const GemvArgs* jobs, int n) {
   const auto bytes = [](const GemvArgs& a) { return static_cast<int64_t>(a.rows) * a.words_per_row * 4; };
   uintptr_t low = ~uintptr_t{0}, high = 0;

@@ -181,8 +181,9 @@ DQ_API int32_t dq_gemv_shards(const void* x, int32_t x_dtype, int64_t m, const d
 DQ_API int32_t dq_gemv_shards_rows(const void* x, int32_t x_dtype, int64_t m, const dq_weight* shards,
                                    int32_t num_shards, const void* bias, void* out, int64_t out_stride,
                                    int32_t out_dtype, void* stream);
-/* The same product for any number of activation rows (prefill), in one launch per four shards on
- * the tcgen05 tensor cores: no dense weight is written.  16-bit activations and metadata, out_dtype
+/* The same product for any number of activation rows (prefill), in one launch per four shards
+ * (two where a last wave of few row tiles is better off as a launch of its own) on the tcgen05 tensor
+ * cores: no dense weight is written.  16-bit activations and metadata, out_dtype
  * == x_dtype, groups of 64 * 2^n values, in_features % 8 == 0, 16-byte aligned x and packed rows;
  * anything else returns DQ_ERR_UNSUPPORTED (outputs then undefined): dequantize + dense serves it. */
 DQ_API int32_t dq_gemm_shards(const void* x, int32_t x_dtype, int64_t m, const dq_weight* shards,

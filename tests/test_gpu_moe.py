@@ -55,6 +55,7 @@ def test_moe_matches_the_composition_oracle(tokens, bits_gu, bits_dn):
     (6, 4, 2048, 512, 2, (2, 2), [8, 2]),     # slices with the routing worked out, several tokens per expert
     (4, 6, 2816, 256, 2, (4, 3), [2]),        # an odd number of steps per slice: ring stages of one step
     (24, 4, 2816, 1408, 2, (3, 8), [2, 1]),   # ... past eight tokens of an expert; 11 steps that no slice divides
+    (24, 4, 4096, 512, 2, (4, 2), [8, 2]),    # ... with stages of two steps
     (3, 8, 4096, 256, 8, (8, 4), [2]),        # a staged activation that leaves one CTA per SM
     (1, 16, 2048, 1408, 4, (4, 4), [4, 1]),   # eight slices of two steps would fill more than 0.6 of the chip
     (4, 8, 4096, 7168, 2, (2, 2), [1, 2]),    # long slices of the down projection in a second round
@@ -65,7 +66,7 @@ def test_moe_with_the_reduction_axis_sliced(tokens, experts, hidden, inter, topk
 
     got, want, layer, ids, w, x = run_case(tokens, experts, hidden, inter, topk, *widths)
     assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 2e-3
-    if tokens == 24:
+    if tokens == 24:  # a second pass over the rows of an expert
         assert int(torch.bincount(ids.flatten()).max()) > 8
     x, ids, w = x.cuda(), ids.cuda(), w.cuda()
     assert slices_of(lambda: ops.moe_gemv(x, ids, w, layer.gate_up, layer.down, num_experts=experts, out_dtype=torch.float32)) == slices
